@@ -1,6 +1,6 @@
 // huffman.cu -- GPU side of the SZ-1.x Huffman codec used by the reference
-// (src/sz_huffman.cpp): symbol histograms, the MSB-first bit packer and a
-// self-synchronising parallel decoder.
+// (src/sz_huffman.cpp): symbol histograms and the MSB-first bit packer (the
+// decoder is huff_decode.cu).
 //
 // Encoder.  The reference's packer (encode, src/sz_huffman.cpp:217-320) emits
 // the MSB-first concatenation of the codes, zero padded to a byte.  Here one
@@ -11,17 +11,6 @@
 // grid and stores it with coalesced stores (atomicOr for the two edge words,
 // shared with the neighbouring tiles).  Words are stored byte-swapped so
 // memory holds the big-endian byte stream the reference writes.
-//
-// Decoder.  The reference stream has no chunk index, so decoding uses
-// self-synchronisation (after Weissenberger & Schmidt, ICPP 2018): the stream
-// is cut into S-bit subsequences, each thread first decodes its subsequence
-// from its nominal start (finding the codeword boundary at which it leaves),
-// then subsequences whose assumed start differs from their predecessor's exit
-// are re-decoded from that exit until nothing changes (prefix codes
-// resynchronise within a few codewords, so this settles in one or two
-// rounds), then counts are scanned and every thread decodes again, writing its
-// symbols.  Lookup is a 2^12-entry first-level table with a bit-serial tree
-// walk for longer codes.
 #include "kernels.h"
 #include "lookback.cuh"
 
@@ -310,41 +299,6 @@ int encode_impl(cpsz_b200_ctx* ctx, const Sym* sym, size_t n, bool map_id_zero, 
   return CPSZ_OK;
 }
 
-// Exclusive scan of the per-CTA bit counts (single CTA, sequential over chunks).
-__global__ void __launch_bounds__(1024) scan_u64_kernel(const unsigned long long* __restrict__ in,
-                                                        unsigned long long* __restrict__ out, size_t n) {
-  __shared__ unsigned long long warp_tot[32];
-  __shared__ unsigned long long carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (size_t base = 0; base < n; base += 1024) {
-    size_t i = base + threadIdx.x;
-    unsigned long long v = i < n ? in[i] : 0ull;
-    unsigned long long x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
-      if ((threadIdx.x & 31) >= o) x += y;
-    }
-    if ((threadIdx.x & 31) == 31) warp_tot[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      unsigned long long w = warp_tot[threadIdx.x];
-      for (int o = 1; o < 32; o <<= 1) {
-        unsigned long long y = __shfl_up_sync(0xffffffffu, w, o);
-        if (threadIdx.x >= o) w += y;
-      }
-      warp_tot[threadIdx.x] = w;
-    }
-    __syncthreads();
-    unsigned long long pre = carry + (threadIdx.x >= 32 ? warp_tot[(threadIdx.x >> 5) - 1] : 0ull) + x - v;
-    if (i < n) out[i] = pre;
-    __syncthreads();
-    if (threadIdx.x == 1023) carry = pre + v;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[n] = carry;
-}
-
 // ---- histogram -------------------------------------------------------------------
 constexpr int HIST_NT = 512;
 constexpr int HIST_LO = 32768 - 4096;  // shared window of the code histogram
@@ -500,238 +454,6 @@ __global__ void __launch_bounds__(HIST_NT) hist_follow_kernel(const uint16_t* __
   hist_flush(sh, hist, c_lo, c_mid, c_hi);
 }
 
-// ---- decoder ---------------------------------------------------------------------
-constexpr int DEC_S = 1024;  // bits per subsequence
-constexpr int DEC_NT = 256;
-
-struct BitReader {
-  const uint32_t* w;  // big-endian words
-  __device__ __forceinline__ uint32_t peek32(unsigned long long pos) const {
-    size_t wi = pos >> 5;
-    uint32_t a = bswap32(__ldg(w + wi)), b = bswap32(__ldg(w + wi + 1));
-    return __funnelshift_l(b, a, (unsigned)(pos & 31));
-  }
-};
-
-// Decodes one symbol at `pos`; returns its length in bits (0 on a corrupt walk).
-__device__ __forceinline__ int decode_one(const BitReader& br, const uint32_t* lut, const HuffDecTable& T,
-                                          unsigned long long pos, uint32_t* sym) {
-  uint32_t p = br.peek32(pos);
-  uint32_t e = lut[p >> (32 - HUFF_LUT_BITS)];
-  if (!(e & 0x80)) {
-    *sym = e >> 8;
-    return (int)(e & 0x7f);
-  }
-  uint32_t node = e >> 8;
-  int l = HUFF_LUT_BITS;
-  while (l < 64) {
-    uint32_t bit = (br.peek32(pos + l) >> 31) & 1u;
-    node = T.child[2 * node + bit];
-    l++;
-    if (node == 0 || node >= (uint32_t)T.node_count) return 0;
-    if (T.leaf[node]) {
-      *sym = T.sym[node];
-      return l;
-    }
-  }
-  return 0;
-}
-
-// A sequential reader: the next bits MSB-first in a 64-bit register, refilled
-// a word at a time, so a symbol found by the table costs no memory access.
-// Holds at least 32 valid bits between symbols.
-struct BitCursor {
-  const uint32_t* w;
-  unsigned long long buf;
-  unsigned long long wi;  // the next word to load
-  int nb;                 // valid bits in buf
-  __device__ __forceinline__ void seek(unsigned long long pos) {
-    wi = pos >> 5;
-    const unsigned long long a = bswap32(__ldg(w + wi)), b = bswap32(__ldg(w + wi + 1));
-    buf = ((a << 32) | b) << (pos & 31);
-    nb = 64 - (int)(pos & 31);
-    wi += 2;
-  }
-  __device__ __forceinline__ void skip(int l) {  // 1 <= l <= 32
-    buf <<= l;
-    nb -= l;
-    if (nb <= 32) {
-      buf |= (unsigned long long)bswap32(__ldg(w + wi)) << (32 - nb);
-      nb += 32;
-      wi++;
-    }
-  }
-};
-
-// decode_one on the cursor, which sits at `pos`; advances it past the symbol.
-__device__ __forceinline__ int decode_cur(BitCursor& c, const BitReader& br, const uint32_t* lut,
-                                          const HuffDecTable& T, unsigned long long pos, uint32_t* sym) {
-  const uint32_t e = lut[(uint32_t)(c.buf >> (64 - HUFF_LUT_BITS))];
-  if (!(e & 0x80)) {
-    *sym = e >> 8;
-    const int l = (int)(e & 0x7f);
-    c.skip(l);
-    return l;
-  }
-  const int l = decode_one(br, lut, T, pos, sym);  // a code longer than the table: walk the tree
-  if (l > 0) c.seek(pos + l);
-  return l;
-}
-
-__device__ __forceinline__ void load_lut(uint32_t* slut, const uint32_t* lut) {
-  for (int k = threadIdx.x; k < (1 << HUFF_LUT_BITS); k += blockDim.x) slut[k] = lut[k];
-  __syncthreads();
-}
-
-// Count word bit: the subsequence's decode ran into an invalid code (possible
-// from an unsynchronised start; on the true path only in a corrupt stream).
-constexpr unsigned int DEC_INVALID = 0x80000000u;
-
-// Phase 1: decode subsequence t from its nominal start to its limit.
-// Phase 2 (resync): subsequence t restarts from its predecessor's exit when
-// that differs from its start.  Huffman codes resynchronise within a few
-// symbols, so the new path runs in lockstep with the previous one (always
-// advancing the one behind): once both reach the same bit position the rest
-// equals the previous decode, whose exit and count (less the symbols before
-// that position) carry over.
-__global__ void __launch_bounds__(DEC_NT) dec_scan_kernel(BitReader br, HuffDecTable T, unsigned long long nbits,
-                                                          int nsub, unsigned long long* __restrict__ start,
-                                                          unsigned long long* __restrict__ end,
-                                                          unsigned int* __restrict__ cnt, int resync,
-                                                          int* __restrict__ changed, int* flag) {
-  __shared__ uint32_t slut[1 << HUFF_LUT_BITS];
-  int t = blockIdx.x * DEC_NT + threadIdx.x;
-  // a resynchronisation round leaves at once the blocks with no start to
-  // move (most of them after the first round), without loading the table
-  if (resync && !__syncthreads_or(t > 0 && t < nsub && end[t - 1] != start[t])) return;
-  load_lut(slut, T.lut);
-  if (t >= nsub) return;
-  unsigned long long lim = (unsigned long long)(t + 1) * DEC_S;
-  if (lim > nbits) lim = nbits;
-  uint32_t sym;
-  if (!resync) {
-    unsigned long long pos = (unsigned long long)t * DEC_S;
-    start[t] = pos;
-    BitCursor cur{br.w};
-    cur.seek(pos);
-    unsigned int c = 0;
-    while (pos < lim) {
-      const int l = decode_cur(cur, br, slut, T, pos, &sym);
-      if (l == 0) {
-        if (t == 0) atomicOr(flag, FLAG_HUFF_CORRUPT);
-        c |= DEC_INVALID;
-        pos = lim;
-        break;
-      }
-      pos += l;
-      c++;
-    }
-    end[t] = pos;
-    cnt[t] = c;
-    return;
-  }
-  if (t == 0) return;
-  const unsigned long long s = end[t - 1], s_old = start[t];
-  if (s == s_old) return;
-  const unsigned long long e_old = end[t];
-  const unsigned int c_old = cnt[t];
-  start[t] = s;
-  *changed = 1;
-  unsigned long long a = s, b = s_old;  // the new path, the previous one
-  unsigned int ca = 0, cb = 0;
-  bool old_ok = true;
-  while (a < lim) {
-    if (old_ok && b < a) {  // b < a < lim: still on the previous decode
-      const int l = decode_one(br, slut, T, b, &sym);
-      if (l == 0) old_ok = false;
-      b += l;
-      cb++;
-      continue;
-    }
-    if (old_ok && a == b) {
-      if (c_old & DEC_INVALID) atomicOr(flag, FLAG_HUFF_CORRUPT);
-      end[t] = e_old;
-      cnt[t] = ca + ((c_old & ~DEC_INVALID) - cb);
-      return;
-    }
-    const int l = decode_one(br, slut, T, a, &sym);
-    if (l == 0) {
-      atomicOr(flag, FLAG_HUFF_CORRUPT);
-      a = lim;
-      break;
-    }
-    a += l;
-    ca++;
-  }
-  end[t] = a;
-  cnt[t] = ca;
-}
-
-// Phase 3: subsequence t writes its symbols from output index off[t].  A
-// thread's symbols are packed into aligned 64-bit stores (single stores at the
-// unaligned head and tail of its range): one store per symbol, each to its
-// own line, made the write rate the limit.
-template <class Out>
-__global__ void __launch_bounds__(DEC_NT) dec_write_kernel(BitReader br, HuffDecTable T, unsigned long long nbits,
-                                                           int nsub, const unsigned long long* __restrict__ start,
-                                                           const unsigned long long* __restrict__ off,
-                                                           size_t n, Out* __restrict__ out) {
-  constexpr int PER = 8 / sizeof(Out);
-  constexpr int SB = 8 * sizeof(Out);
-  __shared__ uint32_t slut[1 << HUFF_LUT_BITS];
-  load_lut(slut, T.lut);
-  int t = blockIdx.x * DEC_NT + threadIdx.x;
-  if (t >= nsub) return;
-  unsigned long long lim = (unsigned long long)(t + 1) * DEC_S;
-  if (lim > nbits) lim = nbits;
-  unsigned long long pos = start[t];
-  unsigned long long o = off[t];
-  const bool packed = (reinterpret_cast<uintptr_t>(out) & 7) == 0;
-  BitCursor cur{br.w};
-  cur.seek(pos);
-  unsigned long long acc = 0;
-  int na = 0;  // symbols in acc, which starts at an aligned index
-  while (pos < lim && o < n) {
-    uint32_t sym;
-    const int l = decode_cur(cur, br, slut, T, pos, &sym);
-    if (l == 0) break;
-    pos += l;
-    if (na == 0 && (!packed || (o % PER) != 0)) {
-      out[o++] = (Out)sym;
-      continue;
-    }
-    acc |= (unsigned long long)(Out)sym << (SB * na);
-    o++;
-    if (++na == PER) {
-      *reinterpret_cast<unsigned long long*>(out + (o - PER)) = acc;
-      acc = 0;
-      na = 0;
-    }
-  }
-  for (int k = 0; k < na; k++) out[o - na + k] = (Out)(acc >> (SB * k));
-}
-
-__global__ void fill_kernel_u8(uint8_t* out, size_t n, uint8_t v) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) out[i] = v;
-}
-__global__ void fill_kernel_u16(uint16_t* out, size_t n, uint16_t v) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) out[i] = v;
-}
-
-__global__ void u32_to_u64_kernel(const unsigned int* in, unsigned long long* out, int n, unsigned int mask) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = in[i] & mask;
-}
-
-__global__ void clear_invalid_kernel(unsigned int* cnt, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) cnt[i] &= ~DEC_INVALID;
-}
-
-__global__ void check_total_kernel(const unsigned long long* off, int nsub, size_t n, int* flag) {
-  if (off[nsub] < n) atomicOr(flag, FLAG_HUFF_CORRUPT);
-}
-
 }  // namespace
 
 int launch_codebook_scatter(cpsz_b200_ctx* ctx, const HuffEntry* d_entries, size_t n, unsigned long long* code,
@@ -788,73 +510,6 @@ int launch_hist_follow(cpsz_b200_ctx* ctx, const uint16_t* const codes[2], const
                                                             hist[0], hist[1], tickets, gave_up);
   count_launch(ctx);
   return check_launch("hist_follow_kernel");
-}
-
-size_t huff_decode_tmp_bytes(size_t nbits) {
-  size_t nsub = (nbits + DEC_S - 1) / DEC_S + 1;
-  return align_up(nsub + 1, 32) * 8 * 3 + align_up(nsub + 1, 32) * 4 * 2 + 4096 + scan_u32_tmp_bytes(nsub + 1);
-}
-
-int launch_huff_decode(cpsz_b200_ctx* ctx, const uint8_t* bytes, size_t nbytes, size_t n, HuffDecTable tab, void* out,
-                       int out_bytes_per_sym, void* tmp) {
-  if (n == 0) return CPSZ_OK;
-  if (tab.root_is_leaf) {
-    unsigned grid = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)ctx->num_sms * 8);
-    if (out_bytes_per_sym == 1) fill_kernel_u8<<<grid, 256, 0, ctx->stream>>>((uint8_t*)out, n, (uint8_t)tab.root_sym);
-    else fill_kernel_u16<<<grid, 256, 0, ctx->stream>>>((uint16_t*)out, n, (uint16_t)tab.root_sym);
-    count_launch(ctx);
-    return check_launch("huffman fill");
-  }
-  unsigned long long nbits = (unsigned long long)nbytes * 8;
-  int nsub = (int)((nbits + DEC_S - 1) / DEC_S);
-  if (nsub == 0) return set_error(CPSZ_ERR_FORMAT, "empty Huffman stream for %zu symbols", n);
-  char* p = (char*)tmp;
-  size_t a = align_up((size_t)nsub + 1, 32);
-  unsigned long long* start = (unsigned long long*)p;
-  p += a * 8;
-  unsigned long long* end = (unsigned long long*)p;
-  p += a * 8;
-  unsigned long long* off = (unsigned long long*)p;
-  p += a * 8;
-  unsigned int* cnt = (unsigned int*)p;
-  p += a * 4;
-  int* changed = (int*)p;
-  BitReader br{(const uint32_t*)bytes};
-  unsigned grid = (unsigned)((nsub + DEC_NT - 1) / DEC_NT);
-  dec_scan_kernel<<<grid, DEC_NT, 0, ctx->stream>>>(br, tab, nbits, nsub, start, end, cnt, 0, changed, ctx->d_flag);
-  count_launch(ctx);
-  // resynchronisation rounds; each round fixes at least one more subsequence,
-  // in practice the first round already converges.
-  int* h_changed = (int*)ctx->pinned;
-  for (int round = 0; round < nsub; round++) {
-    cudaMemsetAsync(changed, 0, sizeof(int), ctx->stream);
-    dec_scan_kernel<<<grid, DEC_NT, 0, ctx->stream>>>(br, tab, nbits, nsub, start, end, cnt, 1, changed, ctx->d_flag);
-    count_launch(ctx);
-    cudaMemcpyAsync(h_changed, changed, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-    CPSZ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    if (!*h_changed) break;
-  }
-  // output offsets: a device-wide u32 scan when every offset fits 32 bits (a
-  // subsequence decodes at most one symbol per bit, plus the one crossing its
-  // end), else one CTA over 64-bit counts; the exits are no longer needed
-  // after the final round, so their array holds the counts' copy
-  if (nbits + (unsigned long long)nsub < (1ull << 32)) {
-    unsigned int* off32 = reinterpret_cast<unsigned int*>(end);
-    clear_invalid_kernel<<<(nsub + 255) / 256, 256, 0, ctx->stream>>>(cnt, nsub);
-    CPSZ_TRY(launch_scan_u32(ctx, cnt, off32, (size_t)nsub, p + 256));  // off32[nsub] = the total
-    u32_to_u64_kernel<<<(nsub + 256) / 256, 256, 0, ctx->stream>>>(off32, off, nsub + 1, 0xffffffffu);
-  } else {
-    unsigned long long* cnt64 = end;
-    u32_to_u64_kernel<<<(nsub + 255) / 256, 256, 0, ctx->stream>>>(cnt, cnt64, nsub, ~DEC_INVALID);
-    scan_u64_kernel<<<1, 1024, 0, ctx->stream>>>(cnt64, off, (size_t)nsub);
-  }
-  check_total_kernel<<<1, 1, 0, ctx->stream>>>(off, nsub, n, ctx->d_flag);
-  if (out_bytes_per_sym == 1)
-    dec_write_kernel<uint8_t><<<grid, DEC_NT, 0, ctx->stream>>>(br, tab, nbits, nsub, start, off, n, (uint8_t*)out);
-  else
-    dec_write_kernel<uint16_t><<<grid, DEC_NT, 0, ctx->stream>>>(br, tab, nbits, nsub, start, off, n, (uint16_t*)out);
-  count_launch(ctx, 4);
-  return check_launch("huffman decode");
 }
 
 // ---- Huffman packing without any allocation ---------------------------------------------

@@ -269,67 +269,54 @@ bool huff_parse(const unsigned char* p, size_t avail, size_t max_symbol, HuffDec
               avail);
     return false;
   }
-  const unsigned char* tb = p + 12 + 1;
   const size_t nc = (size_t)node_count;
   const int wdt = nc <= 256 ? 1 : (nc <= 65536 ? 2 : 4);
-  auto rd = [&](const unsigned char* base, size_t i) -> uint32_t {
-    uint32_t v = 0;
-    memcpy(&v, base + i * wdt, wdt);
-    return v;
-  };
+  const unsigned char* L = p + 12 + 1;
+  const unsigned char* R = L + nc * wdt;
+  const unsigned char* C = R + nc * wdt;
+  const unsigned char* t = C + 4 * nc;
   out->node_count = (int)nc;
-  out->child.assign(2 * nc, 0);
-  out->sym.assign(nc, 0);
-  out->leaf.assign(nc, 0);
-  for (size_t i = 0; i < nc; i++) {
-    out->child[2 * i] = rd(tb, i);
-    out->child[2 * i + 1] = rd(tb + nc * wdt, i);
-    memcpy(&out->sym[i], tb + 2 * nc * wdt + 4 * i, 4);
-    out->leaf[i] = tb[2 * nc * wdt + 4 * nc + i];
-  }
+  out->tree_offset = 13;
+  out->tree_bytes = tree_size - 1;
   // The reference rebuilds the root with t = C[0]/t[0] only for <= 256 nodes
   // (reconstruct_HuffTree_from_bytes_anyStates, src/sz_huffman.cpp:570-596);
   // larger trees get an inner root.
-  out->root_is_leaf = (nc <= 256) && out->leaf[0];
-  out->root_sym = out->sym[0];
-  if (!out->root_is_leaf) out->leaf[0] = 0;
-  // validate: inner nodes have two children with larger indices; leaves carry
-  // an in-range symbol.
-  for (size_t i = 0; i < nc; i++) {
-    if (out->leaf[i] || (i == 0 && out->root_is_leaf)) {
-      if (out->sym[i] > max_symbol) {
-        set_error(CPSZ_ERR_FORMAT, "Huffman leaf symbol %u out of range", out->sym[i]);
-        return false;
+  out->root_is_leaf = (nc <= 256) && t[0];
+  memcpy(&out->root_sym, C, 4);
+  // inner nodes have two children with larger indices; leaves carry an
+  // in-range symbol
+  uint32_t max_sym = 0;
+  size_t bad_leaf = nc, bad_node = nc;
+  auto check = [&](auto tag) {
+    using Wd = decltype(tag);
+    for (size_t i = 0; i < nc; i++) {
+      Wd l, r;
+      uint32_t c;
+      memcpy(&l, L + i * sizeof(Wd), sizeof(Wd));
+      memcpy(&r, R + i * sizeof(Wd), sizeof(Wd));
+      memcpy(&c, C + 4 * i, 4);
+      max_sym = std::max(max_sym, c);
+      const bool leaf = t[i] && (i || out->root_is_leaf);
+      if (leaf ? c > max_symbol : (l <= i || r <= i || l >= nc || r >= nc)) {
+        (leaf ? bad_leaf : bad_node) = i;
+        return;
       }
-      continue;
     }
-    uint32_t l = out->child[2 * i], r = out->child[2 * i + 1];
-    if (l <= i || r <= i || l >= nc || r >= nc) {
-      set_error(CPSZ_ERR_FORMAT, "Huffman tree node %zu has invalid children", i);
-      return false;
-    }
+  };
+  if (wdt == 1) check(uint8_t{});
+  else if (wdt == 2) check(uint16_t{});
+  else check(uint32_t{});
+  if (bad_leaf < nc) {
+    uint32_t c;
+    memcpy(&c, C + 4 * bad_leaf, 4);
+    set_error(CPSZ_ERR_FORMAT, "Huffman leaf symbol %u out of range", c);
+    return false;
   }
-  // first-level table
-  out->lut.assign(1u << HUFF_LUT_BITS, 0);
-  if (!out->root_is_leaf) {
-    for (uint32_t pat = 0; pat < (1u << HUFF_LUT_BITS); pat++) {
-      uint32_t node = 0;
-      uint32_t e = 0;
-      bool done = false;
-      for (int k = 0; k < HUFF_LUT_BITS; k++) {
-        uint32_t bit = (pat >> (HUFF_LUT_BITS - 1 - k)) & 1u;
-        node = out->child[2 * node + bit];
-        if (out->leaf[node]) {
-          e = (out->sym[node] << 8) | (uint32_t)(k + 1);
-          done = true;
-          break;
-        }
-      }
-      if (!done) e = 0x80u | (node << 8);
-      out->lut[pat] = e;
-    }
+  if (bad_node < nc) {
+    set_error(CPSZ_ERR_FORMAT, "Huffman tree node %zu has invalid children", bad_node);
+    return false;
   }
-  out->tree_size = tree_size;
+  out->max_sym = max_sym;
   memcpy(&out->nbytes, p + 12 + tree_size, 8);
   out->bits_offset = 12 + (size_t)tree_size + 8;
   if (out->nbytes > avail - out->bits_offset) {

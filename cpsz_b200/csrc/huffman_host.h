@@ -39,17 +39,16 @@ void huff_tables(const HuffCodebook& cb, size_t bins, unsigned long long* code, 
 // Section size: 8 + 4 + tree_size + 8 + ceil(total_bits/8).
 inline size_t huff_section_bytes(const HuffCodebook& cb) { return cb.tree_bytes.size() + 8 + (cb.total_bits + 7) / 8; }
 
+// A parsed Huffman section; offsets are from its start.
 struct HuffDecoderHost {
-  std::vector<uint32_t> lut;    // 1 << 12 entries
-  std::vector<uint32_t> child;  // 2 per node
-  std::vector<uint32_t> sym;
-  std::vector<uint8_t> leaf;
   int node_count = 0;
   bool root_is_leaf = false;
   uint32_t root_sym = 0;
-  size_t tree_size = 0;
+  uint32_t max_sym = 0;        // largest C entry of any node
+  size_t tree_offset = 0;      // the arrays L, R, C, t
+  size_t tree_bytes = 0;
   size_t nbytes = 0;           // bit-stream bytes
-  size_t bits_offset = 0;      // offset of the bit stream from the section start
+  size_t bits_offset = 0;
   size_t section_bytes = 0;    // whole section
 };
 

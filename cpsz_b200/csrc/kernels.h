@@ -23,6 +23,7 @@ constexpr int FLAG_TIMEOUT = 2;       // a bounded inter-CTA wait gave up
 constexpr int FLAG_HUFF_CORRUPT = 4;  // a Huffman stream does not decode to the expected symbols
 constexpr int FLAG_RAW_RANGE = 8;     // an unpredictable-value index fell outside the stored list
 constexpr int FLAG_OUT_CAPACITY = 16; // an output stream did not fit its buffer
+constexpr int FLAG_HUFF_RESYNC = 32;  // a Huffman stream needs more synchronisation rounds (launch_huff_decode)
 
 // ---- 2D error bounds ---------------------------------------------------------
 // The bound kernel beside the wavefront runs unit by unit: a unit is a
@@ -233,25 +234,26 @@ int launch_hist_u16_pair(cpsz_b200_ctx* ctx, const uint16_t* a, const uint16_t* 
 int launch_hist_follow(cpsz_b200_ctx* ctx, const uint16_t* const codes[2], const unsigned* const group_done[2], int r1,
                        int r2, unsigned long long* const hist[2], unsigned* tickets, int* gave_up, cudaStream_t stream);
 
-// Decoder table: first-level lookup of HUFF_LUT_BITS bits; entries
-//   leaf:  (sym << 8) | len            (len in 1..HUFF_LUT_BITS)
-//   inner: 0x80 | (node << 8)          (walk the tree from `node` bit by bit)
-// Tree arrays: child[2*node + bit] (node index; leaves have t = 1 and sym in C).
-constexpr int HUFF_LUT_BITS = 12;
-struct HuffDecTable {
-  const uint32_t* lut;       // 1 << HUFF_LUT_BITS entries
-  const uint32_t* child;     // 2 * node_count
-  const uint32_t* sym;       // node_count (leaf symbol)
-  const uint8_t* leaf;       // node_count
-  int node_count;
-  int root_is_leaf;          // single-symbol stream (no bits)
-  uint32_t root_sym;
+// One Huffman stream to decode (huff_decode.cu): exactly n symbols, u8 or u16.
+constexpr size_t HUFF_DEC_PAD = 16;  // zero bytes behind a stream's bits
+struct HuffDecJob {
+  const uint8_t* bits = nullptr;  // device, 4-byte aligned, nbytes + HUFF_DEC_PAD readable
+  size_t nbytes = 0;
+  const uint8_t* tree = nullptr;  // device, 16-byte aligned: L, R, C, t as serialized, checked by huff_parse
+  int node_count = 0;
+  bool root_is_leaf = false;      // single-symbol stream (no bits): n times root_sym
+  uint32_t root_sym = 0;
+  size_t n = 0;
+  void* out = nullptr;            // device
+  int out_bytes = 1;              // 1: symbols <= 255, 2: symbols <= 65535
 };
-size_t huff_decode_tmp_bytes(size_t nbits);
-// Decodes exactly n symbols from a bit stream of nbits bits (words: big-endian
-// byte order, padded with >= 8 zero bytes).  Output u8 or u16.
-int launch_huff_decode(cpsz_b200_ctx* ctx, const uint8_t* bytes, size_t nbytes, size_t n, HuffDecTable tab,
-                       void* out, int out_bytes_per_sym, void* tmp);
+// Up to three streams at once.  A stream whose subsequences did not settle in
+// the fixed rounds raises FLAG_HUFF_RESYNC (its output is then incomplete):
+// the caller decodes again with settle, which waits on the host until they
+// have.  A stream that does not decode to n symbols raises FLAG_HUFF_CORRUPT.
+// tmp: huff_decode_tmp_bytes(jobs, nj).
+size_t huff_decode_tmp_bytes(const HuffDecJob* jobs, int nj);
+int launch_huff_decode(cpsz_b200_ctx* ctx, const HuffDecJob* jobs, int nj, void* tmp, bool settle);
 
 // ---- 3D offline (log) path ----------------------------------------------------------
 // Id written for predictable-bound points that still end unpredictable

@@ -132,7 +132,7 @@ int flag_error(int flag) {
   if (flag & FLAG_TIMEOUT) return set_error(CPSZ_ERR_TIMEOUT, "a bounded device-side wait gave up");
   if (flag & FLAG_ID_OVERFLOW)
     return set_error(CPSZ_ERR_UNSUPPORTED, "an error-bound id does not fit the 8-bit id stream (max_pwr_eb too large)");
-  if (flag & FLAG_HUFF_CORRUPT) return set_error(CPSZ_ERR_FORMAT, "Huffman stream does not decode");
+  if (flag & (FLAG_HUFF_CORRUPT | FLAG_HUFF_RESYNC)) return set_error(CPSZ_ERR_FORMAT, "Huffman stream does not decode");
   if (flag & FLAG_RAW_RANGE) return set_error(CPSZ_ERR_FORMAT, "unpredictable-value list shorter than its codes");
   if (flag & FLAG_OUT_CAPACITY) return set_error(CPSZ_ERR_INVALID, "an output stream exceeded its buffer");
   return CPSZ_OK;
@@ -1263,9 +1263,9 @@ int decompress_2d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
   HuffDecoderHost hid;
   if (!huff_parse(blob + BLOB_HDR, eb_size, 2047, &hid)) return CPSZ_ERR_FORMAT;
   if (hid.section_bytes > eb_size) return set_error(CPSZ_ERR_FORMAT, "id section overruns");
-  for (uint32_t s : hid.sym)
-    if (s > (uint32_t)ID_MAX_2D)
-      return set_error(CPSZ_ERR_UNSUPPORTED, "error-bound id %u beyond the supported range (<= %d)", s, ID_MAX_2D);
+  if (hid.max_sym > (uint32_t)ID_MAX_2D)
+    return set_error(CPSZ_ERR_UNSUPPORTED, "error-bound id %u beyond the supported range (<= %d)", hid.max_sym,
+                     ID_MAX_2D);
   FieldView fv[2];
   CPSZ_TRY(parse_field(blob, fields_at, u_size, N, nblocks, &fv[0]));
   CPSZ_TRY(parse_field(blob, fields_at + u_size, v_size, N, nblocks, &fv[1]));
@@ -1273,102 +1273,80 @@ int decompress_2d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
   if (log_form) CPSZ_TRY(libm_tables_device(ctx, &libm));
   const bool dev_out = is_device_ptr(U_out) && is_device_ptr(V_out);
 
-  // ---- workspace ----
+  // ---- workspace: what goes up (one image), what starts at zero, the rest ----
+  int r1v[2] = {r1, r1};
+  std::vector<WaveItem> items;
+  const int n_items = build_wave_items(2, r1v, items);
+  WaveField hf[2] = {};
   const HuffDecoderHost* hs[3] = {&hid, &fv[0].huff, &fv[1].huff};
+  const size_t sec_at[3] = {BLOB_HDR, fv[0].huff_off, fv[1].huff_off};
+  Upload up;
+  const size_t up_fields = up.add(hf, sizeof(hf)), up_items = up.add(items.data(), n_items * sizeof(WaveItem));
+  size_t up_tree[3], up_bits[3], up_unpred[2];
+  for (int k = 0; k < 3; k++) up_tree[k] = up.add(blob + sec_at[k] + hs[k]->tree_offset, hs[k]->tree_bytes);
+  const size_t up_signs = up.add(blob + BLOB_HDR + eb_size, 2 * sign_bytes);
+  up_bits[0] = up.add(blob + sec_at[0] + hid.bits_offset, hid.nbytes, HUFF_DEC_PAD);
+  up.cut();
+  for (int f = 0; f < 2; f++) {
+    up_bits[1 + f] = up.add(blob + sec_at[1 + f] + hs[1 + f]->bits_offset, hs[1 + f]->nbytes, HUFF_DEC_PAD);
+    up_unpred[f] = up.add(blob + fv[f].unpred_off, 4 * fv[f].n_unpred);
+    up.cut();
+  }
+  HuffDecJob dec[3];
+  for (int k = 0; k < 3; k++) {
+    dec[k].nbytes = hs[k]->nbytes;
+    dec[k].node_count = hs[k]->node_count;
+    dec[k].root_is_leaf = hs[k]->root_is_leaf;
+    dec[k].root_sym = hs[k]->root_sym;
+    dec[k].n = k ? N : n_ids;
+    dec[k].out_bytes = k ? 2 : 1;
+  }
+  // a small blob goes up and is decoded in one piece, a large one stream by
+  // stream, each decoded while the next one goes up
+  const bool whole = up.bytes() <= UPLOAD_WHOLE;
+  size_t dec_bytes[3];
+  for (int k = 0; k < 3; k++) dec_bytes[k] = whole ? (k ? 0 : huff_decode_tmp_bytes(dec, 3)) : huff_decode_tmp_bytes(&dec[k], 1);
+  const size_t strip_bytes = align_up(strip_scratch_bytes(r1, r2), 256), gbnd_bytes = 2 * (size_t)ngroups * r2 * 8;
+  const size_t zero_bytes = 256 + 2 * strip_bytes + gbnd_bytes;
   size_t bytes = 0;
   auto add = [&](size_t b) { bytes += align_up(b, 256) + 256; };
-  if (!dev_out) add(8 * N);
-  add(n_ids);  // ids
-  add(2 * sign_bytes + 16);
-  for (int k = 0; k < 3; k++) {
-    add(hs[k]->nbytes + 64);
-    add((1u << HUFF_LUT_BITS) * 4 + hs[k]->child.size() * 4 + hs[k]->sym.size() * 4 + hs[k]->leaf.size());
-    add(huff_decode_tmp_bytes(hs[k]->nbytes * 8));
+  add(up.bytes());
+  add(zero_bytes);
+  for (int f = 0; f < 2; f++) {
+    if (!dev_out) add(4 * N);
+    add(2 * N);  // codes in block order
+    add(8 * N);  // raster pairs
   }
-  add(4 * N);  // codes blocks
-  add(8 * N);  // (pairs: the raw raster below holds 16 N)
-  add(8 * N);  // raw raster
-  add(2 * 4 * N);  // unpred lists
-  add(2 * strip_scratch_bytes(r1, r2));
-  add(2 * (size_t)ngroups * r2 * 8);
-  add(64);
-  add(2 * sizeof(WaveField) + 2 * (size_t)ngroups * sizeof(WaveItem));
+  add(n_ids);
+  for (int k = 0; k < 3; k++) add(dec_bytes[k]);
   CPSZ_TRY(arena_reserve(ctx, bytes));
   CPSZ_TRY(pinned_reserve(ctx, 4096));
-  auto A = [&](size_t b) { return arena_alloc(ctx, b); };
+  auto A = [&](size_t b) { return (uint8_t*)arena_alloc(ctx, b); };
   cudaStream_t st = ctx->stream;
+  uint8_t* d_up = A(up.bytes());
+  uint8_t* d_zero = A(zero_bytes);  // the wavefront's queue, strip scratch, boundary rows
   float* dU = dev_out ? U_out : (float*)A(4 * N);
   float* dV = dev_out ? V_out : (float*)A(4 * N);
-  uint8_t* ids = (uint8_t*)A(n_ids);
-  uint8_t* signs = (uint8_t*)A(2 * sign_bytes + 16);
-  if (sign_bytes) CPSZ_TRY(h2d(ctx, signs, blob + BLOB_HDR + eb_size, 2 * sign_bytes, st));
-  uint8_t* bits[3];
-  HuffDecTable tab[3];
-  void* dtmp[3];
-  for (int k = 0; k < 3; k++) {
-    const HuffDecoderHost& h = *hs[k];
-    bits[k] = (uint8_t*)A(h.nbytes + 64);
-    size_t tb = (1u << HUFF_LUT_BITS) * 4 + h.child.size() * 4 + h.sym.size() * 4 + h.leaf.size();
-    uint8_t* t = (uint8_t*)A(tb);
-    dtmp[k] = A(huff_decode_tmp_bytes(h.nbytes * 8));
-    const size_t off_bits = (k == 0) ? BLOB_HDR + h.bits_offset : fv[k - 1].huff_off + h.bits_offset;
-    CPSZ_CUDA_TRY(cudaMemsetAsync(bits[k], 0, h.nbytes + 64, st));
-    if (h.nbytes) CPSZ_TRY(h2d(ctx, bits[k], blob + off_bits, h.nbytes, st));
-    uint32_t* lut = (uint32_t*)t;
-    uint32_t* child = lut + (1u << HUFF_LUT_BITS);
-    uint32_t* sym = child + h.child.size();
-    uint8_t* leaf = (uint8_t*)(sym + h.sym.size());
-    CPSZ_CUDA_TRY(cudaMemcpyAsync(lut, h.lut.data(), h.lut.size() * 4, cudaMemcpyHostToDevice, st));
-    CPSZ_CUDA_TRY(cudaMemcpyAsync(child, h.child.data(), h.child.size() * 4, cudaMemcpyHostToDevice, st));
-    CPSZ_CUDA_TRY(cudaMemcpyAsync(sym, h.sym.data(), h.sym.size() * 4, cudaMemcpyHostToDevice, st));
-    CPSZ_CUDA_TRY(cudaMemcpyAsync(leaf, h.leaf.data(), h.leaf.size(), cudaMemcpyHostToDevice, st));
-    tab[k] = HuffDecTable{lut, child, sym, leaf, h.node_count, h.root_is_leaf ? 1 : 0, h.root_sym};
-  }
+  uint8_t* ids = A(n_ids);
   uint16_t* cblocks[2];
   float2* raw[2];  // (addend, raw flag) per point; .x holds the raw value where the code is 0
-  float* unpred[2];
-  void* strip[2];
   for (int f = 0; f < 2; f++) {
     cblocks[f] = (uint16_t*)A(2 * N);
     raw[f] = (float2*)A(8 * N);
-    unpred[f] = (float*)A(4 * fv[f].n_unpred + 4);
-    strip[f] = A(strip_scratch_bytes(r1, r2));
-    if (fv[f].n_unpred)
-      CPSZ_TRY(h2d(ctx, unpred[f], blob + fv[f].unpred_off, 4 * fv[f].n_unpred, st));
   }
-  unsigned long long* gbnd = (unsigned long long*)A(2 * (size_t)ngroups * r2 * 8);
-  int* queue = (int*)A(64);
-  WaveField* dfields = (WaveField*)A(2 * sizeof(WaveField));
-  WaveItem* ditems = (WaveItem*)A(2 * (size_t)ngroups * sizeof(WaveItem));
-  if (!ditems) return set_error(CPSZ_ERR_NOMEM, "workspace layout overflow");
-  CPSZ_CUDA_TRY(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), st));
-  reset_marks(ctx);
-  mark(ctx, "huffman_decode");
-
-  // ---- Huffman decode ----
-  CPSZ_TRY(launch_huff_decode(ctx, bits[0], hid.nbytes, n_ids, tab[0], ids, 1, dtmp[0]));
-  for (int f = 0; f < 2; f++)
-    CPSZ_TRY(launch_huff_decode(ctx, bits[1 + f], fv[f].huff.nbytes, N, tab[1 + f], cblocks[f], 2, dtmp[1 + f]));
-  // ---- raster pairs, unpredictable scatter ----
-  mark(ctx, "raster+scatter");
-  unsigned int* h_cnt = (unsigned int*)ctx->pinned + 16;
-  {
-    const uint16_t* cb[2] = {cblocks[0], cblocks[1]};
-    // offline_log: one id stream for both components, base 2
-    const uint8_t* idf[2] = {ids, log_form ? ids : ids + N};
-    const float* un[2] = {unpred[0], unpred[1]};
-    const unsigned long long nun[2] = {fv[0].n_unpred, fv[1].n_unpred};
-    CPSZ_TRY(launch_strip_unpass(ctx, cb, idf, un, nun, r1, r2, raw, strip, log_form ? 1 : 2));
-    for (int f = 0; f < 2; f++)
-      CPSZ_CUDA_TRY(cudaMemcpyAsync(h_cnt + f, strip_total(strip[f], r1, r2), 4, cudaMemcpyDeviceToHost, st));
+  void* dtmp[3];
+  for (int k = 0; k < 3; k++) dtmp[k] = A(dec_bytes[k]);
+  if (!dtmp[2]) return set_error(CPSZ_ERR_NOMEM, "workspace layout overflow");
+  void* strip[2] = {d_zero + 256, d_zero + 256 + strip_bytes};
+  unsigned long long* gbnd = (unsigned long long*)(d_zero + 256 + 2 * strip_bytes);
+  for (int k = 0; k < 3; k++) {
+    dec[k].bits = d_up + up_bits[k];
+    dec[k].tree = d_up + up_tree[k];
+    dec[k].out = k ? (void*)cblocks[k - 1] : (void*)ids;
   }
-  // ---- wavefront ----
-  WaveField hf[2] = {};
   for (int f = 0; f < 2; f++) {
     WaveField& F = hf[f];
     F.pair = raw[f];
-    F.codes = nullptr;
-    F.trace = nullptr;
     F.out = f ? dV : dU;
     F.gbnd = gbnd + (size_t)f * ngroups * r2;
     F.pair_pitch = r2;
@@ -1377,28 +1355,73 @@ int decompress_2d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
     F.r1 = r1;
     F.r2 = r2;
   }
-  int r1v[2] = {r1, r1};
-  std::vector<WaveItem> items;
-  int n_items = build_wave_items(2, r1v, items);
-  CPSZ_CUDA_TRY(cudaMemcpyAsync(dfields, hf, sizeof(hf), cudaMemcpyHostToDevice, st));
-  CPSZ_CUDA_TRY(cudaMemcpyAsync(ditems, items.data(), n_items * sizeof(WaveItem), cudaMemcpyHostToDevice, st));
-  CPSZ_CUDA_TRY(cudaMemsetAsync(gbnd, 0, 2 * (size_t)ngroups * r2 * 8, st));
-  CPSZ_CUDA_TRY(cudaMemsetAsync(queue, 0, 64, st));
-  mark(ctx, "wave2d_decompress");
-  CPSZ_TRY(launch_wave2d(ctx, true, dfields, ditems, n_items, queue, (size_t)r1 * r2));
-  if (log_form) {
-    mark(ctx, "exp2d");
-    CPSZ_TRY(launch_exp2d(ctx, dU, dV, signs, signs + sign_bytes, N, libm.exp2f));
+  uint8_t* d_signs = d_up + up_signs;
+  unsigned int* h_cnt = (unsigned int*)ctx->pinned + 16;
+
+  // a copy from the caller's page-locked blob must not outlive the call
+  struct AuxDrain {
+    cudaStream_t s = nullptr;
+    ~AuxDrain() {
+      if (s) cudaStreamSynchronize(s);
+    }
+  } aux_drain;
+
+  // A stream whose subsequences did not settle in the decoder's fixed rounds
+  // (FLAG_HUFF_RESYNC) is decoded again, with rounds until they have.
+  for (int attempt = 0;; attempt++) {
+    const bool settle = attempt > 0;
+    CPSZ_CUDA_TRY(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), st));
+    CPSZ_CUDA_TRY(cudaMemsetAsync(d_zero, 0, zero_bytes, st));
+    reset_marks(ctx);
+    mark(ctx, "huffman_decode");
+    if (whole || settle) {
+      if (!settle) CPSZ_TRY(up.send_whole(ctx, d_up, st));
+      if (whole) {
+        CPSZ_TRY(launch_huff_decode(ctx, dec, 3, dtmp[0], settle));
+      } else {
+        for (int k = 0; k < 3; k++) CPSZ_TRY(launch_huff_decode(ctx, &dec[k], 1, dtmp[k], settle));
+      }
+    } else {
+      aux_drain.s = ctx->aux;
+      for (int k = 0; k < 3; k++) {
+        CPSZ_TRY(up.send_part(ctx, d_up, k, ctx->aux));
+        CPSZ_CUDA_TRY(cudaEventRecord(ctx->up_ev[k], ctx->aux));
+        CPSZ_CUDA_TRY(cudaStreamWaitEvent(st, ctx->up_ev[k], 0));
+        CPSZ_TRY(launch_huff_decode(ctx, &dec[k], 1, dtmp[k], false));
+      }
+    }
+    // ---- raster pairs, unpredictable scatter ----
+    mark(ctx, "raster+scatter");
+    {
+      const uint16_t* cb[2] = {cblocks[0], cblocks[1]};
+      // offline_log: one id stream for both components, base 2
+      const uint8_t* idf[2] = {ids, log_form ? ids : ids + N};
+      const float* un[2] = {(const float*)(d_up + up_unpred[0]), (const float*)(d_up + up_unpred[1])};
+      const unsigned long long nun[2] = {fv[0].n_unpred, fv[1].n_unpred};
+      CPSZ_TRY(launch_strip_unpass(ctx, cb, idf, un, nun, r1, r2, raw, strip, log_form ? 1 : 2));
+      for (int f = 0; f < 2; f++)
+        CPSZ_CUDA_TRY(cudaMemcpyAsync(h_cnt + f, strip_total(strip[f], r1, r2), 4, cudaMemcpyDeviceToHost, st));
+    }
+    // ---- wavefront ----
+    mark(ctx, "wave2d_decompress");
+    CPSZ_TRY(launch_wave2d(ctx, true, (const WaveField*)(d_up + up_fields), (const WaveItem*)(d_up + up_items), n_items,
+                           (int*)d_zero, (size_t)r1 * r2));
+    if (log_form) {
+      mark(ctx, "exp2d");
+      CPSZ_TRY(launch_exp2d(ctx, dU, dV, d_signs, d_signs + sign_bytes, N, libm.exp2f));
+    }
+    mark(ctx, "d2h");
+    if (!dev_out) {
+      CPSZ_TRY(d2h(ctx, U_out, dU, 4 * N, st));
+      CPSZ_TRY(d2h(ctx, V_out, dV, 4 * N, st));
+    }
+    mark(ctx, "end");
+    int flag = 0;
+    CPSZ_TRY(read_flag(ctx, &flag));
+    if ((flag & FLAG_HUFF_RESYNC) && !settle) continue;
+    if (flag) return flag_error(flag);
+    break;
   }
-  mark(ctx, "d2h");
-  if (!dev_out) {
-    CPSZ_TRY(d2h(ctx, U_out, dU, 4 * N, st));
-    CPSZ_TRY(d2h(ctx, V_out, dV, 4 * N, st));
-  }
-  mark(ctx, "end");
-  int flag = 0;
-  CPSZ_TRY(read_flag(ctx, &flag));
-  if (flag) return flag_error(flag);
   for (int f = 0; f < 2; f++)
     if (h_cnt[f] != fv[f].n_unpred)
       return set_error(CPSZ_ERR_FORMAT, "field %d: %u zero codes but %zu unpredictable values", f, h_cnt[f],

@@ -41,7 +41,7 @@ int flag_error3(int flag) {
     return set_error(CPSZ_ERR_UNSUPPORTED,
                      "an error-bound id reaches the reference's unpredictable marker 24 (max_pwr_eb >= 3)");
   if (flag & FLAG_RAW_RANGE) return set_error(CPSZ_ERR_FORMAT, "code or unpredictable stream shorter than its ids");
-  if (flag & FLAG_HUFF_CORRUPT) return set_error(CPSZ_ERR_FORMAT, "Huffman stream does not decode");
+  if (flag & (FLAG_HUFF_CORRUPT | FLAG_HUFF_RESYNC)) return set_error(CPSZ_ERR_FORMAT, "Huffman stream does not decode");
   if (flag & FLAG_OUT_CAPACITY) return set_error(CPSZ_ERR_INVALID, "an output stream exceeded its buffer");
   if (flag & FLAG_TIMEOUT) return set_error(CPSZ_ERR_TIMEOUT, "a bounded device-side wait gave up");
   return set_error(CPSZ_ERR_CUDA, "device flag %d", flag);
@@ -302,9 +302,9 @@ int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
   if (n_ids != N) return set_error(CPSZ_ERR_FORMAT, "id count %llu != %zu points", n_ids, N);
   HuffDecoderHost hs[2];
   if (!huff_parse(blob + at, blob_size - at, 511, &hs[0])) return CPSZ_ERR_FORMAT;
-  for (uint32_t s : hs[0].sym)
-    if (s > (uint32_t)ID_RAW_3D)
-      return set_error(CPSZ_ERR_UNSUPPORTED, "error-bound id %u beyond the supported range (<= %d)", s, ID_RAW_3D);
+  if (hs[0].max_sym > (uint32_t)ID_RAW_3D)
+    return set_error(CPSZ_ERR_UNSUPPORTED, "error-bound id %u beyond the supported range (<= %d)", hs[0].max_sym,
+                     ID_RAW_3D);
   const size_t ids_at = at;
   at += hs[0].section_bytes;
   if (blob_size - at < 8) return set_error(CPSZ_ERR_FORMAT, "blob truncated before the code section");
@@ -317,18 +317,37 @@ int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
   LibmTables lt;
   CPSZ_TRY(libm_tables_device(ctx, &lt));
 
+  // what goes up, as one image: a small blob whole, a large one stream by
+  // stream, each decoded while the next one goes up
+  const size_t sec_at[2] = {ids_at, codes_at};
+  Upload up;
+  size_t up_tree[2], up_bits[2];
+  for (int k = 0; k < 2; k++) up_tree[k] = up.add(blob + sec_at[k] + hs[k].tree_offset, hs[k].tree_bytes);
+  up_bits[0] = up.add(blob + ids_at + hs[0].bits_offset, hs[0].nbytes, HUFF_DEC_PAD);
+  up.cut();
+  up_bits[1] = up.add(blob + codes_at + hs[1].bits_offset, hs[1].nbytes, HUFF_DEC_PAD);
+  up.cut();
+  const size_t up_unpred = up.add(blob + unpred_at, 4 * n_unpred), up_signs = up.add(blob + 8, 3 * smap, 16);
+  up.cut();
+  HuffDecJob dec[2];
+  for (int k = 0; k < 2; k++) {
+    dec[k].nbytes = hs[k].nbytes;
+    dec[k].node_count = hs[k].node_count;
+    dec[k].root_is_leaf = hs[k].root_is_leaf;
+    dec[k].root_sym = hs[k].root_sym;
+    dec[k].n = k ? n_codes : N;
+    dec[k].out_bytes = k ? 2 : 1;
+  }
+  const bool whole = up.bytes() <= UPLOAD_WHOLE;
+  size_t dec_bytes[2];
+  for (int k = 0; k < 2; k++) dec_bytes[k] = whole ? (k ? 0 : huff_decode_tmp_bytes(dec, 2)) : huff_decode_tmp_bytes(&dec[k], 1);
   size_t bytes = 0;
   auto add = [&](size_t b) { bytes += align_up(b, 256) + 256; };
+  add(up.bytes());
   if (!dev_out) add(12 * N);
-  add(3 * smap + 16);
-  add(4 * n_unpred + 16);
   add(N);
   add(2 * n_codes + 16);
-  for (int k = 0; k < 2; k++) {
-    add(hs[k].nbytes + 64);
-    add((1u << HUFF_LUT_BITS) * 4 + hs[k].child.size() * 4 + hs[k].sym.size() * 4 + hs[k].leaf.size());
-    add(huff_decode_tmp_bytes(hs[k].nbytes * 8));
-  }
+  for (int k = 0; k < 2; k++) add(dec_bytes[k]);
   add(2 * (nchunks + 1) * 4);
   add(scan_u32_tmp_bytes(nchunks));
   add(16 * N);
@@ -338,38 +357,17 @@ int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
   CPSZ_TRY(pinned_reserve(ctx, 4096));
   auto A = [&](size_t b) { return arena_alloc(ctx, b); };
   cudaStream_t st = ctx->stream;
+  uint8_t* d_up = (uint8_t*)A(up.bytes());
   float* out = dev_out ? nullptr : (float*)A(12 * N);
   float* dU = dev_out ? U_out : out;
   float* dV = dev_out ? V_out : out + N;
   float* dW = dev_out ? W_out : out + 2 * N;
-  uint8_t* signs = (uint8_t*)A(3 * smap + 16);
-  float* unpred = (float*)A(4 * n_unpred + 16);
+  const uint8_t* signs = d_up + up_signs;
+  const float* unpred = (const float*)(d_up + up_unpred);
   uint8_t* ids = (uint8_t*)A(N);
   uint16_t* codes = (uint16_t*)A(2 * n_codes + 16);
-  uint8_t* bits[2];
-  HuffDecTable tab[2];
   void* dtmp[2];
-  const size_t sec_at[2] = {ids_at, codes_at};
-  for (int k = 0; k < 2; k++) {
-    const HuffDecoderHost& h = hs[k];
-    bits[k] = (uint8_t*)A(h.nbytes + 64);
-    const size_t tb = (1u << HUFF_LUT_BITS) * 4 + h.child.size() * 4 + h.sym.size() * 4 + h.leaf.size();
-    uint8_t* t = (uint8_t*)A(tb);
-    dtmp[k] = A(huff_decode_tmp_bytes(h.nbytes * 8));
-    if (!dtmp[k]) return set_error(CPSZ_ERR_NOMEM, "workspace layout overflow");
-    CPSZ_CUDA_TRY(cudaMemsetAsync(bits[k], 0, h.nbytes + 64, st));
-    if (h.nbytes)
-      CPSZ_TRY(h2d(ctx, bits[k], blob + sec_at[k] + h.bits_offset, h.nbytes, st));
-    uint32_t* lut = (uint32_t*)t;
-    uint32_t* child = lut + (1u << HUFF_LUT_BITS);
-    uint32_t* sym = child + h.child.size();
-    uint8_t* leaf = (uint8_t*)(sym + h.sym.size());
-    CPSZ_CUDA_TRY(cudaMemcpyAsync(lut, h.lut.data(), h.lut.size() * 4, cudaMemcpyHostToDevice, st));
-    CPSZ_CUDA_TRY(cudaMemcpyAsync(child, h.child.data(), h.child.size() * 4, cudaMemcpyHostToDevice, st));
-    CPSZ_CUDA_TRY(cudaMemcpyAsync(sym, h.sym.data(), h.sym.size() * 4, cudaMemcpyHostToDevice, st));
-    CPSZ_CUDA_TRY(cudaMemcpyAsync(leaf, h.leaf.data(), h.leaf.size(), cudaMemcpyHostToDevice, st));
-    tab[k] = HuffDecTable{lut, child, sym, leaf, h.node_count, h.root_is_leaf ? 1 : 0, h.root_sym};
-  }
+  for (int k = 0; k < 2; k++) dtmp[k] = A(dec_bytes[k]);
   unsigned* chunk_cnt = (unsigned*)A((nchunks + 1) * 4);
   unsigned* chunk_off = (unsigned*)A((nchunks + 1) * 4);
   void* scan_tmp = A(scan_u32_tmp_bytes(nchunks));
@@ -377,29 +375,59 @@ int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
   float4* rec = (float4*)A(16 * N);
   void* wave_sync = A(wave3d_scratch_bytes(r1, r2));
   if (!wave_sync) return set_error(CPSZ_ERR_NOMEM, "workspace layout overflow");
-  CPSZ_CUDA_TRY(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), st));
-  CPSZ_TRY(h2d(ctx, signs, blob + 8, 3 * smap, st));
-  if (n_unpred) CPSZ_TRY(h2d(ctx, unpred, blob + unpred_at, 4 * n_unpred, st));
-  reset_marks(ctx);
-  mark(ctx, "huffman_decode");
-  CPSZ_TRY(launch_huff_decode(ctx, bits[0], hs[0].nbytes, N, tab[0], ids, 1, dtmp[0]));
-  if (n_codes) CPSZ_TRY(launch_huff_decode(ctx, bits[1], hs[1].nbytes, n_codes, tab[1], codes, 2, dtmp[1]));
-  mark(ctx, "prep3d");
-  CPSZ_TRY(launch_chunk_count_3d(ctx, false, ids, N, chunk_cnt));
-  CPSZ_TRY(launch_scan_u32(ctx, chunk_cnt, chunk_off, nchunks, scan_tmp));
-  CPSZ_TRY(launch_prep3d(ctx, ids, N, chunk_off, codes, n_codes, unpred, n_unpred, pairs));
-  mark(ctx, "wave3d_decompress");
-  CPSZ_TRY(launch_wave3d(ctx, true, pairs, rec, nullptr, signs, smap, &lt, dU, dV, dW, r1, r2, r3, wave_sync));
-  mark(ctx, "d2h");
-  if (!dev_out) {
-    CPSZ_TRY(d2h(ctx, U_out, dU, 4 * N, st));
-    CPSZ_TRY(d2h(ctx, V_out, dV, 4 * N, st));
-    CPSZ_TRY(d2h(ctx, W_out, dW, 4 * N, st));
+  for (int k = 0; k < 2; k++) {
+    dec[k].bits = d_up + up_bits[k];
+    dec[k].tree = d_up + up_tree[k];
+    dec[k].out = k ? (void*)codes : (void*)ids;
   }
-  mark(ctx, "end");
-  int flag = 0;
-  CPSZ_TRY(read_flag3(ctx, &flag));
-  if (flag) return flag_error3(flag);
+  // a copy from the caller's page-locked blob must not outlive the call
+  struct AuxDrain {
+    cudaStream_t s = nullptr;
+    ~AuxDrain() {
+      if (s) cudaStreamSynchronize(s);
+    }
+  } aux_drain;
+
+  // A stream whose subsequences did not settle in the decoder's fixed rounds
+  // (FLAG_HUFF_RESYNC) is decoded again, with rounds until they have.
+  for (int attempt = 0;; attempt++) {
+    const bool settle = attempt > 0;
+    CPSZ_CUDA_TRY(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), st));
+    reset_marks(ctx);
+    mark(ctx, "huffman_decode");
+    if (whole) {
+      if (!settle) CPSZ_TRY(up.send_whole(ctx, d_up, st));
+      CPSZ_TRY(launch_huff_decode(ctx, dec, 2, dtmp[0], settle));
+    } else {
+      for (int k = 0; k < 3; k++) {
+        if (!settle) {
+          aux_drain.s = ctx->aux;
+          CPSZ_TRY(up.send_part(ctx, d_up, k, ctx->aux));
+          CPSZ_CUDA_TRY(cudaEventRecord(ctx->up_ev[k], ctx->aux));
+          CPSZ_CUDA_TRY(cudaStreamWaitEvent(st, ctx->up_ev[k], 0));
+        }
+        if (k < 2) CPSZ_TRY(launch_huff_decode(ctx, &dec[k], 1, dtmp[k], settle));
+      }
+    }
+    mark(ctx, "prep3d");
+    CPSZ_TRY(launch_chunk_count_3d(ctx, false, ids, N, chunk_cnt));
+    CPSZ_TRY(launch_scan_u32(ctx, chunk_cnt, chunk_off, nchunks, scan_tmp));
+    CPSZ_TRY(launch_prep3d(ctx, ids, N, chunk_off, codes, n_codes, unpred, n_unpred, pairs));
+    mark(ctx, "wave3d_decompress");
+    CPSZ_TRY(launch_wave3d(ctx, true, pairs, rec, nullptr, signs, smap, &lt, dU, dV, dW, r1, r2, r3, wave_sync));
+    mark(ctx, "d2h");
+    if (!dev_out) {
+      CPSZ_TRY(d2h(ctx, U_out, dU, 4 * N, st));
+      CPSZ_TRY(d2h(ctx, V_out, dV, 4 * N, st));
+      CPSZ_TRY(d2h(ctx, W_out, dW, 4 * N, st));
+    }
+    mark(ctx, "end");
+    int flag = 0;
+    CPSZ_TRY(read_flag3(ctx, &flag));
+    if ((flag & FLAG_HUFF_RESYNC) && !settle) continue;
+    if (flag) return flag_error3(flag);
+    break;
+  }
   return CPSZ_OK;
 }
 

@@ -179,4 +179,25 @@ int d2h(cpsz_b200_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t s
   return CPSZ_OK;
 }
 
+int Upload::send_whole(cpsz_b200_ctx* ctx, uint8_t* dst, cudaStream_t st) const {
+  if (!bytes_) return CPSZ_OK;
+  CPSZ_TRY(upload_reserve(ctx, bytes_));
+  char* h = (char*)ctx->up_pinned;
+  for (const Piece& p : pieces_) {
+    CopyPool::get().copy(h + p.at, p.src, p.n);
+    memset(h + p.at + p.n, 0, p.pad);
+  }
+  CPSZ_CUDA_TRY(cudaMemcpyAsync(dst, h, bytes_, cudaMemcpyHostToDevice, st));
+  return CPSZ_OK;
+}
+
+int Upload::send_part(cpsz_b200_ctx* ctx, uint8_t* dst, int part, cudaStream_t st) const {
+  for (const Piece& p : pieces_) {
+    if (p.part != part) continue;
+    if (p.pad) CPSZ_CUDA_TRY(cudaMemsetAsync(dst + p.at + p.n, 0, p.pad, st));
+    CPSZ_TRY(h2d(ctx, dst + p.at, p.src, p.n, st));
+  }
+  return CPSZ_OK;
+}
+
 }  // namespace cpsz

@@ -9,6 +9,8 @@
 // destination holds the data.  Device-side ordering is that of `st`.
 #pragma once
 
+#include <vector>
+
 #include "runtime.h"
 
 namespace cpsz {
@@ -18,5 +20,38 @@ HostKind host_kind(const void* p);
 
 int h2d(cpsz_b200_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t st);
 int d2h(cpsz_b200_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t st);
+
+// Several host pieces that go up to one device buffer: add() places a piece
+// (256-byte aligned, `pad` zero bytes behind it) and returns its offset there;
+// cut() ends a part.  Either the whole image goes up in one copy from the
+// context's page-locked staging (send_whole: no other copy from it may be in
+// flight), or part by part (send_part, h2d's rules).  Sources are read when
+// they are sent.
+class Upload {
+ public:
+  size_t add(const void* src, size_t n, size_t pad = 0) {
+    const size_t at = align_up(bytes_, 256);
+    pieces_.push_back(Piece{src, n, pad, at, part_});
+    bytes_ = at + n + pad;
+    return at;
+  }
+  void cut() { part_++; }
+  size_t bytes() const { return bytes_; }
+  int send_whole(cpsz_b200_ctx* ctx, uint8_t* dst, cudaStream_t st) const;
+  int send_part(cpsz_b200_ctx* ctx, uint8_t* dst, int part, cudaStream_t st) const;
+
+ private:
+  struct Piece {
+    const void* src;
+    size_t n, pad, at;
+    int part;
+  };
+  std::vector<Piece> pieces_;
+  size_t bytes_ = 0;
+  int part_ = 0;
+};
+// Images up to this size go up whole: one copy and no gap between the
+// streams' decoders; above it the staging copy takes longer than they do.
+constexpr size_t UPLOAD_WHOLE = (size_t)4 << 20;
 
 }  // namespace cpsz

@@ -1,0 +1,114 @@
+"""The GPU Huffman decoder against the oracle, on 2D blobs with made-up streams.
+
+Any code and id sequence is a valid blob, so the streams aim at the decoder's
+own edges: codes longer than one and both look-up tables, trees of every index
+width, streams that end at, before and after a subsequence's or a tile's end,
+and fixed-length codes that never synchronise (the settling rounds)."""
+import struct
+
+import numpy as np
+import pytest
+
+import cpsz_b200
+from tests._util import assert_bits_equal
+
+pytestmark = pytest.mark.gpu
+
+SUB_BITS, SCAN_TILE, WRITE_TILE = 512, 240, 256  # the decoder's subsequence and its tiles
+
+
+def blob_2d(oracle, ids, codes, r1, r2, rng):
+    """A 2D offline blob of the given streams (unpredictable values made up)."""
+    nblocks = ((r1 - 1) // 12 + 1) * ((r2 - 1) // 12 + 1)
+    sec = oracle.huffman_encode(2048, ids.astype(np.int32))
+    fields = []
+    for c in codes:
+        un = rng.standard_normal(int((c == 0).sum())).astype(np.float32)
+        fields.append(struct.pack("<iBi8xQQ", 12, 0, 32768, 0, un.size) + un.tobytes() +
+                      bytes((nblocks - 1) // 8 + 1) + oracle.huffman_encode(131072, c.astype(np.int32)))
+    head = struct.pack("<idQQQ", 4, 2.0 ** -52, len(sec), *map(len, fields))
+    return head + sec + fields[0] + fields[1]
+
+
+def fibonacci(rng, n, symbols):
+    """n symbols with Fibonacci-like shares: code lengths 1, 2, 3, ... symbols."""
+    f = [1, 1]
+    while len(f) < symbols:
+        f.append(f[-1] + f[-2])
+    s = np.repeat(32768 + np.arange(symbols), np.array(f[::-1]))
+    s = np.concatenate([s, np.full(n - s.size, 32768)])
+    rng.shuffle(s)
+    return s
+
+
+def streams(kind, n, rng):
+    if kind == "fixed3":       # eight equal shares: 3-bit codes never synchronise
+        return 32764 + rng.permutation(np.arange(n) % 8)
+    if kind == "fixed16":      # every symbol: 16-bit codes and 32-bit tree indices
+        return rng.permutation(np.arange(n) % 65535 + 1)
+    if kind == "two":          # one bit each
+        return 32768 + (rng.random(n) < 0.5)
+    if kind == "one":
+        return np.full(n, 32768)
+    if kind == "deep":         # codes over 20 bits: beyond both tables
+        return fibonacci(rng, n, 29)
+    if kind == "wide":         # many distinct symbols, most codes over 12 bits, and unpredictable points
+        c = (32768 + np.round(rng.standard_normal(n) * 3000)).clip(1, 65535)
+        return np.where(rng.random(n) < 0.01, 0, c)
+    return (32768 + np.round(rng.standard_cauchy(n) * 2)).clip(0, 65535)
+
+
+def ids_of(kind, n, rng):
+    if kind == "one":
+        return np.full(n, 21)
+    if kind == "fixed3":
+        return 20 + rng.permutation(np.arange(n) % 8)
+    return np.where(rng.random(n) < 0.6, 22, rng.integers(0, 30, n))
+
+
+@pytest.mark.parametrize("kind,r1,r2", [
+    ("cauchy", 1, 1), ("one", 1, 1), ("cauchy", 1, 7), ("cauchy", 13, 1), ("two", 25, 13), ("one", 40, 60),
+    # one-bit codes: exactly one subsequence, one symbol more, one scan / write tile, and around them
+    ("two", 1, SUB_BITS), ("two", 1, SUB_BITS + 1), ("two", SCAN_TILE, SUB_BITS), ("two", WRITE_TILE, SUB_BITS),
+    ("two", WRITE_TILE, SUB_BITS + 1), ("two", 2 * SCAN_TILE + 1, SUB_BITS - 1),
+    ("fixed3", 300, 501), ("fixed16", 300, 500), ("deep", 1100, 1300), ("wide", 401, 999), ("cauchy", 800, 1201),
+])
+def test_gpu_decoder_matches_oracle(ctx, oracle, kind, r1, r2):
+    rng = np.random.default_rng(r1 * 4099 + r2)
+    n = r1 * r2
+    codes = [streams(kind, n, rng), streams(kind, n, rng)]
+    blob = blob_2d(oracle, ids_of(kind, 2 * n, rng), codes, r1, r2, rng)
+    du, dv = cpsz_b200.sz_decompress_cp_preserve_2d_offline(blob, r1, r2, ctx=ctx)
+    ou, ov = oracle.decompress_2d(blob, r1, r2)
+    assert_bits_equal(du, ou)
+    assert_bits_equal(dv, ov)
+
+
+def test_gpu_decoder_streams_sent_one_by_one(ctx, oracle):
+    """A blob above 4 MiB goes up and is decoded stream by stream, here with a
+    code stream that needs the settling rounds."""
+    rng = np.random.default_rng(5)
+    r1, r2 = 1000, 3001
+    codes = [streams("wide", r1 * r2, rng), streams("fixed3", r1 * r2, rng)]
+    blob = blob_2d(oracle, ids_of("cauchy", 2 * r1 * r2, rng), codes, r1, r2, rng)
+    assert len(blob) > 4 << 20
+    du, dv = cpsz_b200.sz_decompress_cp_preserve_2d_offline(blob, r1, r2, ctx=ctx)
+    ou, ov = oracle.decompress_2d(blob, r1, r2)
+    assert_bits_equal(du, ou)
+    assert_bits_equal(dv, ov)
+
+
+def test_gpu_decoder_refuses_short_streams(ctx, oracle):
+    """Streams that hold fewer symbols than the field has points, and a tree
+    that is not one."""
+    rng = np.random.default_rng(6)
+    r1, r2 = 60, 70
+    codes = [streams("wide", r1 * r2, rng), streams("wide", r1 * r2, rng)]
+    ids = ids_of("cauchy", 2 * r1 * r2, rng)
+    short = [codes[0], codes[1][: r1 * r2 // 2]]
+    with pytest.raises(cpsz_b200.CpszError):
+        cpsz_b200.sz_decompress_cp_preserve_2d_offline(blob_2d(oracle, ids, short, r1, r2, rng), r1, r2, ctx=ctx)
+    blob = bytearray(blob_2d(oracle, ids, codes, r1, r2, rng))
+    blob[36 + 13] = 0  # the id tree's root is its own left child
+    with pytest.raises(cpsz_b200.CpszError):
+        cpsz_b200.sz_decompress_cp_preserve_2d_offline(bytes(blob), r1, r2, ctx=ctx)
