@@ -48,3 +48,26 @@ def test_device_buffers(ctx):
     small = torch.zeros(16, dtype=torch.uint8, device="cuda")
     with pytest.raises(cpsz_b200.CpszError):
         cpsz_b200.lossless_compress_gpu(d_in, out=small, ctx=ctx)
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 8191, 8192, 8193, 8192 * 8 - 1, 8192 * 8 + 5, 8192 * 9])
+@pytest.mark.parametrize("kind", ["text", "sparse", "long", "mixed"])
+def test_block_edges(ctx, n, kind):
+    """Blocks of every sequence count and literal header: a few matches and
+    many (batches of 32 sequences, one- and two-byte counts), literal runs over
+    31 and 4095 bytes, matches that reach a block's end."""
+    rng = np.random.default_rng(n)
+    if kind == "text":  # short matches everywhere
+        a = rng.integers(0, 4, n).astype(np.uint8)
+    elif kind == "sparse":  # mostly literals, a repeated run now and then
+        a = rng.integers(0, 256, n).astype(np.uint8)
+        for at in range(0, n - 600, 1500):
+            a[at + 300:at + 500] = a[at:at + 200]
+    elif kind == "long":  # matches of thousands of bytes
+        a = np.resize(rng.integers(0, 256, 97), n).astype(np.uint8)
+    else:
+        a = rng.integers(0, 256, n).astype(np.uint8)
+        a[: n // 2] = rng.integers(0, 3, n // 2)
+        a[-20:] = 5
+    frame = _roundtrip(a.tobytes(), ctx)
+    assert len(frame) <= cpsz_b200.lib().cpsz_b200_lossless_bound(n)
