@@ -185,11 +185,10 @@ constexpr long long LOOKBACK_SPIN = 1ll << 24;
 
 // Warp 0 of a strip's CTA: the exclusive prefix of its blocks' zero counts
 // (bpre), its own count published, and the count of all earlier strips
-// (s_excl); the last strip also stores the component's total beside the
-// ticket.  A look-back that waits past its bound sets FLAG_TIMEOUT.
+// (s_excl); the last strip also stores the component's total.  A look-back that waits past its bound sets FLAG_TIMEOUT.
 __device__ __forceinline__ void strip_prefix(unsigned long long* status, unsigned int s, unsigned int ns,
                                              const StripGeom& g, const unsigned int* bz, unsigned int* bpre,
-                                             unsigned long long* s_excl, int lane, int* flag) {
+                                             unsigned long long* s_excl, int lane, unsigned* total, int* flag) {
   const unsigned int v = lane < g.nb ? bz[lane] : 0u;
   unsigned int inc = v;  // inclusive scan of the block counts
 #pragma unroll
@@ -203,30 +202,45 @@ __device__ __forceinline__ void strip_prefix(unsigned long long* status, unsigne
   const unsigned long long excl = lookback_warp(status, s, tot, lane, LOOKBACK_SPIN, flag);
   if (lane == 0) {
     *s_excl = excl;
-    if (s == ns - 1) reinterpret_cast<unsigned int*>(status + ns)[1] = (unsigned int)(excl + tot);
+    if (s == ns - 1) *total = (unsigned int)(excl + tot);
   }
 }
 
 __device__ __forceinline__ unsigned int lanemask_lt(int lane) { return (1u << lane) - 1u; }
 
+// Compression, one launch for both components of every field: codes raster ->
+// block order, and the unpredictable values (code 0) in block order.
 struct StripPass {
   const uint16_t* raster;
   const float* x;
   uint16_t* blocks;
   float* unpred;
-  unsigned long long* status;  // ns words, then the ticket and the component total (u32 each); zeroed
+  unsigned long long* status;  // ns words, then the ticket
 };
-
-// Compression, one launch for both components: codes raster -> block order,
-// and the unpredictable values (code 0) in block order.
-__global__ void __launch_bounds__(STRIP_NT) strip_pass_kernel(StripPass P0, StripPass P1, long long pitch,
-                                                              long long x_pitch, int r1, int r2, int nsc,
-                                                              unsigned int ns, int* flag) {
+__global__ void __launch_bounds__(STRIP_NT) strip_pass_kernel(const __grid_constant__ StripJob one,
+                                                              const StripJob* __restrict__ jobs, int njobs, int* flag) {
   __shared__ __align__(16) uint16_t t[BS][STRIP_TP];
   __shared__ unsigned int bz[STRIP_BLOCKS], bpre[STRIP_BLOCKS];
   __shared__ unsigned int s_idx;
   __shared__ unsigned long long s_excl;
-  const StripPass P = blockIdx.y ? P1 : P0;
+  __shared__ int s_job;
+  if (jobs) {
+    if (threadIdx.x == 0) {
+      int lo = 0, hi = njobs - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (jobs[mid].strip0 <= blockIdx.x) lo = mid;
+        else hi = mid - 1;
+      }
+      s_job = lo;
+    }
+    __syncthreads();
+  }
+  const StripJob& J = jobs ? jobs[s_job] : one;
+  const int c = blockIdx.y, r1 = J.r1, r2 = J.r2, nsc = (r2 + STRIP_W - 1) / STRIP_W;
+  const long long pitch = r2;
+  const unsigned int ns = (unsigned)((r1 + BS - 1) / BS) * (unsigned)nsc;
+  const StripPass P{J.raster[c], J.x[c], J.blocks[c], J.unpred[c], J.status[c]};
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) s_idx = atomicAdd(reinterpret_cast<unsigned int*>(P.status + ns), 1u);
   if (threadIdx.x < STRIP_BLOCKS) bz[threadIdx.x] = 0;
@@ -303,7 +317,7 @@ __global__ void __launch_bounds__(STRIP_NT) strip_pass_kernel(StripPass P0, Stri
     if (v == 0) atomicAdd(&bz[p.b], 1u);
   }
   __syncthreads();
-  if (warp == 0) strip_prefix(P.status, s, ns, g, bz, bpre, &s_excl, lane, flag);
+  if (warp == 0) strip_prefix(P.status, s, ns, g, bz, bpre, &s_excl, lane, J.total + c, flag);
   __syncthreads();
 
   // unpredictable values, in block order
@@ -323,7 +337,7 @@ __global__ void __launch_bounds__(STRIP_NT) strip_pass_kernel(StripPass P0, Stri
         z = t[li][col] == 0;
       }
       const unsigned int m = __ballot_sync(FULLM, z);
-      if (z) P.unpred[run + __popc(m & lanemask_lt(lane))] = P.x[(long long)(g.bi * BS + li) * x_pitch + g.c0 + col];
+      if (z) P.unpred[run + __popc(m & lanemask_lt(lane))] = P.x[(long long)(g.bi * BS + li) * pitch + g.c0 + col];
       run += __popc(m);
     }
   }
@@ -336,6 +350,7 @@ struct StripUnpass {
   unsigned long long n_unpred;
   float2* pair;                // raster (pitch r2)
   unsigned long long* status;  // as in StripPass
+  unsigned* total;
   int id_shift;                // p = 2^(id_shift * id) * 2^-52: 2 (offline), 1 (offline_log)
 };
 
@@ -411,7 +426,7 @@ __global__ void __launch_bounds__(STRIP_NT) strip_unpass_kernel(StripUnpass P0, 
     if (c == 0) atomicAdd(&bz[p.b], 1u);
   }
   __syncthreads();
-  if (warp == 0) strip_prefix(P.status, s, ns, g, bz, bpre, &s_excl, lane, flag);
+  if (warp == 0) strip_prefix(P.status, s, ns, g, bz, bpre, &s_excl, lane, P.total, flag);
 
   // raster pairs (the other warps start while warp 0 looks back)
   const long long row0 = (long long)g.bi * BS;
@@ -480,6 +495,48 @@ __global__ void __launch_bounds__(STRIP_NT) strip_unpass_kernel(StripUnpass P0, 
   }
 }
 
+// ---- byte runs ------------------------------------------------------------------------
+// Whole words of the destination from two source words each (the two sides'
+// alignments differ), single bytes at a chunk's ends.
+constexpr int PIECE_CHUNK = 8192;
+__global__ void __launch_bounds__(256) copy_pieces_kernel(const CopyPiece* __restrict__ pieces, int n) {
+  __shared__ int s_piece;
+  if (threadIdx.x == 0) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (pieces[mid].chunk0 <= blockIdx.x) lo = mid;
+      else hi = mid - 1;
+    }
+    s_piece = lo;
+  }
+  __syncthreads();
+  const CopyPiece P = pieces[s_piece];
+  const size_t c0 = (size_t)(blockIdx.x - P.chunk0) * PIECE_CHUNK;
+  if (c0 >= P.n) return;
+  const int len = (int)(P.n - c0 < (size_t)PIECE_CHUNK ? P.n - c0 : (size_t)PIECE_CHUNK);
+  uint8_t* d = P.dst + c0;
+  const uint8_t* s = P.src ? P.src + c0 : nullptr;
+  const int head = min(len, (int)((4 - ((uintptr_t)d & 3)) & 3)), words = (len - head) >> 2, tail = head + 4 * words;
+  if (threadIdx.x < 8) {
+    const int i = threadIdx.x < 4 ? (int)threadIdx.x : tail + (int)threadIdx.x - 4;
+    if (threadIdx.x < 4 ? i < head : i < len) d[i] = s ? s[i] : 0;
+  }
+  uint32_t* dw = reinterpret_cast<uint32_t*>(d + head);
+  if (!s) {
+    for (int k = threadIdx.x; k < words; k += 256) dw[k] = 0;
+    return;
+  }
+  const uint8_t* sb = s + head;
+  const unsigned sh = 8 * ((uintptr_t)sb & 3);
+  const uint32_t* sw = reinterpret_cast<const uint32_t*>(sb - ((uintptr_t)sb & 3));
+  if (sh == 0) {
+    for (int k = threadIdx.x; k < words; k += 256) dw[k] = sw[k];
+  } else {  // sw[k + 1] holds a byte of the run, so it is readable
+    for (int k = threadIdx.x; k < words; k += 256) dw[k] = __funnelshift_r(sw[k], sw[k + 1], sh);
+  }
+}
+
 }  // namespace
 
 size_t scan_u32_tmp_bytes(size_t n) { return ((n + SCAN_CHUNK - 1) / SCAN_CHUNK + 2) * sizeof(unsigned int) + 256; }
@@ -498,6 +555,22 @@ int launch_scan_u32(cpsz_b200_ctx* ctx, const unsigned int* in, unsigned int* ou
   return check_launch("scan_u32");
 }
 
+unsigned assign_piece_chunks(CopyPiece* pieces, size_t n) {
+  unsigned at = 0;
+  for (size_t k = 0; k < n; k++) {
+    pieces[k].chunk0 = at;
+    at += (unsigned)std::max<size_t>(1, (pieces[k].n + PIECE_CHUNK - 1) / PIECE_CHUNK);
+  }
+  return at;
+}
+
+int launch_copy_pieces(cpsz_b200_ctx* ctx, const CopyPiece* d_pieces, int n, unsigned ctas) {
+  if (n <= 0) return CPSZ_OK;
+  copy_pieces_kernel<<<ctas, 256, 0, ctx->stream>>>(d_pieces, n);
+  count_launch(ctx);
+  return check_launch("copy_pieces_kernel");
+}
+
 size_t strip_count(int r1, int r2) {
   const long long nbx = (r1 + BS - 1) / BS, nsc = (r2 + STRIP_W - 1) / STRIP_W;
   return (size_t)(nbx * nsc);
@@ -505,39 +578,25 @@ size_t strip_count(int r1, int r2) {
 
 size_t strip_scratch_bytes(int r1, int r2) { return 8 * strip_count(r1, r2) + 8; }
 
-const unsigned int* strip_total(const void* scratch, int r1, int r2) {
-  return (const unsigned int*)((const char*)scratch + 8 * strip_count(r1, r2) + 4);
-}
-
-int launch_strip_pass(cpsz_b200_ctx* ctx, const uint16_t* const raster[2], long long pitch, const float* const x[2],
-                      long long x_pitch, int r1, int r2, uint16_t* const blocks[2], float* const unpred[2],
-                      void* const scratch[2]) {
-  const size_t ns = strip_count(r1, r2);
+int launch_strip_pass(cpsz_b200_ctx* ctx, const StripJob* jobs, const StripJob* d_jobs, int n) {
+  const size_t ns = jobs[n - 1].strip0 + strip_count(jobs[n - 1].r1, jobs[n - 1].r2);
   if (ns > 0x7fffffffu) return set_error(CPSZ_ERR_UNSUPPORTED, "field of %zu strips", ns);
-  for (int f = 0; f < 2; f++)  // the totals of an empty field read 0
-    CPSZ_CUDA_TRY(cudaMemsetAsync(scratch[f], 0, strip_scratch_bytes(r1, r2), ctx->stream));
-  if (ns == 0) return CPSZ_OK;
-  const int nsc = (r2 + STRIP_W - 1) / STRIP_W;
-  StripPass P[2];
-  for (int f = 0; f < 2; f++) P[f] = StripPass{raster[f], x[f], blocks[f], unpred[f], (unsigned long long*)scratch[f]};
-  strip_pass_kernel<<<dim3((unsigned)ns, 2), STRIP_NT, 0, ctx->stream>>>(P[0], P[1], pitch, x_pitch, r1, r2, nsc,
-                                                                         (unsigned)ns, ctx->d_flag);
+  strip_pass_kernel<<<dim3((unsigned)ns, 2), STRIP_NT, 0, ctx->stream>>>(jobs[0], n == 1 ? nullptr : d_jobs, n,
+                                                                         ctx->d_flag);
   count_launch(ctx);
   return check_launch("strip_pass_kernel");
 }
 
 int launch_strip_unpass(cpsz_b200_ctx* ctx, const uint16_t* const blocks[2], const uint8_t* const ids[2],
                         const float* const unpred[2], const unsigned long long n_unpred[2], int r1, int r2,
-                        float2* const pair[2], void* const scratch[2], int id_shift) {
+                        float2* const pair[2], void* const scratch[2], unsigned* total, int id_shift) {
   const size_t ns = strip_count(r1, r2);
   if (ns > 0x7fffffffu) return set_error(CPSZ_ERR_UNSUPPORTED, "field of %zu strips", ns);
-  for (int f = 0; f < 2; f++)  // the totals of an empty field read 0
-    CPSZ_CUDA_TRY(cudaMemsetAsync(scratch[f], 0, strip_scratch_bytes(r1, r2), ctx->stream));
-  if (ns == 0) return CPSZ_OK;
   const int nsc = (r2 + STRIP_W - 1) / STRIP_W;
   StripUnpass P[2];
   for (int f = 0; f < 2; f++)
-    P[f] = StripUnpass{blocks[f], ids[f], unpred[f], n_unpred[f], pair[f], (unsigned long long*)scratch[f], id_shift};
+    P[f] = StripUnpass{blocks[f], ids[f], unpred[f], n_unpred[f], pair[f], (unsigned long long*)scratch[f], total + f,
+                       id_shift};
   strip_unpass_kernel<<<dim3((unsigned)ns, 2), STRIP_NT, 0, ctx->stream>>>(P[0], P[1], r1, r2, nsc, (unsigned)ns,
                                                                            ctx->d_flag);
   count_launch(ctx);

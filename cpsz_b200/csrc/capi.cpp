@@ -277,8 +277,16 @@ int cpsz_b200_huffman_encode_u16(cpsz_b200_ctx* ctx, const uint16_t* sym, size_t
   CPSZ_CUDA_TRY(cudaMemsetAsync(out, 0, out_cap, ctx->stream));
   CPSZ_CUDA_TRY(cudaMemsetAsync(d_total, 0, 8, ctx->stream));
   CPSZ_CUDA_TRY(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
-  CPSZ_TRY(launch_huff_encode_u16(ctx, sym, n, HuffEncTable{(const unsigned long long*)code, len, 65536},
-                                  (uint32_t*)out, out_cap, d_total, tmp));
+  PackJob job;
+  job.sym = sym;
+  job.n = n;
+  job.sym_bytes = 2;
+  job.tab = HuffEncTable{(const unsigned long long*)code, len, 65536};
+  job.out = (uint32_t*)out;
+  job.cap_words = out_cap / 4;
+  job.scratch = (unsigned long long*)tmp;
+  job.total_bits = d_total;
+  CPSZ_TRY(launch_huff_encode(ctx, job));
   unsigned long long* h = (unsigned long long*)ctx->pinned;
   CPSZ_CUDA_TRY(cudaMemcpyAsync(h, d_total, 8, cudaMemcpyDeviceToHost, ctx->stream));
   CPSZ_CUDA_TRY(cudaMemcpyAsync(h + 1, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -332,10 +340,10 @@ int cpsz_b200_compress_3d_offline_log_f32_into(cpsz_b200_ctx* ctx, const float* 
   if (!out || !blob_size) return set_error(CPSZ_ERR_INVALID, "null output pointer");
   RESOLVE(ctx);
   Blob3D b;
-  CPSZ_TRY(compress_3d(ctx, U, V, W, r1, r2, r3, max_pwr_eb, &b));
+  CPSZ_TRY(compress_3d(ctx, U, V, W, r1, r2, r3, max_pwr_eb, &b, is_device_ptr(out) ? out : nullptr, out_cap));
   *blob_size = b.size;
   if (b.size > out_cap) return set_error(CPSZ_ERR_INVALID, "output capacity %zu < blob size %zu", out_cap, b.size);
-  CPSZ_TRY(copy_out(ctx, out, b.d_blob, b.size));
+  if (b.d_blob != out) CPSZ_TRY(copy_out(ctx, out, b.d_blob, b.size));
   CPSZ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return CPSZ_OK;
 }

@@ -11,6 +11,8 @@
 // grid and stores it with coalesced stores (atomicOr for the two edge words,
 // shared with the neighbouring tiles).  Words are stored byte-swapped so
 // memory holds the big-endian byte stream the reference writes.
+#include <algorithm>
+
 #include "kernels.h"
 #include "lookback.cuh"
 
@@ -36,6 +38,18 @@ struct PackWin {
   static constexpr int n = sizeof(Sym) == 1 ? 256 : PK_WIN;
   static constexpr int per_word = 4 / (int)sizeof(Sym);  // symbols per 32-bit register
 };
+
+// The job whose CTAs include x: the last with cta0 <= x.
+template <class Job>
+__device__ __forceinline__ int find_job(const Job* __restrict__ jobs, int n, unsigned x) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (jobs[mid].cta0 <= x) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
 
 struct PackShared {
   uint32_t words[PK_WORDS];     // the tile's packed bits from its first bit (tile-relative)
@@ -80,16 +94,21 @@ __device__ __forceinline__ uint32_t pk_lcode(const PackShared& sh, unsigned s, u
 // histograms) finds its starting bit first and ORs its words straight into
 // global memory.  The stream starts at bit `bit0` (0-31) of out[0].
 template <class Sym, bool MAP0>
-__global__ void __launch_bounds__(PK_NT, PK_CTAS_PER_SM)
-    pack_kernel(const Sym* __restrict__ sym, size_t n, const unsigned long long* __restrict__ code,
-                const uint8_t* __restrict__ len, int nsym, uint32_t* __restrict__ out, size_t cap_words, int bit0,
-                unsigned long long* __restrict__ state, unsigned int* __restrict__ ticket, unsigned long long ntiles,
-                unsigned long long* __restrict__ d_total, int* __restrict__ flag) {
+__device__ __forceinline__ void pack_stream(const PackJob& J, PackShared& sh, int* __restrict__ flag) {
+  const Sym* __restrict__ sym = static_cast<const Sym*>(J.sym);
+  const size_t n = J.n, cap_words = J.cap_words;
+  const unsigned long long* __restrict__ code = J.tab.code;
+  const uint8_t* __restrict__ len = J.tab.len;
+  const int nsym = J.tab.nsym, bit0 = J.bit0;
+  uint32_t* __restrict__ out = J.out;
+  unsigned long long* __restrict__ state = J.scratch + 1;
+  unsigned int* __restrict__ ticket = reinterpret_cast<unsigned int*>(J.scratch);
+  const unsigned long long ntiles = (n + PK_TILE - 1) / PK_TILE;
+  unsigned long long* __restrict__ d_total = J.total_bits;
   using W = PackWin<Sym>;
   constexpr int NW = PK_SPT / W::per_word;  // registers of packed symbols
   constexpr int SB = 8 * (int)sizeof(Sym);
   constexpr unsigned SMASK = sizeof(Sym) == 1 ? 0xffu : 0xffffu;
-  __shared__ PackShared sh;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < W::n; i += PK_NT) {
     const int s = W::lo + i;
@@ -256,47 +275,63 @@ __global__ void __launch_bounds__(PK_NT, PK_CTAS_PER_SM)
   }
 }
 
-__global__ void __launch_bounds__(256) codebook_scatter_kernel(const HuffEntry* __restrict__ e, size_t n,
-                                                               unsigned long long* __restrict__ code,
-                                                               uint8_t* __restrict__ len) {
-  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
-  if (i < n) {
-    const HuffEntry v = e[i];
-    code[v.sym] = v.code;
-    len[v.sym] = (uint8_t)v.len;
+// The CTAs of a launch are shared out among its streams (PackJob::cta0); a CTA
+// takes tiles of its own stream until they run out.  SYM: 1 u8, 2 u16, 0 both.
+template <int SYM>
+__global__ void __launch_bounds__(PK_NT, PK_CTAS_PER_SM)
+    pack_kernel(const __grid_constant__ PackJob one, const PackJob* __restrict__ jobs, int njobs,
+                int* __restrict__ flag) {
+  __shared__ PackShared sh;
+  __shared__ PackJob s_job;
+  if (jobs) {
+    if (threadIdx.x == 0) s_job = jobs[find_job(jobs, njobs, blockIdx.x)];
+    __syncthreads();
   }
+  const PackJob& J = jobs ? s_job : one;
+  if (SYM == 2 || (SYM == 0 && J.sym_bytes == 2)) pack_stream<uint16_t, false>(J, sh, flag);
+  else if (J.map_id_zero) pack_stream<uint8_t, true>(J, sh, flag);
+  else pack_stream<uint8_t, false>(J, sh, flag);
+}
+
+// Before the packers: the codebook entries of a stream scattered into its
+// tables, and the bytes its bits go to zeroed (the packer ORs the words two
+// tiles share).  grid.y: the stream; grid.x CTAs take its entries and bytes in
+// chunks of 256 and PREP_BYTES.
+constexpr unsigned PREP_BYTES = 16384;
+__global__ void __launch_bounds__(256) pack_prep_kernel(const PackPrep* __restrict__ jobs) {
+  const PackPrep J = jobs[blockIdx.y];
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (i < J.n) {
+    const HuffEntry v = J.entries[i];
+    J.code[v.sym] = v.code;
+    J.len[v.sym] = (uint8_t)v.len;
+  }
+  const size_t b0 = (size_t)blockIdx.x * PREP_BYTES;
+  if (b0 >= J.zero_bytes) return;
+  const size_t b1 = b0 + PREP_BYTES < J.zero_bytes ? b0 + PREP_BYTES : J.zero_bytes;
+  uint8_t* p = J.zero + b0;
+  uint8_t* const e = J.zero + b1;
+  uint8_t* const lo = (uint8_t*)(((uintptr_t)p + 15) & ~(uintptr_t)15);
+  if (lo >= e) {
+    for (uint8_t* q = p + threadIdx.x; q < e; q += 256) *q = 0;
+    return;
+  }
+  uint8_t* const hi = (uint8_t*)((uintptr_t)e & ~(uintptr_t)15);
+  if (p + threadIdx.x < lo) p[threadIdx.x] = 0;
+  if (hi + threadIdx.x < e) hi[threadIdx.x] = 0;
+  for (uint8_t* q = lo + 16 * threadIdx.x; q < hi; q += 16 * 256) *reinterpret_cast<uint4*>(q) = make_uint4(0, 0, 0, 0);
 }
 
 size_t pack_scratch_words(size_t n) { return (n + PK_TILE - 1) / PK_TILE + 1; }
 
-// scratch: pack_scratch_words(n) words (ticket, then one state per tile), zeroed here.
-template <class Sym>
-int pack_launch(int num_sms, cudaStream_t st, const Sym* sym, size_t n, bool map_id_zero, HuffEncTable tab,
-                uint32_t* out, size_t out_cap_bytes, int bit0, unsigned long long* scratch,
-                unsigned long long* d_total_bits, int* flag) {
-  if (n == 0) return CPSZ_OK;
-  if (bit0 < 0 || bit0 > 31) return set_error(CPSZ_ERR_INVALID, "internal: stream start bit %d", bit0);
-  const unsigned long long ntiles = (n + PK_TILE - 1) / PK_TILE;
-  CPSZ_CUDA_TRY(cudaMemsetAsync(scratch, 0, (ntiles + 1) * 8, st));
-  const unsigned long long cap = (unsigned long long)num_sms * PK_CTAS_PER_SM;
-  const unsigned grid = (unsigned)(ntiles < cap ? ntiles : cap);
-  auto k = pack_kernel<Sym, false>;
-  if constexpr (sizeof(Sym) == 1) {
-    if (map_id_zero) k = pack_kernel<Sym, true>;
-  }
-  k<<<grid, PK_NT, 0, st>>>(sym, n, tab.code, tab.len, tab.nsym, out, out_cap_bytes / 4, bit0, scratch + 1,
-                            reinterpret_cast<unsigned int*>(scratch), ntiles, d_total_bits, flag);
-  return check_launch("pack_kernel");
-}
-
-template <class Sym>
-int encode_impl(cpsz_b200_ctx* ctx, const Sym* sym, size_t n, bool map_id_zero, HuffEncTable tab, uint32_t* out,
-                size_t out_cap_bytes, unsigned long long* d_total_bits, void* tmp, int bit0) {
-  if (n == 0) return CPSZ_OK;
-  CPSZ_TRY(pack_launch<Sym>(ctx->num_sms, ctx->stream, sym, n, map_id_zero, tab, out, out_cap_bytes, bit0,
-                            (unsigned long long*)tmp, d_total_bits, ctx->d_flag));
-  count_launch(ctx);
-  return CPSZ_OK;
+// CTAs of one of `streams` streams: its share of a full device, or one per
+// PK_TILES_PER_CTA tiles if that is more (a CTA loads its stream's codebook
+// window once, about a quarter of a tile's time).
+constexpr size_t PK_TILES_PER_CTA = 4;
+unsigned pack_ctas(int num_sms, size_t n, int streams) {
+  const size_t ntiles = (n + PK_TILE - 1) / PK_TILE, cap = (size_t)num_sms * PK_CTAS_PER_SM;
+  const size_t share = std::max((ntiles + PK_TILES_PER_CTA - 1) / PK_TILES_PER_CTA, cap / (size_t)streams);
+  return (unsigned)std::min(ntiles, std::min(cap, share));
 }
 
 // ---- histogram -------------------------------------------------------------------
@@ -366,22 +401,59 @@ __device__ __forceinline__ void hist_flush(unsigned* sh, unsigned long long* his
   if (threadIdx.x == 0 && sh[HIST_W]) atomicAdd(&hist[0], (unsigned long long)sh[HIST_W]);
 }
 
-// Stream blockIdx.y (s0 / s1, n symbols each) into its histogram (h0 / h1);
-// SKIP0: symbol 0 is not counted.
+// Component blockIdx.y of a field's codes into its histogram, by the field's
+// share of the CTAs; SKIP0: symbol 0 is not counted.
 template <bool SKIP0>
-__global__ void __launch_bounds__(HIST_NT) hist_u16_kernel(const uint16_t* __restrict__ s0,
-                                                           const uint16_t* __restrict__ s1, size_t n,
-                                                           unsigned long long* __restrict__ h0,
-                                                           unsigned long long* __restrict__ h1) {
-  const uint16_t* __restrict__ s = blockIdx.y ? s1 : s0;
-  unsigned long long* __restrict__ hist = blockIdx.y ? h1 : h0;
+__global__ void __launch_bounds__(HIST_NT) hist_u16_kernel(const __grid_constant__ HistJob one,
+                                                           const HistJob* __restrict__ jobs, int njobs) {
   __shared__ unsigned int sh[HIST_W + 1];  // window + symbol 0
+  __shared__ int s_job;
+  if (threadIdx.x == 0) s_job = jobs ? find_job(jobs, njobs, blockIdx.x) : 0;
   for (int k = threadIdx.x; k <= HIST_W; k += HIST_NT) sh[k] = 0;
   __syncthreads();
+  const HistJob& J = jobs ? jobs[s_job] : one;
+  unsigned long long* __restrict__ hist = J.hist[blockIdx.y];
   unsigned c_lo = 0, c_mid = 0, c_hi = 0;
-  hist_span<SKIP0>(sh, hist, s, n, (size_t)blockIdx.x * HIST_NT + threadIdx.x, (size_t)gridDim.x * HIST_NT, c_lo,
-                   c_mid, c_hi);
+  hist_span<SKIP0>(sh, hist, J.sym[blockIdx.y], J.n, (size_t)(blockIdx.x - J.cta0) * HIST_NT + threadIdx.x,
+                   (size_t)J.ctas * HIST_NT, c_lo, c_mid, c_hi);
   hist_flush(sh, hist, c_lo, c_mid, c_hi);
+}
+
+// ---- histogram -> list ---------------------------------------------------------------
+// The symbols that occur, ascending, as symbol << 40 | count, and their number,
+// written straight into page-locked host memory: the host reads a few thousand
+// words where it would copy and scan 65536 bins (512 KB and about 20 us each).
+// One CTA per histogram; warp w has bins 2048 w .. 2048 w + 2047, 32 per step,
+// so a step's ballot gives every lane its place.
+constexpr int LIST_NT = 1024;
+constexpr int LIST_STEPS = 65536 / LIST_NT;
+__global__ void __launch_bounds__(LIST_NT) hist_list_kernel(const HistList* __restrict__ jobs) {
+  const HistList J = jobs[blockIdx.x];
+  __shared__ unsigned s_warp[LIST_NT / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned bin0 = (unsigned)warp * 32 * LIST_STEPS + lane;
+  unsigned n = 0;  // this lane's occurring bins
+#pragma unroll 16
+  for (int k = 0; k < LIST_STEPS; k++) n += J.hist[bin0 + 32 * k] != 0;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) n += __shfl_xor_sync(0xffffffffu, n, d);
+  if (lane == 0) s_warp[warp] = n;
+  __syncthreads();
+  unsigned v = s_warp[lane], x = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, x, d);
+    if (lane >= d) x += y;
+  }
+  if (threadIdx.x == 31) *J.count = x;
+  unsigned at = __shfl_sync(0xffffffffu, x - v, warp);
+#pragma unroll 16
+  for (int k = 0; k < LIST_STEPS; k++) {
+    const unsigned long long c = J.hist[bin0 + 32 * k];
+    const unsigned m = __ballot_sync(0xffffffffu, c != 0);
+    if (c) J.list[at + __popc(m & ((1u << lane) - 1u))] = (unsigned long long)(bin0 + 32 * k) << 40 | c;
+    at += __popc(m);
+  }
 }
 
 // ---- histogram follower ----------------------------------------------------------
@@ -456,49 +528,83 @@ __global__ void __launch_bounds__(HIST_NT) hist_follow_kernel(const uint16_t* __
 
 }  // namespace
 
-int launch_codebook_scatter(cpsz_b200_ctx* ctx, const HuffEntry* d_entries, size_t n, unsigned long long* code,
-                            uint8_t* len) {
-  if (n == 0) return CPSZ_OK;
-  codebook_scatter_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(d_entries, n, code, len);
-  count_launch(ctx);
-  return check_launch("codebook_scatter_kernel");
-}
-
 size_t huff_encode_tmp_bytes(size_t n) { return align_up(pack_scratch_words(n), 32) * sizeof(unsigned long long); }
 
-int launch_huff_encode_u8(cpsz_b200_ctx* ctx, const uint8_t* sym, size_t n, bool map_id_zero, HuffEncTable tab,
-                          uint32_t* out_words, size_t out_cap_bytes, unsigned long long* d_total_bits, void* tmp,
-                          int bit0) {
-  return encode_impl<uint8_t>(ctx, sym, n, map_id_zero, tab, out_words, out_cap_bytes, d_total_bits, tmp, bit0);
+int launch_pack_prep(cpsz_b200_ctx* ctx, const PackPrep* d_jobs, int n, size_t max_entries, size_t max_zero_bytes) {
+  const size_t gx = std::max((max_entries + 255) / 256, (max_zero_bytes + PREP_BYTES - 1) / PREP_BYTES);
+  if (n <= 0 || gx == 0) return CPSZ_OK;
+  pack_prep_kernel<<<dim3((unsigned)gx, (unsigned)n), 256, 0, ctx->stream>>>(d_jobs);
+  count_launch(ctx);
+  return check_launch("pack_prep_kernel");
 }
 
-int launch_huff_encode_u16(cpsz_b200_ctx* ctx, const uint16_t* sym, size_t n, HuffEncTable tab, uint32_t* out_words,
-                           size_t out_cap_bytes, unsigned long long* d_total_bits, void* tmp, int bit0) {
-  return encode_impl<uint16_t>(ctx, sym, n, false, tab, out_words, out_cap_bytes, d_total_bits, tmp, bit0);
+unsigned pack_assign_ctas(int num_sms, PackJob* jobs, int n) {
+  unsigned at = 0;
+  for (int k = 0; k < n; k++) {
+    jobs[k].cta0 = at;
+    at += pack_ctas(num_sms, jobs[k].n, n);
+  }
+  return at;
 }
 
-int launch_hist_u16(cpsz_b200_ctx* ctx, const uint16_t* sym, size_t n, unsigned long long* hist) {
-  return launch_hist_u16_pair(ctx, sym, nullptr, n, hist, nullptr);
+int launch_pack(cudaStream_t st, const PackJob* jobs, const PackJob* d_jobs, int n, unsigned ctas, int* flag) {
+  if (ctas == 0) return CPSZ_OK;
+  bool u8 = false, u16 = false;
+  for (int k = 0; k < n; k++) {
+    if (jobs[k].bit0 < 0 || jobs[k].bit0 > 31)
+      return set_error(CPSZ_ERR_INVALID, "internal: stream start bit %d", jobs[k].bit0);
+    (jobs[k].sym_bytes == 2 ? u16 : u8) = true;
+  }
+  const PackJob* table = n == 1 ? nullptr : d_jobs;
+  if (u8 && u16) pack_kernel<0><<<ctas, PK_NT, 0, st>>>(jobs[0], table, n, flag);
+  else if (u16) pack_kernel<2><<<ctas, PK_NT, 0, st>>>(jobs[0], table, n, flag);
+  else pack_kernel<1><<<ctas, PK_NT, 0, st>>>(jobs[0], table, n, flag);
+  return check_launch("pack_kernel");
 }
-int launch_hist_u16_pair(cpsz_b200_ctx* ctx, const uint16_t* a, const uint16_t* b, size_t n, unsigned long long* ha,
-                         unsigned long long* hb) {
-  if (n == 0) return CPSZ_OK;
-  const int k = b ? 2 : 1;
-  int grid = ctx->num_sms * 2 / k;
-  size_t need = (n + HIST_NT - 1) / HIST_NT;
-  if ((size_t)grid > need) grid = (int)need;
-  hist_u16_kernel<false><<<dim3(grid, k), HIST_NT, 0, ctx->stream>>>(a, b, n, ha, hb);
+
+int launch_huff_encode(cpsz_b200_ctx* ctx, PackJob job) {
+  if (job.n == 0) return CPSZ_OK;
+  CPSZ_CUDA_TRY(cudaMemsetAsync(job.scratch, 0, pack_scratch_words(job.n) * 8, ctx->stream));
+  CPSZ_TRY(launch_pack(ctx->stream, &job, nullptr, 1, pack_assign_ctas(ctx->num_sms, &job, 1), ctx->d_flag));
+  count_launch(ctx);
+  return CPSZ_OK;
+}
+
+// About two CTAs per SM in all, each with at least 16 symbols a thread: a CTA
+// clears and flushes an 8192-bin window whatever it counts.
+unsigned hist_assign_ctas(int num_sms, HistJob* jobs, int n) {
+  size_t total = 0;
+  for (int k = 0; k < n; k++) total += jobs[k].n;
+  const size_t share = std::max<size_t>(16 * HIST_NT, (total + num_sms - 1) / num_sms);
+  unsigned at = 0;
+  for (int k = 0; k < n; k++) {
+    jobs[k].cta0 = at;
+    jobs[k].ctas = (unsigned)std::max<size_t>(1, (jobs[k].n + share - 1) / share);
+    at += jobs[k].ctas;
+  }
+  return at;
+}
+
+int launch_hist_u16(cpsz_b200_ctx* ctx, const HistJob* jobs, const HistJob* d_jobs, int n, unsigned ctas) {
+  hist_u16_kernel<false><<<dim3(ctas, 2), HIST_NT, 0, ctx->stream>>>(jobs[0], n == 1 ? nullptr : d_jobs, n);
   count_launch(ctx);
   return check_launch("hist_u16_kernel");
 }
+
 int launch_hist_u16_nonzero(cpsz_b200_ctx* ctx, const uint16_t* sym, size_t n, unsigned long long* hist) {
   if (n == 0) return CPSZ_OK;
-  int grid = ctx->num_sms * 2;
-  size_t need = (n + HIST_NT - 1) / HIST_NT;
-  if ((size_t)grid > need) grid = (int)need;
-  hist_u16_kernel<true><<<dim3(grid, 1), HIST_NT, 0, ctx->stream>>>(sym, nullptr, n, hist, nullptr);
+  HistJob job{{sym, nullptr}, {hist, nullptr}, n, 0, 0};
+  job.ctas = (unsigned)std::min<size_t>((size_t)ctx->num_sms * 2, (n + HIST_NT - 1) / HIST_NT);
+  hist_u16_kernel<true><<<dim3(job.ctas, 1), HIST_NT, 0, ctx->stream>>>(job, nullptr, 1);
   count_launch(ctx);
   return check_launch("hist_u16_kernel");
+}
+
+int launch_hist_list(cpsz_b200_ctx* ctx, const HistList* d_jobs, int n, cudaStream_t stream) {
+  if (n <= 0) return CPSZ_OK;
+  hist_list_kernel<<<n, LIST_NT, 0, stream>>>(d_jobs);
+  count_launch(ctx);
+  return check_launch("hist_list_kernel");
 }
 
 int launch_hist_follow(cpsz_b200_ctx* ctx, const uint16_t* const codes[2], const unsigned* const group_done[2], int r1,
@@ -578,7 +684,16 @@ extern "C" int cpsz_b200_huffman_encode_u16_noalloc(const uint16_t* sym, size_t 
   int dev = 0, sms = 0;
   CPSZ_CUDA_TRY(cudaGetDevice(&dev));
   CPSZ_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  CPSZ_TRY(pack_launch<uint16_t>(sms, st, sym, n, false, HuffEncTable{(const unsigned long long*)code, len, 65536},
-                                 (uint32_t*)out, out_cap, 0, scratch, (unsigned long long*)total_bits, flag));
+  PackJob job;
+  job.sym = sym;
+  job.n = n;
+  job.sym_bytes = 2;
+  job.tab = HuffEncTable{(const unsigned long long*)code, len, 65536};
+  job.out = (uint32_t*)out;
+  job.cap_words = out_cap / 4;
+  job.scratch = scratch;
+  job.total_bits = (unsigned long long*)total_bits;
+  CPSZ_CUDA_TRY(cudaMemsetAsync(scratch, 0, pack_scratch_words(n) * 8, st));
+  CPSZ_TRY(launch_pack(st, &job, nullptr, 1, pack_assign_ctas(sms, &job, 1), flag));
   return check_launch("huffman no-alloc encode");
 }

@@ -119,20 +119,16 @@ size_t tree_size_for(size_t nodes) {
 
 }  // namespace
 
-bool huff_build(const unsigned long long* hist, size_t bins, size_t state_num, HuffCodebook* out) {
+namespace {
+
+// The codebook of the leaves in the thread's scratch.
+bool build_leaves(size_t bins, size_t state_num, HuffCodebook* out) {
+  Scratch& sc = scratch();
   // Leaves are nodes 0..distinct-1 in symbol order (the reference inserts them
   // that way); merged nodes follow.  Node data lives in two small arrays so
   // the merge loop and the walk stay cache-resident.
-  Scratch& sc = scratch();
   std::vector<uint32_t>& leaf_sym = sc.leaf_sym;
   std::vector<unsigned long long>& leaf_freq = sc.leaf_freq;
-  leaf_sym.clear();
-  leaf_freq.clear();
-  for (size_t s = 0; s < bins; s++)
-    if (hist[s]) {
-      leaf_sym.push_back((uint32_t)s);
-      leaf_freq.push_back(hist[s]);
-    }
   const size_t distinct = leaf_sym.size();
   if (distinct == 0) {
     set_error(CPSZ_ERR_INVALID, "Huffman: empty histogram");
@@ -232,16 +228,29 @@ bool huff_build(const unsigned long long* hist, size_t bins, size_t state_num, H
   return true;
 }
 
-int huff_upload(cpsz_b200_ctx* ctx, const HuffCodebook& cb, HuffEntry* h_stage, HuffEntry* d_ent,
-                unsigned long long* code, uint8_t* len) {
-  const size_t n = cb.entries.size();
-  const HuffEntry* src = cb.entries.data();
-  if (h_stage) {
-    memcpy(h_stage, src, n * sizeof(HuffEntry));
-    src = h_stage;
+}  // namespace
+
+bool huff_build(const unsigned long long* hist, size_t bins, size_t state_num, HuffCodebook* out) {
+  Scratch& sc = scratch();
+  sc.leaf_sym.clear();
+  sc.leaf_freq.clear();
+  for (size_t s = 0; s < bins; s++)
+    if (hist[s]) {
+      sc.leaf_sym.push_back((uint32_t)s);
+      sc.leaf_freq.push_back(hist[s]);
+    }
+  return build_leaves(bins, state_num, out);
+}
+
+bool huff_build_list(const unsigned long long* list, size_t n, size_t bins, size_t state_num, HuffCodebook* out) {
+  Scratch& sc = scratch();
+  sc.leaf_sym.resize(n);
+  sc.leaf_freq.resize(n);
+  for (size_t k = 0; k < n; k++) {
+    sc.leaf_sym[k] = (uint32_t)(list[k] >> 40);
+    sc.leaf_freq[k] = list[k] & ((1ull << 40) - 1);
   }
-  CPSZ_CUDA_TRY(cudaMemcpyAsync(d_ent, src, n * sizeof(HuffEntry), cudaMemcpyHostToDevice, ctx->stream));
-  return launch_codebook_scatter(ctx, d_ent, n, code, len);
+  return build_leaves(bins, state_num, out);
 }
 
 void huff_tables(const HuffCodebook& cb, size_t bins, unsigned long long* code, uint8_t* len) {

@@ -25,13 +25,9 @@ struct HuffCodebook {
 // exceed 64 bits.
 bool huff_build(const unsigned long long* hist, size_t bins, size_t state_num, HuffCodebook* out);
 
-// Device tables of the codebook: its entries go up to d_ent (room for
-// cb.entries.size()) on ctx->stream and are scattered into code / len.  With
-// h_stage (page-locked, room for the entries) the entries are copied there
-// first, so the upload is asynchronous; without, they go up from the
-// codebook's own (pageable) memory.
-int huff_upload(cpsz_b200_ctx* ctx, const HuffCodebook& cb, HuffEntry* h_stage, HuffEntry* d_ent,
-                unsigned long long* code, uint8_t* len);
+// The same from the symbols that occur: n words symbol << 40 | count, ascending,
+// every symbol below `bins`.
+bool huff_build_list(const unsigned long long* list, size_t n, size_t bins, size_t state_num, HuffCodebook* out);
 
 // Full per-symbol tables over `bins` symbols (code right-aligned; len 0 = absent).
 void huff_tables(const HuffCodebook& cb, size_t bins, unsigned long long* code, uint8_t* len);

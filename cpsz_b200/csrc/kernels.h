@@ -152,27 +152,47 @@ int launch_wave2d(cpsz_b200_ctx* ctx, bool decompress, const WaveField* d_fields
 // ---- block-order plumbing (12 x 12 blocks) ---------------------------------------
 // Both directions run as one pass over strips (a 12-row block row cut into
 // runs of 32 blocks), one launch for both components of a field, with a
-// decoupled look-back for the unpredictable values' offsets.
-// scratch[f]: strip_scratch_bytes(r1, r2) bytes (zeroed by the launch); after
-// it, *strip_total(scratch[f], ...) holds the component's number of zero codes.
+// decoupled look-back for the unpredictable values' offsets (scratch:
+// strip_scratch_bytes(r1, r2) zeroed bytes per component).
 size_t strip_count(int r1, int r2);
 size_t strip_scratch_bytes(int r1, int r2);
-const unsigned int* strip_total(const void* scratch, int r1, int r2);
 // Compression: codes raster -> 12x12-block order, and the values x at zero
-// codes (unpredictable) into unpred[f] in block order.
-int launch_strip_pass(cpsz_b200_ctx* ctx, const uint16_t* const raster[2], long long pitch, const float* const x[2],
-                      long long x_pitch, int r1, int r2, uint16_t* const blocks[2], float* const unpred[2],
-                      void* const scratch[2]);
+// codes (unpredictable) into unpred[f] in block order; several fields in one
+// launch, a CTA per strip and component (strip0: the field's first strip).
+struct StripJob {
+  const uint16_t* raster[2];
+  const float* x[2];
+  uint16_t* blocks[2];
+  float* unpred[2];
+  unsigned long long* status[2];  // strip_scratch_bytes(r1, r2) each, zeroed
+  unsigned* total;                // page-locked host memory: zero codes per component
+  int r1, r2;
+  unsigned strip0;
+};
+int launch_strip_pass(cpsz_b200_ctx* ctx, const StripJob* jobs, const StripJob* d_jobs, int n);
 // Decompression: block-order codes -> per raster point (pitch r2) the pair the
 // wavefront reads: (addend 2(code - 32768) * 4^id * 2^-52 (0 for id 0), raw
 // flag bits 0), or for code 0 (raw value, raw flag bits 1), the raw values
 // taken from unpred[f] in block order (an index past n_unpred[f] raises
 // FLAG_RAW_RANGE).
 // id_shift: 2 for the offline ids (p = 4^id * 2^-52), 1 for the offline_log
-// ids (p = 2^id * 2^-52).
+// ids (p = 2^id * 2^-52).  total (page-locked host memory) receives the number
+// of zero codes per component.
 int launch_strip_unpass(cpsz_b200_ctx* ctx, const uint16_t* const blocks[2], const uint8_t* const ids[2],
                         const float* const unpred[2], const unsigned long long n_unpred[2], int r1, int r2,
-                        float2* const pair[2], void* const scratch[2], int id_shift = 2);
+                        float2* const pair[2], void* const scratch[2], unsigned* total, int id_shift = 2);
+
+// Byte runs copied inside device memory (src null: zeros), several in one
+// launch, a CTA per PIECE_CHUNK bytes: assign_piece_chunks sets chunk0 and
+// returns the CTAs.  Runs must not overlap.
+struct CopyPiece {
+  uint8_t* dst;
+  const uint8_t* src;
+  size_t n;
+  unsigned chunk0;
+};
+unsigned assign_piece_chunks(CopyPiece* pieces, size_t n);
+int launch_copy_pieces(cpsz_b200_ctx* ctx, const CopyPiece* d_pieces, int n, unsigned ctas);
 
 // ---- 2D offline_log (log2d.cu) ------------------------------------------------------
 // Compression: per vertex the host library's log2f of |U| and |V| (-100 for 0)
@@ -193,44 +213,76 @@ struct HuffEntry {
   uint32_t sym;
   uint32_t len;
 };
-// Device codebook tables from n entries: code[e.sym] = e.code, len[e.sym] =
-// e.len.  Entries of symbols not in the list keep what the tables held: the
-// packer looks up only symbols that occur.
-int launch_codebook_scatter(cpsz_b200_ctx* ctx, const HuffEntry* d_entries, size_t n, unsigned long long* code,
-                            uint8_t* len);
 // Codebook for the encoder: per symbol, code right-aligned (bit len-1 = first bit).
 struct HuffEncTable {
   const unsigned long long* code;
   const uint8_t* len;
   int nsym;
 };
-// Symbols: u8 (map 255 -> 0 when map_id_zero) or u16.  Output: MSB-first bit
-// stream, zero padded, written as bytes at out (device, zero-initialised for
-// ceil(bits/8) bytes rounded up to 4).
+// Before a stream is packed (one launch for several streams): its n entries
+// scattered into code / len (entries of symbols not among them keep what the
+// tables held: the packer looks up only symbols that occur), and zero_bytes
+// bytes at `zero` cleared, the bytes its bits go to.
+struct PackPrep {
+  const HuffEntry* entries = nullptr;
+  size_t n = 0;
+  unsigned long long* code = nullptr;
+  uint8_t* len = nullptr;
+  uint8_t* zero = nullptr;
+  size_t zero_bytes = 0;
+};
+int launch_pack_prep(cpsz_b200_ctx* ctx, const PackPrep* d_jobs, int n, size_t max_entries, size_t max_zero_bytes);
+// One stream to pack.  Symbols: u8 (map_id_zero: 255 -> 0) or u16.  Output:
+// MSB-first bit stream, zero padded, written as bytes at out (zero-initialised
+// for ceil(bits/8) bytes).  Words at or beyond cap_words are not written
+// (FLAG_OUT_CAPACITY is raised).  The stream starts at bit bit0 (0-31, most
+// significant first) of out[0]; the bits before it are left as they are (the
+// first word is ORed), so a stream can be written straight after other bytes.
+struct PackJob {
+  const void* sym = nullptr;
+  size_t n = 0;
+  HuffEncTable tab{nullptr, nullptr, 0};
+  uint32_t* out = nullptr;
+  size_t cap_words = 0;
+  unsigned long long* scratch = nullptr;     // huff_encode_tmp_bytes(n), zeroed
+  unsigned long long* total_bits = nullptr;  // optional
+  int bit0 = 0, sym_bytes = 1, map_id_zero = 0;
+  unsigned cta0 = 0;
+};
 size_t huff_encode_tmp_bytes(size_t n);
-// Words at or beyond out_cap_bytes / 4 are not written (FLAG_OUT_CAPACITY is raised).
-// The stream starts at bit bit0 (0-31, most significant first) of out_words[0];
-// the bits before it are left as they are (the first word is ORed), so a
-// stream can be written straight after other bytes.  tmp: huff_encode_tmp_bytes(n).
-int launch_huff_encode_u8(cpsz_b200_ctx* ctx, const uint8_t* sym, size_t n, bool map_id_zero, HuffEncTable tab,
-                          uint32_t* out_words, size_t out_cap_bytes, unsigned long long* d_total_bits, void* tmp,
-                          int bit0 = 0);
-int launch_huff_encode_u16(cpsz_b200_ctx* ctx, const uint16_t* sym, size_t n, HuffEncTable tab,
-                           uint32_t* out_words, size_t out_cap_bytes, unsigned long long* d_total_bits, void* tmp,
-                           int bit0 = 0);
-// Histograms (global, 64-bit bins).
-int launch_hist_u16(cpsz_b200_ctx* ctx, const uint16_t* sym, size_t n, unsigned long long* hist);
-// The same without symbol 0 (its bin stays as it was).
+// Streams' shares of a launch's CTAs (cta0 of each); returns the total.
+unsigned pack_assign_ctas(int num_sms, PackJob* jobs, int n);
+// Packs n streams in one launch (d_jobs: the jobs on the device; not used for one).
+int launch_pack(cudaStream_t st, const PackJob* jobs, const PackJob* d_jobs, int n, unsigned ctas, int* flag);
+// One stream on ctx->stream; its scratch is zeroed here.
+int launch_huff_encode(cpsz_b200_ctx* ctx, PackJob job);
+// Histograms (global, 64-bit bins) of fields' two code components, n symbols
+// each, in one launch: CTAs [cta0, cta0 + ctas) of the launch are a field's
+// (hist_assign_ctas returns the total).
+struct HistJob {
+  const uint16_t* sym[2];
+  unsigned long long* hist[2];
+  size_t n;
+  unsigned cta0, ctas;
+};
+unsigned hist_assign_ctas(int num_sms, HistJob* jobs, int n);
+int launch_hist_u16(cpsz_b200_ctx* ctx, const HistJob* jobs, const HistJob* d_jobs, int n, unsigned ctas);
+// One stream, without symbol 0 (its bin stays as it was).
 int launch_hist_u16_nonzero(cpsz_b200_ctx* ctx, const uint16_t* sym, size_t n, unsigned long long* hist);
-// Two streams of n symbols each in one launch.
-int launch_hist_u16_pair(cpsz_b200_ctx* ctx, const uint16_t* a, const uint16_t* b, size_t n, unsigned long long* ha,
-                         unsigned long long* hb);
+// A 65536-bin histogram as the list of its occurring symbols (ascending,
+// symbol << 40 | count, counts below 2^40) in page-locked host memory.
+struct HistList {
+  const unsigned long long* hist;
+  unsigned long long* list;  // room for 65536
+  unsigned* count;
+};
+int launch_hist_list(cpsz_b200_ctx* ctx, const HistList* d_jobs, int n, cudaStream_t stream);
 // The two code histograms of one field (r1 x r2 raster codes, pitch r2)
 // while its wavefront runs: row groups are counted as their group_done flags
 // (WaveField::group_done) appear.  tickets: 2 words, zeroed.  A wait that
 // outlasts its bound sets *gave_up (zeroed by the caller) and leaves the
 // histograms incomplete; the caller then counts them with
-// launch_hist_u16_pair.  Enqueued on `stream`.
+// launch_hist_u16.  Enqueued on `stream`.
 int launch_hist_follow(cpsz_b200_ctx* ctx, const uint16_t* const codes[2], const unsigned* const group_done[2], int r1,
                        int r2, unsigned long long* const hist[2], unsigned* tickets, int* gave_up, cudaStream_t stream);
 

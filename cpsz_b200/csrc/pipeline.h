@@ -61,8 +61,10 @@ struct Blob3D {
   size_t n_unpred = 0;  // floats (3 per unpredictable point)
   size_t n_codes = 0;   // codes (3 per predicted point)
 };
+// dev_out (optional): device memory of dev_cap bytes that gets the blob if it
+// has room (out->d_blob == dev_out then).
 int compress_3d(cpsz_b200_ctx* ctx, const float* U, const float* V, const float* W, size_t r1, size_t r2, size_t r3,
-                double max_pwr_eb, Blob3D* out);
+                double max_pwr_eb, Blob3D* out, unsigned char* dev_out = nullptr, size_t dev_cap = 0);
 int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_size, size_t r1, size_t r2, size_t r3,
                   float* U, float* V, float* W);
 

@@ -32,6 +32,7 @@
 #include "host_pool.h"
 #include "huffman_host.h"
 #include "kernels.h"
+#include "pack_group.h"
 #include "tuning.h"
 #include "pipeline.h"
 #include "transfer.h"
@@ -43,13 +44,22 @@ namespace {
 constexpr int BS = 12;
 constexpr size_t FIELD_HDR = 4 + 1 + 4 + 8 + 8 + 8;  // up to and including n_unpred
 constexpr size_t BLOB_HDR = 4 + 8 + 8 + 8 + 8;
-// pinned staging per field: id histogram, two code histograms, unpredictable
-// counts, the id codebook's entries
-constexpr size_t JOB_PINNED = (256 + 2 * 65536) * 8 + 64 + 256 * sizeof(HuffEntry);
+// pinned staging per field, behind the fields' id histograms (256 words each):
+// the two code histograms' lists and their lengths, the unpredictable counts
+constexpr size_t ID_HIST = 256 * 8;
+constexpr size_t JOB_PINNED = 2 * 65536 * 8 + 64;
 constexpr size_t PINNED_BASE = 4096;  // the flag word and scalars live below
 // sub-batch limits: fields per pass (pinned staging) and points per pass (workspace)
 constexpr int BATCH_MAX_FIELDS = 32;
 constexpr size_t BATCH_MAX_POINTS = (size_t)1 << 27;
+// A single field of at least this many points packs its ids on the second
+// stream while the wavefront's tail runs; a smaller one (and a batch) packs
+// its three streams in one launch once every tree is known: below it the
+// extra copy, launches and events cost more than the packing they hide.
+constexpr size_t EARLY_IDS_POINTS = (size_t)1 << 19;
+
+// upload staging of that packing
+constexpr size_t EARLY_UP = 256 * sizeof(HuffEntry) + sizeof(PackPrep) + sizeof(PackJob) + 512;
 
 struct DevBuf {
   // arena sub-allocations of one field
@@ -65,15 +75,13 @@ struct DevBuf {
   unsigned* gdone;            // per component and row group: the wavefront is done with it; then 2 tickets, gave_up
   unsigned long long* units;  // eb2d progress word, then per-unit counters of finished vertices
   int2* uorder;               // eb2d's unit order (every band's units, band after band)
-  void* strip[2];            // strip-pass look-back words and counters
+  unsigned long long* strip[2];  // strip-pass look-back words and ticket
   float* unpred[2];
   unsigned long long* enc_code[3];
   uint8_t* enc_len[3];
-  HuffEntry* enc_ent[3];  // codebook entries as uploaded
-  void* enc_tmp[3];
+  unsigned long long* enc_tmp[3];
   uint32_t* bits[3];
   uint8_t* blob;
-  uint8_t* stage;       // the blob's small pieces and their descriptors, as uploaded
   float* logs[2];       // offline_log: log2f |U|, |V| (the unpredictable values it stores)
   uint32_t* signs[2];   // offline_log: sign maps
 };
@@ -83,24 +91,24 @@ struct Job2D {
   const float* U_in = nullptr;
   const float* V_in = nullptr;
   int r1 = 0, r2 = 0, ngroups = 0, ncb = 0;
-  size_t N = 0, nseg = 0, nblocks = 0;
+  size_t N = 0, nblocks = 0;
   double eb = 0;
   const double* eb_ext = nullptr;  // given per-vertex bounds (device), else derived
   bool dev_in = false;
   size_t ids_bits_cap = 0, codes_bits_cap = 0, blob_cap = 0;
   DevBuf d{};
-  unsigned long long* h_hist_ids = nullptr;    // pinned
-  unsigned long long* h_hist_codes = nullptr;  // pinned, 2 x 65536
-  unsigned int* h_nunpred = nullptr;           // pinned, 2
-  HuffEntry* h_ids_ent = nullptr;              // pinned, 256
+  unsigned long long* h_hist_ids = nullptr;  // pinned, 256
+  unsigned long long* h_list[2] = {nullptr, nullptr};  // pinned, 65536 each
+  unsigned* h_nlist = nullptr;               // pinned, 2
+  unsigned* h_nunpred = nullptr;             // pinned, 2
   HuffCodebook cb[3];
   bool tree_ok[3] = {false, false, false};
   size_t n_unpred[2] = {0, 0};
   size_t sec_bytes[3] = {0, 0, 0}, bits_bytes[3] = {0, 0, 0};
   size_t size = 0;  // blob bytes
   // device output: the blob is built in place at blob_base (blob_room bytes
-  // there), the caller's buffer when it is a device buffer with room for the
-  // blob's bound, else the workspace blob
+  // there), the caller's buffer when it is a device buffer with room for it,
+  // else the workspace blob
   unsigned char* dev_out = nullptr;
   size_t dev_cap = 0;
   uint8_t* blob_base = nullptr;
@@ -112,7 +120,7 @@ struct Job2D {
   // the offline_log form: base 2, one id stream of N symbols, the two sign
   // maps (device, MSB-first bit streams) between the id section and the fields
   bool log_form = false;
-  const uint32_t* d_signs[2] = {nullptr, nullptr};
+  size_t n_syms(int k) const { return k || log_form ? N : 2 * N; }  // stream k: ids, codes of U / V
 };
 
 int read_flag(cpsz_b200_ctx* ctx, int* out) {
@@ -162,7 +170,6 @@ int job_init(Job2D& j, const float* U, const float* V, size_t r1s, size_t r2s, d
   j.ngroups = (j.r1 + WAVE_GROUP_ROWS - 1) / WAVE_GROUP_ROWS;
   j.ncb = (j.r2 + UNIT_COLS - 1) / UNIT_COLS;
   const int nby = (j.r2 - 1) / BS + 1, nbx = (j.r1 - 1) / BS + 1;
-  j.nseg = (size_t)j.r1 * nby;
   j.nblocks = (size_t)nbx * nby;
   j.dev_in = is_device_ptr(U) && is_device_ptr(V);
   // bit streams: Huffman averages < log2(distinct) + 1 bits per symbol
@@ -174,123 +181,156 @@ int job_init(Job2D& j, const float* U, const float* V, size_t r1s, size_t r2s, d
   return CPSZ_OK;
 }
 
-// Bound of the blob's small pieces (header, three trees with their stream
-// sizes, field headers, indicators) and their descriptors.
-size_t stage_bytes(const Job2D& j) {
-  const size_t tree = 12 + 1 + 13 * std::min<size_t>(131072, 2 * j.N + 1) + 8;
-  return BLOB_HDR + 2 * FIELD_HDR + 2 * ((j.nblocks + 7) / 8) + (12 + 1 + 13 * 512 + 8) + 2 * tree + 64 + 24 * 32;
+// Bound of a field's uploads once its trees are known: code entries and
+// their tables' jobs, then the blob's small pieces (header, three trees with
+// their stream sizes, field headers) and their descriptors.
+size_t up_bytes_bound(const Job2D& j) {
+  const size_t sym = std::min<size_t>(65536, j.N), tree = 12 + 1 + 13 * std::min<size_t>(131072, 2 * j.N + 1) + 8;
+  return (256 + 2 * sym) * sizeof(HuffEntry) + BLOB_HDR + 2 * FIELD_HDR + (12 + 1 + 13 * 512 + 8) + 2 * tree +
+         3 * (sizeof(PackPrep) + sizeof(PackJob)) + 24 * sizeof(CopyPiece) + 1024;
 }
 
-// Workspace of one field (each piece padded as the arena pads it).
-size_t job_bytes(const Job2D& j) {
+// Pass-wide device pieces.
+struct PassBuf {
+  // the setup image, one upload: thresholds, wavefront fields and items, jobs
+  // of the batched kernels, eb2d's unit order
+  uint8_t* image;
+  size_t image_bytes;
+  double* thr;
+  WaveField* fields;
+  WaveItem* items;
+  Eb2dJob* eb;
+  HistJob* hist;
+  HistList* list;
+  StripJob* strip;
+  int2* uorder;
+  // zeroed in one piece: the wavefront's queue, histograms, look-back words
+  uint8_t* zero;
+  size_t zero_bytes;
+  int* queue;
+  unsigned long long* hist_ids;
+  uint8_t* gbnd;  // boundary rows, right behind (a pass over some row groups keeps part of them)
+  size_t gbnd_bytes;
+  uint8_t* up_ids;  // early id entries
+  uint8_t* up;      // later uploads
+  size_t up_bytes;
+};
+
+// The pass's workspace: with a null arena every piece is only counted (each
+// padded as the arena pads it).
+struct Alloc {
+  cpsz_b200_ctx* ctx;  // null: count
   size_t bytes = 0;
-  auto add = [&](size_t b) { bytes += align_up(b, 256) + 256; };
-  const size_t N = j.N;
-  if (!j.dev_in) add(8 * N);
-  add(2 * N);                           // ids
-  add(256 * 8);                         // hist ids
-  add(4 * N);                           // codes raster
-  add(16 * N);                          // wavefront input pairs
-  add(4 * N);                           // codes blocks
-  add(2 * 65536 * 8);                   // hist codes
-  add(2 * (size_t)j.ngroups * j.r2 * 8);  // boundary rows (tagged words)
-  add((2 * (size_t)j.ngroups + 4) * 4);   // row-group done flags, follower tickets and flag
-  add(((size_t)j.ngroups * j.ncb + 1) * 8);       // eb2d progress word + unit counters
-  add((size_t)j.ngroups * j.ncb * sizeof(int2));  // eb2d unit order
-  add(2 * strip_scratch_bytes(j.r1, j.r2));
-  add(2 * 4 * N);  // unpred
-  add(256 * 9);
-  add(2 * 65536 * 9);
-  add(256 * sizeof(HuffEntry));
-  add(std::min<size_t>(65536, N) * sizeof(HuffEntry));
-  add(std::min<size_t>(65536, N) * sizeof(HuffEntry));
-  add(huff_encode_tmp_bytes(2 * N));
-  add(2 * huff_encode_tmp_bytes(N));
-  add(j.ids_bits_cap);
-  add(2 * j.codes_bits_cap);
-  add(j.blob_cap);
-  add(stage_bytes(j));
-  if (j.log_form) {
-    add(2 * 4 * N);                        // log values
-    add(2 * 4 * ((N + 31) / 32));          // sign maps
-  }
-  return bytes;
-}
-
-int job_alloc(cpsz_b200_ctx* ctx, Job2D& j) {
-  // a request that does not fit fails every later one too (no smaller piece
-  // may land behind a failed one): the check of the last piece covers all
   bool failed = false;
-  auto A = [&](size_t b) -> void* {
-    void* p = failed ? nullptr : arena_alloc(ctx, b);
-    failed = failed || !p;
+  void* operator()(size_t b) {
+    bytes += align_up(b, 256) + 256;
+    if (!ctx || failed) return nullptr;
+    // a request that does not fit fails every later one too (no smaller piece
+    // may land behind a failed one)
+    void* p = arena_alloc(ctx, b);
+    failed = !p;
     return p;
+  }
+};
+// A run of pieces inside one allocation, 256-byte aligned each.
+struct Run {
+  uint8_t* base;
+  size_t at = 0;
+  uint8_t* take(size_t b) {
+    uint8_t* p = base ? base + at : nullptr;
+    at += align_up(b, 256);
+    return p;
+  }
+};
+
+void pass_alloc(std::vector<Job2D>& jobs, PassBuf& P, Alloc& A) {
+  const size_t nj = jobs.size();
+  auto image = [&](Run r) {
+    P.thr = (double*)r.take(QUANT_TAB_MAX * 8);
+    P.fields = (WaveField*)r.take(2 * nj * sizeof(WaveField));
+    size_t groups = 0, units = 0;
+    for (const Job2D& j : jobs) {
+      groups += j.ngroups;
+      units += (size_t)j.ngroups * j.ncb;
+    }
+    P.items = (WaveItem*)r.take(2 * groups * sizeof(WaveItem));
+    P.eb = (Eb2dJob*)r.take(nj * sizeof(Eb2dJob));
+    P.hist = (HistJob*)r.take(nj * sizeof(HistJob));
+    P.list = (HistList*)r.take(2 * nj * sizeof(HistList));
+    P.strip = (StripJob*)r.take(nj * sizeof(StripJob));
+    P.uorder = (int2*)r.take(nj == 1 ? units * sizeof(int2) : 0);
+    return r.at;
   };
-  DevBuf& d = j.d;
-  const size_t N = j.N;
-  if (j.dev_in) {
-    d.U = const_cast<float*>(j.U_in);
-    d.V = const_cast<float*>(j.V_in);
-  } else {
-    d.U = (float*)A(4 * N);
-    d.V = (float*)A(4 * N);
-  }
-  d.ids = (uint8_t*)A(2 * N);
-  d.hist_ids = (unsigned long long*)A(256 * 8);
-  for (int f = 0; f < 2; f++) {
-    d.craster[f] = (uint16_t*)A(2 * N);
-    d.pairs[f] = (float2*)A(8 * N);
-    d.cblocks[f] = (uint16_t*)A(2 * N);
-    d.hist_codes[f] = (unsigned long long*)A(65536 * 8);
-  }
-  d.gbnd = (unsigned long long*)A(2 * (size_t)j.ngroups * j.r2 * 8);
-  d.gdone = (unsigned*)A((2 * (size_t)j.ngroups + 4) * 4);
-  d.units = (unsigned long long*)A(((size_t)j.ngroups * j.ncb + 1) * 8);
-  d.uorder = (int2*)A((size_t)j.ngroups * j.ncb * sizeof(int2));
-  for (int f = 0; f < 2; f++) {
-    d.strip[f] = A(strip_scratch_bytes(j.r1, j.r2));
-    d.unpred[f] = (float*)A(4 * N);
-  }
-  d.enc_code[0] = (unsigned long long*)A(256 * 8);
-  d.enc_len[0] = (uint8_t*)A(256);
-  for (int f = 1; f < 3; f++) {
-    d.enc_code[f] = (unsigned long long*)A(65536 * 8);
-    d.enc_len[f] = (uint8_t*)A(65536);
-  }
-  d.enc_ent[0] = (HuffEntry*)A(256 * sizeof(HuffEntry));
-  d.enc_ent[1] = (HuffEntry*)A(std::min<size_t>(65536, N) * sizeof(HuffEntry));
-  d.enc_ent[2] = (HuffEntry*)A(std::min<size_t>(65536, N) * sizeof(HuffEntry));
-  d.enc_tmp[0] = A(huff_encode_tmp_bytes(2 * N));
-  d.enc_tmp[1] = A(huff_encode_tmp_bytes(N));
-  d.enc_tmp[2] = A(huff_encode_tmp_bytes(N));
-  d.bits[0] = (uint32_t*)A(j.ids_bits_cap);
-  d.bits[1] = (uint32_t*)A(j.codes_bits_cap);
-  d.bits[2] = (uint32_t*)A(j.codes_bits_cap);
-  d.blob = (uint8_t*)A(j.blob_cap);
-  d.stage = (uint8_t*)A(stage_bytes(j));
-  if (!d.stage) return set_error(CPSZ_ERR_NOMEM, "workspace layout overflow");
-  if (j.dev_out && j.dev_cap >= j.blob_cap + 8) {
-    j.blob_base = j.dev_out;
-    j.blob_room = j.dev_cap;
-  } else {
+  P.image_bytes = image(Run{nullptr});
+  P.image = (uint8_t*)A(P.image_bytes);
+  image(Run{P.image});
+  auto zero = [&](Run r) {
+    P.queue = (int*)r.take(256);
+    P.hist_ids = (unsigned long long*)r.take(nj * ID_HIST);
+    for (size_t k = 0; k < nj; k++) {
+      Job2D& j = jobs[k];
+      DevBuf& d = j.d;
+      d.hist_ids = P.hist_ids + 256 * k;
+      d.units = (unsigned long long*)r.take(((size_t)j.ngroups * j.ncb + 1) * 8);
+      d.gdone = (unsigned*)r.take((2 * (size_t)j.ngroups + 4) * 4);
+      for (int f = 0; f < 2; f++) {
+        d.hist_codes[f] = (unsigned long long*)r.take(65536 * 8);
+        d.strip[f] = (unsigned long long*)r.take(strip_scratch_bytes(j.r1, j.r2));
+      }
+      for (int f = 0; f < 3; f++) d.enc_tmp[f] = (unsigned long long*)r.take(huff_encode_tmp_bytes(j.n_syms(f)));
+    }
+    P.zero_bytes = r.at;
+    P.gbnd = r.take(0);
+    for (Job2D& j : jobs) j.d.gbnd = (unsigned long long*)r.take(2 * (size_t)j.ngroups * j.r2 * 8);
+    P.gbnd_bytes = r.at - P.zero_bytes;
+    return r.at;
+  };
+  const size_t zb = zero(Run{nullptr});
+  P.zero = (uint8_t*)A(zb);
+  zero(Run{P.zero});
+  P.up_bytes = 0;
+  for (const Job2D& j : jobs) P.up_bytes += up_bytes_bound(j);
+  P.up = (uint8_t*)A(P.up_bytes);
+  P.up_ids = (uint8_t*)A(EARLY_UP);
+  for (Job2D& j : jobs) {
+    DevBuf& d = j.d;
+    const size_t N = j.N;
+    if (j.dev_in) {
+      d.U = const_cast<float*>(j.U_in);
+      d.V = const_cast<float*>(j.V_in);
+    } else {
+      d.U = (float*)A(4 * N);
+      d.V = (float*)A(4 * N);
+    }
+    d.ids = (uint8_t*)A(2 * N);
+    for (int f = 0; f < 2; f++) {
+      d.craster[f] = (uint16_t*)A(2 * N);
+      d.pairs[f] = (float2*)A(8 * N);
+      d.cblocks[f] = (uint16_t*)A(2 * N);
+      d.unpred[f] = (float*)A(4 * N);
+    }
+    d.uorder = P.uorder;
+    for (int f = 0; f < 3; f++) {
+      const size_t n = f ? 65536 : 256;
+      d.enc_code[f] = (unsigned long long*)A(n * 8);
+      d.enc_len[f] = (uint8_t*)A(n);
+      d.bits[f] = (uint32_t*)A(f ? j.codes_bits_cap : j.ids_bits_cap);
+    }
+    d.blob = (uint8_t*)A(j.blob_cap);
+    if (j.log_form)
+      for (int f = 0; f < 2; f++) {
+        d.logs[f] = (float*)A(4 * N);
+        d.signs[f] = (uint32_t*)A(4 * ((N + 31) / 32));
+      }
     j.blob_base = d.blob;
     j.blob_room = align_up(j.blob_cap, 256);
+    if (j.dev_out && j.dev_cap >= j.blob_cap + 8) {
+      j.blob_base = j.dev_out;
+      j.blob_room = j.dev_cap;
+    }
   }
-  if (j.log_form) {
-    d.logs[0] = (float*)A(4 * N);
-    d.logs[1] = (float*)A(4 * N);
-    d.signs[0] = (uint32_t*)A(4 * ((N + 31) / 32));
-    d.signs[1] = (uint32_t*)A(4 * ((N + 31) / 32));
-    if (!d.signs[1]) return set_error(CPSZ_ERR_NOMEM, "workspace layout overflow");
-    j.d_signs[0] = d.signs[0];
-    j.d_signs[1] = d.signs[1];
-  }
-  return CPSZ_OK;
 }
 
-// Blob assembly of one field in device memory (header, id tree, two field
-// blobs); the small host-made pieces go up in one copy and are scattered
-// with device-to-device copies.
 // The reference's 2D blob (sz_compress_cp_preserve_2d_offline,
 // src/sz_compress_cp_preserve_2d.cpp): header, the id stream's Huffman
 // section, then per component its header, unpredictable floats, the all-zero
@@ -380,81 +420,47 @@ int job_layout(const Job2D& j, BlobLayout& L) {
   return CPSZ_OK;
 }
 
-// The small pieces of a blob in one launch: CTA (x, y) copies bytes
-// [x * 4096, (x + 1) * 4096) of piece y from the staged bytes (byte stores:
-// the bytes around a piece belong to other sections, some written before it).
-constexpr int PIECE_CHUNK = 4096;
-__global__ void __launch_bounds__(256) pieces_kernel(const uint8_t* __restrict__ small,
-                                                     const unsigned long long* __restrict__ desc,
-                                                     uint8_t* __restrict__ blob) {
-  const unsigned long long dst = desc[3 * blockIdx.y], src = desc[3 * blockIdx.y + 1], n = desc[3 * blockIdx.y + 2];
-  const unsigned long long c0 = (unsigned long long)blockIdx.x * PIECE_CHUNK;
-  const unsigned long long c1 = n < c0 + PIECE_CHUNK ? n : c0 + PIECE_CHUNK;
-  if (src == ~0ull) {  // a run of zeros
-    for (unsigned long long i = c0 + threadIdx.x; i < c1; i += 256) blob[dst + i] = 0;
-    return;
-  }
-  for (unsigned long long i = c0 + threadIdx.x; i < c1; i += 256) blob[dst + i] = small[src + i];
-}
-
-// Bytes job_assemble uploads: the small pieces and the referenced ones, then
-// their descriptors.
-size_t assemble_payload_bytes(const BlobLayout& L) {
-  size_t n = L.small.size();
+// Upload staging that job_pieces takes for a field, its copies' table included.
+size_t piece_up_bytes(const BlobLayout& L) {
+  size_t b = align_up(L.small.size(), 16) + (L.pieces.size() + 5) * sizeof(CopyPiece) + 64;
   for (const BlobLayout::Piece& pc : L.pieces)
-    if (pc.ext) n += pc.n;
-  return align_up(n, 8);
+    if (pc.ext) b += align_up(pc.n, 16) + 16;
+  return b;
 }
-size_t assemble_upload_bytes(const BlobLayout& L) { return assemble_payload_bytes(L) + 24 * L.pieces.size(); }
 
-// The sections of a device blob that the packers do not write: the staged
-// small pieces (header, trees, stream sizes, field headers, indicators), the
-// unpredictable values and the sign maps.  h_up: page-locked staging of
-// assemble_upload_bytes(L), which must stay untouched until the pass ends.
-int job_assemble(cpsz_b200_ctx* ctx, Job2D& j, const BlobLayout& L, uint8_t* h_up) {
-  cudaStream_t st = ctx->stream;
+// The sections of a device blob that the packers do not write, as copies for
+// launch_copy_pieces: the staged small pieces (header, trees, stream sizes,
+// field headers), the zero indicators, the unpredictable values, the sign maps.
+int job_pieces(Job2D& j, const BlobLayout& L, UpImage& up, std::vector<CopyPiece>& out) {
   uint8_t* blob = j.blob_base;
-  // pieces and their descriptors go up in one copy
-  const size_t up_size = assemble_upload_bytes(L), payload = assemble_payload_bytes(L);
-  memcpy(h_up, L.small.data(), L.small.size());
-  size_t ext_at = L.small.size();
-  unsigned long long* desc = (unsigned long long*)(h_up + payload);
-  for (size_t i = 0; i < L.pieces.size(); i++) {
-    const BlobLayout::Piece& pc = L.pieces[i];
-    size_t src = pc.src;
+  uint8_t *d_small, *d_ext;
+  uint8_t* h = up.take(L.small.size(), &d_small);
+  if (!h) return up_overrun();
+  memcpy(h, L.small.data(), L.small.size());
+  for (const BlobLayout::Piece& pc : L.pieces) {
+    CopyPiece c{blob + pc.dst, pc.zero ? nullptr : d_small + pc.src, pc.n, 0};
     if (pc.ext) {
-      memcpy(h_up + ext_at, pc.ext, pc.n);
-      src = ext_at;
-      ext_at += pc.n;
+      if (!(h = up.take(pc.n, &d_ext))) return up_overrun();
+      memcpy(h, pc.ext, pc.n);
+      c.src = d_ext;
     }
-    desc[3 * i] = pc.dst;
-    desc[3 * i + 1] = pc.zero ? ~0ull : src;
-    desc[3 * i + 2] = pc.n;
+    out.push_back(c);
   }
-  if (up_size > stage_bytes(j)) return set_error(CPSZ_ERR_INVALID, "internal: blob pieces exceed their bound");
-  uint8_t* d_up = j.d.stage;
-  CPSZ_CUDA_TRY(cudaMemcpyAsync(d_up, h_up, up_size, cudaMemcpyHostToDevice, st));
-  if (!L.pieces.empty()) {
-    size_t longest = 0;
-    for (const BlobLayout::Piece& pc : L.pieces) longest = std::max(longest, pc.n);
-    const dim3 grid((unsigned)std::max<size_t>(1, (longest + PIECE_CHUNK - 1) / PIECE_CHUNK), (unsigned)L.pieces.size());
-    pieces_kernel<<<grid, 256, 0, st>>>(d_up, (const unsigned long long*)(d_up + payload), blob);
-    count_launch(ctx);
-    CPSZ_TRY(check_launch("pieces_kernel"));
-  }
-  for (int f = 0; f < 2; f++)
+  for (int f = 0; f < 2; f++) {
     if (j.n_unpred[f])
-      CPSZ_CUDA_TRY(
-          cudaMemcpyAsync(blob + L.unpred_dst[f], j.d.unpred[f], 4 * j.n_unpred[f], cudaMemcpyDeviceToDevice, st));
-  for (int f = 0; f < 2 && L.sign_bytes; f++)
-    CPSZ_CUDA_TRY(cudaMemcpyAsync(blob + L.sign_dst + f * L.sign_bytes, j.d_signs[f], L.sign_bytes,
-                                  cudaMemcpyDeviceToDevice, st));
+      out.push_back(CopyPiece{blob + L.unpred_dst[f], (const uint8_t*)j.d.unpred[f], 4 * j.n_unpred[f], 0});
+    if (L.sign_bytes)
+      out.push_back(
+          CopyPiece{blob + L.sign_dst + f * L.sign_bytes, (const uint8_t*)j.d.signs[f], L.sign_bytes, 0});
+  }
   j.size = L.total;
   return CPSZ_OK;
 }
 
 // One compression pass over `jobs` (workspace reserved by the caller).
-int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) {
+// dev_at (device memory with room for dev_room bytes, or null): the blobs are
+// built there back to back if they fit.
+int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap, uint8_t* dev_at, size_t dev_room) {
   cudaStream_t st = ctx->stream;
   const int nj = (int)jobs.size();
   // the offline_log form runs as a pass of one field
@@ -462,22 +468,19 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
   const QuantTable& qt = log_form ? quant_table_2d_log() : quant_table_2d();
   LibmTables libm{};
   if (log_form) CPSZ_TRY(libm_tables_device(ctx, &libm));
-  // pass-wide device pieces
-  double* thr_tab = (double*)arena_alloc(ctx, QUANT_TAB_MAX * 8);
-  int* queue = (int*)arena_alloc(ctx, 64);
-  WaveField* d_fields = (WaveField*)arena_alloc(ctx, 2 * nj * sizeof(WaveField));
-  int total_groups = 0;
-  for (const Job2D& j : jobs) total_groups += j.ngroups;
-  WaveItem* d_items = (WaveItem*)arena_alloc(ctx, 2 * (size_t)total_groups * sizeof(WaveItem));
-  Eb2dJob* d_ebjobs = (Eb2dJob*)arena_alloc(ctx, nj * sizeof(Eb2dJob));
-  if (!d_items || !d_ebjobs) return set_error(CPSZ_ERR_NOMEM, "workspace layout overflow");
-  for (Job2D& j : jobs) CPSZ_TRY(job_alloc(ctx, j));
-  for (int k = 0; k < nj; k++) {
-    uint8_t* base = (uint8_t*)ctx->pinned + PINNED_BASE + (size_t)k * JOB_PINNED;
-    jobs[k].h_hist_ids = (unsigned long long*)base;
-    jobs[k].h_hist_codes = jobs[k].h_hist_ids + 256;
-    jobs[k].h_nunpred = (unsigned int*)(jobs[k].h_hist_codes + 2 * 65536);
-    jobs[k].h_ids_ent = (HuffEntry*)(base + (256 + 2 * 65536) * 8 + 64);
+  PassBuf P{};
+  Alloc arena{ctx};
+  pass_alloc(jobs, P, arena);
+  if (arena.failed) return set_error(CPSZ_ERR_NOMEM, "workspace layout overflow");
+  {
+    uint8_t* base = (uint8_t*)ctx->pinned + PINNED_BASE;
+    for (int k = 0; k < nj; k++) jobs[k].h_hist_ids = (unsigned long long*)(base + k * ID_HIST);
+    base += nj * ID_HIST;
+    for (int k = 0; k < nj; k++, base += JOB_PINNED) {
+      for (int f = 0; f < 2; f++) jobs[k].h_list[f] = (unsigned long long*)base + (size_t)f * 65536;
+      jobs[k].h_nlist = (unsigned*)(base + 2 * 65536 * 8);
+      jobs[k].h_nunpred = jobs[k].h_nlist + 2;
+    }
   }
 
   // Derived bounds (eb2d) signal per 128-row group, so for one field the
@@ -496,14 +499,15 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
     return (int)align_up((size_t)(j.r1 + K - 1) / K, WAVE_GROUP_ROWS);
   };
 
-  // ---- setup: flags, tables, wavefront descriptors ----
+  // ---- setup: one image with the tables and every kernel's jobs, built in
+  // the page-locked upload staging (no copy from it is in flight yet; the
+  // pass's later uploads reuse it after this copy has run) ----
   reset_marks(ctx);
   mark(ctx, "h2d+setup");
-  CPSZ_CUDA_TRY(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), st));
-  CPSZ_CUDA_TRY(cudaMemcpyAsync(thr_tab, qt.t, QUANT_TAB_MAX * 8, cudaMemcpyHostToDevice, st));
-  for (Job2D& j : jobs) CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.hist_ids, 0, 256 * 8, st));
-  std::vector<WaveField> hf(2 * nj);
-  std::vector<int> r1v(2 * nj);
+  CPSZ_TRY(upload_reserve(ctx, P.image_bytes));
+  uint8_t* const h_image = (uint8_t*)ctx->up_pinned;
+  auto host = [&](auto* dev) { return reinterpret_cast<decltype(dev)>(h_image + ((uint8_t*)dev - P.image)); };
+  memcpy(host(P.thr), qt.t, QUANT_TAB_MAX * 8);
   // a pass that quantizes again only some vertices starts the recursion at
   // their first row group: the groups above (and their boundary rows, which
   // the first group run reads) are the previous pass's
@@ -515,33 +519,39 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
   // groups finish, instead of after it (below 2^22 points the histograms take
   // a few microseconds and the follower's own launch and waits cost more).
   const bool follow = overlap && nj == 1 && !tap && jobs[0].N >= ((size_t)1 << 22);
+  std::vector<WaveField> hf(2 * nj);
+  std::vector<int> r1v(2 * nj);
+  std::vector<HistJob> hist_jobs(nj);
+  std::vector<StripJob> strip_jobs(nj);
+  size_t strips = 0;
   for (int k = 0; k < nj; k++) {
     Job2D& j = jobs[k];
-    if (follow) CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.gdone, 0, (2 * (size_t)j.ngroups + 4) * 4, st));
-    for (int f = 0; f < 2; f++) {
-      CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.gbnd + ((size_t)f * j.ngroups + g0) * j.r2, 0,
-                                    (size_t)(j.ngroups - g0) * j.r2 * 8, st));
-      CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.hist_codes[f], 0, 65536 * 8, st));  // stage 3's histograms
-    }
     if (overlap) {
-      // eb2d's unit counters and its unit order, band by band (units along
-      // diagonals of slope eb2d.skew column blocks per group)
-      CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.units, 0, ((size_t)j.ngroups * j.ncb + 1) * 8, st));
+      // eb2d's unit order, band by band (units along diagonals of slope
+      // eb2d.skew column blocks per group)
       const int R = band_rows(j), skew = tune_get(TUNE_EB2D_SKEW, j.N);
-      std::vector<int2> order, part;
+      std::vector<int2> part;
+      int2* order = host(P.uorder);
       for (int r0 = 0; r0 < j.r1; r0 += R) {
         unit_order(r0 / WAVE_GROUP_ROWS, (std::min(j.r1, r0 + R) + WAVE_GROUP_ROWS - 1) / WAVE_GROUP_ROWS, j.ncb, skew,
                    part);
-        order.insert(order.end(), part.begin(), part.end());
+        order = std::copy(part.begin(), part.end(), order);
       }
-      // through the page-locked upload staging (no copy from it is in flight
-      // yet; the pass's later uploads reuse it after this copy has run)
-      CPSZ_TRY(upload_reserve(ctx, order.size() * sizeof(int2)));
-      memcpy(ctx->up_pinned, order.data(), order.size() * sizeof(int2));
-      CPSZ_CUDA_TRY(
-          cudaMemcpyAsync(j.d.uorder, ctx->up_pinned, order.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
     }
+    StripJob& S = strip_jobs[k];
+    S = StripJob{{j.d.craster[0], j.d.craster[1]},
+                 {j.log_form ? j.d.logs[0] : j.d.U, j.log_form ? j.d.logs[1] : j.d.V},
+                 {j.d.cblocks[0], j.d.cblocks[1]},
+                 {j.d.unpred[0], j.d.unpred[1]},
+                 {j.d.strip[0], j.d.strip[1]},
+                 j.h_nunpred,
+                 j.r1,
+                 j.r2,
+                 (unsigned)strips};
+    strips += strip_count(j.r1, j.r2);
+    hist_jobs[k] = HistJob{{j.d.craster[0], j.d.craster[1]}, {j.d.hist_codes[0], j.d.hist_codes[1]}, j.N, 0, 0};
     for (int f = 0; f < 2; f++) {
+      host(P.list)[2 * k + f] = HistList{j.d.hist_codes[f], j.h_list[f], j.h_nlist + f};
       WaveField& F = hf[2 * k + f];
       F.pair = j.d.pairs[f];
       F.codes = j.d.craster[f];
@@ -563,14 +573,17 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
       r1v[2 * k + f] = j.r1;
     }
   }
+  if (strips > 0x7fffffffu) return set_error(CPSZ_ERR_UNSUPPORTED, "fields of %zu strips", strips);
+  const unsigned hist_ctas = hist_assign_ctas(ctx->num_sms, hist_jobs.data(), nj);
   std::vector<WaveItem> items;
   build_wave_items(2 * nj, r1v.data(), items);
   if (g0 > 0) items.erase(std::remove_if(items.begin(), items.end(), [&](const WaveItem& w) { return w.group < g0; }),
                           items.end());
   const int n_items = (int)items.size();
-  CPSZ_CUDA_TRY(cudaMemcpyAsync(d_fields, hf.data(), hf.size() * sizeof(WaveField), cudaMemcpyHostToDevice, st));
-  CPSZ_CUDA_TRY(cudaMemcpyAsync(d_items, items.data(), n_items * sizeof(WaveItem), cudaMemcpyHostToDevice, st));
-  CPSZ_CUDA_TRY(cudaMemsetAsync(queue, 0, 64, st));
+  std::copy(hf.begin(), hf.end(), host(P.fields));
+  std::copy(items.begin(), items.end(), host(P.items));
+  std::copy(hist_jobs.begin(), hist_jobs.end(), host(P.hist));
+  std::copy(strip_jobs.begin(), strip_jobs.end(), host(P.strip));
   // A batch of device-resident fields derives its bounds in one bound-kernel
   // launch: every field's tiles in one grid (largest field first, so the
   // small fields' tiles fill the launch's tail), each CTA finding its field in
@@ -589,7 +602,7 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
     std::vector<int> by_size(nj);
     for (int k = 0; k < nj; k++) by_size[k] = k;
     std::stable_sort(by_size.begin(), by_size.end(), [&](int a, int b) { return jobs[a].N > jobs[b].N; });
-    std::vector<Eb2dJob> ebj;
+    Eb2dJob* ebj = host(P.eb);
     for (int k : by_size) {
       const Job2D& j = jobs[k];
       Eb2dJob e;
@@ -611,11 +624,24 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
         break;
       }
       eb_tiles += (int)t;
-      ebj.push_back(e);
+      *ebj++ = e;
     }
-    if (eb_batched)
-      CPSZ_CUDA_TRY(cudaMemcpyAsync(d_ebjobs, ebj.data(), nj * sizeof(Eb2dJob), cudaMemcpyHostToDevice, st));
   }
+  CPSZ_CUDA_TRY(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), st));
+  CPSZ_CUDA_TRY(cudaMemcpyAsync(P.image, h_image, P.image_bytes, cudaMemcpyHostToDevice, st));
+  if (g0 == 0) {
+    CPSZ_CUDA_TRY(cudaMemsetAsync(P.zero, 0, P.zero_bytes + P.gbnd_bytes, st));
+  } else {
+    const Job2D& j = jobs[0];
+    CPSZ_CUDA_TRY(cudaMemsetAsync(P.zero, 0, P.zero_bytes, st));
+    for (int f = 0; f < 2; f++)
+      CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.gbnd + ((size_t)f * j.ngroups + g0) * j.r2, 0,
+                                    (size_t)(j.ngroups - g0) * j.r2 * 8, st));
+  }
+  double* const thr_tab = P.thr;
+  int* const queue = P.queue;
+  const WaveField* const d_fields = P.fields;
+  const WaveItem* const d_items = P.items;
   size_t pass_points = 0;
   for (const Job2D& j : jobs) pass_points += j.N;
   // a wavefront launched beside its producer must be finished before this
@@ -668,7 +694,7 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
       CPSZ_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->ev[2], 0));
     }
     if (eb_batched)
-      CPSZ_TRY(launch_eb2d_batch(ctx, d_ebjobs, nj, eb_tiles, eb_shape, thr_tab, qt.n, qt.float_pow4));
+      CPSZ_TRY(launch_eb2d_batch(ctx, P.eb, nj, eb_tiles, eb_shape, thr_tab, qt.n, qt.float_pow4));
     for (Job2D& j : jobs) {
       // beside the wavefront, eb2d runs unit by unit in the order made in the
       // setup; band_units(g0, g1) is the slice for the rows of groups [g0, g1)
@@ -738,12 +764,13 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
           CPSZ_TRY(band_launch(c));
         }
       }
-      CPSZ_CUDA_TRY(cudaMemcpyAsync(j.h_hist_ids, j.d.hist_ids, 256 * 8, cudaMemcpyDeviceToHost, st));
     }
+    if (!(tap && tap->recon_only))
+      CPSZ_CUDA_TRY(cudaMemcpyAsync(jobs[0].h_hist_ids, P.hist_ids, nj * ID_HIST, cudaMemcpyDeviceToHost, st));
     CPSZ_CUDA_TRY(record(ctx->ev[0]));
     if (follow) {
       // the code histograms, counted on the second stream as the wavefront
-      // finishes its row groups; the flag and the histograms come back there
+      // finishes its row groups; the flag and the lists come back there
       Job2D& j = jobs[0];
       follow_drain.s = ctx->aux;
       CPSZ_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->ev[0], 0));
@@ -754,11 +781,12 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
       CPSZ_TRY(launch_hist_follow(ctx, codes, gd, j.r1, j.r2, hc, tix, (int*)(tix + 2), ctx->aux));
       CPSZ_CUDA_TRY(
           cudaMemcpyAsync(follow_flag_snapshot(ctx), tix + 2, sizeof(int), cudaMemcpyDeviceToHost, ctx->aux));
-      for (int f = 0; f < 2; f++) {
-        CPSZ_CUDA_TRY(cudaMemcpyAsync(j.h_hist_codes + (size_t)f * 65536, j.d.hist_codes[f], 65536 * 8,
-                                      cudaMemcpyDeviceToHost, ctx->aux));
-        CPSZ_CUDA_TRY(cudaEventRecord(ctx->job_ev[f], ctx->aux));
-      }
+      // on the high-priority stream: its two CTAs would otherwise wait for the
+      // block-order pass's tens of thousands (the host's trees start with them)
+      CPSZ_CUDA_TRY(cudaEventRecord(ctx->ev[6], ctx->aux));
+      CPSZ_CUDA_TRY(cudaStreamWaitEvent(ctx->hi, ctx->ev[6], 0));
+      CPSZ_TRY(launch_hist_list(ctx, P.list, 2, ctx->hi));
+      CPSZ_CUDA_TRY(cudaEventRecord(ctx->ev[6], ctx->hi));
     }
     if (tap && tap->ids)
       CPSZ_CUDA_TRY(cudaMemcpyAsync(tap->ids, jobs[0].d.ids, 2 * jobs[0].N, cudaMemcpyDeviceToDevice, st));
@@ -779,15 +807,9 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
     return CPSZ_OK;
   };
   auto count_codes = [&]() -> int {
-    for (int k = 0; k < nj; k++) {
-      Job2D& j = jobs[k];
-      CPSZ_TRY(launch_hist_u16_pair(ctx, j.d.craster[0], j.d.craster[1], j.N, j.d.hist_codes[0], j.d.hist_codes[1]));
-      for (int f = 0; f < 2; f++) {
-        CPSZ_CUDA_TRY(cudaMemcpyAsync(j.h_hist_codes + (size_t)f * 65536, j.d.hist_codes[f], 65536 * 8,
-                                      cudaMemcpyDeviceToHost, st));
-        CPSZ_CUDA_TRY(record(ctx->job_ev[2 * k + f]));
-      }
-    }
+    CPSZ_TRY(launch_hist_u16(ctx, hist_jobs.data(), P.hist, nj, hist_ctas));
+    CPSZ_TRY(launch_hist_list(ctx, P.list, 2 * nj, st));
+    CPSZ_CUDA_TRY(record(ctx->ev[6]));
     return CPSZ_OK;
   };
   bool hist_in_stage3 = !follow;
@@ -798,14 +820,7 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
     // them while the GPU converts to block order and gathers unpredictables);
     // a single field beside its bounds has them from the follower ----
     if (hist_in_stage3) CPSZ_TRY(count_codes());
-    for (int k = 0; k < nj; k++) {
-      Job2D& j = jobs[k];
-      const float* x[2] = {j.log_form ? j.d.logs[0] : j.d.U, j.log_form ? j.d.logs[1] : j.d.V};
-      CPSZ_TRY(launch_strip_pass(ctx, j.d.craster, j.r2, x, j.r2, j.r1, j.r2, j.d.cblocks, j.d.unpred, j.d.strip));
-      for (int f = 0; f < 2; f++)
-        CPSZ_CUDA_TRY(cudaMemcpyAsync(j.h_nunpred + f, strip_total(j.d.strip[f], j.r1, j.r2), 4,
-                                      cudaMemcpyDeviceToHost, st));
-    }
+    CPSZ_TRY(launch_strip_pass(ctx, strip_jobs.data(), P.strip, nj));
     CPSZ_CUDA_TRY(record(ctx->ev[5]));  // the unpredictable counts are on the host
     return CPSZ_OK;
   };
@@ -890,28 +905,21 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
     return d2h(ctx, dst, src, n, ctx->aux);
   };
   // Bit packing of stream k (0: ids, 1-2: codes of U / V).  A device blob gets
-  // the bits in place, at byte `at` (the sections around it are written later
+  // the bits in place, at byte `at` (the sections around it are written
   // byte by byte, and the packer ORs only zero bits into their bytes); host
   // output packs into a buffer of the stream's own that is copied out.
-  auto pack = [&](Job2D& j, int k, size_t at, HuffEntry* h_stage) -> int {
+  auto add_stream = [&](PackGroup& G, Job2D& j, int k, size_t at) {
     uint8_t* dst = j.host_out ? (uint8_t*)j.d.bits[k] : j.blob_base + at;
     const size_t room = j.host_out ? (k ? j.codes_bits_cap : j.ids_bits_cap) : j.blob_room - at;
-    const size_t mis = (uintptr_t)dst & 3;
-    CPSZ_CUDA_TRY(cudaMemsetAsync(dst, 0, j.bits_bytes[k], ctx->stream));
-    CPSZ_TRY(huff_upload(ctx, j.cb[k], h_stage, j.d.enc_ent[k], j.d.enc_code[k], j.d.enc_len[k]));
-    const HuffEncTable tab{j.d.enc_code[k], j.d.enc_len[k], k ? 65536 : 256};
-    uint32_t* w = (uint32_t*)(dst - mis);
-    if (k == 0)
-      return launch_huff_encode_u8(ctx, j.d.ids, j.log_form ? j.N : 2 * j.N, true, tab, w, room + mis, nullptr,
-                                   j.d.enc_tmp[0], (int)(8 * mis));
-    return launch_huff_encode_u16(ctx, j.d.cblocks[k - 1], j.N, tab, w, room + mis, nullptr, j.d.enc_tmp[k],
-                                  (int)(8 * mis));
+    G.add(j.cb[k], k ? (const void*)j.d.cblocks[k - 1] : (const void*)j.d.ids, k ? 2 : 1, k == 0, j.n_syms(k), dst,
+          j.bits_bytes[k], room, j.d.enc_code[k], j.d.enc_len[k], j.d.enc_tmp[k]);
   };
 
-  // host: the id trees (their histograms arrive with the bounds), and their
-  // bit packing on the aux stream as soon as the bounds are done: it runs
-  // beside the wavefront's tail, which leaves most SMs idle, and the main
-  // stream joins aux before the blob is finished
+  // host: the id trees (their histograms arrive with the bounds); a large
+  // field's ids are packed on the aux stream as soon as the bounds are done:
+  // that runs beside the wavefront's tail, which leaves most SMs idle, and the
+  // main stream joins aux before the blob is finished
+  const bool early_ids = nj == 1 && jobs[0].N >= EARLY_IDS_POINTS;
   auto tree_failure = [&]() {
     int fl = 0;
     CPSZ_TRY(read_flag(ctx, &fl));
@@ -920,41 +928,53 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
   };
   CPSZ_CUDA_TRY(cudaEventSynchronize(ctx->ev[0]));
   host_parallel_for(nj, [&](int k) { jobs[k].tree_ok[0] = huff_build(jobs[k].h_hist_ids, 256, 2048, &jobs[k].cb[0]); });
-  CPSZ_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->ev[0], 0));
-  aux_drain.s = ctx->aux;
   for (Job2D& j : jobs) {
     if (!j.tree_ok[0]) return tree_failure();
     j.sec_bytes[0] = huff_section_bytes(j.cb[0]);
     j.bits_bytes[0] = (j.cb[0].total_bits + 7) / 8;
     if (j.bits_bytes[0] + 8 > j.ids_bits_cap) return set_error(CPSZ_ERR_UNSUPPORTED, "Huffman stream larger than its bound");
+  }
+  if (early_ids) {
+    Job2D& j = jobs[0];
+    CPSZ_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->ev[0], 0));
+    aux_drain.s = ctx->aux;
+    // the setup image has been copied (ev[0] follows it), so its staging is
+    // free; the later uploads are staged behind these entries
+    CPSZ_TRY(upload_reserve(ctx, EARLY_UP));
+    UpImage up{(uint8_t*)ctx->up_pinned, P.up_ids, EARLY_UP};
+    PackGroup G;
+    add_stream(G, j, 0, ids_bits_at(j));
+    CPSZ_TRY(G.stage(up, ctx->num_sms));
     OnStream on_aux(ctx, ctx->aux);
-    CPSZ_TRY(pack(j, 0, ids_bits_at(j), j.h_ids_ent));
+    CPSZ_TRY(up.send(ctx->aux));
+    CPSZ_TRY(G.launch(ctx));
+    if (h_async) {
+      const size_t at = ids_bits_at(j);
+      if (at + j.bits_bytes[0] > j.host_cap)
+        return set_error(CPSZ_ERR_INVALID, "output capacity %zu too small for the blob", j.host_cap);
+      CPSZ_TRY(d2h(ctx, j.host_out + at, j.d.bits[0], j.bits_bytes[0], ctx->aux));
+    }
   }
-  if (h_async) {
-    const size_t at = ids_bits_at(*hj);
-    if (at + hj->bits_bytes[0] > hj->host_cap)
-      return set_error(CPSZ_ERR_INVALID, "output capacity %zu too small for the blob", hj->host_cap);
-    CPSZ_TRY(d2h(ctx, hj->host_out + at, hj->d.bits[0], hj->bits_bytes[0], ctx->aux));
-  }
-  // code trees, each as soon as its histogram is on the host
-  auto code_trees = [&]() {
+  // code trees, as soon as the histograms' lists are on the host
+  auto code_trees = [&]() -> int {
+    CPSZ_CUDA_TRY(cudaEventSynchronize(ctx->ev[6]));
     host_parallel_for(2 * nj, [&](int q) {
       Job2D& j = jobs[q / 2];
       const int f = q % 2;
-      j.tree_ok[1 + f] = cudaSetDevice(ctx->device) == cudaSuccess && cudaEventSynchronize(ctx->job_ev[q]) == cudaSuccess &&
-                         huff_build(j.h_hist_codes + (size_t)f * 65536, 65536, 131072, &j.cb[1 + f]);
+      j.tree_ok[1 + f] = huff_build_list(j.h_list[f], j.h_nlist[f], 65536, 131072, &j.cb[1 + f]);
     });
+    return CPSZ_OK;
   };
   if (follow) {
     // the follower's histograms; one that gave up (its wavefront was not
     // running beside it) leaves them to be counted here
-    CPSZ_CUDA_TRY(cudaEventSynchronize(ctx->job_ev[1]));
+    CPSZ_CUDA_TRY(cudaEventSynchronize(ctx->ev[6]));
     if (*(volatile int*)follow_flag_snapshot(ctx)) {
       for (int f = 0; f < 2; f++) CPSZ_CUDA_TRY(cudaMemsetAsync(jobs[0].d.hist_codes[f], 0, 65536 * 8, st));
       CPSZ_TRY(count_codes());
     }
   }
-  code_trees();
+  CPSZ_TRY(code_trees());
   if (overlap) {
     // The histograms are on the host, so is the flag snapshot taken before
     // them.  A wavefront wait that gave up (the bound kernel was held back
@@ -971,16 +991,19 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
         F.unit_done = nullptr;
         F.group_done = nullptr;
       }
-      CPSZ_CUDA_TRY(cudaMemcpyAsync(d_fields, hf.data(), hf.size() * sizeof(WaveField), cudaMemcpyHostToDevice, st));
+      CPSZ_CUDA_TRY(cudaMemcpyAsync(P.fields, hf.data(), hf.size() * sizeof(WaveField), cudaMemcpyHostToDevice, st));
       for (Job2D& j : jobs) {
         CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.gbnd, 0, 2 * (size_t)j.ngroups * j.r2 * 8, st));
-        for (int f = 0; f < 2; f++) CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.hist_codes[f], 0, 65536 * 8, st));
+        for (int f = 0; f < 2; f++) {
+          CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.hist_codes[f], 0, 65536 * 8, st));
+          CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.strip[f], 0, strip_scratch_bytes(j.r1, j.r2), st));
+        }
       }
       CPSZ_CUDA_TRY(cudaMemsetAsync(queue, 0, 64, st));
       CPSZ_TRY(launch_wave2d(ctx, false, d_fields, d_items, n_items, queue, pass_points));
       hist_in_stage3 = true;
       CPSZ_TRY(stage_3());
-      code_trees();
+      CPSZ_TRY(code_trees());
       ctx->wave_reruns++;
     }
   }
@@ -999,11 +1022,13 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
   }
   CPSZ_CUDA_TRY(cudaEventSynchronize(ctx->ev[5]));
   std::vector<BlobLayout> lay(nj);
+  size_t all_bytes = 0;
   for (int q = 0; q < nj; q++) {
     Job2D& j = jobs[q];
     j.n_unpred[0] = j.h_nunpred[0];
     j.n_unpred[1] = j.h_nunpred[1];
     CPSZ_TRY(job_layout(j, lay[q]));
+    all_bytes += lay[q].total;
     if (j.host_out) {
       if (lay[q].total > j.host_cap)
         return set_error(CPSZ_ERR_INVALID, "output capacity %zu < blob size %zu", j.host_cap, lay[q].total);
@@ -1011,22 +1036,16 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
       return set_error(CPSZ_ERR_UNSUPPORTED, "blob larger than its bound");
     }
   }
-  // page-locked staging of the pass's remaining uploads: code entries, and
-  // the device blobs' small pieces (no copy from it is in flight here)
-  // (each piece taken at a 16-byte boundary, as counted here)
-  size_t up_bytes = 0;
-  for (int q = 0; q < nj; q++)
-    up_bytes += align_up(jobs[q].cb[1].entries.size() * sizeof(HuffEntry), 16) +
-                align_up(jobs[q].cb[2].entries.size() * sizeof(HuffEntry), 16) +
-                (jobs[q].host_out ? 0 : align_up(assemble_upload_bytes(lay[q]), 16));
-  CPSZ_TRY(upload_reserve(ctx, up_bytes));
-  uint8_t* up_at = (uint8_t*)ctx->up_pinned;
-  uint8_t* const up_end = up_at + up_bytes;
-  auto up_take = [&](size_t n) -> uint8_t* {
-    uint8_t* p = up_at;
-    up_at += align_up(n, 16);
-    return up_at <= up_end ? p : nullptr;
-  };
+  // every size is known now: blobs with room in the caller's device memory are
+  // built there (8 bytes over: the packers touch the last word of a stream)
+  if (!early_ids && dev_at && all_bytes + 8 <= dev_room) {
+    size_t at = 0;
+    for (int q = 0; q < nj; q++) {
+      jobs[q].blob_base = dev_at + at;
+      jobs[q].blob_room = dev_room - at;
+      at += lay[q].total;
+    }
+  }
   if (hj) {
     const BlobLayout& hl = lay[0];
     for (const BlobLayout::Piece& pc : hl.pieces) {
@@ -1037,36 +1056,65 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
       for (int f = 0; f < 2; f++) {
         CPSZ_TRY(d2h_beside(hj->host_out + hl.unpred_dst[f], hj->d.unpred[f], 4 * hj->n_unpred[f]));
         if (hl.sign_bytes)
-          CPSZ_TRY(d2h_beside(hj->host_out + hl.sign_dst + f * hl.sign_bytes, hj->d_signs[f], hl.sign_bytes));
+          CPSZ_TRY(d2h_beside(hj->host_out + hl.sign_dst + f * hl.sign_bytes, hj->d.signs[f], hl.sign_bytes));
       }
   }
-  for (int q = 0; q < nj; q++) {
-    Job2D& j = jobs[q];
-    for (int k = 1; k < 3; k++) {
-      HuffEntry* h_stage = (HuffEntry*)up_take(j.cb[k].entries.size() * sizeof(HuffEntry));
-      if (!h_stage) return set_error(CPSZ_ERR_INVALID, "internal: upload staging overrun");
-      CPSZ_TRY(pack(j, k, lay[q].bit_dst[k], h_stage));
-      if (h_async) CPSZ_TRY(d2h_beside(j.host_out + lay[q].bit_dst[k], j.d.bits[k], j.bits_bytes[k]));
+  // The streams still to be packed, in one launch; or, to page-locked host
+  // output, one by one, each copied out while the next is packed.
+  const int k_first = early_ids ? 1 : 0;
+  std::vector<PackGroup> groups(h_async ? 3 - k_first : 1);
+  for (int q = 0; q < nj; q++)
+    for (int k = k_first; k < 3; k++) add_stream(groups[h_async ? k - k_first : 0], jobs[q], k, lay[q].bit_dst[k]);
+  // page-locked staging of the pass's remaining uploads, behind the early id
+  // entries' (whose copy may still be in flight)
+  const size_t early_up = early_ids ? align_up(EARLY_UP, 256) : 0;
+  size_t up_bytes = 1024;
+  for (const PackGroup& G : groups) up_bytes += G.up_bytes();
+  for (const BlobLayout& L : lay) up_bytes += piece_up_bytes(L);
+  if (up_bytes > P.up_bytes) return set_error(CPSZ_ERR_INVALID, "internal: uploads exceed their bound");
+  if (early_ids && ctx->up_cap < early_up + up_bytes) CPSZ_CUDA_TRY(cudaStreamSynchronize(ctx->aux));
+  CPSZ_TRY(upload_reserve(ctx, early_up + up_bytes));
+  UpImage up{(uint8_t*)ctx->up_pinned + early_up, P.up, up_bytes};
+  for (PackGroup& G : groups) CPSZ_TRY(G.stage(up, ctx->num_sms));
+  // the rest of a device blob (header, trees, unpredictable values, sign
+  // maps): uploaded with the entries, or, for a large field, staged once the
+  // packers are running
+  std::vector<CopyPiece> pieces;
+  uint8_t* d_pieces = nullptr;
+  unsigned piece_ctas = 0;
+  auto stage_pieces = [&]() -> int {
+    for (int q = 0; q < nj; q++) CPSZ_TRY(job_pieces(jobs[q], lay[q], up, pieces));
+    piece_ctas = assign_piece_chunks(pieces.data(), pieces.size());
+    uint8_t* h = up.take(pieces.size() * sizeof(CopyPiece), &d_pieces);
+    if (!h) return up_overrun();
+    memcpy(h, pieces.data(), pieces.size() * sizeof(CopyPiece));
+    return CPSZ_OK;
+  };
+  if (!hj && !early_ids) CPSZ_TRY(stage_pieces());
+  CPSZ_TRY(up.send(st));
+  for (size_t g = 0; g < groups.size(); g++) {
+    CPSZ_TRY(groups[g].launch(ctx));
+    if (h_async) {
+      const int k = k_first + (int)g;
+      CPSZ_TRY(d2h_beside(hj->host_out + lay[0].bit_dst[k], hj->d.bits[k], hj->bits_bytes[k]));
     }
   }
   if (aux_drain.s) {  // the aux stream's work (id packing, section copies) joins the main stream
     CPSZ_CUDA_TRY(cudaEventRecord(ctx->ev[7], ctx->aux));
     CPSZ_CUDA_TRY(cudaStreamWaitEvent(st, ctx->ev[7], 0));
   }
-  // ---- stage 5: the rest of a device blob (header, trees, unpredictable
-  // values, sign maps), enqueued behind the packers, or, for host output
-  // without page-locked memory, the sections not yet copied ----
+  // ---- stage 5: the rest of a device blob, or, for host output without
+  // page-locked memory, the sections not yet copied ----
   mark(ctx, "blob_assembly");
   int assembled = CPSZ_OK;
-  if (!hj)
-    for (int q = 0; q < nj; q++) {
-      uint8_t* h_up = up_take(assemble_upload_bytes(lay[q]));
-      if (!h_up) {
-        assembled = set_error(CPSZ_ERR_INVALID, "internal: upload staging overrun");
-        break;
-      }
-      if ((assembled = job_assemble(ctx, jobs[q], lay[q], h_up)) != CPSZ_OK) break;
+  if (!hj) {
+    if (early_ids) {
+      assembled = stage_pieces();
+      if (assembled == CPSZ_OK) assembled = up.send(st);
     }
+    if (assembled == CPSZ_OK)
+      assembled = launch_copy_pieces(ctx, (const CopyPiece*)d_pieces, (int)pieces.size(), piece_ctas);
+  }
   {
     int flag = 0;
     CPSZ_TRY(read_flag(ctx, &flag));  // synchronizes the stream; a kernel's error outranks the assembly's
@@ -1080,7 +1128,7 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
       for (int f = 0; f < 2; f++) {
         CPSZ_TRY(d2h(ctx, hj->host_out + hl.unpred_dst[f], hj->d.unpred[f], 4 * hj->n_unpred[f], st));
         if (hl.sign_bytes)
-          CPSZ_TRY(d2h(ctx, hj->host_out + hl.sign_dst + f * hl.sign_bytes, hj->d_signs[f], hl.sign_bytes, st));
+          CPSZ_TRY(d2h(ctx, hj->host_out + hl.sign_dst + f * hl.sign_bytes, hj->d.signs[f], hl.sign_bytes, st));
       }
       for (int k = 1; k < 3; k++) CPSZ_TRY(d2h(ctx, hj->host_out + hl.bit_dst[k], hj->d.bits[k], hj->bits_bytes[k], st));
     }
@@ -1100,17 +1148,13 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap) 
   return CPSZ_OK;
 }
 
-size_t pass_bytes(const std::vector<Job2D>& jobs) {
-  size_t bytes = 0;
-  int total_groups = 0;
-  for (const Job2D& j : jobs) {
-    bytes += job_bytes(j);
-    total_groups += j.ngroups;
-  }
-  bytes += align_up(QUANT_TAB_MAX * 8, 256) + 256 + 512 + align_up(2 * jobs.size() * sizeof(WaveField), 256) + 256 +
-           align_up(2 * (size_t)total_groups * sizeof(WaveItem), 256) + 256 + align_up(jobs.size() * sizeof(Eb2dJob), 256) +
-           256;
-  return bytes;
+// Workspace and page-locked staging of a pass (its pieces are placed by run_pass).
+int pass_reserve(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs) {
+  PassBuf P{};
+  Alloc count{nullptr};
+  pass_alloc(jobs, P, count);
+  CPSZ_TRY(arena_reserve(ctx, count.bytes));
+  return pinned_reserve(ctx, PINNED_BASE + jobs.size() * (ID_HIST + JOB_PINNED));
 }
 
 }  // namespace
@@ -1141,9 +1185,8 @@ int compress_2d(cpsz_b200_ctx* ctx, const float* U_in, const float* V_in, size_t
     jobs[0].host_out = host_out;
     jobs[0].host_cap = host_cap;
   }
-  CPSZ_TRY(arena_reserve(ctx, pass_bytes(jobs)));
-  CPSZ_TRY(pinned_reserve(ctx, PINNED_BASE + JOB_PINNED));
-  CPSZ_TRY(run_pass(ctx, jobs, tap));
+  CPSZ_TRY(pass_reserve(ctx, jobs));
+  CPSZ_TRY(run_pass(ctx, jobs, tap, jobs[0].dev_out, jobs[0].dev_cap));
   out->d_blob = jobs[0].host_out ? nullptr : jobs[0].blob_base;
   out->size = jobs[0].size;
   out->n_unpred[0] = jobs[0].n_unpred[0];
@@ -1172,14 +1215,13 @@ int compress_2d_batch(cpsz_b200_ctx* ctx, int n, const float* const* U, const fl
       jobs.push_back(std::move(j));
       k++;
     }
-    CPSZ_TRY(arena_reserve(ctx, pass_bytes(jobs)));
-    CPSZ_TRY(pinned_reserve(ctx, PINNED_BASE + jobs.size() * JOB_PINNED));
-    CPSZ_TRY(run_pass(ctx, jobs, nullptr));
+    CPSZ_TRY(pass_reserve(ctx, jobs));
+    CPSZ_TRY(run_pass(ctx, jobs, nullptr, dev_out && at < out_cap ? out + at : nullptr, at < out_cap ? out_cap - at : 0));
     for (size_t q = 0; q < jobs.size(); q++) {
       const Job2D& j = jobs[q];
       if (at + j.size > out_cap)
         return set_error(CPSZ_ERR_INVALID, "output capacity %zu < %zu bytes of blobs", out_cap, at + j.size);
-      CPSZ_TRY(d2h(ctx, out + at, j.blob_base, j.size, ctx->stream));
+      if (j.blob_base != out + at) CPSZ_TRY(d2h(ctx, out + at, j.blob_base, j.size, ctx->stream));
       at += j.size;
       offsets[k0 + q + 1] = at;
     }
@@ -1398,9 +1440,7 @@ int decompress_2d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
       const uint8_t* idf[2] = {ids, log_form ? ids : ids + N};
       const float* un[2] = {(const float*)(d_up + up_unpred[0]), (const float*)(d_up + up_unpred[1])};
       const unsigned long long nun[2] = {fv[0].n_unpred, fv[1].n_unpred};
-      CPSZ_TRY(launch_strip_unpass(ctx, cb, idf, un, nun, r1, r2, raw, strip, log_form ? 1 : 2));
-      for (int f = 0; f < 2; f++)
-        CPSZ_CUDA_TRY(cudaMemcpyAsync(h_cnt + f, strip_total(strip[f], r1, r2), 4, cudaMemcpyDeviceToHost, st));
+      CPSZ_TRY(launch_strip_unpass(ctx, cb, idf, un, nun, r1, r2, raw, strip, h_cnt, log_form ? 1 : 2));
     }
     // ---- wavefront ----
     mark(ctx, "wave2d_decompress");

@@ -22,6 +22,7 @@
 
 #include "huffman_host.h"
 #include "kernels.h"
+#include "pack_group.h"
 #include "transfer.h"
 #include "pipeline.h"
 
@@ -58,7 +59,7 @@ int check_dims(size_t r1, size_t r2, size_t r3) {
 }  // namespace
 
 int compress_3d(cpsz_b200_ctx* ctx, const float* U_in, const float* V_in, const float* W_in, size_t r1s, size_t r2s,
-                size_t r3s, double max_pwr_eb, Blob3D* out) {
+                size_t r3s, double max_pwr_eb, Blob3D* out, unsigned char* dev_out, size_t dev_cap) {
   if (!U_in || !V_in || !W_in) return set_error(CPSZ_ERR_INVALID, "null input field");
   CPSZ_TRY(check_dims(r1s, r2s, r3s));
   if (max_pwr_eb != max_pwr_eb) return set_error(CPSZ_ERR_INVALID, "max_pwr_eb is NaN");
@@ -85,20 +86,19 @@ int compress_3d(cpsz_b200_ctx* ctx, const float* U_in, const float* V_in, const 
   add(12 * N);         // unpredictable triples
   add(3 * sign_words * 4);
   add(wave3d_scratch_bytes(r1, r2));
-  add(256 * 8);
-  add(65536 * 8);
-  add(QUANT_TAB_MAX * 8);
+  // zeroed in one piece: both histograms, the packers' look-back words
+  const size_t tmp_ids = align_up(huff_encode_tmp_bytes(N), 256);
+  const size_t zero_bytes = 256 * 8 + 65536 * 8 + tmp_ids + huff_encode_tmp_bytes(3 * N);
+  add(zero_bytes);
+  const size_t image_bytes = QUANT_TAB_MAX * 8 + sizeof(HistList);
+  add(image_bytes);
   add(256 * 9);
   add(65536 * 9);
-  add(256 * sizeof(HuffEntry));
-  add(std::min<size_t>(65536, 3 * N + 1) * sizeof(HuffEntry));
-  add(huff_encode_tmp_bytes(N));
-  add(huff_encode_tmp_bytes(3 * N));
+  const size_t syms = std::min<size_t>(65536, 3 * N + 1), tree = 12 + 13 * std::min<size_t>(131072, 2 * syms) + 8;
+  const size_t up_cap = (256 + syms) * sizeof(HuffEntry) + tree + 12 + 13 * 512 + 4096;
+  add(up_cap);
   const size_t ids_bits_cap = (N * 8 + 7) / 8 + 64;
   const size_t codes_bits_cap = (3 * N * 17 + 7) / 8 + 64;
-  add(ids_bits_cap);
-  add(codes_bits_cap);
-  add(64);
   const size_t blob_cap = 8 + 3 * smap + 8 + 12 * N + 8 + 8 + 2 * (12 + 13 * 131072 + 8) + ids_bits_cap +
                           codes_bits_cap + 4096;
   add(blob_cap);
@@ -131,25 +131,32 @@ int compress_3d(cpsz_b200_ctx* ctx, const float* U_in, const float* V_in, const 
   float* unpred = (float*)A(12 * N);
   uint32_t* signs = (uint32_t*)A(3 * sign_words * 4);
   void* wave_sync = A(wave3d_scratch_bytes(r1, r2));
-  unsigned long long* hist_ids = (unsigned long long*)A(256 * 8);
-  unsigned long long* hist_codes = (unsigned long long*)A(65536 * 8);
-  double* thr_tab = (double*)A(QUANT_TAB_MAX * 8);
+  uint8_t* zero = (uint8_t*)A(zero_bytes);
+  unsigned long long* hist_ids = (unsigned long long*)zero;
+  unsigned long long* hist_codes = hist_ids + 256;
+  unsigned long long* enc_tmp[2] = {hist_codes + 65536,
+                                    (unsigned long long*)((uint8_t*)(hist_codes + 65536) + tmp_ids)};
+  uint8_t* image = (uint8_t*)A(image_bytes);
+  double* thr_tab = (double*)image;
+  HistList* d_list = (HistList*)(thr_tab + QUANT_TAB_MAX);
   unsigned long long* enc_code[2] = {(unsigned long long*)A(256 * 8), (unsigned long long*)A(65536 * 8)};
   uint8_t* enc_len[2] = {(uint8_t*)A(256), (uint8_t*)A(65536)};
-  HuffEntry* enc_ent[2] = {(HuffEntry*)A(256 * sizeof(HuffEntry)),
-                           (HuffEntry*)A(std::min<size_t>(65536, 3 * N + 1) * sizeof(HuffEntry))};
-  void* enc_tmp[2] = {A(huff_encode_tmp_bytes(N)), A(huff_encode_tmp_bytes(3 * N))};
-  uint32_t* bits[2] = {(uint32_t*)A(ids_bits_cap), (uint32_t*)A(codes_bits_cap)};
-  (void)A(64);
+  uint8_t* d_up = (uint8_t*)A(up_cap);
   uint8_t* blob = (uint8_t*)A(blob_cap);
   if (!blob) return set_error(CPSZ_ERR_NOMEM, "workspace layout overflow");
 
   reset_marks(ctx);
   mark(ctx, "h2d+setup");
+  unsigned* h_npred = (unsigned*)ctx->pinned + 4;  // the flag word lives at offset 0
+  unsigned* h_nlist = h_npred + 1;
+  unsigned long long* h_hist_ids = (unsigned long long*)ctx->pinned + 8;
+  unsigned long long* h_list = h_hist_ids + 256;
+  CPSZ_TRY(upload_reserve(ctx, image_bytes));
+  memcpy(ctx->up_pinned, qt.t, QUANT_TAB_MAX * 8);
+  *(HistList*)((double*)ctx->up_pinned + QUANT_TAB_MAX) = HistList{hist_codes, h_list, h_nlist};
   CPSZ_CUDA_TRY(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), st));
-  CPSZ_CUDA_TRY(cudaMemsetAsync(hist_ids, 0, 256 * 8, st));
-  CPSZ_CUDA_TRY(cudaMemsetAsync(hist_codes, 0, 65536 * 8, st));
-  CPSZ_CUDA_TRY(cudaMemcpyAsync(thr_tab, qt.t, QUANT_TAB_MAX * 8, cudaMemcpyHostToDevice, st));
+  CPSZ_CUDA_TRY(cudaMemsetAsync(zero, 0, zero_bytes, st));
+  CPSZ_CUDA_TRY(cudaMemcpyAsync(image, ctx->up_pinned, image_bytes, cudaMemcpyHostToDevice, st));
   mark(ctx, "eb3d");
   CPSZ_TRY(launch_eb3d(ctx, dU, dV, dW, r1, r2, r3, max_pwr_eb, thr_tab, qt.n, ids));
   mark(ctx, "log3d");
@@ -163,11 +170,8 @@ int compress_3d(cpsz_b200_ctx* ctx, const float* U_in, const float* V_in, const 
   // are never 0 (|q| <= 32767 around 32768), an unpredictable point's are,
   // and so is every fourth lane, so the count without symbol 0 is the
   // compacted codes' histogram.
-  unsigned* h_npred = (unsigned*)ctx->pinned + 4;  // the flag word lives at offset 0
-  unsigned long long* h_hist_ids = (unsigned long long*)ctx->pinned + 8;
-  unsigned long long* h_hist_codes = h_hist_ids + 256;
   CPSZ_TRY(launch_hist_u16_nonzero(ctx, reinterpret_cast<const uint16_t*>(codes), 4 * N, hist_codes));
-  CPSZ_CUDA_TRY(cudaMemcpyAsync(h_hist_codes, hist_codes, 65536 * 8, cudaMemcpyDeviceToHost, st));
+  CPSZ_TRY(launch_hist_list(ctx, d_list, 1, st));
   CPSZ_CUDA_TRY(cudaEventRecord(ctx->ev[1], st));
   CPSZ_TRY(launch_chunk_count_3d(ctx, true, codes, N, chunk_cnt));
   CPSZ_TRY(launch_scan_u32(ctx, chunk_cnt, chunk_off, nchunks, scan_tmp));
@@ -177,10 +181,11 @@ int compress_3d(cpsz_b200_ctx* ctx, const float* U_in, const float* V_in, const 
   mark(ctx, "host_trees");
   HuffCodebook cb[2];
   CPSZ_CUDA_TRY(cudaEventSynchronize(ctx->ev[1]));
-  bool any_code = false;
-  for (size_t s = 1; s < 65536 && !any_code; s++) any_code = h_hist_codes[s] != 0;
-  if (!any_code) h_hist_codes[0] = 1;  // no predictable point: one-leaf tree of symbol 0, no bits
-  if (!huff_build(h_hist_codes, 65536, 131072, &cb[1])) return CPSZ_ERR_INVALID;
+  if (*h_nlist == 0) {  // no predictable point: one-leaf tree of symbol 0, no bits
+    h_list[0] = 1;
+    *h_nlist = 1;
+  }
+  if (!huff_build_list(h_list, *h_nlist, 65536, 131072, &cb[1])) return CPSZ_ERR_INVALID;
   CPSZ_CUDA_TRY(cudaStreamSynchronize(st));
   int flag = 0;
   CPSZ_TRY(read_flag3(ctx, &flag));
@@ -189,79 +194,75 @@ int compress_3d(cpsz_b200_ctx* ctx, const float* U_in, const float* V_in, const 
   const size_t n_codes = 3 * n_pred, n_unpred = 3 * (N - n_pred);
   if (!huff_build(h_hist_ids, 256, 512, &cb[0])) return CPSZ_ERR_INVALID;
 
+  // ---- blob layout, then the streams packed in place (the caller's device
+  // buffer if it has room: 8 bytes over, the packers touch a stream's last
+  // word), the rest copied behind them ----
   mark(ctx, "huffman_encode");
   const size_t sec_bytes[2] = {huff_section_bytes(cb[0]), huff_section_bytes(cb[1])};
   const size_t bits_bytes[2] = {(cb[0].total_bits + 7) / 8, (cb[1].total_bits + 7) / 8};
   if (bits_bytes[0] + 8 > ids_bits_cap || bits_bytes[1] + 8 > codes_bits_cap)
     return set_error(CPSZ_ERR_UNSUPPORTED, "Huffman stream larger than its bound");
-  for (int k = 0; k < 2; k++) {
-    CPSZ_TRY(huff_upload(ctx, cb[k], nullptr, enc_ent[k], enc_code[k], enc_len[k]));
-    CPSZ_CUDA_TRY(cudaMemsetAsync(bits[k], 0, align_up(bits_bytes[k], 4) + 8, st));
-  }
-  CPSZ_TRY(launch_huff_encode_u8(ctx, ids, N, false, HuffEncTable{enc_code[0], enc_len[0], 256}, bits[0],
-                                 ids_bits_cap, nullptr, enc_tmp[0]));
-  if (n_codes)
-    CPSZ_TRY(launch_huff_encode_u16(ctx, codes_out, n_codes, HuffEncTable{enc_code[1], enc_len[1], 65536}, bits[1],
-                                    codes_bits_cap, nullptr, enc_tmp[1]));
-
-  mark(ctx, "blob_assembly");
   const size_t total = 8 + 3 * smap + 8 + 4 * n_unpred + 8 + sec_bytes[0] + 8 + sec_bytes[1];
   if (total > blob_cap) return set_error(CPSZ_ERR_UNSUPPORTED, "blob larger than its bound");
-  std::vector<uint8_t> small;
-  struct Piece {
-    size_t dst, src, n;
-  };
-  std::vector<Piece> pieces;
-  auto stage = [&](size_t dst, const void* p, size_t n) {
-    pieces.push_back(Piece{dst, small.size(), n});
-    small.insert(small.end(), (const uint8_t*)p, (const uint8_t*)p + n);
+  size_t room = blob_cap;
+  if (dev_out && total + 8 <= dev_cap) {
+    blob = dev_out;
+    room = dev_cap;
+  }
+  // (the setup image has been copied: its staging is free)
+  CPSZ_TRY(upload_reserve(ctx, up_cap));
+  UpImage up{(uint8_t*)ctx->up_pinned, d_up, up_cap};
+  std::vector<CopyPiece> pieces;
+  auto stage = [&](size_t dst, const void* p, size_t n) -> int {
+    uint8_t* dev;
+    uint8_t* h = up.take(n, &dev);
+    if (!h) return up_overrun();
+    memcpy(h, p, n);
+    pieces.push_back(CopyPiece{blob + dst, dev, n, 0});
+    return CPSZ_OK;
   };
   size_t at = 0;
   const int hdr[2] = {2, 32768};
-  stage(at, hdr, 8);
+  CPSZ_TRY(stage(at, hdr, 8));
   at += 8;
-  const size_t sign_at = at;
-  at += 3 * smap;
+  for (int c = 0; c < 3; c++, at += smap)
+    pieces.push_back(CopyPiece{blob + at, (const uint8_t*)(signs + c * sign_words), smap, 0});
   unsigned long long v64 = n_unpred;
-  stage(at, &v64, 8);
+  CPSZ_TRY(stage(at, &v64, 8));
   at += 8;
-  const size_t unpred_at = at;
+  if (n_unpred) pieces.push_back(CopyPiece{blob + at, (const uint8_t*)unpred, 4 * n_unpred, 0});
   at += 4 * n_unpred;
   v64 = N;
-  stage(at, &v64, 8);
+  CPSZ_TRY(stage(at, &v64, 8));
   at += 8;
-  size_t bit_at[2];
+  PackGroup G;
   for (int k = 0; k < 2; k++) {
     if (k == 1) {
       v64 = n_codes;
-      stage(at, &v64, 8);
+      CPSZ_TRY(stage(at, &v64, 8));
       at += 8;
     }
-    stage(at, cb[k].tree_bytes.data(), cb[k].tree_bytes.size());
+    CPSZ_TRY(stage(at, cb[k].tree_bytes.data(), cb[k].tree_bytes.size()));
     at += cb[k].tree_bytes.size();
     unsigned long long nb = bits_bytes[k];
-    stage(at, &nb, 8);
+    CPSZ_TRY(stage(at, &nb, 8));
     at += 8;
-    bit_at[k] = at;
+    if (k == 0 || n_codes)
+      G.add(cb[k], k ? (const void*)codes_out : (const void*)ids, k ? 2 : 1, false, k ? n_codes : N, blob + at,
+            bits_bytes[k], room - at, enc_code[k], enc_len[k], enc_tmp[k]);
     at += bits_bytes[k];
   }
   if (at != total) return set_error(CPSZ_ERR_INVALID, "internal: blob layout mismatch (%zu != %zu)", at, total);
-  uint8_t* d_small = blob + align_up(total, 256);
-  if (align_up(total, 256) + small.size() > blob_cap) {
-    for (const Piece& p : pieces)
-      CPSZ_CUDA_TRY(cudaMemcpyAsync(blob + p.dst, small.data() + p.src, p.n, cudaMemcpyHostToDevice, st));
-  } else {
-    CPSZ_CUDA_TRY(cudaMemcpyAsync(d_small, small.data(), small.size(), cudaMemcpyHostToDevice, st));
-    for (const Piece& p : pieces)
-      CPSZ_CUDA_TRY(cudaMemcpyAsync(blob + p.dst, d_small + p.src, p.n, cudaMemcpyDeviceToDevice, st));
-  }
-  for (int c = 0; c < 3; c++)
-    CPSZ_CUDA_TRY(cudaMemcpyAsync(blob + sign_at + c * smap, signs + c * sign_words, smap, cudaMemcpyDeviceToDevice, st));
-  if (n_unpred)
-    CPSZ_CUDA_TRY(cudaMemcpyAsync(blob + unpred_at, unpred, 4 * n_unpred, cudaMemcpyDeviceToDevice, st));
-  for (int k = 0; k < 2; k++)
-    if (bits_bytes[k])
-      CPSZ_CUDA_TRY(cudaMemcpyAsync(blob + bit_at[k], bits[k], bits_bytes[k], cudaMemcpyDeviceToDevice, st));
+  CPSZ_TRY(G.stage(up, ctx->num_sms));
+  const unsigned piece_ctas = assign_piece_chunks(pieces.data(), pieces.size());
+  uint8_t* d_pieces;
+  uint8_t* h_pieces = up.take(pieces.size() * sizeof(CopyPiece), &d_pieces);
+  if (!h_pieces) return up_overrun();
+  memcpy(h_pieces, pieces.data(), pieces.size() * sizeof(CopyPiece));
+  CPSZ_TRY(up.send(st));
+  CPSZ_TRY(G.launch(ctx));
+  mark(ctx, "blob_assembly");
+  CPSZ_TRY(launch_copy_pieces(ctx, (const CopyPiece*)d_pieces, (int)pieces.size(), piece_ctas));
   mark(ctx, "end");
   CPSZ_TRY(read_flag3(ctx, &flag));
   if (flag) return flag_error3(flag);

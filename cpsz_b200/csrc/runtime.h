@@ -93,9 +93,6 @@ struct cpsz_b200_ctx {
   // chunked host-to-device uploads (one event per chunk, recorded on `aux`)
   static constexpr int kUploadChunks = 32;
   cudaEvent_t up_ev[kUploadChunks] = {};
-  // per (field, component) "histogram on the host" events of a compression pass
-  static constexpr int kJobEvents = 64;
-  cudaEvent_t job_ev[kJobEvents] = {};
   cpsz::Arena arena;
   // pinned ring for bulk copies of pageable host memory (transfer.h)
   static constexpr int kStageSlots = 4;
