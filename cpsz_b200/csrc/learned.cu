@@ -194,13 +194,14 @@ int compress_2d_learned(cpsz_b200_ctx* ctx, cpsz_b200_mlp* mlp, const float* U_i
   const size_t N = r1s * r2s, ncell = 2 * (r1s - 1) * (r2s - 1);
   cudaStream_t st = ctx->stream;
   const bool dev_in = is_device_ptr(U_in) && is_device_ptr(V_in);
-  // workspace of the loop (the compressor's own arena is reused by every pass)
-  DevMem mem;
+  // workspace of the loop (the compressor's own arena is reused by every
+  // pass), kept by the context: a cudaMalloc and cudaFree per call wait for
+  // the device and cost 1 to 10 ms
   const size_t bytes = align_up(8 * N, 256) * 2 + align_up(QUANT_TAB_MAX * 8, 256) + align_up(4 * N, 256) * 3 +
                        align_up(2 * N, 256) +
                        align_up(ncell, 256) * 2 + align_up(N, 256) * 2 + 4096 + (dev_in ? 0 : align_up(8 * N, 256));
-  CPSZ_TRY(mem.alloc(bytes));
-  uint8_t* w = (uint8_t*)mem.p;
+  CPSZ_TRY(loop_reserve(ctx, bytes));
+  uint8_t* w = (uint8_t*)ctx->loop_mem;
   auto take = [&](size_t b) {
     void* p = w;
     w += align_up(b, 256);

@@ -248,6 +248,25 @@ int pinned_reserve(cpsz_b200_ctx* ctx, size_t bytes) {
   return CPSZ_OK;
 }
 
+int loop_reserve(cpsz_b200_ctx* ctx, size_t bytes) {
+  if (ctx->loop_cap >= bytes) return CPSZ_OK;
+  if (ctx->loop_mem) {
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(ctx->loop_mem);
+    ctx->loop_mem = nullptr;
+    ctx->loop_cap = 0;
+  }
+  bytes = align_up(bytes, 1 << 20);
+  cudaError_t e = cudaMalloc(&ctx->loop_mem, bytes);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    ctx->loop_mem = nullptr;
+    return set_error(CPSZ_ERR_NOMEM, "device workspace of %zu bytes: %s", bytes, cudaGetErrorString(e));
+  }
+  ctx->loop_cap = bytes;
+  return CPSZ_OK;
+}
+
 int upload_reserve(cpsz_b200_ctx* ctx, size_t bytes) {
   if (ctx->up_cap >= bytes) return CPSZ_OK;
   if (ctx->up_pinned) cudaFreeHost(ctx->up_pinned);
@@ -338,6 +357,7 @@ int cpsz_b200_ctx_destroy(cpsz_b200_ctx* c) {
   if (c->hi) cudaStreamSynchronize(c->hi);
   for (auto& g : c->pass_graphs) cudaGraphExecDestroy(g.exec);
   if (c->arena.base) cudaFree(c->arena.base);
+  if (c->loop_mem) cudaFree(c->loop_mem);
   if (c->pinned) cudaFreeHost(c->pinned);
   if (c->up_pinned) cudaFreeHost(c->up_pinned);
   if (c->stage) cudaFreeHost(c->stage);

@@ -94,6 +94,9 @@ struct cpsz_b200_ctx {
   static constexpr int kUploadChunks = 32;
   cudaEvent_t up_ev[kUploadChunks] = {};
   cpsz::Arena arena;
+  // workspace of the learned bounds' loop, beside the arena its passes use
+  void* loop_mem = nullptr;
+  size_t loop_cap = 0;
   // pinned ring for bulk copies of pageable host memory (transfer.h)
   static constexpr int kStageSlots = 4;
   static constexpr size_t kStageBytes = (size_t)16 << 20;
@@ -140,6 +143,8 @@ int arena_reserve(cpsz_b200_ctx* ctx, size_t bytes);
 void* arena_alloc(cpsz_b200_ctx* ctx, size_t bytes);
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 int pinned_reserve(cpsz_b200_ctx* ctx, size_t bytes);
+// Grows ctx->loop_mem to at least `bytes`.
+int loop_reserve(cpsz_b200_ctx* ctx, size_t bytes);
 // Grows ctx->up_pinned to at least `bytes` (its old contents are dropped:
 // call it only when no copy from it is in flight).
 int upload_reserve(cpsz_b200_ctx* ctx, size_t bytes);
