@@ -758,8 +758,8 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap, 
         for (int c = 0; c < nch; c++) {
           const size_t off = (size_t)c * R * j.r2;
           const size_t cnt = (size_t)(std::min(j.r1, (c + 1) * R + 1) - c * R) * j.r2;
-          CPSZ_CUDA_TRY(cudaMemcpyAsync(j.d.U + off, j.U_in + off, 4 * cnt, cudaMemcpyHostToDevice, ctx->aux));
-          CPSZ_CUDA_TRY(cudaMemcpyAsync(j.d.V + off, j.V_in + off, 4 * cnt, cudaMemcpyHostToDevice, ctx->aux));
+          CPSZ_TRY(h2d(ctx, j.d.U + off, j.U_in + off, 4 * cnt, ctx->aux));
+          CPSZ_TRY(h2d(ctx, j.d.V + off, j.V_in + off, 4 * cnt, ctx->aux));
           CPSZ_CUDA_TRY(cudaEventRecord(ctx->up_ev[c], ctx->aux));
           CPSZ_TRY(band_launch(c));
         }

@@ -98,8 +98,9 @@ struct cpsz_b200_ctx {
   void* loop_mem = nullptr;
   size_t loop_cap = 0;
   // pinned ring for bulk copies of pageable host memory (transfer.h)
-  static constexpr int kStageSlots = 4;
-  static constexpr size_t kStageBytes = (size_t)16 << 20;
+  static constexpr int kStageSlots = 32;
+  static constexpr size_t kStageBytes = (size_t)2 << 20;
+  int stage_pos = 0;  // the next copy's first slot
   void* stage = nullptr;
   cudaEvent_t stage_ev[kStageSlots] = {};
   void* pinned = nullptr;
