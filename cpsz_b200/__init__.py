@@ -495,14 +495,16 @@ def debug_eb2d(U, V, max_pwr_eb: float, ctx: Context | None = None, exact: bool 
     return eb, ids
 
 
-def debug_eb3d(U, V, W, max_pwr_eb: float, ctx: Context | None = None):
-    """Per-vertex 3D bound (float64) and id bytes (255 = bound not positive) from the GPU kernel."""
+def debug_eb3d(U, V, W, max_pwr_eb: float, ctx: Context | None = None, exact: bool = True):
+    """Per-vertex 3D bound (float64) and id bytes (255 = bound not positive) from the GPU kernel.
+
+    exact=False runs the compressor's filtered path and returns (None, ids)."""
     U, V, W = (np.ascontiguousarray(a, np.float32) for a in (U, V, W))
     r1, r2, r3 = U.shape
-    eb = np.empty(U.shape, np.float64)
+    eb = np.empty(U.shape, np.float64) if exact else None
     ids = np.empty(U.shape, np.uint8)
     _check(lib().cpsz_b200_debug_eb3d(_h(ctx), U.ctypes.data, V.ctypes.data, W.ctypes.data, r1, r2, r3,
-                                      float(max_pwr_eb), eb.ctypes.data, ids.ctypes.data))
+                                      float(max_pwr_eb), eb.ctypes.data if exact else None, ids.ctypes.data))
     return eb, ids
 
 
@@ -639,11 +641,17 @@ def debug_filter_premises(ctx: Context | None = None) -> dict:
     the filtered 2D / 3D bounds rely on: acbrt1 relative error above / below a
     double cube root ("acbrt1_hi", "acbrt1_lo"), the relative errors of
     rcp.approx, ex2.approx and sqrt.approx, and lg2.approx's absolute error
-    per binade ("lg2": {e: max over [2^e, 2^(e+1))}, e = -126..0)."""
-    out = np.zeros(132, np.float64)
+    per binade ("lg2": {e: max over [2^e, 2^(e+1))}, e = -126..0); acbrt1's
+    rounding error above / below its two Newton steps ("root_hi", "root_lo")
+    and, of those steps' own relative deviation, the largest slope over the
+    argument's logarithm across 64 floats ("root_slope") and the largest change
+    from a float to the next ("root_step")."""
+    out = np.zeros(136, np.float64)
     _check(lib().cpsz_b200_debug_filter_premises(_h(ctx), out.ctypes.data, out.size))
     return {"acbrt1_hi": out[0], "acbrt1_lo": out[1], "rcp": out[2], "ex2": out[3], "sqrt": out[4],
-            "lg2": {e: out[5 + e + 126] for e in range(-126, 1)}}
+            "lg2": {e: out[5 + e + 126] for e in range(-126, 1)},
+            "root_hi": out[132], "root_lo": out[133], "root_slope": out[134],
+            "root_step": out[135]}
 
 
 def debug_libm(which: str, x, ctx: Context | None = None):

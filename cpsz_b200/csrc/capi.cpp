@@ -384,7 +384,9 @@ int cpsz_b200_debug_eb3d(cpsz_b200_ctx* ctx, const float* U, const float* V, con
   double *deb = nullptr, *dtab = nullptr;
   uint8_t* dids = nullptr;
   CPSZ_CUDA_TRY(cudaMalloc((void**)&dF, 12 * N));
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&deb, 8 * N));
+  void* dscr = nullptr;
+  if (eb_out) CPSZ_CUDA_TRY(cudaMalloc((void**)&deb, 8 * N));
+  else CPSZ_CUDA_TRY(cudaMalloc(&dscr, eb3d_scratch_bytes(N)));
   CPSZ_CUDA_TRY(cudaMalloc((void**)&dids, N));
   CPSZ_CUDA_TRY(cudaMalloc((void**)&dtab, QUANT_TAB_MAX * 8));
   cudaMemcpy(dF, U, 4 * N, cudaMemcpyHostToDevice);
@@ -392,12 +394,13 @@ int cpsz_b200_debug_eb3d(cpsz_b200_ctx* ctx, const float* U, const float* V, con
   cudaMemcpy(dF + 2 * N, W, 4 * N, cudaMemcpyHostToDevice);
   cudaMemcpy(dtab, qt.t, QUANT_TAB_MAX * 8, cudaMemcpyHostToDevice);
   cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream);
-  int rc = launch_eb3d(ctx, dF, dF + N, dF + 2 * N, (int)r1, (int)r2, (int)r3, max_pwr_eb, dtab, qt.n, dids, deb);
+  int rc = launch_eb3d(ctx, dF, dF + N, dF + 2 * N, (int)r1, (int)r2, (int)r3, max_pwr_eb, dtab, qt.n, dids, dscr, deb);
   cudaStreamSynchronize(ctx->stream);
   if (rc == CPSZ_OK) {
     if (eb_out) cudaMemcpy(eb_out, deb, 8 * N, cudaMemcpyDeviceToHost);
     if (id_codes) cudaMemcpy(id_codes, dids, N, cudaMemcpyDeviceToHost);
   }
+  cudaFree(dscr);
   cudaFree(dF);
   cudaFree(deb);
   cudaFree(dids);
@@ -454,7 +457,7 @@ int cpsz_b200_debug_libm(cpsz_b200_ctx* ctx, int which, const float* in, size_t 
 
 int cpsz_b200_debug_filter_premises(cpsz_b200_ctx* ctx, double* out, size_t n) {
   RESOLVE(ctx);
-  if (!out || n < (size_t)FP_COUNT) return set_error(CPSZ_ERR_INVALID, "need %d output doubles", (int)FP_COUNT);
+  if (!out || n < (size_t)FP_ROOT_HI) return set_error(CPSZ_ERR_INVALID, "need %d output doubles", (int)FP_ROOT_HI);
   unsigned* d = nullptr;
   CPSZ_CUDA_TRY(cudaMalloc((void**)&d, FP_COUNT * sizeof(unsigned)));
   unsigned h[FP_COUNT];
@@ -467,7 +470,7 @@ int cpsz_b200_debug_filter_premises(cpsz_b200_ctx* ctx, double* out, size_t n) {
   }
   cudaFree(d);
   if (rc != CPSZ_OK) return rc;
-  for (int i = 0; i < FP_COUNT; i++) {
+  for (int i = 0; i < FP_COUNT && (size_t)i < n; i++) {
     float f;
     memcpy(&f, &h[i], 4);
     out[i] = f;

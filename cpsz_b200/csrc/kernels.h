@@ -313,9 +313,25 @@ int launch_huff_decode(cpsz_b200_ctx* ctx, const HuffDecJob* jobs, int nj, void*
 constexpr int ID_RAW_3D = 24;
 // Per-vertex bound (24 tets, reference order) -> id byte (ID_ZERO when the
 // bound is not positive; ids >= ID_RAW_3D raise FLAG_ID_OVERFLOW).  eb_out
-// (optional) receives the bound before quantization.
+// (optional) receives the bound before quantization.  scratch: eb3d_scratch_bytes(N)
+// bytes for the ids alone (null with eb_out).
+size_t eb3d_scratch_bytes(size_t n);
 int launch_eb3d(cpsz_b200_ctx* ctx, const float* U, const float* V, const float* W, int r1, int r2, int r3,
-                double max_pwr_eb, const double* d_thr, int thr_n, uint8_t* id_q, double* eb_out = nullptr);
+                double max_pwr_eb, const double* d_thr, int thr_n, uint8_t* id_q, void* scratch, double* eb_out = nullptr);
+// The ids alone, by enclosures of the bounds (eb3d_filter.cu): launch_eb3d
+// goes there when no bounds are asked for and eb3d_filter_takes says so.
+// chunk: i-planes a CTA marches over; list: room for `limit` entries; count:
+// zeroed; once more than `limit` vertices stay open (*count > limit) the ids
+// are incomplete.
+struct Eb3dOpen {
+  unsigned at_lo, at_hi;  // the vertex
+  unsigned tets;          // those to evaluate (bit k: the k-th around it)
+  unsigned pad;
+};
+bool eb3d_filter_takes(int r1, int r2, int r3, double max_pwr_eb);
+int launch_eb3d_filter(cpsz_b200_ctx* ctx, const float* U, const float* V, const float* W, int r1, int r2, int r3,
+                       double max_pwr_eb, const double* d_thr, int thr_n, uint8_t* id_q, int chunk, Eb3dOpen* list,
+                       unsigned* count, unsigned limit);
 // Log transform: pairs[i] = (log2f|U|, log2f|V|, log2f|W| (-100 for 0), 1/precision
 // or NaN); sign bitmaps (bit 7-(i%8) of byte i/8 = value > 0) as 3 arrays of
 // sign_words 32-bit words.
@@ -323,7 +339,10 @@ int launch_log3d(cpsz_b200_ctx* ctx, const float* U, const float* V, const float
                  const LibmFn& L, float4* pairs, uint32_t* signs, size_t sign_words);
 // Exhaustive maxima of the operations the filtered bounds rely on
 // (selfcheck.cu), FP_COUNT floats as bit patterns in d_out (device).
-enum FilterPremise { FP_ACBRT_HI = 0, FP_ACBRT_LO = 1, FP_RCP = 2, FP_EX2 = 3, FP_SQRT = 4, FP_LG2 = 5, FP_COUNT = 132 };
+enum FilterPremise {
+  FP_ACBRT_HI = 0, FP_ACBRT_LO = 1, FP_RCP = 2, FP_EX2 = 3, FP_SQRT = 4, FP_LG2 = 5,
+  FP_ROOT_HI = 132, FP_ROOT_LO = 133, FP_ROOT_SLOPE = 134, FP_ROOT_STEP = 135, FP_COUNT = 136
+};
 int launch_filter_premises(cpsz_b200_ctx* ctx, unsigned* d_out);
 // Host-library log2f (which 0) / exp2f (which 1) of n device floats.
 int launch_libm_eval(cpsz_b200_ctx* ctx, int which, const float* in, size_t n, const LibmTables& L, float* out);

@@ -6,6 +6,7 @@
 //            wavefront's per-point input (log values, 1/precision)
 //   compact3d / prep3d   raster-order compaction of codes and unpredictable
 //            values (compress) and its inverse (decompress)
+#include <algorithm>
 #include <cfloat>
 
 #include "eb_math.cuh"
@@ -39,7 +40,9 @@ __global__ void __launch_bounds__(EB_NT, 3) eb3d_kernel(const float* __restrict_
                                                      const float* __restrict__ W, int r1, int r2, int r3,
                                                      int i_chunk, double max_pwr_eb, const double* __restrict__ thr,
                                                      int thr_n, uint8_t* __restrict__ id_q,
-                                                     double* __restrict__ eb_out, int* __restrict__ flag) {
+                                                     double* __restrict__ eb_out, int* __restrict__ flag,
+                                                     const unsigned* __restrict__ open, unsigned limit) {
+  if (open && *open <= limit) return;  // the filtered path has every id
   __shared__ float vtx[2][3][VJ][VK];
   __shared__ float tets[2][6][CJ][CK];
   const int k0 = blockIdx.x * EB_TK, j0 = blockIdx.y * EB_TJ;
@@ -355,10 +358,18 @@ int grid_for(size_t n, int per_block, int cap) {
   return (int)(g ? g : 1);
 }
 
+// Vertices that may stay open: at one in 8 their evaluation costs about what
+// the filtered path saves.
+unsigned eb3d_open_limit(size_t points) {
+  return (unsigned)std::min<size_t>(std::max<size_t>(4096, points / 8), 0x7fffffffu);
+}
+
 }  // namespace
 
+size_t eb3d_scratch_bytes(size_t n) { return 256 + (size_t)eb3d_open_limit(n) * sizeof(Eb3dOpen); }
+
 int launch_eb3d(cpsz_b200_ctx* ctx, const float* U, const float* V, const float* W, int r1, int r2, int r3,
-                double max_pwr_eb, const double* d_thr, int thr_n, uint8_t* id_q, double* eb_out) {
+                double max_pwr_eb, const double* d_thr, int thr_n, uint8_t* id_q, void* scratch, double* eb_out) {
   dim3 grid((r3 + EB_TK - 1) / EB_TK, (r2 + EB_TJ - 1) / EB_TJ, 1);
   if (grid.y > 65535)
     return set_error(CPSZ_ERR_UNSUPPORTED, "3D field with r2 = %d exceeds the bound kernel's grid", r2);
@@ -372,8 +383,19 @@ int launch_eb3d(cpsz_b200_ctx* ctx, const float* U, const float* V, const float*
   int chunk = (int)((r1 + want - 1) / want);
   if (chunk < min_chunk) chunk = min_chunk < r1 ? min_chunk : r1;
   grid.z = (r1 + chunk - 1) / chunk;
+  // The ids alone: the filtered path, and behind it the fully evaluated one,
+  // which runs only if too many vertices stayed open (a field of degenerate
+  // tets: there every tet would be evaluated once per vertex instead of once).
+  unsigned* open = nullptr;
+  const unsigned limit = eb3d_open_limit(points);
+  if (!eb_out && scratch && eb3d_filter_takes(r1, r2, r3, max_pwr_eb)) {
+    open = (unsigned*)scratch;
+    CPSZ_CUDA_TRY(cudaMemsetAsync(open, 0, 4, ctx->stream));
+    CPSZ_TRY(launch_eb3d_filter(ctx, U, V, W, r1, r2, r3, max_pwr_eb, d_thr, thr_n, id_q, chunk,
+                                (Eb3dOpen*)((char*)scratch + 256), open, limit));
+  }
   eb3d_kernel<<<grid, EB_NT, 0, ctx->stream>>>(U, V, W, r1, r2, r3, chunk, max_pwr_eb, d_thr, thr_n, id_q, eb_out,
-                                                ctx->d_flag);
+                                                ctx->d_flag, open, limit);
   count_launch(ctx);
   return check_launch("eb3d_kernel");
 }

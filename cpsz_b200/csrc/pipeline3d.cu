@@ -77,7 +77,7 @@ int compress_3d(cpsz_b200_ctx* ctx, const float* U_in, const float* V_in, const 
   auto add = [&](size_t b) { bytes += align_up(b, 256) + 256; };
   if (!dev_in) add(12 * N);
   add(N);              // ids
-  add(16 * N);         // pairs
+  add(std::max(16 * N, eb3d_scratch_bytes(N)));  // pairs
   add(16 * N);         // reconstruction
   add(8 * N);          // codes per point
   add(2 * (nchunks + 1) * 4);
@@ -121,7 +121,7 @@ int compress_3d(cpsz_b200_ctx* ctx, const float* U_in, const float* V_in, const 
     dW = h + 2 * N;
   }
   uint8_t* ids = (uint8_t*)A(N);
-  float4* pairs = (float4*)A(16 * N);
+  float4* pairs = (float4*)A(std::max(16 * N, eb3d_scratch_bytes(N)));
   float4* rec = (float4*)A(16 * N);
   ushort4* codes = (ushort4*)A(8 * N);
   unsigned* chunk_cnt = (unsigned*)A((nchunks + 1) * 4);
@@ -158,7 +158,7 @@ int compress_3d(cpsz_b200_ctx* ctx, const float* U_in, const float* V_in, const 
   CPSZ_CUDA_TRY(cudaMemsetAsync(zero, 0, zero_bytes, st));
   CPSZ_CUDA_TRY(cudaMemcpyAsync(image, ctx->up_pinned, image_bytes, cudaMemcpyHostToDevice, st));
   mark(ctx, "eb3d");
-  CPSZ_TRY(launch_eb3d(ctx, dU, dV, dW, r1, r2, r3, max_pwr_eb, thr_tab, qt.n, ids));
+  CPSZ_TRY(launch_eb3d(ctx, dU, dV, dW, r1, r2, r3, max_pwr_eb, thr_tab, qt.n, ids, pairs));  // (pairs: not yet written)
   mark(ctx, "log3d");
   CPSZ_TRY(launch_log3d(ctx, dU, dV, dW, ids, N, lt.log2f, pairs, signs, sign_words));
   mark(ctx, "wave3d_compress");

@@ -9,6 +9,13 @@
 //   acbrt1 (the reference's cube root, bit for bit the product path's) against
 //     a double cube root, relative, over all positive normal floats (above
 //     and below 1 separately);
+//   acbrt1 against its own two Newton steps from the same first guess in
+//     double (what its float roundings add, above and below separately), and
+//     how fast the relative deviation of those exact steps from the cube root
+//     changes: the largest change over ROOT_STRIDE floats, divided by the
+//     logarithm of their ratio, and the largest from a float to the next
+//     (between any two floats it is at most the first times the logarithm of
+//     their ratio plus ROOT_STRIDE - 1 times the second);
 //   rcp.approx.ftz.f32, relative, over the normal floats below 2^126;
 //   ex2.approx.ftz.f32, relative, over [-87, 0];
 //   sqrt.approx.f32, relative, over all positive normal floats;
@@ -32,10 +39,25 @@ __device__ __forceinline__ void raise_max(unsigned* out, int slot, double e) {
   atomicMax(out + slot, __float_as_uint((float)e));
 }
 
+constexpr int ROOT_STRIDE = 64;
+
+// acbrt1's two Newton steps without rounding, from its own first guess.
+__device__ __forceinline__ double acbrt1_steps(float x0) {
+  int ix = __float_as_int(x0);
+  ix = (ix >> 2) + (ix >> 4);
+  ix = ix + (ix >> 4);
+  ix = ix + (ix >> 8);
+  const double a = x0;
+  double x = __int_as_float(0x2a5137a0 + ix);
+  x = (2.0 * x + a / (x * x)) / 3.0;
+  x = (2.0 * x + a / (x * x)) / 3.0;
+  return x;
+}
+
 __global__ void filter_premises_kernel(unsigned* __restrict__ out) {
   const unsigned long long tid = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
   const unsigned long long nt = (unsigned long long)gridDim.x * blockDim.x;
-  double hi = 0, lo = 0, rc = 0, ex = 0, sq = 0, lg = 0;
+  double hi = 0, lo = 0, rc = 0, ex = 0, sq = 0, lg = 0, rhi = 0, rlo = 0, slope = 0, step = 0;
   int lg_slot = -1;  // the binade lg accumulates (a thread's b rises, so binades come in order)
   for (unsigned long long b = 0x00800000ull + tid; b < 0x7f800000ull; b += nt) {
     const float x = __uint_as_float((unsigned)b);
@@ -43,6 +65,16 @@ __global__ void filter_premises_kernel(unsigned* __restrict__ out) {
     const double e = (double)dev::acbrt1_nonneg(x) / cbrt(xd) - 1.0;
     hi = fmax(hi, e);
     lo = fmax(lo, -e);
+    const double steps = acbrt1_steps(x);
+    const double r = (double)dev::acbrt1_nonneg(x) / steps - 1.0;
+    rhi = fmax(rhi, r);
+    rlo = fmax(rlo, -r);
+    const double dev0 = steps / cbrt(xd);
+    if (b + ROOT_STRIDE < 0x7f800000ull) {
+      const float y = __uint_as_float((unsigned)b + 1), z = __uint_as_float((unsigned)b + ROOT_STRIDE);
+      step = fmax(step, fabs(acbrt1_steps(y) / cbrt((double)y) - dev0));
+      slope = fmax(slope, fabs(acbrt1_steps(z) / cbrt((double)z) - dev0) / log1p(((double)z - xd) / xd));
+    }
     sq = fmax(sq, fabs((double)sqrt_approx_f(x) / sqrt(xd) - 1.0));
     if (b < 0x7e800000ull) rc = fmax(rc, fabs((double)dev::rcp_approx(x) * xd - 1.0));
     if (b < 0x40000000ull) {
@@ -66,6 +98,10 @@ __global__ void filter_premises_kernel(unsigned* __restrict__ out) {
   raise_max(out, FP_RCP, rc);
   raise_max(out, FP_EX2, ex);
   raise_max(out, FP_SQRT, sq);
+  raise_max(out, FP_ROOT_HI, rhi);
+  raise_max(out, FP_ROOT_LO, rlo);
+  raise_max(out, FP_ROOT_SLOPE, slope);
+  raise_max(out, FP_ROOT_STEP, step);
 }
 
 }  // namespace

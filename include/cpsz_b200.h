@@ -296,7 +296,8 @@ size_t cpsz_b200_blob_size_2d(const unsigned char* blob);
 int cpsz_b200_debug_eb2d(cpsz_b200_ctx* ctx, const float* U, const float* V, size_t r1, size_t r2,
                          double max_pwr_eb, double* eb_out, uint8_t* id_codes);
 /* The 3D bound kernel alone: per-vertex bound (N doubles) and id bytes (N;
- * 255 = bound not positive).  Host buffers. */
+ * 255 = bound not positive).  Host buffers.  eb_out NULL takes the
+ * compressor's filtered path (ids only), which must give the same ids. */
 int cpsz_b200_debug_eb3d(cpsz_b200_ctx* ctx, const float* U, const float* V, const float* W, size_t r1, size_t r2,
                          size_t r3, double max_pwr_eb, double* eb_out, uint8_t* id_codes);
 /* The wavefront's per-group wait for the bound kernel gives up once the bound
@@ -323,7 +324,12 @@ int cpsz_b200_debug_wave_trace(cpsz_b200_ctx* ctx, size_t len, long long* out);
  * positive normal floats; out[2] rcp.approx.ftz.f32 (relative, normal floats
  * below 2^126); out[3] ex2.approx.ftz.f32 (relative, [-87, 0]); out[4]
  * sqrt.approx.f32 (relative, positive normal floats); out[5 + e + 126]
- * lg2.approx.ftz.f32 (absolute) on [2^e, 2^(e+1)), e = -126..0.  n >= 132. */
+ * lg2.approx.ftz.f32 (absolute) on [2^e, 2^(e+1)), e = -126..0.  n >= 132;
+ * with n >= 136 also out[132] / out[133] how far acbrt1's roundings take it
+ * above / below its own two Newton steps (relative), and of those exact steps'
+ * relative deviation from the cube root out[134] the largest change over 64
+ * floats, divided by the change of the argument's logarithm, and out[135] the
+ * largest change from a float to the next. */
 int cpsz_b200_debug_filter_premises(cpsz_b200_ctx* ctx, double* out, size_t n);
 /* Host-computed quantization thresholds (which = 2: 2D offline, 1: 2D
  * offline_log, 3: 3D): t[k] is the smallest bound with id >= k under the host

@@ -85,3 +85,54 @@ def test_filtered_eb3d_equals_oracle(ctx, oracle, eb):
             assert_bits_equal(e, ref, nan_equal=True)
         except AssertionError as err:
             raise AssertionError(f"{name}: {err}") from None
+
+
+EB3_ABS, EB3_REL = 3.0e-7, 2.0e-4
+
+
+def test_id_enclosure_budget_holds_on_this_device(ctx):
+    """The error budget of the compression path's enclosure (the proof in
+    eb3d_filter.cu), recomputed over the bounds it is used for (k <= 0.3) from
+    the operations' maxima on this GPU, stays below EB3_ABS + EB3_REL k."""
+    m = cpsz_b200.debug_filter_premises(ctx=ctx)
+    assert m["root_hi"] + m["root_lo"] <= 2.9e-7 and m["root_slope"] <= 5e-5 and m["root_step"] <= 1e-10
+    u = 2.0 ** -24
+    k = np.linspace(0.0, 0.3, 20001)
+    q = np.tanh(3 * np.arctanh(k))
+    dk = (1 - k ** 2) / (3 * (1 - q ** 2))
+    # the reference's K: its cube roots' roundings and steps, sum and quotient; its float sums
+    ref = 0.5 * (m["root_hi"] + m["root_lo"] + 63 * m["root_step"]) + 3 * m["root_slope"] * k + 2 * u * k + 6.2 * u / 6
+    # q: minors 5.2 u, sums 7 u, rcp.approx, product
+    term_q = dk * (5.2 * u + q * (7 * u + m["rcp"] + u))
+    total = ref + term_q + 6 * u * k
+    assert np.all(total <= EB3_ABS + EB3_REL * k - u * (k + EB3_ABS)), np.max(total - EB3_REL * k)
+
+
+# vertices around the kernel's tiles (32 x 8 columns, cubes 33 x 9) and its smallest fields
+SHAPES = [(2, 2, 2), (3, 8, 32), (3, 9, 33), (2, 17, 65), (5, 7, 31), (4, 10, 34), (40, 3, 2)]
+
+
+@pytest.mark.parametrize("eb", [0.25, 0.1, 0.01, 1e-5, 0.0])
+def test_filtered_ids_equal_exact_ids(ctx, eb):
+    """The compression path's ids against those of the fully evaluated bounds."""
+    rng = np.random.default_rng(12)
+    fields = list(_fields())
+    U, V, Wf = (a for a in fields[0][1])
+    land = rng.random(SHAPE) < 0.3
+    fields.append(("land", tuple(np.where(land, np.float32(0), a) for a in (U, V, Wf))))
+    fields.append(("constant", tuple(np.full(SHAPE, x, np.float32) for x in (0.3, -0.7, 0.1))))
+    lin = np.indices(SHAPE).astype(np.float32)
+    fields.append(("linear", (lin[0] - 9.5, lin[1] - 11.5, lin[2] - 13.5)))
+    fields.append(("nearly parallel", (U, U * np.float32(1 + 1e-6), U * np.float32(1 - 1e-6) + V * np.float32(1e-5))))
+    bad = np.array(U)
+    bad[7, 9, 11], bad[12, 3, 20], bad[5:7, 18, 4] = np.nan, np.inf, 1e38
+    fields.append(("not finite", (bad, V, Wf)))
+    for s in SHAPES:
+        fields.append((f"noise {s}", tuple(rng.standard_normal(s).astype(np.float32) for _ in range(3))))
+        fields.append((f"smooth {s}", W.field_3d(95, *s, 3, 5.0)))
+    fields.append(("large smooth", W.field_3d(96, 70, 90, 100, 8, 12.0)))
+    for name, f in fields:
+        _, want = cpsz_b200.debug_eb3d(*f, eb, ctx=ctx)
+        _, got = cpsz_b200.debug_eb3d(*f, eb, ctx=ctx, exact=False)
+        bad = np.nonzero(want != got)
+        assert bad[0].size == 0, (name, bad[0].size, [x[:4] for x in bad], want[bad][:4], got[bad][:4])
