@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(NT, 2048 / 64 / (NT / 32)) eb2d_kernel(const f
   static_assert(UNIT_COLS % TX == 0, "a tile's columns must lie in one unit");
   __shared__ float su[TY + 2][TX + 3];
   __shared__ float sv[TY + 2][TX + 3];
-  // compression (FAST): the float bound of an ordinary triangle, or +inf when
+  // compression (FAST): the q (cell_eb_float) of an ordinary triangle, or +inf when
   // the triangle took the exact path (its bound is in tri) or does not exist;
   // exact mode: tri alone
   __shared__ float trf[2][CY][CX];
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(NT, 2048 / 64 / (NT / 32)) eb2d_kernel(const f
   __syncthreads();
   // cells (ci, cj) = (i0-1+a, j0-1+b), a in [0, CY), b in [0, CX).
   // Compression (FAST): both triangles of a cell per thread and round
-  // (1089 cells over 256 threads at 32x32), the float bound in trf, or +inf
+  // (1089 cells over 256 threads at 32x32), the q in trf, or +inf
   // there and the exact bound in tri for a triangle that takes the exact
   // path; a cell outside the field holds +inf in both (it has no triangles,
   // and +inf leaves every vertex minimum unchanged).  Exact mode: one
@@ -127,6 +127,8 @@ __global__ void __launch_bounds__(NT, 2048 / 64 / (NT / 32)) eb2d_kernel(const f
   // bound is a call (tri_eb_exact is not inlined), so its code is in the
   // instruction cache once.
   bool any_exact = false;
+  // q's near 1 are beyond every max_pwr_eb up to 0.9 (cell_eb_float)
+  const float q_max = max_pwr_eb <= 0.9 ? INFINITY : 0.999f;
   if (FAST) {
     for (int c = tid; c < CY * CX; c += NT) {
       const int a = c / CX, b = c - (c / CX) * CX;
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(NT, 2048 / 64 / (NT / 32)) eb2d_kernel(const f
       bool ok[2] = {false, false};
       if (in)
         dev::cell_eb_float(su[a][b], su[a + 1][b], su[a][b + 1], su[a + 1][b + 1], sv[a][b], sv[a + 1][b],
-                           sv[a][b + 1], sv[a + 1][b + 1], t[0], t[1], ok[0], ok[1]);
+                           sv[a][b + 1], sv[a + 1][b + 1], q_max, t[0], t[1], ok[0], ok[1]);
 #pragma unroll
       for (int kind = 0; kind < 2; kind++) {
         if (!ok[kind]) {
@@ -206,13 +208,14 @@ __global__ void __launch_bounds__(NT, 2048 / 64 / (NT / 32)) eb2d_kernel(const f
     int code[2];
     double eb = 0;
     if (FAST) {
-      // enclosure of the vertex bound: the float bounds of its ordinary
-      // triangles (min mf, each within FFILT_REL and FFILT_ABS of the
+      // enclosure of the vertex bound: the bound of its ordinary triangles (mf,
+      // from the least of their q's, within FFILT_REL and FFILT_ABS of the
       // reference's value) and the exact ones (min md).  The six incident
       // triangles are read unconditionally: a missing one (a cell outside the
       // field) holds +inf.
-      const float mf = fminf(fminf(fminf(trf[0][a][b], trf[1][a][b]), fminf(trf[0][a][b + 1], trf[1][a + 1][b])),
-                             fminf(trf[0][a + 1][b + 1], trf[1][a + 1][b + 1]));
+      const float mf = dev::keep_sign2_of_q(
+          fminf(fminf(fminf(trf[0][a][b], trf[1][a][b]), fminf(trf[0][a][b + 1], trf[1][a + 1][b])),
+                fminf(trf[0][a + 1][b + 1], trf[1][a + 1][b + 1])));
       double md = INFINITY;
       bool nan = false;
       if (tile_exact) {

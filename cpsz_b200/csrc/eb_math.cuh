@@ -225,32 +225,37 @@ __device__ __forceinline__ float rcp_approx(float x) {
 //    reference's flag equals (sign s_k == sign x_k) and its det is not zero.
 //    Otherwise, and when all three flags hold (a critical point), the
 //    triangle is exact.
-//  * bounds.  keep_sign2(P, N) = |sqrt P - sqrt N| / (sqrt P + sqrt N) =
-//    |P - N| / (sqrt P + sqrt N)^2 (1 when P or N is 0), P and N the sums of
-//    the positive / negated negative terms.  Its numerator P - N is one of the
-//    accurate values above: x_k for the two-term bounds, s_k for the
-//    four-term ones (p01 - p10 + p12 - p21 = x3 + x2, and so on).  The
-//    denominator d = P + N + 2 sqrt(P N) comes from float sums of the terms
-//    (3u relative each) and sqrt.approx: within 2^-20 relative.  Each value
-//    is |D| times rcp.approx(d) (at most 9.9e-8 relative on these operands,
-//    measured with the other premises) rounded once: within 2^-19.6 of the
-//    real one.  The triangle's bound is the max over failing flags of the
-//    min of two such values, both exact, so it too is within 2^-19.6 of the
-//    real value's; the result t is within 2^-18 t of the real value, and the
-//    reference's double value within 2^-50 r + 2^-52 of it; the enclosure
-//    uses 2^-16 relative and 2^-40 absolute.
-//  * range.  Exact path when S is not finite, S > 2^40 or S < 2^-60, or a
-//    product P N is below 2^-110 and not 0 (sqrt of a subnormal product).
+//  * bounds.  keep_sign2(P, N) = |sqrt P - sqrt N| / (sqrt P + sqrt N) (1 when
+//    P or N is 0), P and N the sums of the positive / negated negative terms,
+//    is k(q) = q / (1 + sqrt(1 - q^2)) of q = |P - N| / (P + N), which grows with
+//    q.  So the triangle's bound is k of the max over failing flags of the
+//    min of two q's, the min over a vertex's triangles is taken on the q's,
+//    too, and k is evaluated once per vertex: no square root per triangle.  A
+//    q's numerator is one of the accurate values above: x_k for the two-term
+//    bounds, s_k for the four-term ones (p01 - p10 + p12 - p21 = x3 + x2, and
+//    so on); its denominator a sum of two or four |p|, within 3u; rcp.approx
+//    (at most 9.9e-8 = 1.7u, measured with the other premises) and a product:
+//    each q is within 7.7u of the real one, relative, and so is the triangle's.
+//    k moves 1 / sqrt(1 - q^2) times as much, and its evaluation adds 6u: at
+//    most 80u for bounds up to 0.9 (q <= 0.9945), and 180u up to q = 0.999.  The
+//    enclosure uses 2^-16 (256u) relative and 2^-40 absolute, which also covers
+//    the reference's own double arithmetic (2^-50 relative, 2^-52).  A q near 1
+//    stands for a bound above 0.96, beyond a max_pwr_eb of at most 0.9; with a
+//    larger one (q_max) a triangle of q > 0.999 is exact.
+//  * range.  Exact path when S is not finite, S > 2^40 or S < 2^-60, or one of
+//    the |p| + |p'| is below 2^-100 (its rcp.approx may flush).
 constexpr float FFILT_REL = 1.0f / 65536.0f;           // 2^-16
 constexpr float FFILT_ABS = 9.09494702e-13f;           // 2^-40
 
-__device__ __forceinline__ float pos_part(float t) { return t > 0.f ? t : 0.f; }
-__device__ __forceinline__ float neg_part(float t) { return t < 0.f ? -t : 0.f; }
+// k(q) for q >= 0 (1 from q = 1 up to a rounding above, +inf at +inf).
+__device__ __forceinline__ float keep_sign2_of_q(float q) {
+  return q * rcp_approx(1.f + sqrt_approx(fmaxf((1.f - q) * (1.f + q), 0.f)));
+}
 
 // ---- both triangles of a cell at once --------------------------------------------
 // Cell (a, b) of the grid holds the "upper" triangle {(a,b), (a+1,b), (a+1,b+1)}
 // and the "lower" one {(a,b), (a,b+1), (a+1,b+1)}: vertices 0 and 2 are
-// shared, so p02, p20, x1 and the two-term bound of x1 are the same for both.
+// shared, so p02, p20, x1 and the two-term q of x1 are the same for both.
 // cell_eb_float runs the filter above for the two triangles together, the
 // upper one in the low word and the lower one in the high word of packed
 // f32x2 operands: add / sub / mul.rn.f32x2 round each word exactly as the
@@ -296,49 +301,16 @@ __device__ __forceinline__ void two_diff2(f32x2 a, f32x2 c, f32x2& s, f32x2& e) 
   const f32x2 bb = sub2(s, a);
   e = sub2(sub2(a, sub2(s, bb)), add2(c, bb));
 }
-// keep_sign2 of both words: 1 where P or N is 0, else +-|D| / d with
-// d = (P + N) + 2 sqrt(P N) (PpN = P + N) as D * rcp.approx(d); the sign is
-// D's (callers take |.|)
-__device__ __forceinline__ f32x2 ks2_val2(f32x2 D, f32x2 P, f32x2 N, f32x2 PpN, bool& bad_x, bool& bad_y) {
-  const f32x2 pn = mul2(P, N);
-  float P0, P1, N0, N1, q0, q1;
-  unpk2(P, P0, P1);
-  unpk2(N, N0, N1);
-  unpk2(pn, q0, q1);
-  const bool one0 = P0 == 0.f || N0 == 0.f, one1 = P1 == 0.f || N1 == 0.f;
-  bad_x |= !one0 && !(q0 >= 1.2924697e-33f);  // 2^-110
-  bad_y |= !one1 && !(q1 >= 1.2924697e-33f);
-  const f32x2 sq = pk2(sqrt_approx(q0), sqrt_approx(q1));
-  float d0, d1, v0, v1;
-  unpk2(add2(PpN, add2(sq, sq)), d0, d1);
-  unpk2(mul2(D, pk2(rcp_approx(d0), rcp_approx(d1))), v0, v1);
-  return pk2(one0 ? 1.f : v0, one1 ? 1.f : v1);
-}
-__device__ __forceinline__ f32x2 pos2(f32x2 t) {
-  float a, b;
-  unpk2(t, a, b);
-  return pk2(pos_part(a), pos_part(b));
-}
-__device__ __forceinline__ f32x2 neg2(f32x2 t) {
-  float a, b;
-  unpk2(t, a, b);
-  return pk2(neg_part(a), neg_part(b));
-}
-// The float bounds of the cell's upper (t_up) and lower (t_lo) triangles, with
-// ok_* false for a triangle that takes the exact path.  Vertices: U00 = (a,b),
-// U10 = (a+1,b), U01 = (a,b+1), U11 = (a+1,b+1); the upper triangle is
+// The q's of the cell's upper (t_up) and lower (t_lo) triangles, with ok_* false
+// for a triangle that takes the exact path.  Vertices: U00 = (a,b), U10 =
+// (a+1,b), U01 = (a,b+1), U11 = (a+1,b+1); the upper triangle is
 // (U00, U10, U11), the lower (U00, U01, U11) -- tri_eb's (u0, u1, u2).
-//
-// Sums of parts.  Every bound's P and N are sums of the positive / negated
-// negative parts of two or four of the terms (p20, -p02), (p12, -p21),
-// (p01, -p10), whose pairs give P_k = pos(a) + neg(c), N_k = neg(a) + pos(c)
-// for edge k = (a, -c): the two-term bound of x_k uses P_k, N_k, the
-// four-term bound of s_k = x_i + x_j uses P_i + P_j, N_i + N_j, and
-// S = (PN_1 + PN_2) + PN_3 with PN_k = P_k + N_k = |a| + |c|.  Summed in
-// pairs, each is within 2u of its exact value (the filter allows 3u).
+// PN_k = |a| + |c| are the sums of an edge k's two terms (a, -c): the two-term
+// bound of x_k has the denominator PN_k, the four-term one of s_k = x_i + x_j
+// PN_i + PN_j, and S = (PN_1 + PN_2) + PN_3.
 __device__ __forceinline__ void cell_eb_float(float U00, float U10, float U01, float U11, float V00, float V10,
-                                              float V01, float V11, float& t_up, float& t_lo, bool& ok_up,
-                                              bool& ok_lo) {
+                                              float V01, float V11, float q_max, float& t_up, float& t_lo,
+                                              bool& ok_up, bool& ok_lo) {
   const f32x2 u0 = pk2(U00, U00), u1 = pk2(U10, U01), u2 = pk2(U11, U11);
   const f32x2 v0 = pk2(V00, V00), v1 = pk2(V10, V01), v2 = pk2(V11, V11);
   const f32x2 p01 = mul2(u0, v1), p10 = mul2(u1, v0), p02 = mul2(u0, v2), p20 = mul2(u2, v0), p12 = mul2(u1, v2),
@@ -357,12 +329,14 @@ __device__ __forceinline__ void cell_eb_float(float U00, float U10, float U01, f
   const f32x2 s2 = add2(h2, add2(g2, add2(e1, e3)));
   const f32x2 s3 = add2(h3, add2(g3, e12));
   const f32x2 det = add2(hd, add2(gd, add2(g1, add2(e12, e3))));
-  const f32x2 P1 = add2(pos2(p20), neg2(p02)), N1 = add2(neg2(p20), pos2(p02));
-  const f32x2 P2 = add2(pos2(p12), neg2(p21)), N2 = add2(neg2(p12), pos2(p21));
-  const f32x2 P3 = add2(pos2(p01), neg2(p10)), N3 = add2(neg2(p01), pos2(p10));
-  const f32x2 PN1 = add2(P1, N1), PN2 = add2(P2, N2), PN3 = add2(P3, N3);
-  float S[2], X1[2], X2[2], X3[2], S1[2], S2[2], S3[2], DT[2];
-  unpk2(add2(add2(PN1, PN2), PN3), S[0], S[1]);
+  float a20[2], a02[2], a12[2], a21[2], a01[2], a10[2];
+  unpk2(p20, a20[0], a20[1]);
+  unpk2(p02, a02[0], a02[1]);
+  unpk2(p12, a12[0], a12[1]);
+  unpk2(p21, a21[0], a21[1]);
+  unpk2(p01, a01[0], a01[1]);
+  unpk2(p10, a10[0], a10[1]);
+  float X1[2], X2[2], X3[2], S1[2], S2[2], S3[2], DT[2];
   unpk2(x1, X1[0], X1[1]);
   unpk2(x2, X2[0], X2[1]);
   unpk2(x3, X3[0], X3[1]);
@@ -370,54 +344,35 @@ __device__ __forceinline__ void cell_eb_float(float U00, float U10, float U01, f
   unpk2(s2, S2[0], S2[1]);
   unpk2(s3, S3[0], S3[1]);
   unpk2(det, DT[0], DT[1]);
-  bool bad[2], f1[2], f2[2], f3[2];
-#pragma unroll
-  for (int w = 0; w < 2; w++) {
-    // x1 is bitwise the same in both words: word 0's serves both
-    const float T = S[w] * 5.68434189e-14f;  // 2^-44
-    bool b = !(S[w] >= 8.67361738e-19f && S[w] <= 1.09951163e12f);  // [2^-60, 2^40], false for NaN
-    b |= !(fabsf(S1[w]) > T && fabsf(S2[w]) > T && fabsf(S3[w]) > T && fabsf(DT[w]) > T);
-    b |= X1[0] == 0.f || X2[w] == 0.f || X3[w] == 0.f;
-    f1[w] = (S1[w] > 0.f) == (X1[0] > 0.f);
-    f2[w] = (S2[w] > 0.f) == (X2[w] > 0.f);
-    f3[w] = (S3[w] > 0.f) == (X3[w] > 0.f);
-    bad[w] = b || (f1[w] && f2[w] && f3[w]);  // a critical point: exact path
-  }
-  // max over failing flags of min(two-term, four-term bound), all three
-  // evaluated (no divergence); the two-term bound of x1 is the same for both
-  // triangles and is evaluated once
-  float k1;
-  {
-    float P1w, N1w, PN1w, unused;
-    unpk2(P1, P1w, unused);
-    unpk2(N1, N1w, unused);
-    unpk2(PN1, PN1w, unused);
-    const bool one = P1w == 0.f || N1w == 0.f;
-    const float q = P1w * N1w;
-    const bool b1 = !one && !(q >= 1.2924697e-33f);  // 2^-110
-    bad[0] |= b1;
-    bad[1] |= b1;
-    k1 = one ? 1.f : X1[0] * rcp_approx(PN1w + 2.f * sqrt_approx(q));
-  }
-  float a1[2], a2[2], a3[2], b2[2], b3[2];
-  unpk2(ks2_val2(s1, add2(P2, P3), add2(N2, N3), add2(PN2, PN3), bad[0], bad[1]), a1[0], a1[1]);
-  unpk2(ks2_val2(x2, P2, N2, PN2, bad[0], bad[1]), a2[0], a2[1]);
-  unpk2(ks2_val2(s2, add2(P1, P3), add2(N1, N3), add2(PN1, PN3), bad[0], bad[1]), b2[0], b2[1]);
-  unpk2(ks2_val2(x3, P3, N3, PN3, bad[0], bad[1]), a3[0], a3[1]);
-  unpk2(ks2_val2(s3, add2(P1, P2), add2(N1, N2), add2(PN1, PN2), bad[0], bad[1]), b3[0], b3[1]);
+  // x1, PN1 and the two-term q of x1 are the same in both words
+  const float PN1 = fabsf(a20[0]) + fabsf(a02[0]);
+  const float q1 = fabsf(X1[0]) * rcp_approx(PN1);
   float t[2];
+  bool ok[2];
 #pragma unroll
   for (int w = 0; w < 2; w++) {
-    float e = 0.f;
-    if (!f1[w]) e = fmaxf(e, fminf(fabsf(k1), fabsf(a1[w])));
-    if (!f2[w]) e = fmaxf(e, fminf(fabsf(a2[w]), fabsf(b2[w])));
-    if (!f3[w]) e = fmaxf(e, fminf(fabsf(a3[w]), fabsf(b3[w])));
+    const float PN2 = fabsf(a12[w]) + fabsf(a21[w]), PN3 = fabsf(a01[w]) + fabsf(a10[w]);
+    const float P12 = PN1 + PN2, S = P12 + PN3;
+    const float T = S * 5.68434189e-14f;  // 2^-44
+    bool b = S >= 8.67361738e-19f && S <= 1.09951163e12f;  // [2^-60, 2^40], false for NaN
+    b &= fminf(fminf(fabsf(S1[w]), fabsf(S2[w])), fminf(fabsf(S3[w]), fabsf(DT[w]))) > T;
+    b &= X1[0] != 0.f && X2[w] != 0.f && X3[w] != 0.f;
+    b &= fminf(fminf(PN1, PN2), PN3) >= 7.88860905e-31f;  // 2^-100
+    const float m1 = fminf(q1, fabsf(S1[w]) * rcp_approx(PN2 + PN3));
+    const float m2 = fminf(fabsf(X2[w]) * rcp_approx(PN2), fabsf(S2[w]) * rcp_approx(PN1 + PN3));
+    const float m3 = fminf(fabsf(X3[w]) * rcp_approx(PN3), fabsf(S3[w]) * rcp_approx(P12));
+    // flag k holds when s_k and x_k have one sign; a triangle where all three
+    // do is a critical point: exact path
+    const int f1 = __float_as_int(S1[w]) ^ __float_as_int(X1[0]), f2 = __float_as_int(S2[w]) ^ __float_as_int(X2[w]),
+              f3 = __float_as_int(S3[w]) ^ __float_as_int(X3[w]);
+    const float e = fmaxf(f1 < 0 ? m1 : 0.f, fmaxf(f2 < 0 ? m2 : 0.f, f3 < 0 ? m3 : 0.f));
     t[w] = e;
+    ok[w] = b && (f1 | f2 | f3) < 0 && e <= q_max;
   }
   t_up = t[0];
   t_lo = t[1];
-  ok_up = !bad[0];
-  ok_lo = !bad[1];
+  ok_up = ok[0];
+  ok_lo = ok[1];
 }
 
 // ---- 3D (src/sz_compress_cp_preserve_3d.cpp:266-358) --------------------------

@@ -54,3 +54,18 @@ def test_compressor_uses_the_filtered_path_consistently(ctx):
     st = cpsz_b200.compress_2d_stages(U, V, 0.1, ctx=ctx)
     _, exact = cpsz_b200.debug_eb2d(U, V, 0.1, ctx=ctx, exact=True)
     assert np.array_equal(st["ids"], np.where(exact == 255, 0, exact).astype(np.int32))
+
+
+@pytest.mark.parametrize("eb", [0.900001, 1.0])
+def test_filtered_ids_at_bounds_near_one(ctx, eb):
+    """Above 0.9 a triangle's ratio near 1 takes the exact path: fields whose
+    sums have one small side (bounds close to 1), and the others."""
+    rng = np.random.default_rng(8)
+    U = np.abs(rng.standard_normal((400, 500))).astype(np.float32)
+    V = (rng.standard_normal((400, 500)) * 1e-3).astype(np.float32)
+    fields = list(_fields())[4:] + [("one side small", (U, V)), ("one sign", (U, np.abs(V) + np.float32(1)))]
+    for name, (U, V) in fields:
+        _, exact = cpsz_b200.debug_eb2d(U, V, eb, ctx=ctx, exact=True)
+        _, fast = cpsz_b200.debug_eb2d(U, V, eb, ctx=ctx, exact=False)
+        bad = np.flatnonzero(exact != fast)
+        assert bad.size == 0, f"{name}: {bad.size} ids differ, first at {bad[:5]}"
