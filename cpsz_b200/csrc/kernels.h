@@ -96,14 +96,18 @@ int launch_requant2d(cpsz_b200_ctx* ctx, const float* U, const float* V, size_t 
 
 // ---- 2D Lorenzo wavefront ------------------------------------------------------
 // One field of the wavefront.  Raster arrays carry their own row pitch (elements).
+// Words per boundary row: the last lane of a group stores eight columns at a
+// time, the first block from column -31, the last up to r2 + 30.
+inline __host__ __device__ size_t wave_gbnd_pitch(int r2) { return ((size_t)r2 + 63) & ~(size_t)1; }
 struct WaveField {
   // per-point input pair: compress (value, bits of 1/precision; NaN for
   // precision 0), decompress (addend 2(code-32768)*p or the raw value, raw flag)
   const float2* pair;
   uint16_t* codes;     // compress: quantization codes out (raster)
   float* out;          // compress: reconstruction (optional tap); decompress: decoded field
-  // last row of every WAVE_GROUP_ROWS-row group, ngroups * r2 tagged words
-  // ((column + 1) << 32 | float bits); zeroed before every launch
+  // last row of every WAVE_GROUP_ROWS-row group, ngroups * wave_gbnd_pitch(r2)
+  // tagged words ((column + 1) << 32 | float bits), column c in word c + 31 of
+  // its row; 16-byte aligned, zeroed before every launch
   unsigned long long* gbnd;
   long long pair_pitch, code_pitch, out_pitch;
   int r1, r2;

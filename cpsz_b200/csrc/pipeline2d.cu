@@ -281,7 +281,7 @@ void pass_alloc(std::vector<Job2D>& jobs, PassBuf& P, Alloc& A) {
     }
     P.zero_bytes = r.at;
     P.gbnd = r.take(0);
-    for (Job2D& j : jobs) j.d.gbnd = (unsigned long long*)r.take(2 * (size_t)j.ngroups * j.r2 * 8);
+    for (Job2D& j : jobs) j.d.gbnd = (unsigned long long*)r.take(2 * j.ngroups * wave_gbnd_pitch(j.r2) * 8);
     P.gbnd_bytes = r.at - P.zero_bytes;
     return r.at;
   };
@@ -559,7 +559,7 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap, 
                     ? ctx->d_wave_trace + (size_t)f * j.ngroups * WAVE_WARPS * 4
                     : nullptr;
       F.out = tap ? tap->recon[f] : nullptr;
-      F.gbnd = j.d.gbnd + (size_t)f * j.ngroups * j.r2;
+      F.gbnd = j.d.gbnd + f * j.ngroups * wave_gbnd_pitch(j.r2);
       F.pair_pitch = j.r2;
       F.code_pitch = j.r2;
       F.out_pitch = j.r2;
@@ -634,9 +634,10 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap, 
   } else {
     const Job2D& j = jobs[0];
     CPSZ_CUDA_TRY(cudaMemsetAsync(P.zero, 0, P.zero_bytes, st));
+    const size_t pitch = wave_gbnd_pitch(j.r2);
     for (int f = 0; f < 2; f++)
-      CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.gbnd + ((size_t)f * j.ngroups + g0) * j.r2, 0,
-                                    (size_t)(j.ngroups - g0) * j.r2 * 8, st));
+      CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.gbnd + ((size_t)f * j.ngroups + g0) * pitch, 0,
+                                    (size_t)(j.ngroups - g0) * pitch * 8, st));
   }
   double* const thr_tab = P.thr;
   int* const queue = P.queue;
@@ -993,7 +994,7 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap, 
       }
       CPSZ_CUDA_TRY(cudaMemcpyAsync(P.fields, hf.data(), hf.size() * sizeof(WaveField), cudaMemcpyHostToDevice, st));
       for (Job2D& j : jobs) {
-        CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.gbnd, 0, 2 * (size_t)j.ngroups * j.r2 * 8, st));
+        CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.gbnd, 0, 2 * j.ngroups * wave_gbnd_pitch(j.r2) * 8, st));
         for (int f = 0; f < 2; f++) {
           CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.hist_codes[f], 0, 65536 * 8, st));
           CPSZ_CUDA_TRY(cudaMemsetAsync(j.d.strip[f], 0, strip_scratch_bytes(j.r1, j.r2), st));
@@ -1348,7 +1349,7 @@ int decompress_2d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
   const bool whole = up.bytes() <= UPLOAD_WHOLE;
   size_t dec_bytes[3];
   for (int k = 0; k < 3; k++) dec_bytes[k] = whole ? (k ? 0 : huff_decode_tmp_bytes(dec, 3)) : huff_decode_tmp_bytes(&dec[k], 1);
-  const size_t strip_bytes = align_up(strip_scratch_bytes(r1, r2), 256), gbnd_bytes = 2 * (size_t)ngroups * r2 * 8;
+  const size_t strip_bytes = align_up(strip_scratch_bytes(r1, r2), 256), gbnd_bytes = 2 * ngroups * wave_gbnd_pitch(r2) * 8;
   const size_t zero_bytes = 256 + 2 * strip_bytes + gbnd_bytes;
   size_t bytes = 0;
   auto add = [&](size_t b) { bytes += align_up(b, 256) + 256; };
@@ -1390,7 +1391,7 @@ int decompress_2d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
     WaveField& F = hf[f];
     F.pair = raw[f];
     F.out = f ? dV : dU;
-    F.gbnd = gbnd + (size_t)f * ngroups * r2;
+    F.gbnd = gbnd + f * ngroups * wave_gbnd_pitch(r2);
     F.pair_pitch = r2;
     F.code_pitch = r2;
     F.out_pitch = r2;

@@ -20,25 +20,30 @@
 //    the raw value, and a raw flag), staged per 32-step window k as a
 //    "parallelogram" tile -- row l holds columns [32k - l, 32k - l + 32),
 //    exactly what lane l touches during steps [32k, 32k + 32) -- filled with
-//    coalesced 8-byte cp.async row copies one window ahead (double buffered)
-//    and drained with coalesced row stores one window behind.  A 33-element
-//    row pitch makes the per-step accesses tile[l][t] bank-conflict free.
-//    Points outside the field are staged as pairs that reconstruct to 0, so a
-//    step has no bounds branches;
+//    coalesced 8-byte cp.async row copies one window ahead (double buffered;
+//    the lines asked for three windows before that, so a copy meets them in
+//    L2) and drained with coalesced row stores one window behind.  A lane
+//    reads two steps and writes four per 16-byte access; the row pitches (34
+//    pairs, 36 words) keep those free of bank conflicts.  Points outside the
+//    field are staged as pairs that reconstruct to 0, so a step has no bounds
+//    branches;
 //  * the staging and draining run in a helper warp paired with each compute
 //    warp (same scheduler; a named barrier per window), so the compute warp's
 //    instruction stream holds only the recurrence, and the helper's
 //    instructions issue in the compute warp's dependency stalls;
-//  * a step has no branches: the hand-off below and the test tap are single
-//    predicated stores, and the tap is a template parameter (a branch in the
-//    step splits it into basic blocks the compiler cannot overlap);
+//  * steps run in blocks of eight without a branch (the test tap is a
+//    predicated store and a template parameter: a branch splits the steps into
+//    basic blocks the compiler cannot overlap).  A block is entered through
+//    one test: the eight columns above are there, and so is room for the eight
+//    that lane 31 writes; what waits is out of line;
 //  * a CTA owns a WAVE_GROUP_ROWS-row group (WAVE_WARPS compute warps; 128
 //    rows, 4 warps: one per scheduler, plus their helpers).  Warp w takes the
-//    row above from warp w-1 through a shared-memory ring of tagged words, 8
-//    columns at a time (one warp-uniform tag test per 8 steps); lane 31
-//    stores one tagged word per step.  The CTA's first warp takes the previous
-//    group's last row from global memory, a whole 32-column window at a time,
-//    validated once per window and loaded coalesced one window ahead;
+//    row above from warp w-1 through a shared-memory ring of tagged words,
+//    read a few steps before the block that needs them; lane 31 stores a
+//    block's eight words as four 16-byte stores at its end.  The CTA's first
+//    warp takes the previous group's last row from global memory: it copies
+//    the words two blocks ahead (an L2 round trip is about a block) into a
+//    ring of its own and reads that like the others;
 //  * CTAs are persistent and pull (field, group) items from a device work
 //    queue (atomic counter).  An item's predecessor (same field, previous
 //    group) was dequeued earlier by a running CTA, so every wait ends;
@@ -54,9 +59,9 @@
 //    when the producer has finished no tile for a while (it is not running
 //    beside it), and the host then runs the wavefront again after it.
 //
-// Tagged words are 64-bit (column + 1) << 32 | float bits, written and read as
-// single aligned 64-bit accesses, so a reader that sees the expected tag holds
-// that column's value and no memory fence is needed.  Every wait is bounded;
+// Tagged words are 64-bit (column + 1) << 32 | float bits, aligned, written and
+// read whole (a 16-byte access moves two of them), so a reader that sees the
+// expected tag holds that column's value and no memory fence is needed.  Every wait is bounded;
 // on expiry the kernel sets FLAG_TIMEOUT and stops waiting.
 //
 // Arithmetic (bit-identical to include/sz_compression_utils.hpp:52-65 and
@@ -65,15 +70,30 @@
 //   reference's capacity test |diff|/p + 1 < 65536 is y < 65535 (y + 1 is
 //   exact in double below 2^16);
 //   (int)((|diff|/p + 1) / 2) = (trunc(y) + 1) >> 1 = floor(y/2 + 1/2), taken
-//   without a conversion: y/2 + 1/2 rounded down keeps its floor, and that
-//   plus 2^23 rounded down is 2^23 + floor exactly;
+//   without a conversion: y/2 + 1/2 rounded down keeps its floor (one
+//   fused multiply-add, the product being exact), and that plus 2^23 rounded
+//   down is 2^23 + floor exactly;
 //   the reference's (float)((double)pred + (double)(2q) * p) equals the float
 //   sum pred + 2q*p: 2q*p is exact in float (|2q| < 2^17), and whenever the
 //   exact sum does not fit a double one addend lies below 2^-5 ulp of the
-//   other, where rounding through double and rounding once agree;
+//   other, where rounding through double and rounding once agree.  It is one
+//   fused multiply-add of q and +-2p; pred + 0 in it makes a zero pred +0, as
+//   adding q = 0's +0 does, and a 2q*p past the largest float (q >= 2^127/p)
+//   stays unpredictable, as it is where the product is rounded;
 //   |dec - x| <= p compares a float against a power of two.
 // Decompression adds the precomputed 2(code - 32768) * p (0 when id = 0) or
 // takes the stored raw value.
+//
+// What bounds it: the step's dependency chain (a shuffle, eleven dependent
+// operations and a select: about 80 cycles when compressing, 48 for the
+// inverse, timed by themselves), the warp's other instructions between them,
+// and the SM's shared-memory pipe, which the four warps' steps and their
+// helpers' copies share.  Compressing, a warp alone takes 57 ns a step (78 with
+// a separate multiply and sign select in the chain, 8-byte tile accesses and a
+// tagged store per step), inside 8192 x 8192 70 ns (100), and a group follows
+// its predecessor by 4.5 us beyond its own rows' skew (10 with a 32-column
+// window of the row above as the unit of waiting): 1.39 ms for both fields of
+// 8192 x 8192 by itself (2.16), 1.08 ms for the inverse (1.61).
 #include "kernels.h"
 #include "tuning.h"
 
@@ -83,9 +103,9 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int RING = 128;
-constexpr int TP = 33;         // tile row pitch (elements)
-constexpr int TILE = 32 * TP;  // elements per tile
-constexpr long long SPIN_LIMIT = 1ll << 22;
+constexpr int TP = 34;  // input tile row pitch (pairs): 16-byte rows whose 16-byte reads meet no bank twice
+constexpr int OP = 36;  // output tile row pitch (words), likewise
+constexpr unsigned SPIN_LIMIT = 1u << 22;
 // A wait for the producer gives up after this long without any of its tiles
 // finishing (it is not running: a tool serialises kernels, or the device is
 // held by other work); the host then runs the wavefront again after it.
@@ -111,15 +131,38 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void cp_async16_if(bool p, unsigned smem, const void* gmem) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q cp.async.cg.shared.global [%1], [%2], 16;\n\t}" ::"r"((unsigned)p),
+               "r"(smem), "l"(gmem)
+               : "memory");
+}
 // Named barrier of one compute warp and its helper warp (ids 1..WAVE_WARPS).
 __device__ __forceinline__ void pair_sync(int strip) { asm volatile("bar.sync %0, 64;" ::"r"(1 + strip) : "memory"); }
 // Stores that only some lanes perform, as single predicated instructions: the
 // per-step hand-off then never splits the warp into divergent paths.
-__device__ __forceinline__ void st_u64_if(bool p, void* addr, unsigned long long v) {
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.volatile.u64 [%1], %2;\n\t}" ::"r"((unsigned)p),
-               "l"(addr), "l"(v));
+__device__ __forceinline__ void sts_2u64_if(unsigned p, unsigned addr, unsigned long long a, unsigned long long b) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.volatile.shared.v2.u64 [%1], {%2, %3};\n\t}" ::"r"(p),
+               "r"(addr), "l"(a), "l"(b));
+}
+__device__ __forceinline__ void stg_2u64_if(unsigned p, void* addr, unsigned long long a, unsigned long long b) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.relaxed.gpu.global.v2.u64 [%1], {%2, %3};\n\t}" ::"r"(p),
+               "l"(addr), "l"(a), "l"(b));
+}
+__device__ __forceinline__ void ldg_u64_if(bool p, unsigned long long& v, const unsigned long long* addr) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t@q ld.relaxed.gpu.global.u64 %0, [%2];\n\t}"
+               : "+l"(v)
+               : "r"((unsigned)p), "l"(addr));
+}
+__device__ __forceinline__ void lds_u64_if(bool p, unsigned long long& v, unsigned addr) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t@q ld.volatile.shared.u64 %0, [%2];\n\t}"
+               : "+l"(v)
+               : "r"((unsigned)p), "r"(addr));
 }
 __device__ __forceinline__ void st_global_f32_if(bool p, void* g, float v) {
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.global.f32 [%1], %2;\n\t}" ::"r"((unsigned)p),
@@ -127,13 +170,24 @@ __device__ __forceinline__ void st_global_f32_if(bool p, void* g, float v) {
                : "memory");
 }
 
-struct WarpTiles {
-  float2 in[2][TILE];
-  uint32_t out[2][TILE];
+__device__ __forceinline__ float4 lds_f4(unsigned addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void sts_u128(unsigned addr, const uint32_t (&v)[4]) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]));
+}
+
+struct __align__(16) WarpTiles {
+  float2 in[2][32 * TP];
+  uint32_t out[2][32 * OP];
 };
 
 struct Shared {
-  unsigned long long ring[WAVE_WARPS][RING];
+  // column c in word c + 31 (mod RING); the last ring holds the previous
+  // group's row, copied ahead by the CTA's first warp
+  __align__(16) unsigned long long ring[WAVE_WARPS + 1][RING];
   volatile int cons[WAVE_WARPS];  // ring columns its consumer has finished with
   int item;
 };
@@ -148,13 +202,19 @@ __device__ __forceinline__ void tile_fill(const WaveField& F, WarpTiles& T, long
                                           int k, int buf) {
   // staged pair of a point outside the field: reconstructs to 0
   const float2 pad = DECOMP ? make_float2(0.f, __int_as_float(1)) : make_float2(0.f, __int_as_float(0x7FC00000));
-  const float2* rp = F.pair + row0 * F.pair_pitch;
-  int c = 32 * k + lane;
+  const float2* rp = F.pair + row0 * F.pair_pitch + (32 * k + lane);
+  const long long step = (long long)F.pair_pitch - 1;
   float2* d = &T.in[buf][lane];
+  if (nrows == 32 && 32 * k >= 31 && 32 * k + 31 < F.r2) {  // every point is in the field
+#pragma unroll 8
+    for (int l = 0; l < 32; l++, rp += step) cp_async8(d + l * TP, rp);
+  } else {
+    int c = 32 * k + lane;
 #pragma unroll 4
-  for (int l = 0; l < 32; l++, c--, d += TP, rp += F.pair_pitch) {
-    if (l < nrows && (unsigned)c < (unsigned)F.r2) cp_async8(d, rp + c);
-    else *d = pad;
+    for (int l = 0; l < 32; l++, c--, d += TP, rp += step) {
+      if (l < nrows && (unsigned)c < (unsigned)F.r2) cp_async8(d, rp);
+      else *d = pad;
+    }
   }
   cp_commit();
 }
@@ -162,14 +222,24 @@ __device__ __forceinline__ void tile_fill(const WaveField& F, WarpTiles& T, long
 template <bool DECOMP>
 __device__ __forceinline__ void tile_drain(const WaveField& F, const WarpTiles& T, long long row0, int nrows, int lane,
                                            int k, int buf) {
-  int c = 32 * k + lane;
   const uint32_t* s = &T.out[buf][lane];
-  long long r = row0;
-  for (int l = 0; l < nrows; l++, c--, s += TP, r++) {
-    if ((unsigned)c < (unsigned)F.r2) {
-      const uint32_t v = *s;
-      if (DECOMP) F.out[r * F.out_pitch + c] = __uint_as_float(v);
-      else F.codes[r * F.code_pitch + c] = (uint16_t)v;
+  const int c0 = 32 * k + lane;
+  float* of = DECOMP ? F.out + row0 * F.out_pitch + c0 : nullptr;
+  uint16_t* oc = DECOMP ? nullptr : F.codes + row0 * F.code_pitch + c0;
+  const bool inner = nrows == 32 && 32 * k >= 31 && 32 * k + 31 < F.r2;
+  // eight rows are read before the first is written: one shared-memory latency
+  for (int l0 = 0; l0 < nrows; l0 += 8) {
+    uint32_t v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = s[(l0 + j) * OP];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      if (inner || (l0 + j < nrows && (unsigned)(c0 - l0 - j) < (unsigned)F.r2)) {
+        if (DECOMP) *of = __uint_as_float(v[j]);
+        else *oc = (uint16_t)v[j];
+      }
+      if (DECOMP) of += F.out_pitch - 1;
+      else oc += F.code_pitch - 1;
     }
   }
 }
@@ -225,13 +295,18 @@ __device__ __forceinline__ void run_helper(const WaveField& F, int group, int st
   int ready = 0;
   if (waits) wait_units(F, group, 0, lane, ready, flag);
   tile_fill<DECOMP>(F, T, row0, nrows, lane, 0, 0);
-  cp_wait_all();
+  cp_wait<0>();
   for (int k = 0; k < nwin; k++) {
     pair_sync(strip);  // the compute warp starts window k (tiles buf = k & 1)
     if (waits && k + 1 < nwin) wait_units(F, group, k + 1, lane, ready, flag);
     if (k + 1 < nwin) tile_fill<DECOMP>(F, T, row0, nrows, lane, k + 1, (k + 1) & 1);
+    if (lane < nrows && 32 * (k + 4) < F.r2) {
+      const float2* pf = F.pair + (row0 + lane) * F.pair_pitch + (32 * (k + 4) - lane);
+      prefetch_l2(pf);
+      prefetch_l2(pf - 16);
+    }
     if (k >= 1) tile_drain<DECOMP>(F, T, row0, nrows, lane, k - 1, (k - 1) & 1);
-    cp_wait_all();
+    cp_wait<0>();
   }
   pair_sync(strip);  // the compute warp has finished the last window
   tile_drain<DECOMP>(F, T, row0, nrows, lane, nwin - 1, (nwin - 1) & 1);
@@ -250,159 +325,146 @@ __device__ __forceinline__ void run_strip(const WaveField& F, int group, int war
   const bool has_below = row0 + 32 < r1;
   const bool below_global = has_below && warp == WAVE_WARPS - 1;
   const bool below_ring = has_below && !below_global;
-  const unsigned long long* gb_in = above_global ? F.gbnd + (size_t)(group - 1) * r2 : nullptr;
-  unsigned long long* gb_out = F.gbnd + (size_t)group * r2;
+  const unsigned to_ring = below_ring & (lane == 31), to_global = below_global & (lane == 31);
+  const unsigned long long* gb_in = above_global ? F.gbnd + (size_t)(group - 1) * wave_gbnd_pitch(r2) : F.gbnd;
+  unsigned long long* gb_out = F.gbnd + (size_t)group * wave_gbnd_pitch(r2);
+  const unsigned ring_in = (unsigned)__cvta_generic_to_shared(&sh.ring[warp > 0 ? warp - 1 : WAVE_WARPS][0]);
+  const unsigned ring_out = (unsigned)__cvta_generic_to_shared(&sh.ring[warp][0]);
 
-  int credit = RING;  // ring columns this warp may write before re-reading its consumer's progress
+  // ring columns this warp may write before re-reading its consumer's progress
+  int credit = below_ring ? RING : 0x7fffffff;
   bool aborted = false;
-  long long spin_above = 0, spin_credit = 0;
+  unsigned spin_above = 0, spin_credit = 0;
   const long long t_start = F.trace ? globaltimer_ns() : 0;
   float outPrev = 0.f, upPrev = 0.f;
   const int nwin = (r2 + 31 + 31) / 32;  // windows that contain any step
-  auto ring_word = [&](int c) -> unsigned long long {
-    return *(volatile unsigned long long*)&sh.ring[warp - 1][c & (RING - 1)];
+  // The row above: lane j (mod 8) holds the tagged word of column cb + j, read
+  // from a ring a few steps before the block starts.  The previous group's
+  // words are copied into theirs two blocks ahead (an L2 round trip).
+  const int lane8 = lane & 7;
+  const bool copies = above_global && lane < 5;  // 16-byte pieces of columns c - 1 .. c + 8
+  const int gb_words = (int)wave_gbnd_pitch(r2);
+  auto copy_above = [&](int c) {
+    const int i = c + 30 + 2 * lane;
+    cp_async16_if(copies && i < gb_words, ring_in + 8u * (unsigned)(i & (RING - 1)), gb_in + i);
+    cp_commit();
   };
-  // coalesced prefetch of the previous group's last row, one window ahead
-  unsigned long long gcur = 0, gnext = 0;
-  auto gload = [&](int k) -> unsigned long long {
-    const int c = 32 * k + lane;
-    return (c < r2) ? __ldcg(gb_in + c) : 0ull;
+  auto ring_word = [&](unsigned long long& v, int c) {
+    lds_u64_if(has_above, v, ring_in + 8u * (unsigned)((c + 31) & (RING - 1)));
   };
-
-  if (above_global) gnext = gload(0);
-  for (int k = 0; k < nwin; k++) {
-    const int buf = k & 1;
-    pair_sync(warp);  // window k is staged; window k-1's outputs are handed to the helper
-    if (above_global) {
-      // the whole window of the row above must be present: one poll per window
-      gcur = gnext;
-      const int cl = 32 * k + lane;
-      bool ok = cl >= r2 || tag_is(gcur, cl);
-      long long spins = 0;
-      while (!__all_sync(FULL, ok) && !aborted) {
+  auto global_word = [&](unsigned long long& v, int c) { ldg_u64_if(above_global, v, gb_in + 31 + min(c, r2 - 1)); };
+  unsigned long long wn = 0ull;
+  float av = 0.f;
+  // Everything the block at cb needs is there: the eight columns above, and
+  // room in the ring for the eight that lane 31 writes.  One test, one branch.
+  auto enter_block = [&](int cb, unsigned long long w) {
+    const int c = cb + lane8;
+    const bool ok = !has_above || c >= r2 || tag_is(w, c);
+    if (!__all_sync(FULL, ok & (cb - 24 < credit))) {
+      unsigned spins = 0;
+      bool have = ok;
+      while (!aborted && !__all_sync(FULL, have)) {
         if (++spins > SPIN_LIMIT) {
           if (lane == 0) atomicOr(flag, FLAG_TIMEOUT);
           aborted = true;
           break;
         }
-        __nanosleep(100);
-        if (!ok) {
-          gcur = __ldcg(gb_in + cl);
-          ok = tag_is(gcur, cl);
-        }
+        if (spins > 64) __nanosleep(100);
+        ring_word(w, c);
+        global_word(w, c);
+        have = c >= r2 || tag_is(w, c);
       }
       spin_above += spins;
-      gnext = gload(k + 1);
+      spins = 0;
+      while (!aborted && cb - 24 >= credit) {
+        if (++spins > SPIN_LIMIT) {
+          if (lane == 0) atomicOr(flag, FLAG_TIMEOUT);
+          aborted = true;
+          break;
+        }
+        if (spins > 64) __nanosleep(100);
+        credit = sh.cons[warp + 1] + RING;
+      }
+      spin_credit += spins;
+      if (aborted) w = 0ull;
     }
-    const float2* tin = &T.in[buf][lane * TP];
-    uint32_t* to = &T.out[buf][lane * TP];
+    av = tag_val(w);
+  };
+
+  copy_above(0);
+  copy_above(8);
+  cp_wait<1>();
+  __syncwarp();
+  ring_word(wn, lane8);
+  enter_block(0, wn);
+  for (int k = 0; k < nwin; k++) {
+    pair_sync(warp);  // window k is staged; window k-1's outputs are handed to the helper
+    const unsigned tin = (unsigned)__cvta_generic_to_shared(&T.in[k & 1][lane * TP]);
+    const unsigned to = (unsigned)__cvta_generic_to_shared(&T.out[k & 1][lane * OP]);
 #pragma unroll 1
     for (int tb = 0; tb < 32; tb += 8) {
       const int cb = 32 * k + tb;  // lane 0's column at the block's first step
-      // ---- the row above, 8 columns (all lanes hold lane 0's values) ----
-      float ab[8];
-      if (above_global) {
+      copy_above(cb + 16);
+      float4 e[4];  // (value, 1/precision or flag) of two steps each
+      uint32_t o4[4];
 #pragma unroll
-        for (int j = 0; j < 8; j++) ab[j] = tag_val(__shfl_sync(FULL, gcur, tb + j));
-      } else if (above_ring) {
-        unsigned long long wv[8];
-        bool ok = true;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-          wv[j] = ring_word(cb + j);
-          ok &= (cb + j >= r2) | tag_is(wv[j], cb + j);
-        }
-        if (!ok && !aborted) {  // warp-uniform: all lanes read the same words
-          long long spins = 0;
-          do {
-            if (++spins > SPIN_LIMIT) {
-              if (lane == 0) atomicOr(flag, FLAG_TIMEOUT);
-              aborted = true;
-              break;
-            }
-            ok = true;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-              wv[j] = ring_word(cb + j);
-              ok &= (cb + j >= r2) | tag_is(wv[j], cb + j);
-            }
-          } while (!ok);
-          spin_above += spins;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; j++) ab[j] = tag_val(wv[j]);
-        if (lane == 0) sh.cons[warp] = cb;  // columns below cb have been consumed
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; j++) ab[j] = 0.f;
-      }
-      if (aborted) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) ab[j] = 0.f;
-      }
-      // ---- ring credit for the 8 columns lane 31 writes in this block ----
-      if (below_ring) {
-        const int cmax = cb - 24;
-        if (cmax >= credit && !aborted) {
-          long long spins = 0;
-          int v = sh.cons[warp + 1];
-          while (v + RING <= cmax) {
-            if (++spins > SPIN_LIMIT) {
-              if (lane == 0) atomicOr(flag, FLAG_TIMEOUT);
-              aborted = true;
-              break;
-            }
-            v = sh.cons[warp + 1];
-          }
-          spin_credit += spins;
-          credit = v + RING;
-        }
-      }
+      for (int j = 0; j < 4; j++) e[j] = lds_f4(tin + 8u * (tb + 2 * j));
+      float h8[8];
       // ---- 8 steps ----
 #pragma unroll
       for (int j = 0; j < 8; j++) {
-        const int t = tb + j;
+        const float x = (j & 1) ? e[j / 2].z : e[j / 2].x, second = (j & 1) ? e[j / 2].w : e[j / 2].y;
+        const float ab = __shfl_sync(FULL, av, j);
         const float shfl = __shfl_up_sync(FULL, outPrev, 1);
-        const float U = (lane == 0) ? ab[j] : shfl;
+        const float U = (lane == 0) ? ab : shfl;
         const float pred = (outPrev + U) - upPrev;
-        const float2 e = tin[t];
         float out;
         if (DECOMP) {
-          out = (__float_as_int(e.y) != 0) ? e.x : pred + e.x;
-          to[t] = __float_as_uint(out);
+          out = (__float_as_int(second) != 0) ? x : pred + x;
+          o4[j & 3] = __float_as_uint(out);
         } else {
-          const float x = e.x, inv = e.y;  // inv = 1/p (NaN for precision 0)
+          const float inv = second;  // 1/p (NaN for precision 0)
           const float p = __int_as_float(0x7F000000 - __float_as_int(inv));
+          const float lim = fminf(32768.f, inv * 0x1p127f);
           const float diff = x - pred;
-          // q = (trunc(y) + 1) >> 1 = floor(y/2 + 1/2) for y = |diff|/p >= 0.
-          // y/2 = |diff| * (inv/2) is exact; rounding y/2 + 1/2 down keeps
-          // its floor, and rounding that plus 2^23 down yields 2^23 + floor
-          // exactly (for y >= 2^24 the point is unpredictable anyway).
-          const float h = fabsf(diff) * (0.5f * inv);
-          const float mq = __fadd_rd(__fadd_rd(h, 0.5f), 8388608.0f);
-          const float qf = mq - 8388608.0f;
-          // 0 - qf keeps q = 0 a +0 addend (as the decoder's 2(code - 32768) * p is)
-          const float dec = pred + ((diff > 0.f) ? qf : 0.f - qf) * (p + p);
-          const bool ok = (h < 32767.5f) & (fabsf(dec - x) <= p);
+          const unsigned neg = __float_as_uint(diff) & 0x80000000u;
+          const float m = __fmaf_rd(fabsf(diff), 0.5f * inv, 0.5f);
+          const float qf = __fadd_rd(m, 8388608.0f) - 8388608.0f;
+          const float dec = __fmaf_rn(qf, __uint_as_float(__float_as_uint(p + p) | neg), pred + 0.f);
+          const bool ok = (m < lim) & (fabsf(dec - x) <= p);
           out = ok ? dec : x;
-          const int qa = __float_as_int(mq) - 0x4B000000;
-          to[t] = ok ? (uint32_t)(((diff > 0.f) ? qa : -qa) + 32768) : 0u;
+          const float cf = __fmaf_rn(qf, __uint_as_float(0x3F800000u | neg), 8388608.0f + 32768.0f);
+          o4[j & 3] = ok ? __float_as_uint(cf) : 0u;
           if (TAP) {  // optional reconstruction tap (tests)
             const int c = cb + j - lane;
             st_global_f32_if((lane < nrows) & ((unsigned)c < (unsigned)r2),
                              F.out + (long long)(row0 + lane) * F.out_pitch + c, out);
           }
         }
-        // lane 31 hands its row down (column cb + j - 31)
-        const int c31 = cb + j - 31;
-        const bool w31 = (lane == 31) & ((unsigned)c31 < (unsigned)r2) & has_below;
-        st_u64_if(w31, below_ring ? (void*)&sh.ring[warp][c31 & (RING - 1)] : (void*)(gb_out + c31), tagged(c31, out));
+        if ((j & 3) == 3) sts_u128(to + 4u * (tb + j - 3), o4);
+        h8[j] = out;
         upPrev = U;
         outPrev = out;
+        if (j == 5) {
+          cp_wait<1>();
+          __syncwarp();
+          ring_word(wn, cb + 8 + lane8);
+          if (lane == 0) sh.cons[warp] = cb + 8;  // columns below this have been consumed
+        }
       }
+      // lane 31 hands its row down, columns cb - 31 .. cb - 24 (those outside
+      // the row land in the slack and in ring words no reader waits for)
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) {
+        sts_2u64_if(to_ring, ring_out + 8u * (unsigned)((cb + j) & (RING - 1)), tagged(cb + j - 31, h8[j]),
+                    tagged(cb + j - 30, h8[j + 1]));
+        stg_2u64_if(to_global, gb_out + cb + j, tagged(cb + j - 31, h8[j]), tagged(cb + j - 30, h8[j + 1]));
+      }
+      enter_block(cb + 8, wn);
     }
   }
   pair_sync(warp);  // the last window's outputs go to the helper
+  cp_wait<0>();
   if (lane == 0 && above_ring) sh.cons[warp] = r2 + RING;
   if (F.trace && lane == 0) {
     long long* tr = F.trace + ((long long)group * WAVE_WARPS + warp) * 4;
@@ -423,7 +485,7 @@ __device__ __forceinline__ void wave2d_body(const WaveField* __restrict__ fields
   const int strip = warp % WAVE_WARPS;  // the strip a compute warp runs, or its helper serves
   for (;;) {
     if (threadIdx.x == 0) sh.item = atomicAdd(queue, 1);
-    for (int k = threadIdx.x; k < WAVE_WARPS * RING; k += blockDim.x) (&sh.ring[0][0])[k] = 0ull;
+    for (int k = threadIdx.x; k < (WAVE_WARPS + 1) * RING; k += blockDim.x) (&sh.ring[0][0])[k] = 0ull;
     if (threadIdx.x < WAVE_WARPS) sh.cons[threadIdx.x] = 0;
     __syncthreads();
     const int it = sh.item;
