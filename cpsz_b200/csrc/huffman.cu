@@ -5,11 +5,11 @@
 // Encoder.  The reference's packer (encode, src/sz_huffman.cpp:217-320) emits
 // the MSB-first concatenation of the codes, zero padded to a byte.  Here one
 // persistent kernel reads every symbol once: a tile of 8192 consecutive
-// symbols sums and scans its code lengths, finds its starting bit by a
-// decoupled look-back over the earlier tiles' published bit counts, packs its
-// codes into a shared-memory word buffer aligned to the global 32-bit word
-// grid and stores it with coalesced stores (atomicOr for the two edge words,
-// shared with the neighbouring tiles).  Words are stored byte-swapped so
+// symbols sums and scans its code lengths, packs its codes into a
+// shared-memory word buffer, finds its starting bit by a decoupled look-back
+// over the earlier tiles' published bit counts, and stores the buffer shifted
+// onto the global 32-bit word grid with coalesced stores (atomicOr for the two
+// edge words, shared with the neighbouring tiles).  Words are stored byte-swapped so
 // memory holds the big-endian byte stream the reference writes.
 #include <algorithm>
 
@@ -32,6 +32,12 @@ constexpr long long PK_SPIN_LIMIT = 1ll << 22;  // look-back polls before giving
 
 __device__ __forceinline__ uint32_t bswap32(uint32_t x) { return __byte_perm(x, 0, 0x0123); }
 
+__device__ __forceinline__ void sts_u32_if(bool p, unsigned addr, uint32_t v) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.shared.u32 [%1], %2;\n\t}" ::"r"((unsigned)p),
+               "r"(addr), "r"(v)
+               : "memory");
+}
+
 template <class Sym>
 struct PackWin {
   static constexpr int lo = sizeof(Sym) == 1 ? 0 : PK_WIN_LO;
@@ -52,10 +58,10 @@ __device__ __forceinline__ int find_job(const Job* __restrict__ jobs, int n, uns
 }
 
 struct PackShared {
-  uint32_t words[PK_WORDS];     // the tile's packed bits from its first bit (tile-relative)
-  uint32_t lcode[PK_WIN];       // codes of at most 32 bits, left-aligned (0 for longer codes)
+  uint32_t words[PK_WORDS];  // the tile's packed bits from its first bit (tile-relative)
+  uint32_t lcode[PK_WIN];    // codes of at most 32 bits, left-aligned (0 for longer codes)
   uint8_t len[PK_WIN];
-  unsigned int warp_bits[PK_NT / 32];
+  unsigned int warp_bits[2][PK_NT / 32];
   unsigned long long excl;
   unsigned int tile;
 };
@@ -78,21 +84,36 @@ __device__ __forceinline__ uint32_t pk_lcode(const PackShared& sh, unsigned s, u
 }
 
 // Persistent packer.  Tiles of PK_TILE symbols are taken in order from a
-// ticket; thread t of a tile owns its symbols t*32 .. t*32+31.  Per tile:
-//   1. code lengths (kept in registers) summed and scanned in the CTA; the
-//      tile's bit count is published for the look-back (lookback.cuh);
-//   2. the codes are packed tile-relative into the shared word buffer: each
-//      thread appends its codes to a 64-bit register and stores every word
-//      it completes (a word is completed by exactly one thread, which also
-//      zeroes the bits of earlier threads in it); after a barrier each
-//      thread ORs in its last, partial word;
-//   3. warp 0 finds the tile's starting bit (by now the predecessors have
-//      mostly published); the buffer goes out shifted onto the global word
-//      grid with coalesced stores, the two edge words (shared with the
-//      neighbouring tiles) by atomicOr.
+// ticket; thread t of a tile owns its symbols t*32 .. t*32+31.
+//   1. A tile is taken: its symbols are read, their code lengths (kept in
+//      registers) summed and scanned in the CTA, and its bit count published
+//      for the look-back (lookback.cuh).
+//   2. The codes are packed tile-relative into the shared word buffer: each
+//      thread appends its codes to a 32-bit register and stores every word it
+//      completes (a word is completed by exactly one thread, which also zeroes
+//      the bits of earlier threads in it); after a barrier each thread ORs in
+//      its last, partial word.
+//   3. The next tile is taken (1), and only then does warp 0 find the starting
+//      bit of the one that is packed: its predecessors had that long to
+//      publish, so the look-back is one round trip and waits for nobody.  A
+//      ticket's count is always published without a wait on another CTA in
+//      between, or the look-backs would hold one another up (a ticket taken a
+//      whole tile ahead doubled the kernel's time).
+//   4. The buffer goes out shifted onto the global word grid with coalesced
+//      stores, the two edge words (shared with the neighbouring tiles) by
+//      atomicOr.
 // A tile with a code longer than 32 bits (possible only for skewed
-// histograms) finds its starting bit first and ORs its words straight into
-// global memory.  The stream starts at bit `bit0` (0-31) of out[0].
+// histograms) skips 2 and ORs its words straight into global memory.  The
+// stream starts at bit `bit0` (0-31) of out[0].
+//
+// Bound by the latency between its barriers (a ticket, the symbols, a
+// look-back, the stores) at half the chip's warps, and by issue: 45 thread
+// instructions a u16 symbol, 29 an id.  Both code streams of 8192 x 8192 take
+// .49 ms; .59 with the look-back directly after the packing and a 64-bit
+// append under a branch.  Measured and no better: five or three CTAs an SM,
+// 16 symbols a thread at 256 or 512 threads (.78-.86), codes kept beside the
+// lengths (spills), a window lookup without the fallback (a sixth fewer
+// instructions, the same time).
 template <class Sym, bool MAP0>
 __device__ __forceinline__ void pack_stream(const PackJob& J, PackShared& sh, int* __restrict__ flag) {
   const Sym* __restrict__ sym = static_cast<const Sym*>(J.sym);
@@ -111,21 +132,23 @@ __device__ __forceinline__ void pack_stream(const PackJob& J, PackShared& sh, in
   constexpr unsigned SMASK = sizeof(Sym) == 1 ? 0xffu : 0xffffu;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < W::n; i += PK_NT) {
-    const int s = W::lo + i;
-    const unsigned l = s < nsym ? len[s] : 0u;
+    int v = W::lo + i;
+    if (MAP0 && v == (int)ID_ZERO) v = 0;  // the stream's zero id is symbol 0
+    const unsigned l = v < nsym ? len[v] : 0u;
     sh.len[i] = (uint8_t)l;
-    sh.lcode[i] = (l >= 1 && l <= 32) ? (uint32_t)(code[s] << (32 - l)) : 0u;
+    sh.lcode[i] = (l >= 1 && l <= 32) ? (uint32_t)(code[v] << (32 - l)) : 0u;
   }
   const bool vec_ok = ((uintptr_t)sym & 15) == 0;
-  for (;;) {
-    if (tid == 0) sh.tile = atomicAdd(ticket, 1u);
-    __syncthreads();  // also: the codebook window is in place
-    const unsigned long long tile = sh.tile;
-    if (tile >= ntiles) break;
+  const unsigned words0 = (unsigned)__cvta_generic_to_shared(&sh.words[0]);
+  // A tile in flight: its symbols, their code lengths (4 to a register), the
+  // thread's bits and where they start among the tile's.
+  uint32_t w[NW] = {}, lw[PK_SPT / 4];
+  unsigned int bits = 0, tpre = 0, agg = 0;
+  bool any_long = false;
+  auto sym_k = [&](int k) -> unsigned { return (w[k / W::per_word] >> (SB * (k % W::per_word))) & SMASK; };
+  auto take = [&](unsigned long long tile, int par) {
     const size_t my = (size_t)tile * PK_TILE + (size_t)tid * PK_SPT;
-    const int cnt = my >= n ? 0 : (int)((n - my) < (size_t)PK_SPT ? (n - my) : (size_t)PK_SPT);
-    uint32_t w[NW];
-    if (cnt == PK_SPT && vec_ok) {
+    if (my + PK_SPT <= n && vec_ok) {
       const uint4* src = reinterpret_cast<const uint4*>(sym + my);
 #pragma unroll
       for (int q = 0; q < NW / 4; q++) {
@@ -140,80 +163,99 @@ __device__ __forceinline__ void pack_stream(const PackJob& J, PackShared& sh, in
       for (int q = 0; q < NW; q++) w[q] = 0;
 #pragma unroll
       for (int k = 0; k < PK_SPT; k++)
-        if (k < cnt) w[k / W::per_word] |= (uint32_t)sym[my + k] << (SB * (k % W::per_word));
+        if (my + k < n) w[k / W::per_word] |= (uint32_t)sym[my + k] << (SB * (k % W::per_word));
     }
-    auto sym_k = [&](int k) -> unsigned {
-      unsigned s = (w[k / W::per_word] >> (SB * (k % W::per_word))) & SMASK;
-      if (MAP0 && s == ID_ZERO) s = 0;
-      return s;
-    };
-    // 1. lengths, 4 to a register
-    uint32_t lw[PK_SPT / 4];
-    unsigned int bits = 0;
-    bool lng = false;
+    unsigned int b = 0, lmax = 0;
 #pragma unroll
     for (int k = 0; k < PK_SPT; k++) {
-      const unsigned l = k < cnt ? pk_len<Sym>(sh, sym_k(k), len) : 0u;
-      bits += l;
-      lng |= l > 32;
+      const unsigned l = pk_len<Sym>(sh, sym_k(k), len);
+      b += l;
+      lmax = max(lmax, l);
       lw[k / 4] = (k % 4) ? (lw[k / 4] | (l << (8 * (k % 4)))) : l;
     }
-    unsigned int x = bits;
+    if (my + PK_SPT > n) {  // the stream's end: no bits past it
+      b = lmax = 0;
+      const int cnt = my >= n ? 0 : (int)(n - my);
+#pragma unroll
+      for (int k = 0; k < PK_SPT; k++) {
+        if (k >= cnt) lw[k / 4] &= ~(255u << (8 * (k % 4)));
+        const unsigned l = (lw[k / 4] >> (8 * (k % 4))) & 255u;
+        b += l;
+        lmax = max(lmax, l);
+      }
+    }
+    unsigned int x = b;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned int y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
-    if (lane == 31) sh.warp_bits[warp] = x;
-    const bool any_long = __syncthreads_or(lng) != 0;
-    unsigned int wpre = 0, agg = 0;
+    if (lane == 31) sh.warp_bits[par][warp] = x;
+    any_long = __syncthreads_or(lmax > 32) != 0;
+    unsigned int wpre = 0;
+    agg = 0;
 #pragma unroll
     for (int q = 0; q < PK_NT / 32; q++) {
-      const unsigned int v = sh.warp_bits[q];
+      const unsigned int v = sh.warp_bits[par][q];
       wpre += q < warp ? v : 0u;
       agg += v;
     }
-    const unsigned int tpre = wpre + x - bits;
-    auto len_k = [&](int k) -> unsigned { return (lw[k / 4] >> (8 * (k % 4))) & 255u; };
-    unsigned long long excl;
+    bits = b;
+    tpre = wpre + x - b;
+    if (tid == 0) lookback_publish(state, tile, agg);
+  };
 
-    if (!any_long) {
-      // 2. tile-relative packing; nobody completes the last partial word
-      if (tid == 0) {
-        lookback_publish(state, tile, agg);
-        if (agg & 31) sh.words[agg >> 5] = 0;
-      }
-      int wi = (int)(tpre >> 5);
-      int nacc = (int)(tpre & 31);  // leading bits of word wi belong to earlier threads
-      unsigned long long acc = 0;   // pending bits, most significant first
+  if (tid == 0) sh.tile = atomicAdd(ticket, 1u);
+  __syncthreads();  // also: the codebook window is in place
+  unsigned long long tile = sh.tile;
+  if (tile >= ntiles) return;
+  take(tile, 0);
+  for (int par = 1;; par ^= 1) {
+    unsigned int after = 0;
+    if (tid == 0) after = atomicAdd(ticket, 1u);
+    // 2. tile-relative packing; nobody completes the last partial word
+    const bool packed = !any_long;
+    const unsigned int t_agg = agg, t_pre = tpre;
+    uint32_t acc = 0;  // the word at `at` so far
+    unsigned nacc = tpre & 31;  // leading bits of its first word belong to earlier threads
+    unsigned at = words0 + 4u * (tpre >> 5);
+    if (packed) {
+      if (tid == 0 && (agg & 31)) sh.words[agg >> 5] = 0;
 #pragma unroll
       for (int k = 0; k < PK_SPT; k++) {
-        if (k < cnt) {
-          const unsigned l = len_k(k);
-          acc |= (unsigned long long)pk_lcode<Sym>(sh, sym_k(k), l, code) << (32 - nacc);
-          nacc += (int)l;
-          if (nacc >= 32) {
-            sh.words[wi++] = (uint32_t)(acc >> 32);
-            acc <<= 32;
-            nacc -= 32;
-          }
-        }
+        const unsigned l = (lw[k / 4] >> (8 * (k % 4))) & 255u;
+        const uint32_t c = pk_lcode<Sym>(sh, sym_k(k), l, code);
+        acc |= c >> nacc;
+        const uint32_t rest = __funnelshift_r(0u, c, nacc);  // the code's bits past that word
+        nacc += l;
+        // a completed word, as one predicated store
+        const bool full = nacc >= 32;
+        sts_u32_if(full, at, acc);
+        acc = full ? rest : acc;
+        at += full ? 4u : 0u;
+        nacc &= 31;
       }
-      __syncthreads();  // every completed word is in place
-      if (bits > 0 && nacc > 0) atomicOr(&sh.words[wi], (uint32_t)(acc >> 32));
-      __syncthreads();
-      // 3. the starting bit, then the words onto the global grid
-      if (warp == 0) {
-        const unsigned long long e = lookback_warp(state, tile, agg, lane, PK_SPIN_LIMIT, flag);
-        if (lane == 0) sh.excl = e;
-      }
-      __syncthreads();
-      excl = sh.excl;
-      const unsigned long long s0 = (unsigned long long)bit0 + excl;
+    }
+    if (tid == 0) sh.tile = after;
+    __syncthreads();  // every completed word is in place
+    // (symbols past the stream's end have left bits below the last code's)
+    if (packed && bits > 0 && nacc > 0) atomicOr(&sh.words[(at - words0) >> 2], acc & ~(0xffffffffu >> nacc));
+    const unsigned long long next = sh.tile;
+    if (next < ntiles) take(next, par);
+    else __syncthreads();
+    // 3. the starting bit, then the words onto the global grid
+    if (warp == 0) {
+      const unsigned long long e = lookback_warp(state, tile, t_agg, lane, PK_SPIN_LIMIT, flag);
+      if (lane == 0) sh.excl = e;
+    }
+    __syncthreads();
+    const unsigned long long excl = sh.excl;
+    const unsigned long long s0 = (unsigned long long)bit0 + excl;
+    const unsigned long long w_lo = s0 >> 5;
+    if (packed) {
       const unsigned int shift = (unsigned int)(s0 & 31);
-      const unsigned long long w_lo = s0 >> 5;
-      const int nrel = (int)((agg + 31) >> 5);
-      const int nout = agg ? (int)((shift + agg - 1) >> 5) + 1 : 0;
+      const int nrel = (int)((t_agg + 31) >> 5);
+      const int nout = t_agg ? (int)((shift + t_agg - 1) >> 5) + 1 : 0;
       for (int k = tid; k < nout; k += PK_NT) {
         const unsigned long long g = w_lo + (unsigned long long)k;
         if (g >= cap_words) {
@@ -227,20 +269,13 @@ __device__ __forceinline__ void pack_stream(const PackJob& J, PackShared& sh, in
         else out[g] = v;
       }
     } else {
-      // a code longer than 32 bits: the starting bit first, every word ORed
-      if (warp == 0) {
-        if (lane == 0) lookback_publish(state, tile, agg);
-        const unsigned long long e = lookback_warp(state, tile, agg, lane, PK_SPIN_LIMIT, flag);
-        if (lane == 0) sh.excl = e;
-      }
-      __syncthreads();
-      excl = sh.excl;
-      const unsigned long long s0 = (unsigned long long)bit0 + excl;
-      const unsigned long long w_lo = s0 >> 5;
-      const unsigned int pos = (unsigned int)(s0 & 31) + tpre;
+      // a code longer than 32 bits: every word ORed
+      const size_t my = (size_t)tile * PK_TILE + (size_t)tid * PK_SPT;
+      const unsigned int pos = (unsigned int)(s0 & 31) + t_pre;
       int wi = (int)(pos >> 5);
       int nacc = (int)(pos & 31);
       unsigned long long acc = 0;
+      bool any = false;
       auto emit = [&]() {
         const unsigned long long g = w_lo + (unsigned long long)wi;
         if (g < cap_words) atomicOr(&out[g], bswap32((uint32_t)(acc >> 32)));
@@ -256,11 +291,12 @@ __device__ __forceinline__ void pack_stream(const PackJob& J, PackShared& sh, in
           nacc -= 32;
         }
       };
-      for (int k = 0; k < cnt; k++) {
+      for (int k = 0; k < PK_SPT && my + k < n; k++) {
         unsigned s = (unsigned)sym[my + k];
         if (MAP0 && s == ID_ZERO) s = 0;
         const int l = __ldg(len + s);
         const unsigned long long c = __ldg(code + s);
+        any |= l > 0;
         if (l > 32) {
           put((uint32_t)(c >> 32) & (uint32_t)((1ull << (l - 32)) - 1), l - 32);
           put((uint32_t)c, 32);
@@ -268,10 +304,12 @@ __device__ __forceinline__ void pack_stream(const PackJob& J, PackShared& sh, in
           put((uint32_t)c & (uint32_t)((1ull << l) - 1), l);
         }
       }
-      if (bits > 0 && nacc > 0) emit();
+      if (any && nacc > 0) emit();
     }
-    if (tile == ntiles - 1 && tid == 0 && d_total) *d_total = excl + agg;
-    __syncthreads();  // the shared buffers are reused by the next tile
+    if (tile == ntiles - 1 && tid == 0 && d_total) *d_total = excl + t_agg;
+    if (next >= ntiles) break;
+    tile = next;
+    __syncthreads();  // the words are written again
   }
 }
 
@@ -326,7 +364,7 @@ size_t pack_scratch_words(size_t n) { return (n + PK_TILE - 1) / PK_TILE + 1; }
 
 // CTAs of one of `streams` streams: its share of a full device, or one per
 // PK_TILES_PER_CTA tiles if that is more (a CTA loads its stream's codebook
-// window once, about a quarter of a tile's time).
+// window once, whatever it packs).
 constexpr size_t PK_TILES_PER_CTA = 4;
 unsigned pack_ctas(int num_sms, size_t n, int streams) {
   const size_t ntiles = (n + PK_TILE - 1) / PK_TILE, cap = (size_t)num_sms * PK_CTAS_PER_SM;

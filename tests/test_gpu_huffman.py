@@ -88,6 +88,17 @@ def test_gpu_huffman_unaligned_symbols(ctx, oracle, offset):
     _check_packing(ctx, oracle, sym, offset)
 
 
+@pytest.mark.parametrize("n", [2, 31, 33, 8191, 8192, 8193, 8224, 16384, 16385, 24577])
+@pytest.mark.parametrize("spread", [1.0, 900.0])
+def test_gpu_huffman_tile_edges(ctx, oracle, n, spread):
+    """Streams that end at and around a thread's 32 symbols and a tile's 8192, inside the cached part
+    of the codebook and across its ends."""
+    rng = np.random.default_rng(n)
+    sym = (32768 + np.round(rng.laplace(0, spread, n))).clip(0, 65535).astype(np.int32)
+    sym[rng.integers(0, n)] = 0
+    _check_packing(ctx, oracle, sym)
+
+
 def test_gpu_huffman_rejects_small_output(ctx):
     torch = pytest.importorskip("torch")
     sym = np.random.default_rng(1).integers(100, 5000, 50_000).astype(np.int32)
