@@ -104,15 +104,28 @@ __global__ void __launch_bounds__(SCAN_NT) scan_down_kernel(const unsigned int* 
 
 // ---- strips: a 12-row block row cut into runs of STRIP_BLOCKS blocks ----------------
 // A strip's blocks are consecutive in block order, so its block-order image is
-// one contiguous range.  A CTA stages the strip in shared memory as rows and
-// moves it between the two orders with 16-byte global loads and stores on both
-// sides (a thread issues all of its loads before it stores any: the kernels
-// are bound by memory latency, not by instructions).
+// one contiguous range.  A CTA holds that image in shared memory, at the
+// range's own 16-byte phase, and moves it to or from global memory in 16-byte
+// pieces; on the raster side it is reached four columns at a time (12 = 3 * 4,
+// so four columns never leave a block's row, and their place in the image is
+// 8-byte aligned).  The unpredictable values are the image's zeros in order.
+//
+// Bound by the latency of a strip's few dependent round trips (ticket, rows,
+// look-back), hidden by other strips: small CTAs, as many as 42 registers a
+// thread allow.  Both components of 8192 x 8192 take .32 ms to block order and
+// .34 back (.57 and .58 with rows in shared memory, an element's place worked
+// out by itself and four CTAs of 256 threads an SM; .34 and .35 with eight of
+// 256, .34 and .38 with sixteen of 128).
 constexpr int STRIP_BLOCKS = 32;
 constexpr int STRIP_W = STRIP_BLOCKS * BS;  // 384 columns
-constexpr int STRIP_NT = 256;
-constexpr int STRIP_TP = STRIP_W + 8;  // shared row pitch in u16: 784 bytes, 16-byte rows
-constexpr int STRIP_VEC = (BS * STRIP_W / 8 + STRIP_NT - 1) / STRIP_NT;  // 16-byte vectors per thread: 3
+constexpr int STRIP_NT = 128;
+constexpr int STRIP_E = BS * STRIP_W;                // 4608 elements
+constexpr int STRIP_IMG = STRIP_E + 16;              // shared image, with room for its phase
+constexpr int STRIP_VEC = (STRIP_E / 8 + STRIP_NT - 1) / STRIP_NT;   // 16-byte vectors per thread: 5
+constexpr int STRIP_GRP = (STRIP_E / 4 + STRIP_NT - 1) / STRIP_NT;   // groups of 4 columns per thread: 9
+constexpr int STRIP_CTAS = 12;                       // per SM: latency is hidden by other strips
+constexpr int STRIP_RUN = 36;                        // consecutive elements whose zeros a thread counts
+static_assert(STRIP_NT * STRIP_RUN >= STRIP_E, "every element has its thread");
 
 struct StripGeom {
   int bi, h, c0, W, nb, wl;
@@ -131,48 +144,18 @@ __device__ __forceinline__ StripGeom strip_geom(long long s, int r1, int r2, int
   return g;
 }
 
-// Element e of a strip's block-order image: block b, row li and column lj
-// inside it (w = the block's width).  Every block but the last is 12 wide, so
-// b = e / (12 h) clamped to the last block.
-struct StripPos {
-  int b, li, lj, w;
-};
-__device__ __forceinline__ StripPos strip_pos(const StripGeom& g, int e) {
-  StripPos p;
-  p.b = min(e / (BS * g.h), g.nb - 1);
-  const int k = e - p.b * BS * g.h;
-  p.w = p.b == g.nb - 1 ? g.wl : BS;
-  p.li = k / p.w;
-  p.lj = k - p.li * p.w;
-  return p;
+// Element e of a strip's block-order image: row and column in the strip.
+// Every block but the last is 12 wide, so b = e / (12 h) clamped to the last.
+__device__ __forceinline__ void strip_pos(const StripGeom& g, int e, int& li, int& col) {
+  const int b = min(e / (BS * g.h), g.nb - 1);
+  const int k = e - b * BS * g.h, w = b == g.nb - 1 ? g.wl : BS;
+  li = k / w;
+  col = b * BS + (k - li * w);
 }
-__device__ __forceinline__ void strip_next(const StripGeom& g, StripPos& p) {
-  if (++p.lj == p.w) {
-    p.lj = 0;
-    if (++p.li == g.h) {
-      p.li = 0;
-      ++p.b;
-      p.w = p.b == g.nb - 1 ? g.wl : BS;
-    }
-  }
-}
-
-// The scalar head and tail that align a strip's block-order range to 16
-// bytes: elements [0, head) and [head + 8 nvec, E) go one by one, the nvec
-// vectors between them 8 at a time.  An unaligned base takes the scalar path.
-struct StripSplit {
-  int E, head, nvec;
-};
-__device__ __forceinline__ StripSplit strip_split(const StripGeom& g, const uint16_t* base) {
-  StripSplit sp;
-  sp.E = g.h * g.W;
-  sp.head = sp.E;
-  sp.nvec = 0;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) == 0) {
-    sp.head = min(sp.E, (int)((8 - (g.out0 & 7)) & 7));
-    sp.nvec = (sp.E - sp.head) >> 3;
-  }
-  return sp;
+// The inverse: the image's element at (li, col).
+__device__ __forceinline__ int strip_elem(const StripGeom& g, int li, int col) {
+  const int b = col / BS, w = b == g.nb - 1 ? g.wl : BS;
+  return b * BS * g.h + li * w + (col - b * BS);
 }
 
 // The strips' unpredictable counts are summed by decoupled look-back
@@ -183,163 +166,150 @@ __device__ __forceinline__ StripSplit strip_split(const StripGeom& g, const uint
 // the look-back's several windows per round trip.
 constexpr long long LOOKBACK_SPIN = 1ll << 24;
 
-// Warp 0 of a strip's CTA: the exclusive prefix of its blocks' zero counts
-// (bpre), its own count published, and the count of all earlier strips
-// (s_excl); the last strip also stores the component's total.  A look-back that waits past its bound sets FLAG_TIMEOUT.
-__device__ __forceinline__ void strip_prefix(unsigned long long* status, unsigned int s, unsigned int ns,
-                                             const StripGeom& g, const unsigned int* bz, unsigned int* bpre,
-                                             unsigned long long* s_excl, int lane, unsigned* total, int* flag) {
-  const unsigned int v = lane < g.nb ? bz[lane] : 0u;
-  unsigned int inc = v;  // inclusive scan of the block counts
+// Whether a zero code may be among the two halves of a word (exact when none
+// is: a false alarm needs a true zero below it).
+__device__ __forceinline__ unsigned zero_half(unsigned v) { return (v - 0x00010001u) & ~v & 0x80008000u; }
+
+struct StripShared {
+  __align__(16) uint16_t img[STRIP_IMG];
+  unsigned int warp_z[STRIP_NT / 32];
+  unsigned int idx;
+  unsigned long long excl;
+};
+
+// Zeros of this thread's run of the image (elements [24 tid, 24 tid + 24)),
+// and of all earlier threads'; total in every thread.  All threads call it.
+__device__ __forceinline__ unsigned strip_zeros(StripShared& sh, const uint16_t* img, int E, unsigned& before,
+                                                unsigned& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int e0 = (int)threadIdx.x * STRIP_RUN, n = min(STRIP_RUN, E - e0);
+  unsigned z = 0;
+  for (int k = 0; k < n; k++) z += img[e0 + k] == 0;
+  unsigned x = z;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    const unsigned int y = __shfl_up_sync(FULLM, inc, d);
-    if (lane >= d) inc += y;
+    const unsigned y = __shfl_up_sync(FULLM, x, d);
+    if (lane >= d) x += y;
   }
-  bpre[lane] = inc - v;
-  const unsigned long long tot = __shfl_sync(FULLM, inc, 31);
-  if (lane == 0) lookback_publish(status, s, tot);
-  const unsigned long long excl = lookback_warp(status, s, tot, lane, LOOKBACK_SPIN, flag);
-  if (lane == 0) {
-    *s_excl = excl;
-    if (s == ns - 1) *total = (unsigned int)(excl + tot);
+  if (lane == 31) sh.warp_z[warp] = x;
+  __syncthreads();
+  before = x - z;
+  total = 0;
+#pragma unroll
+  for (int q = 0; q < STRIP_NT / 32; q++) {
+    const unsigned v = sh.warp_z[q];
+    before += q < warp ? v : 0u;
+    total += v;
   }
+  return z;
 }
-
-__device__ __forceinline__ unsigned int lanemask_lt(int lane) { return (1u << lane) - 1u; }
 
 // Compression, one launch for both components of every field: codes raster ->
 // block order, and the unpredictable values (code 0) in block order.
-struct StripPass {
-  const uint16_t* raster;
-  const float* x;
-  uint16_t* blocks;
-  float* unpred;
-  unsigned long long* status;  // ns words, then the ticket
-};
-__global__ void __launch_bounds__(STRIP_NT) strip_pass_kernel(const __grid_constant__ StripJob one,
+__global__ void __launch_bounds__(STRIP_NT, STRIP_CTAS) strip_pass_kernel(const __grid_constant__ StripJob one,
                                                               const StripJob* __restrict__ jobs, int njobs, int* flag) {
-  __shared__ __align__(16) uint16_t t[BS][STRIP_TP];
-  __shared__ unsigned int bz[STRIP_BLOCKS], bpre[STRIP_BLOCKS];
-  __shared__ unsigned int s_idx;
-  __shared__ unsigned long long s_excl;
+  __shared__ StripShared sh;
   __shared__ int s_job;
   if (jobs) {
-    if (threadIdx.x == 0) {
-      int lo = 0, hi = njobs - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].strip0 <= blockIdx.x) lo = mid;
-        else hi = mid - 1;
-      }
-      s_job = lo;
+    // the last job with strip0 <= blockIdx.x: a warp counts them, its loads
+    // independent of one another (a binary search's are a chain)
+    if (threadIdx.x < 32) {
+      int n = 0;
+      for (int k = threadIdx.x; k < njobs; k += 32) n += jobs[k].strip0 <= blockIdx.x;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) n += __shfl_xor_sync(FULLM, n, d);
+      if (threadIdx.x == 0) s_job = n - 1;
     }
     __syncthreads();
   }
   const StripJob& J = jobs ? jobs[s_job] : one;
   const int c = blockIdx.y, r1 = J.r1, r2 = J.r2, nsc = (r2 + STRIP_W - 1) / STRIP_W;
-  const long long pitch = r2;
   const unsigned int ns = (unsigned)((r1 + BS - 1) / BS) * (unsigned)nsc;
-  const StripPass P{J.raster[c], J.x[c], J.blocks[c], J.unpred[c], J.status[c]};
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_idx = atomicAdd(reinterpret_cast<unsigned int*>(P.status + ns), 1u);
-  if (threadIdx.x < STRIP_BLOCKS) bz[threadIdx.x] = 0;
+  unsigned long long* const status = J.status[c];
+  if (threadIdx.x == 0) sh.idx = atomicAdd(reinterpret_cast<unsigned int*>(status + ns), 1u);
   __syncthreads();
-  const unsigned int s = s_idx;
+  const unsigned int s = sh.idx;
   const StripGeom g = strip_geom(s, r1, r2, nsc);
+  const int E = g.h * g.W, phase = (int)(g.out0 & 7);
+  uint16_t* const img = sh.img + phase;
 
-  // rows into shared memory
-  const uint16_t* src = P.raster + (long long)g.bi * BS * pitch + g.c0;
-  if (((reinterpret_cast<uintptr_t>(P.raster) | (uintptr_t)(2 * pitch)) & 15) == 0) {
-    const int nv = g.W >> 3, tot = g.h * nv;  // c0 is a multiple of 8, so every row's vectors are aligned
-    uint4 v[STRIP_VEC];
+  // the raster's rows into the image: four columns of full blocks at a time,
+  // from the two 8-byte words that hold them (one when they are aligned)
+  const uint16_t* src = J.raster[c] + (long long)g.bi * BS * r2 + g.c0;
+  const int nfull = g.W / BS, ng = 3 * nfull, tot = g.h * ng;
+  unsigned any = 0;
+  uint2 v[STRIP_GRP];
 #pragma unroll
-    for (int it = 0; it < STRIP_VEC; it++) {
-      const int q = threadIdx.x + it * STRIP_NT;
-      if (q < tot) {
-        const int li = q / nv;
-        v[it] = __ldg(reinterpret_cast<const uint4*>(src + (long long)li * pitch) + (q - li * nv));
+  for (int it = 0; it < STRIP_GRP; it++) {
+    const int q = threadIdx.x + it * STRIP_NT;
+    if (q < tot) {
+      const int li = ng == 96 ? q / 96 : q / ng, gr = q - li * ng;
+      const uint16_t* p = src + (long long)li * r2 + 4 * gr;
+      const unsigned a = (unsigned)((uintptr_t)p & 7);
+      const uint2* w = reinterpret_cast<const uint2*>(p - a / 2);
+      uint2 x = __ldg(w);
+      if (a) {
+        const uint2 y = __ldg(w + 1);
+        const unsigned sft = 8 * (a & 3);
+        const unsigned t0 = a & 4 ? x.y : x.x, t1 = a & 4 ? y.x : x.y, t2 = a & 4 ? y.y : y.x;
+        x = make_uint2(__funnelshift_r(t0, t1, sft), __funnelshift_r(t1, t2, sft));
       }
-    }
-#pragma unroll
-    for (int it = 0; it < STRIP_VEC; it++) {
-      const int q = threadIdx.x + it * STRIP_NT;
-      if (q < tot) {
-        const int li = q / nv;
-        reinterpret_cast<uint4*>(&t[li][0])[q - li * nv] = v[it];
-      }
-    }
-    const int rem = g.W - 8 * nv;  // the field's last columns
-    for (int q = threadIdx.x; q < g.h * rem; q += STRIP_NT) {
-      const int li = q / rem, c = 8 * nv + (q - li * rem);
-      t[li][c] = src[(long long)li * pitch + c];
-    }
-  } else {
-#pragma unroll 6
-    for (int q = threadIdx.x; q < g.h * g.W; q += STRIP_NT) {
-      const int li = q / g.W, c = q - li * g.W;
-      t[li][c] = src[(long long)li * pitch + c];
+      v[it] = x;
     }
   }
-  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < STRIP_GRP; it++) {
+    const int q = threadIdx.x + it * STRIP_NT;
+    if (q < tot) {
+      const int li = ng == 96 ? q / 96 : q / ng, gr = q - li * ng, b = gr / 3;
+      *reinterpret_cast<uint2*>(img + (b * g.h + li) * BS + 4 * (gr - 3 * b)) = v[it];
+      any |= zero_half(v[it].x) | zero_half(v[it].y);
+    }
+  }
+  const int rem = g.W - BS * nfull;  // the field's last, narrower block
+  for (int q = threadIdx.x; q < g.h * rem; q += STRIP_NT) {
+    const int li = q / rem, cc = q - li * rem;
+    const uint16_t x = src[(long long)li * r2 + BS * nfull + cc];
+    img[nfull * BS * g.h + q] = x;
+    any |= x == 0;
+  }
+  const bool some = __syncthreads_or(any != 0) != 0;
+  unsigned before = 0, total = 0, z = 0;
+  if (some) z = strip_zeros(sh, img, E, before, total);
+  if (threadIdx.x == 0) lookback_publish(status, s, total);
 
-  // block-order image, 8 elements per 16-byte store; zero codes counted per
-  // block (shared atomics only where a thread met zeros)
-  uint16_t* dst = P.blocks + g.out0;
-  const StripSplit sp = strip_split(g, dst);
-  for (int q = threadIdx.x; q < sp.nvec; q += STRIP_NT) {
-    const int e0 = sp.head + 8 * q;
-    StripPos p = strip_pos(g, e0);
-    unsigned int w32[4];
-    int zb = p.b;
-    unsigned int z = 0;
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-      if (p.b != zb) {
-        if (z) atomicAdd(&bz[zb], z);
-        zb = p.b;
-        z = 0;
-      }
-      const unsigned int v = t[p.li][p.b * BS + p.lj];
-      z += v == 0;
-      w32[m >> 1] = (m & 1) ? (w32[m >> 1] | (v << 16)) : v;
-      strip_next(g, p);
+  // the image, 16 bytes at a time between the range's ends
+  uint16_t* const dst = J.blocks[c] + g.out0;
+  const int head = (reinterpret_cast<uintptr_t>(J.blocks[c]) & 15) ? E : min(E, (8 - phase) & 7);
+  const int nvec = (E - head) >> 3, tail0 = head + 8 * nvec;
+  for (int q = threadIdx.x; q < nvec; q += STRIP_NT)
+    *reinterpret_cast<uint4*>(dst + head + 8 * q) = *reinterpret_cast<const uint4*>(img + head + 8 * q);
+  for (int q = threadIdx.x; q < head + (E - tail0); q += STRIP_NT) {
+    const int e = q < head ? q : tail0 + (q - head);
+    dst[e] = img[e];
+  }
+
+  if (threadIdx.x < 32) {
+    const unsigned long long excl = lookback_warp(status, s, total, (int)threadIdx.x, LOOKBACK_SPIN, flag);
+    if (threadIdx.x == 0) {
+      sh.excl = excl;
+      if (s == ns - 1) J.total[c] = (unsigned int)(excl + total);
     }
-    if (z) atomicAdd(&bz[zb], z);
-    *reinterpret_cast<uint4*>(dst + e0) = make_uint4(w32[0], w32[1], w32[2], w32[3]);
   }
-  const int tail0 = sp.head + 8 * sp.nvec;
-  for (int q = threadIdx.x; q < sp.head + (sp.E - tail0); q += STRIP_NT) {
-    const int e = q < sp.head ? q : tail0 + (q - sp.head);
-    const StripPos p = strip_pos(g, e);
-    const uint16_t v = t[p.li][p.b * BS + p.lj];
-    dst[e] = v;
-    if (v == 0) atomicAdd(&bz[p.b], 1u);
-  }
-  __syncthreads();
-  if (warp == 0) strip_prefix(P.status, s, ns, g, bz, bpre, &s_excl, lane, J.total + c, flag);
+  if (!some) return;
   __syncthreads();
 
   // unpredictable values, in block order
-  const unsigned long long excl = s_excl;
-  for (int b = warp; b < g.nb; b += STRIP_NT / 32) {
-    if (bz[b] == 0) continue;
-    const int w = (b == g.nb - 1) ? g.wl : BS;
-    const int nk = g.h * w;
-    unsigned long long run = excl + bpre[b];
-    for (int k0 = 0; k0 < nk; k0 += 32) {
-      const int k = k0 + lane;
-      int li = 0, col = 0;
-      bool z = false;
-      if (k < nk) {
-        li = k / w;
-        col = b * BS + (k - li * w);
-        z = t[li][col] == 0;
+  if (z) {
+    float* out = J.unpred[c] + sh.excl + before;
+    const float* x = J.x[c] + (long long)g.bi * BS * r2 + g.c0;
+    const int e0 = (int)threadIdx.x * STRIP_RUN, n = min(STRIP_RUN, E - e0);
+    for (int k = 0; k < n; k++)
+      if (img[e0 + k] == 0) {
+        int li, col;
+        strip_pos(g, e0 + k, li, col);
+        *out++ = x[(long long)li * r2 + col];
       }
-      const unsigned int m = __ballot_sync(FULLM, z);
-      if (z) P.unpred[run + __popc(m & lanemask_lt(lane))] = P.x[(long long)(g.bi * BS + li) * pitch + g.c0 + col];
-      run += __popc(m);
-    }
   }
 }
 
@@ -369,129 +339,109 @@ __device__ __forceinline__ float2 dec_pair(unsigned int code, unsigned int id, i
 // raster pairs the wavefront reads, with the unpredictable values (block
 // order) scattered into the pairs of the zero codes.  The last strip stores
 // the number of zero codes, which the host checks against the stored list.
-__global__ void __launch_bounds__(STRIP_NT) strip_unpass_kernel(StripUnpass P0, StripUnpass P1, int r1, int r2,
+__global__ void __launch_bounds__(STRIP_NT, STRIP_CTAS) strip_unpass_kernel(StripUnpass P0, StripUnpass P1, int r1, int r2,
                                                                 int nsc, unsigned int ns, int* flag) {
-  __shared__ __align__(16) uint16_t t[BS][STRIP_TP];
-  __shared__ unsigned int bz[STRIP_BLOCKS], bpre[STRIP_BLOCKS];
-  __shared__ unsigned int s_idx;
-  __shared__ unsigned long long s_excl;
+  __shared__ StripShared sh;
   const StripUnpass P = blockIdx.y ? P1 : P0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_idx = atomicAdd(reinterpret_cast<unsigned int*>(P.status + ns), 1u);
-  if (threadIdx.x < STRIP_BLOCKS) bz[threadIdx.x] = 0;
+  if (threadIdx.x == 0) sh.idx = atomicAdd(reinterpret_cast<unsigned int*>(P.status + ns), 1u);
   __syncthreads();
-  const unsigned int s = s_idx;
+  const unsigned int s = sh.idx;
   const StripGeom g = strip_geom(s, r1, r2, nsc);
+  const int E = g.h * g.W, phase = (int)(g.out0 & 7);
+  uint16_t* const img = sh.img + phase;
 
-  // block-order codes into shared rows, zero codes counted per block
+  // the block-order codes, 16 bytes at a time between the range's ends
   const uint16_t* src = P.blocks + g.out0;
-  const StripSplit sp = strip_split(g, src);
-  {
-    uint4 v[STRIP_VEC];
+  const int head = (reinterpret_cast<uintptr_t>(P.blocks) & 15) ? E : min(E, (8 - phase) & 7);
+  const int nvec = (E - head) >> 3, tail0 = head + 8 * nvec;
+  unsigned any = 0;
+  uint4 v[STRIP_VEC];
 #pragma unroll
-    for (int it = 0; it < STRIP_VEC; it++) {
-      const int q = threadIdx.x + it * STRIP_NT;
-      if (q < sp.nvec) v[it] = __ldg(reinterpret_cast<const uint4*>(src + sp.head + 8 * q));
-    }
+  for (int it = 0; it < STRIP_VEC; it++) {
+    const int q = threadIdx.x + it * STRIP_NT;
+    if (q < nvec) v[it] = __ldg(reinterpret_cast<const uint4*>(src + head + 8 * q));
+  }
 #pragma unroll
-    for (int it = 0; it < STRIP_VEC; it++) {
-      const int q = threadIdx.x + it * STRIP_NT;
-      if (q < sp.nvec) {
-        const unsigned int w32[4] = {v[it].x, v[it].y, v[it].z, v[it].w};
-        StripPos p = strip_pos(g, sp.head + 8 * q);
-        int zb = p.b;
-        unsigned int z = 0;
-#pragma unroll
-        for (int m = 0; m < 8; m++) {
-          if (p.b != zb) {
-            if (z) atomicAdd(&bz[zb], z);
-            zb = p.b;
-            z = 0;
-          }
-          const uint16_t c = (uint16_t)(w32[m >> 1] >> ((m & 1) * 16));
-          t[p.li][p.b * BS + p.lj] = c;
-          z += c == 0;
-          strip_next(g, p);
-        }
-        if (z) atomicAdd(&bz[zb], z);
-      }
+  for (int it = 0; it < STRIP_VEC; it++) {
+    const int q = threadIdx.x + it * STRIP_NT;
+    if (q < nvec) {
+      *reinterpret_cast<uint4*>(img + head + 8 * q) = v[it];
+      any |= zero_half(v[it].x) | zero_half(v[it].y) | zero_half(v[it].z) | zero_half(v[it].w);
     }
   }
-  const int tail0 = sp.head + 8 * sp.nvec;
-  for (int q = threadIdx.x; q < sp.head + (sp.E - tail0); q += STRIP_NT) {
-    const int e = q < sp.head ? q : tail0 + (q - sp.head);
-    const StripPos p = strip_pos(g, e);
-    const uint16_t c = src[e];
-    t[p.li][p.b * BS + p.lj] = c;
-    if (c == 0) atomicAdd(&bz[p.b], 1u);
+  for (int q = threadIdx.x; q < head + (E - tail0); q += STRIP_NT) {
+    const int e = q < head ? q : tail0 + (q - head);
+    const uint16_t x = src[e];
+    img[e] = x;
+    any |= x == 0;
   }
-  __syncthreads();
-  if (warp == 0) strip_prefix(P.status, s, ns, g, bz, bpre, &s_excl, lane, P.total, flag);
+  const bool some = __syncthreads_or(any != 0) != 0;
+  unsigned before = 0, total = 0, z = 0;
+  if (some) z = strip_zeros(sh, img, E, before, total);
+  if (threadIdx.x == 0) lookback_publish(P.status, s, total);
 
-  // raster pairs (the other warps start while warp 0 looks back)
+  // raster pairs
   const long long row0 = (long long)g.bi * BS;
   if ((r2 & 3) == 0 && ((reinterpret_cast<uintptr_t>(P.ids) & 3) | (reinterpret_cast<uintptr_t>(P.pair) & 15)) == 0) {
-    // 4 columns per item (W is a multiple of 4 here): one u32 of ids in, two 16-byte pair stores out
-    constexpr int ROW_VEC = (BS * STRIP_W / 4 + STRIP_NT - 1) / STRIP_NT;  // 5
+    // 4 columns per item (W is a multiple of 4 here, and so is every block's
+    // width): one u32 of ids in, two 16-byte pair stores out
     const int nq = g.W >> 2, tot = g.h * nq;
-    unsigned int idv[ROW_VEC];
+    unsigned int idv[STRIP_GRP];
 #pragma unroll
-    for (int u = 0; u < ROW_VEC; u++) {
+    for (int u = 0; u < STRIP_GRP; u++) {
       const int q = threadIdx.x + u * STRIP_NT;
       if (q < tot) {
-        const int li = q / nq;
+        const int li = nq == 96 ? q / 96 : q / nq;
         idv[u] = __ldg(reinterpret_cast<const unsigned int*>(P.ids + (row0 + li) * r2 + g.c0) + (q - li * nq));
       }
     }
 #pragma unroll
-    for (int u = 0; u < ROW_VEC; u++) {
+    for (int u = 0; u < STRIP_GRP; u++) {
       const int q = threadIdx.x + u * STRIP_NT;
       if (q < tot) {
-        const int li = q / nq, c = 4 * (q - li * nq);
-        const uint2 cw = *reinterpret_cast<const uint2*>(&t[li][c]);
+        const int li = nq == 96 ? q / 96 : q / nq, gr = q - li * nq, b = gr / 3;
+        const int w = b == g.nb - 1 ? g.wl : BS;
+        const uint2 cw = *reinterpret_cast<const uint2*>(img + b * BS * g.h + li * w + 4 * (gr - 3 * b));
         const float2 a = dec_pair(cw.x & 0xffffu, idv[u] & 0xffu, P.id_shift),
-                     b = dec_pair(cw.x >> 16, (idv[u] >> 8) & 0xffu, P.id_shift);
-        const float2 d = dec_pair(cw.y & 0xffffu, (idv[u] >> 16) & 0xffu, P.id_shift),
-                     e = dec_pair(cw.y >> 16, idv[u] >> 24, P.id_shift);
-        float4* out = reinterpret_cast<float4*>(P.pair + (row0 + li) * r2 + g.c0 + c);
-        out[0] = make_float4(a.x, a.y, b.x, b.y);
-        out[1] = make_float4(d.x, d.y, e.x, e.y);
+                     d = dec_pair(cw.x >> 16, (idv[u] >> 8) & 0xffu, P.id_shift);
+        const float2 e = dec_pair(cw.y & 0xffffu, (idv[u] >> 16) & 0xffu, P.id_shift),
+                     f = dec_pair(cw.y >> 16, idv[u] >> 24, P.id_shift);
+        float4* out = reinterpret_cast<float4*>(P.pair + (row0 + li) * r2 + g.c0 + 4 * gr);
+        out[0] = make_float4(a.x, a.y, d.x, d.y);
+        out[1] = make_float4(e.x, e.y, f.x, f.y);
       }
     }
   } else {
 #pragma unroll 6
-    for (int q = threadIdx.x; q < g.h * g.W; q += STRIP_NT) {
-      const int li = q / g.W, c = q - li * g.W;
+    for (int q = threadIdx.x; q < E; q += STRIP_NT) {
+      const int li = g.W == STRIP_W ? q / STRIP_W : q / g.W, c = q - li * g.W;
       const long long gi = (row0 + li) * r2 + g.c0 + c;
-      P.pair[gi] = dec_pair(t[li][c], P.ids[gi], P.id_shift);
+      P.pair[gi] = dec_pair(img[strip_elem(g, li, c)], P.ids[gi], P.id_shift);
     }
   }
-  __syncthreads();  // the raw values below overwrite .x of pairs stored above
+
+  if (threadIdx.x < 32) {
+    const unsigned long long excl = lookback_warp(P.status, s, total, (int)threadIdx.x, LOOKBACK_SPIN, flag);
+    if (threadIdx.x == 0) {
+      sh.excl = excl;
+      if (s == ns - 1) *P.total = (unsigned int)(excl + total);
+    }
+  }
+  if (!some) return;
+  __syncthreads();  // also: the raw values below overwrite .x of pairs stored above
 
   // unpredictable values, in block order
-  const unsigned long long excl = s_excl;
-  for (int b = warp; b < g.nb; b += STRIP_NT / 32) {
-    if (bz[b] == 0) continue;
-    const int w = (b == g.nb - 1) ? g.wl : BS;
-    const int nk = g.h * w;
-    unsigned long long run = excl + bpre[b];
-    for (int k0 = 0; k0 < nk; k0 += 32) {
-      const int k = k0 + lane;
-      int li = 0, col = 0;
-      bool z = false;
-      if (k < nk) {
-        li = k / w;
-        col = b * BS + (k - li * w);
-        z = t[li][col] == 0;
-      }
-      const unsigned int m = __ballot_sync(FULLM, z);
-      if (z) {
-        const unsigned long long o = run + __popc(m & lanemask_lt(lane));
+  if (z) {
+    unsigned long long o = sh.excl + before;
+    const int e0 = (int)threadIdx.x * STRIP_RUN, n = min(STRIP_RUN, E - e0);
+    for (int k = 0; k < n; k++)
+      if (img[e0 + k] == 0) {
+        int li, col;
+        strip_pos(g, e0 + k, li, col);
         if (o < P.n_unpred) P.pair[(row0 + li) * r2 + g.c0 + col].x = P.unpred[o];
         else atomicOr(flag, FLAG_RAW_RANGE);
+        o++;
       }
-      run += __popc(m);
-    }
   }
 }
 
