@@ -359,13 +359,15 @@ int launch_chunk_count_3d(cpsz_b200_ctx* ctx, bool compress, const void* src, si
 int launch_compact3d(cpsz_b200_ctx* ctx, const ushort4* codes, uint8_t* ids, const float* U, const float* V,
                      const float* W, size_t n, const unsigned* chunk_off, uint16_t* codes_out, float* unpred,
                      unsigned long long* hist_ids);
-// Decompress: pairs = (3 addends, 0) for predicted points, (3 raw values, raw
-// flag) for the others.  Short streams raise FLAG_RAW_RANGE.
+// Decompress: pairs = (3 addends, 0) for predicted points, (3 logs of the raw
+// values, raw flag) for the others, whose raw values go to U, V, W.  Short
+// streams raise FLAG_RAW_RANGE.
 int launch_prep3d(cpsz_b200_ctx* ctx, const uint8_t* ids, size_t n, const unsigned* chunk_off, const uint16_t* codes,
-                  size_t n_codes, const float* unpred, size_t n_unpred, float4* pairs);
+                  size_t n_codes, const float* unpred, size_t n_unpred, float4* pairs, const LibmTables* L, float* U,
+                  float* V, float* W);
 // Lorenzo recursion in one persistent launch (wave3d.cu).  Compress: in =
 // log3d pairs, codes out (0,0,0 for unpredictable points).  Decompress: in =
-// prep3d pairs, decoded U, V, W out.  rec: reconstructed log values
+// prep3d pairs, U, V, W of the predicted points out.  rec: reconstructed log values
 // (scratch); scratch: wave3d_scratch_bytes(r1, r2) of device memory.
 size_t wave3d_scratch_bytes(int r1, int r2);
 int launch_wave3d(cpsz_b200_ctx* ctx, bool decompress, const float4* in, float4* rec, ushort4* codes,

@@ -297,7 +297,9 @@ __global__ void __launch_bounds__(CH_NT) prep3d_kernel(const uint8_t* __restrict
                                                        const unsigned* __restrict__ chunk_off,
                                                        const uint16_t* __restrict__ codes, size_t n_codes,
                                                        const float* __restrict__ unpred, size_t n_unpred,
-                                                       float4* __restrict__ pairs, int* __restrict__ flag) {
+                                                       float4* __restrict__ pairs, LibmFn Lg, float* __restrict__ U,
+                                                       float* __restrict__ V, float* __restrict__ W,
+                                                       int* __restrict__ flag) {
   const size_t base = (size_t)blockIdx.x * CH + (size_t)threadIdx.x * CH_PER_T;
   uint8_t iv[CH_PER_T];
   unsigned c = 0;
@@ -338,6 +340,13 @@ __global__ void __launch_bounds__(CH_NT) prep3d_kernel(const uint8_t* __restrict
       } else {
         bad = 1;
       }
+      // decoded as it is; its logs feed the neighbours' predictors (here, point
+      // by point: a logarithm in the recursion holds up every row of its unit)
+      U[idx] = r[0];
+      V[idx] = r[1];
+      W[idx] = r[2];
+#pragma unroll
+      for (int x = 0; x < 3; x++) r[x] = (r[x] == 0.f) ? -100.f : dev::host_log2f(fabsf(r[x]), Lg);
       o = make_float4(r[0], r[1], r[2], __int_as_float(1));
       up++;
     }
@@ -435,9 +444,10 @@ int launch_compact3d(cpsz_b200_ctx* ctx, const ushort4* codes, uint8_t* ids, con
 }
 
 int launch_prep3d(cpsz_b200_ctx* ctx, const uint8_t* ids, size_t n, const unsigned* chunk_off, const uint16_t* codes,
-                  size_t n_codes, const float* unpred, size_t n_unpred, float4* pairs) {
+                  size_t n_codes, const float* unpred, size_t n_unpred, float4* pairs, const LibmTables* L, float* U,
+                  float* V, float* W) {
   prep3d_kernel<<<(int)chunk_count(n), CH_NT, 0, ctx->stream>>>(ids, n, chunk_off, codes, n_codes, unpred, n_unpred,
-                                                                 pairs, ctx->d_flag);
+                                                                 pairs, L->log2f, U, V, W, ctx->d_flag);
   count_launch(ctx);
   return check_launch("prep3d_kernel");
 }

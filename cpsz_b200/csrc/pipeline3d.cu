@@ -413,7 +413,7 @@ int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
     mark(ctx, "prep3d");
     CPSZ_TRY(launch_chunk_count_3d(ctx, false, ids, N, chunk_cnt));
     CPSZ_TRY(launch_scan_u32(ctx, chunk_cnt, chunk_off, nchunks, scan_tmp));
-    CPSZ_TRY(launch_prep3d(ctx, ids, N, chunk_off, codes, n_codes, unpred, n_unpred, pairs));
+    CPSZ_TRY(launch_prep3d(ctx, ids, N, chunk_off, codes, n_codes, unpred, n_unpred, pairs, &lt, dU, dV, dW));
     mark(ctx, "wave3d_decompress");
     CPSZ_TRY(launch_wave3d(ctx, true, pairs, rec, nullptr, signs, smap, &lt, dU, dV, dW, r1, r2, r3, wave_sync));
     mark(ctx, "d2h");
