@@ -55,7 +55,9 @@ constexpr size_t BATCH_MAX_POINTS = (size_t)1 << 27;
 // A single field of at least this many points packs its ids on the second
 // stream while the wavefront's tail runs; a smaller one (and a batch) packs
 // its three streams in one launch once every tree is known: below it the
-// extra copy, launches and events cost more than the packing they hide.
+// extra copy, launches and events cost more than the packing they hide (early
+// against together: 512^2 348 and 326 us, 724^2 591 and 584, 1024^2 534 and
+// 545, 2048^2 942 and 970).
 constexpr size_t EARLY_IDS_POINTS = (size_t)1 << 19;
 
 // upload staging of that packing
