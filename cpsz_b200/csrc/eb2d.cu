@@ -21,8 +21,10 @@
 //
 // One CTA per tile (a 2D grid in row-major tile order, so row groups complete
 // roughly in order): measured faster than a persistent grid that takes tiles
-// with a stride or from a counter (3.75 against 4.27 ms at 8192^2 alone, and
-// the wavefront beside it keeps pace only with the per-tile grid).
+// with a stride or from a counter (when the bounds were evaluated in double
+// precision, 3.75 against 4.27 ms at 8192^2 alone; the wavefront beside it
+// kept pace only with the per-tile grid).  Now 1.36 ms alone, 1.86 beside it:
+// 300 M warp instructions at 4096^2, 69 % of the issue slots.
 #include <algorithm>
 
 #include "eb_math.cuh"

@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(HIST_NT) hist_u16_kernel(const __grid_constant
 // ---- histogram -> list ---------------------------------------------------------------
 // The symbols that occur, ascending, as symbol << 40 | count, and their number,
 // written straight into page-locked host memory: the host reads a few thousand
-// words where it would copy and scan 65536 bins (512 KB and about 20 us each).
+// words where it would copy and scan 65536 bins (512 KB each).
 // One CTA per histogram; warp w has bins 2048 w .. 2048 w + 2047, 32 per step,
 // so a step's ballot gives every lane its place.
 constexpr int LIST_NT = 1024;

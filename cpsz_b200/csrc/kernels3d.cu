@@ -19,6 +19,11 @@ namespace cpsz {
 namespace {
 
 // ---- eb3d ------------------------------------------------------------------------
+// The bounds themselves: calls that want them, fields and max_pwr_eb the id
+// filter (eb3d_filter.cu) does not take, and fields that leave it more open
+// vertices than its list holds (then this kernel runs behind it; elsewhere the
+// launch returns at once).  384^3 takes 15.5 ms here, 4.7 through the filter.
+//
 // A CTA owns a 32 (k) x 8 (j) column of vertices and marches over i.  Per step
 // it stages vertex plane i+1 (with a one-vertex halo towards -j/-k), evaluates
 // the 6 tets of every cube of cube-plane i that touches the column (cubes
