@@ -35,15 +35,16 @@
 //  * loads go through L2 (cp.async.cg: another SM's writes must not meet a
 //    stale L1 line).
 //
-// What bounds it: a unit's step, with the helpers' accesses (32 KB in, 48 KB
-// out per window) and the compute warps' on one shared-memory pipe: .39 us a
-// step for a unit by itself, .19 with idle helpers, .14 without the barrier.
-// A thread that fetched its input and stored its own result, eight ring reads a
-// step and progress published behind two fences took .55-.9 us.  384^3
-// compresses in 1.5 ms here (2.9 before), 256^3 decodes in .6 (3.2, most of
-// it logarithms of raw points taken inside the recursion: prep3d takes them
-// now).  One, two or four input warps and two, four or eight storing ones
-// are within 10 %.
+// What bounds it: the helpers' accesses (32 KB in, 48 KB out per window) and the
+// compute warps' on one shared-memory pipe, then the step's chain and barrier.
+// A unit by itself took .39 us a step, .19 with idle helpers, .14 without the
+// barrier, while a 16-byte copy of four rows scattered its lines over eight
+// slots (24 shared-memory wavefronts; 384^3 1.50 ms, 1.27 with a row's points
+// together).  With a thread fetching its own input and storing its own result,
+// eight ring reads a step and progress published behind two fences a step was
+// .55-.9 us: 384^3 2.9 ms, and decoding 256^3 3.2 (most of it logarithms of
+// raw points inside the recursion: prep3d takes them now), .45 here.  One, two
+// or four input warps and two, four or eight storing ones are within 10 %.
 // Every wait is bounded: on expiry (or once any wait has expired) the kernel
 // sets FLAG_TIMEOUT and stops waiting; the host then fails the call.
 //
@@ -86,7 +87,10 @@ struct W3Args {
 // to one slot's 32 lanes, meet no bank twice.
 template <bool DECOMP>
 struct W3Smem {
-  float4 in[W3_P][W3_SR][33];
+  // Input row by row: a row's eight points of a window are 128 bytes, the point
+  // of step m of row l in piece m ^ (l & 7), so that a copied line lands in one
+  // place and a step's 32 lanes still read all banks.
+  float4 in[W3_P][2][32][W3_W];
   float4 ring[W3_P][W3_SR][33];  // plane i0+p
   float4 below[W3_SL][33];       // plane i0-1
   float4 edge[W3_P][W3_SL];      // row j0-1 of plane i0+p: entry 0 of ring[p]'s slots to come
@@ -134,19 +138,20 @@ __device__ __forceinline__ bool w3_inner(const W3Unit& U, int r3, int T, int p) 
 template <bool DECOMP>
 __device__ __forceinline__ void w3_load_input(const W3Args& a, W3Smem<DECOMP>& M, const W3Unit& U, int T, int p0,
                                               int lane) {
-  const int r3 = a.r3, l0 = lane >> 3, t = T + (lane & 7), slot = t & (W3_SR - 1);
+  const int r3 = a.r3, l0 = lane >> 3, m = lane & 7, t = T + m;
   for (int p = p0; p < W3_P; p += W3_IN) {
     const float4* src = a.in + ((long long)(U.i0 + p) * a.r2 + U.j0 + l0) * r3 + (t - l0 - p);
-    float4* dst = &M.in[p][slot][l0];
+    float4 (*const dst)[W3_W] = M.in[p][(T / W3_W) & 1];
     if (w3_inner(U, r3, T, p)) {
 #pragma unroll
-      for (int r = 0; r < 8; r++, src += 4 * (r3 - 1)) cp16(dst + 4 * r, src, true);
+      for (int r = 0; r < 8; r++, src += 4 * (r3 - 1))
+        cp16(&dst[4 * r + l0][m ^ ((4 * r + l0) & 7)], src, true);
     } else {
 #pragma unroll
       for (int r = 0; r < 8; r++, src += 4 * (r3 - 1)) {
         const int l = 4 * r + l0, k = t - l - p;
         const bool act = p < U.np && l < U.nrows && k >= 0 && k < r3;
-        cp16(dst + 4 * r, act ? src : a.in, act);
+        cp16(&dst[l][m ^ (l & 7)], act ? src : a.in, act);
       }
     }
   }
@@ -323,12 +328,12 @@ __device__ __forceinline__ void w3_compute(const W3Args& a, W3Smem<DECOMP>& M, c
     const float4 (*const Rp)[33] = &M.ring[p][prev];
     const float4 (*const B)[33] = p > 0 ? &M.ring[p - 1][cur] : &M.below[W3_W * (w & 3)];
     const float4 (*const Bp)[33] = p > 0 ? &M.ring[p - 1][prev] : &M.below[W3_W * ((w - 1) & 3)];
-    const float4 (*const X)[33] = &M.in[p][cur];
+    const float4* const X = M.in[p][w & 1][lane];
     if (w == 0) {
       q1 = Bp[W3_W - 2][lane];
       q5 = Rp[W3_W - 1][lane];
     }
-    float4 x = X[0][lane];
+    float4 x = X[lane & 7];
 #pragma unroll
     for (int j = 0; j < W3_W; j++) {
       if (j > 0) compute_sync();  // every plane has finished the step before
@@ -385,7 +390,7 @@ __device__ __forceinline__ void w3_compute(const W3Args& a, W3Smem<DECOMP>& M, c
       __syncwarp();
       q5 = R[j][lane];  // the next step's, of the row above
       q1 = Bj[lane];
-      if (j + 1 < W3_W) x = X[j + 1 < W3_W ? j + 1 : 0][lane];
+      if (j + 1 < W3_W) x = X[(j + 1) ^ (lane & 7)];
     }
   }
   __syncthreads();  // the last window is computed
@@ -393,7 +398,7 @@ __device__ __forceinline__ void w3_compute(const W3Args& a, W3Smem<DECOMP>& M, c
 
 template <bool DECOMP>
 __global__ void __launch_bounds__(W3_THREADS, 1) wave3d_kernel(const W3Args a) {
-  extern __shared__ __align__(16) unsigned char w3_smem[];
+  extern __shared__ __align__(128) unsigned char w3_smem[];
   W3Smem<DECOMP>& M = *reinterpret_cast<W3Smem<DECOMP>*>(w3_smem);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int units = ((a.r1 + W3_P - 1) / W3_P) * a.slabs;
