@@ -43,7 +43,7 @@
 // together).  With a thread fetching its own input and storing its own result,
 // eight ring reads a step and progress published behind two fences a step was
 // .55-.9 us: 384^3 2.9 ms, and decoding 256^3 3.2 (most of it logarithms of
-// raw points inside the recursion: prep3d takes them now), .45 here.  One, two
+// raw points inside the recursion: prep3d takes them now), .5 here.  One, two
 // or four input warps and two, four or eight storing ones are within 10 %.
 // Every wait is bounded: on expiry (or once any wait has expired) the kernel
 // sets FLAG_TIMEOUT and stops waiting; the host then fails the call.
