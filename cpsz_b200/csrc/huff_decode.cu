@@ -81,7 +81,7 @@ struct DecStream {
   uint32_t* lut1;   // write entries: LUT1 words, then LUT1 payload words
   uint16_t* lutc;   // count entries
   uint32_t* lut2;
-  unsigned lut2_cap;
+  unsigned lut2_cap;  // second-level tables there is room for; a pattern's table may number past it
   unsigned* lut2_n;
   uint8_t* rel;     // start of each subsequence, bits after its nominal start
   uint8_t* texit;   // exit of each scan tile, bits after its end
@@ -226,10 +226,10 @@ __device__ __forceinline__ void stage_bits(const DecStream& S, long long g0, uin
   }
 }
 
-// The rest of a code longer than both tables: from `node`, whose code has
-// LUT1_BITS + LUT2_BITS bits.  Returns symbol << 8 | length, 0 beyond MAX_CODE.
-__device__ __noinline__ uint32_t deep_code(DecTree T, Bits b, int pos, uint32_t node) {
-  for (int l = LUT1_BITS + LUT2_BITS; l < MAX_CODE;) {
+// The rest of a code that the tables do not end: from `node`, whose code has
+// `l` bits.  Returns symbol << 8 | length, 0 beyond MAX_CODE.
+__device__ __noinline__ uint32_t deep_code(DecTree T, Bits b, int pos, uint32_t node, int l) {
+  while (l < MAX_CODE) {
     const int at = pos + l;
     const uint32_t bit = (b.word(at >> 5) >> (31 - (at & 31))) & 1u;
     const TreeNode nd = tree_node(T, node);
@@ -242,10 +242,12 @@ __device__ __noinline__ uint32_t deep_code(DecTree T, Bits b, int pos, uint32_t 
 }
 
 // A code over 12 bits (second-level table `t`, next8 its bits after them):
-// symbol << 8 | length; 0: no code.
+// symbol << 8 | length; 0: no code.  A pattern past the tables' room has none
+// (lut2_cap): its code is walked from the root.
 __device__ __forceinline__ uint32_t long_code(const DecStream& S, Bits b, int pos, uint32_t t, uint32_t next8) {
+  if (t >= S.lut2_cap) return deep_code(S.tree, b, pos, 0, 0);
   const uint32_t e = __ldg(S.lut2 + (size_t)t * LUT2 + next8);
-  return e & 0x80u ? deep_code(S.tree, b, pos, e >> 8) : e;
+  return e & 0x80u ? deep_code(S.tree, b, pos, e >> 8, LUT1_BITS + LUT2_BITS) : e;
 }
 
 // Length of the one code at `pos` (lut: count entries).
@@ -600,7 +602,11 @@ DecLayout dec_layout(const HuffDecJob& j) {
   L.nsub = sub_count(j.nbytes);
   L.scan_tiles = (L.nsub + DEC_TILE - 1) / DEC_TILE;
   L.write_tiles = (L.nsub + DEC_NT - 1) / DEC_NT;
-  // patterns that no code ends in are inner nodes at depth 12
+  // Patterns that no code ends in are paths to inner nodes at depth 12: in a
+  // tree fewer than half its nodes.  A node array whose nodes are shared (both
+  // children one node, say: huff_parse takes any children with larger numbers)
+  // can have up to 4096 of them whatever its size; those past this room have
+  // no table.
   L.lut2_cap = std::min<size_t>(LUT1, (size_t)j.node_count / 2 + 1);
   L.zero = align_up(8 * L.write_tiles + 16, 256);
   L.rest = align_up(10 * (size_t)LUT1, 256) + align_up(4 * L.lut2_cap * LUT2, 256) + align_up(L.nsub + 1, 256) +

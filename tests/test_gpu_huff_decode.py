@@ -112,3 +112,59 @@ def test_gpu_decoder_refuses_short_streams(ctx, oracle):
     blob[36 + 13] = 0  # the id tree's root is its own left child
     with pytest.raises(cpsz_b200.CpszError):
         cpsz_b200.sz_decompress_cp_preserve_2d_offline(bytes(blob), r1, r2, ctx=ctx)
+
+
+def shared_node_section(oracle, states, sym, rng, chain=12):
+    """The Huffman section of `sym` with `chain` nodes put before its tree,
+    each the next one's parent twice over, and a made-up `chain`-bit prefix
+    before every code: a node array that is no tree, of which every
+    `chain`-bit pattern leads to one inner node."""
+    sec = oracle.huffman_encode(states, sym.astype(np.int32))
+    nc, size = struct.unpack_from("<QI", sec)
+    wdt = lambda k: np.uint8 if k <= 256 else np.uint16 if k <= 65536 else np.uint32  # noqa: E731
+    w, at = np.dtype(wdt(nc)).itemsize, 13
+    left, right = (np.frombuffer(sec, wdt(nc), nc, at + k * w * nc).astype(np.int64) for k in (0, 1))
+    symbols = np.frombuffer(sec, "<u4", nc, at + 2 * w * nc)
+    leaf = np.frombuffer(sec, np.uint8, nc, at + (2 * w + 4) * nc)
+    code, length = {}, {}
+    todo = [(0, 0, 0)]
+    while todo:
+        node, c, n = todo.pop()
+        if leaf[node]:
+            code[int(symbols[node])], length[int(symbols[node])] = c, n
+        else:
+            todo += [(left[node], 2 * c, n + 1), (right[node], 2 * c + 1, n + 1)]
+    step = np.arange(1, chain + 1)
+    shift = lambda a: np.concatenate([step, np.where(leaf != 0, 0, a + chain)]).astype(wdt(nc + chain))  # noqa: E731
+    tree = b"".join([shift(left).tobytes(), shift(right).tobytes(),
+                     np.concatenate([np.zeros(chain, "<u4"), symbols]).astype("<u4").tobytes(),
+                     bytes(chain) + leaf.tobytes()])
+    prefix = rng.integers(0, 1 << chain, sym.size)
+    bits = "".join(f"{p:0{chain}b}{code[s]:0{length[s]}b}" for p, s in zip(prefix.tolist(), sym.tolist()))
+    data = int(bits.ljust(-(-len(bits) // 8) * 8, "0"), 2).to_bytes(-(-len(bits) // 8), "big")
+    return struct.pack("<QI", nc + chain, 1 + len(tree)) + sec[12:13] + tree + struct.pack("<Q", len(data)) + data
+
+
+@pytest.mark.parametrize("kind,chain", [("two", 12), ("fixed3", 12), ("cauchy", 13), ("wide", 12), ("two", 21)])
+def test_gpu_decoder_node_arrays_that_are_no_tree(ctx, oracle, kind, chain):
+    """Nodes shared by several parents: 4096 patterns of 12 bits that no code
+    ends in, where the second-level tables have room for half the nodes (8 of
+    them in the smallest case).  The codes past the room are walked, and the
+    symbols are those of the plain tree."""
+    rng = np.random.default_rng(chain)
+    r1, r2 = 90, 130
+    n = r1 * r2
+    codes = [np.asarray(streams(kind, n, rng)), np.asarray(streams("wide", n, rng))]
+    ids = ids_of("cauchy", 2 * n, rng)
+    blob = blob_2d(oracle, ids, codes, r1, r2, rng)
+    eb_size, u_size = struct.unpack_from("<QQ", blob, 12)
+    v = blob[36 + eb_size + u_size:]
+    n_unpred = struct.unpack_from("<Q", blob, 36 + eb_size + 25)[0]
+    head = 33 + 4 * n_unpred + ((r1 - 1) // 12 * ((r2 - 1) // 12 + 1) + (r2 - 1) // 12) // 8 + 1
+    u = blob[36 + eb_size:36 + eb_size + head] + shared_node_section(oracle, 131072, codes[0], rng, chain)
+    sec = shared_node_section(oracle, 2048, ids, rng, chain)
+    made = blob[:12] + struct.pack("<QQQ", len(sec), len(u), len(v)) + sec + u + v
+    ou, ov = oracle.decompress_2d(blob, r1, r2)
+    du, dv = cpsz_b200.sz_decompress_cp_preserve_2d_offline(made, r1, r2, ctx=ctx)
+    assert_bits_equal(du, ou)
+    assert_bits_equal(dv, ov)
