@@ -265,6 +265,13 @@ __device__ __forceinline__ void w3_help(const W3Args& a, W3Smem<DECOMP>& M, cons
     w3_wait(a, U, 0, lane, have, aborted);
     w3_load_boundary(a, M, U, -W3_W, lane);
     w3_load_boundary(a, M, U, 0, lane);
+    // Slot -1's entry 0 is there when the barrier opens window 0: plane p + 1
+    // reads it in step 0, before the first barrier among the compute warps.
+    // It is row j0-1 at column -p, which exists for p = 0 alone.
+    if (lane < W3_P) {
+      const bool act = U.s > 0 && lane == 0;
+      cp16(&M.ring[lane][W3_SR - 1][0], act ? a.rec + ((long long)U.i0 * a.r2 + U.j0 - 1) * a.r3 : a.rec, act);
+    }
     cp_wait_all();
     __syncthreads();  // window 0 starts
     for (int w = 0; w < nwin; w++) {
@@ -313,16 +320,13 @@ __device__ __forceinline__ void w3_compute(const W3Args& a, W3Smem<DECOMP>& M, c
   // q0 = (i-1,j-1,k-1), q1 = (i-1,j-1,k), q2 = (i-1,j,k-1), q3 = (i-1,j,k),
   // q4 = (i,j-1,k-1), q5 = (i,j-1,k), q6 = (i,j,k-1)
   float4 q0 = Z, q1, q2 = Z, q4 = Z, q5, q6 = Z;
-  for (int sl = W3_SR - 2; sl < W3_SR; sl++) {  // steps -2 and -1
-    M.ring[p][sl][lane + 1] = Z;
-    if (lane == 0) M.ring[p][sl][0] = Z;
-  }
+  for (int sl = W3_SR - 2; sl < W3_SR; sl++) M.ring[p][sl][lane + 1] = Z;  // steps -2 and -1
+  if (lane == 0) M.ring[p][W3_SR - 2][0] = Z;  // (step -1's comes with the boundary)
   const int nwin = (U.t_end + W3_W - 1) / W3_W;
   for (int w = 0; w < nwin; w++) {
     __syncthreads();  // window w's values are loaded, window w-1 is computed
     const int cur = W3_W * (w & 1), prev = W3_W - cur;
     if (lane < W3_W) M.ring[p][cur + lane][0] = M.edge[p][(W3_W * w + lane) & (W3_SL - 1)];
-    if (w == 0 && lane == W3_W) M.ring[p][W3_SR - 1][0] = M.edge[p][W3_SL - 1];
     __syncwarp();
     float4 (*const R)[33] = &M.ring[p][cur];
     const float4 (*const Rp)[33] = &M.ring[p][prev];

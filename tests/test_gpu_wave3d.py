@@ -27,3 +27,19 @@ def test_recursion_edges(ctx, oracle, shape, raw):
     got = cpsz_b200.sz_decompress_cp_preserve_3d_online_log(blob, *shape, ctx=ctx)
     for a, b in zip(got, oracle.decompress_3d(expect, *shape)):
         assert_bits_equal(a, b)
+
+
+@pytest.mark.parametrize("shape", [(2, 33, 1), (2, 64, 2), (9, 97, 1), (16, 160, 3), (2, 1000, 1)])
+def test_first_column_above_a_unit(ctx, oracle, shape):
+    """A unit's second plane predicts its first column from the row above the
+    unit in its first step, before the compute warps' first barrier: thin
+    fields of many units, many times over, always the oracle's bytes."""
+    rng = np.random.default_rng(shape[1])
+    fields = [(rng.standard_normal(shape) * 0.1 + 2.0 ** c).astype(np.float32) for c in (0, 3, -4)]
+    expect = oracle.compress_3d(*fields, 0.1)
+    out = oracle.decompress_3d(expect, *shape)
+    for _ in range(20):
+        blob = cpsz_b200.sz_compress_cp_preserve_3d_offline_log(*fields, max_pwr_eb=0.1, ctx=ctx)
+        assert blob == expect
+        for a, b in zip(cpsz_b200.sz_decompress_cp_preserve_3d_online_log(blob, *shape, ctx=ctx), out):
+            assert_bits_equal(a, b)
