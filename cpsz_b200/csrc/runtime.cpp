@@ -338,6 +338,7 @@ int cpsz_b200_ctx_create(int device, cpsz_b200_ctx** out) {
   for (auto& ev : c->ev) CPSZ_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   for (auto& ev : c->up_ev) CPSZ_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   for (auto& ev : c->stage_ev) CPSZ_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  CPSZ_CUDA_TRY(cudaEventCreateWithFlags(&c->stage_arm, cudaEventDisableTiming));
   CPSZ_CUDA_TRY(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device));
   CPSZ_CUDA_TRY(cudaMalloc((void**)&c->d_flag, 64));
   CPSZ_CUDA_TRY(cudaMemset(c->d_flag, 0, 64));
@@ -370,6 +371,7 @@ int cpsz_b200_ctx_destroy(cpsz_b200_ctx* c) {
     if (ev) cudaEventDestroy(ev);
   for (auto& ev : c->stage_ev)
     if (ev) cudaEventDestroy(ev);
+  if (c->stage_arm) cudaEventDestroy(c->stage_arm);
   for (auto& ev : c->tev)
     if (ev) cudaEventDestroy(ev);
   cudaStreamDestroy(c->stream);

@@ -103,6 +103,7 @@ struct cpsz_b200_ctx {
   int stage_pos = 0;  // the next copy's first slot
   void* stage = nullptr;
   cudaEvent_t stage_ev[kStageSlots] = {};
+  cudaEvent_t stage_arm = nullptr;  // what a download waits for before its first piece
   void* pinned = nullptr;
   size_t pinned_cap = 0;
   // pinned staging of a pass's small uploads made once the pass's trees are

@@ -13,26 +13,13 @@
 #include "transfer.h"
 
 #include <algorithm>
-#include <atomic>
-#include <condition_variable>
 #include <cstring>
-#include <functional>
-#include <mutex>
-#include <thread>
-#include <vector>
-#ifdef __SSE2__
-#include <emmintrin.h>
-#endif
+
+#include "copy_pool.h"
 
 namespace cpsz {
 
 namespace {
-
-inline void relax() {
-#ifdef __SSE2__
-  _mm_pause();
-#endif
-}
 
 // memcpy with streaming stores (complete when it returns).
 void stream_copy(char* d, const char* s, size_t n) {
@@ -55,105 +42,19 @@ void stream_copy(char* d, const char* s, size_t n) {
 #endif
 }
 
-// Process-wide copy threads.  One job at a time (contexts on several threads
-// take turns): run(pieces, work, drive) has the workers take pieces 0, 1, ...
-// and call work(k) for each once `open` exceeds k, while the calling thread
-// runs drive(open, done), which opens pieces and waits for done[k].
-class CopyPool {
- public:
-  static CopyPool& get() {
-    static CopyPool p;
-    return p;
+// dst[0, n) = src[0, n), by the calling thread and the copy threads.
+void parallel_copy(void* dst, const void* src, size_t n) {
+  constexpr size_t P = (size_t)256 << 10;
+  CopyPool& pool = CopyPool::get();
+  if (n < 2 * P || !pool.parallel()) {
+    memcpy(dst, src, n);
+    return;
   }
-  bool parallel() const { return !workers_.empty(); }
-
-  template <class Work, class Drive>
-  int run(int pieces, const Work& work, const Drive& drive) {
-    std::lock_guard<std::mutex> turn(turn_);
-    std::vector<std::atomic<int>> done(pieces);
-    for (auto& d : done) d.store(0, std::memory_order_relaxed);
-    std::atomic<int> open{0}, next{0};
-    std::atomic<bool> stop{false};
-    auto body = [&] {
-      for (int k; (k = next.fetch_add(1)) < pieces;) {
-        while (open.load(std::memory_order_acquire) <= k) {
-          if (stop.load(std::memory_order_relaxed)) return;
-          relax();
-        }
-        work(k);
-        done[k].store(1, std::memory_order_release);
-      }
-    };
-    const std::function<void()> f = body;
-    {
-      std::lock_guard<std::mutex> lk(m_);
-      f_ = &f;
-      active_ = (int)workers_.size();
-      gen_++;
-    }
-    cv_.notify_all();
-    const int rc = drive(open, done);
-    if (rc != CPSZ_OK) stop.store(true);  // pieces that were never opened
-    std::unique_lock<std::mutex> lk(m_);
-    done_.wait(lk, [&] { return active_ == 0; });
-    f_ = nullptr;
-    return rc;
-  }
-
-  void copy(void* dst, const void* src, size_t n) {
-    constexpr size_t P = (size_t)256 << 10;
-    if (n < 2 * P || !parallel()) {
-      memcpy(dst, src, n);
-      return;
-    }
-    const int pieces = (int)((n + P - 1) / P);
-    run(
-        pieces,
-        [&](int k) { stream_copy((char*)dst + k * P, (const char*)src + k * P, std::min(P, n - k * P)); },
-        [&](std::atomic<int>& open, std::vector<std::atomic<int>>&) {
-          open.store(pieces, std::memory_order_release);
-          return CPSZ_OK;
-        });
-  }
-
- private:
-  CopyPool() {
-    const unsigned hw = std::thread::hardware_concurrency();
-    const int nw = (int)std::min(8u, hw > 1 ? hw - 1 : 0u);
-    for (int w = 0; w < nw; w++) workers_.emplace_back([this] { loop(); });
-  }
-  ~CopyPool() {
-    {
-      std::lock_guard<std::mutex> lk(m_);
-      stop_ = true;
-    }
-    cv_.notify_all();
-    for (auto& t : workers_) t.join();
-  }
-  void loop() {
-    unsigned long long seen = 0;
-    for (;;) {
-      const std::function<void()>* f;
-      {
-        std::unique_lock<std::mutex> lk(m_);
-        cv_.wait(lk, [&] { return stop_ || gen_ != seen; });
-        if (stop_) return;
-        seen = gen_;
-        f = f_;
-      }
-      (*f)();
-      std::lock_guard<std::mutex> lk(m_);
-      if (--active_ == 0) done_.notify_one();
-    }
-  }
-  std::vector<std::thread> workers_;
-  std::mutex turn_, m_;
-  std::condition_variable cv_, done_;
-  const std::function<void()>* f_ = nullptr;
-  int active_ = 0;
-  unsigned long long gen_ = 0;
-  bool stop_ = false;
-};
+  auto work = [&](int k) { stream_copy((char*)dst + k * P, (const char*)src + k * P, std::min(P, n - k * P)); };
+  CopyPool::Job job(pool, work);
+  job.open((int)((n + P - 1) / P));
+  job.help();
+}
 
 // copies at least this large from or to pageable memory go through the ring
 constexpr size_t kStageMin = (size_t)1 << 20;
@@ -174,10 +75,6 @@ int stage_reserve(cpsz_b200_ctx* ctx) {
 size_t piece_bytes(size_t n) {
   const size_t step = (size_t)64 << 10, least = (size_t)256 << 10;
   return std::min(cpsz_b200_ctx::kStageBytes, std::max(least, align_up(n / 16, step)));
-}
-
-inline void wait_for(const std::atomic<int>& d) {
-  while (!d.load(std::memory_order_acquire)) relax();
 }
 
 }  // namespace
@@ -205,6 +102,7 @@ int h2d(cpsz_b200_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t s
   CopyPool& pool = CopyPool::get();
   const size_t C = piece_bytes(n), W = cpsz_b200_ctx::kStageBytes;
   const int S = cpsz_b200_ctx::kStageSlots;
+  static_assert(cpsz_b200_ctx::kStageSlots <= CopyPool::kWindow, "a slot's piece is waited for before its next one");
   char* ring = (char*)ctx->stage;
   const int pieces = (int)((n + C - 1) / C), pos = ctx->stage_pos;
   ctx->stage_pos = (pos + pieces) % S;
@@ -213,27 +111,29 @@ int h2d(cpsz_b200_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t s
   auto work = [&](int k) { stream_copy(ring + slot(k) * W, (const char*)src + (size_t)k * C, bytes(k)); };
   // piece k's slot is free once its last transfer is done: that of piece k - S
   // here, or of an earlier call's (its event may still be pending)
-  auto drive = [&](std::atomic<int>& open, std::vector<std::atomic<int>>& done) -> int {
+  if (pool.parallel()) {
+    CopyPool::Job job(pool, work);
     int opened = 0;
     for (int k = 0; k < pieces; k++) {
-      while (opened < pieces && opened < k + S) {
-        const cudaError_t e = cudaEventQuery(ctx->stage_ev[slot(opened)]);
+      int free = opened;
+      while (free < pieces && free < k + S) {
+        const cudaError_t e = cudaEventQuery(ctx->stage_ev[slot(free)]);
         if (e == cudaErrorNotReady) {
-          if (opened > k) break;  // enough to go on with
-          CPSZ_CUDA_TRY(cudaEventSynchronize(ctx->stage_ev[slot(opened)]));
+          if (free > k) break;  // enough to go on with
+          CPSZ_CUDA_TRY(cudaEventSynchronize(ctx->stage_ev[slot(free)]));
         } else {
           CPSZ_CUDA_TRY(e);
         }
-        open.store(++opened, std::memory_order_release);
+        if (++free == opened + 4) job.open(opened = free);  // copied while the other slots are looked at
       }
-      wait_for(done[k]);
+      job.open(opened = free);
+      job.wait(k);
       CPSZ_CUDA_TRY(cudaMemcpyAsync((char*)dst + (size_t)k * C, ring + slot(k) * W, bytes(k), cudaMemcpyHostToDevice,
                                     st));
       CPSZ_CUDA_TRY(cudaEventRecord(ctx->stage_ev[slot(k)], st));
     }
     return CPSZ_OK;
-  };
-  if (pool.parallel()) return pool.run(pieces, work, drive);
+  }
   for (int k = 0; k < pieces; k++) {
     CPSZ_CUDA_TRY(cudaEventSynchronize(ctx->stage_ev[slot(k)]));
     work(k);
@@ -255,6 +155,7 @@ int d2h(cpsz_b200_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t s
   CopyPool& pool = CopyPool::get();
   const size_t C = piece_bytes(n), W = cpsz_b200_ctx::kStageBytes;
   const int S = cpsz_b200_ctx::kStageSlots;
+  static_assert(cpsz_b200_ctx::kStageSlots <= CopyPool::kWindow, "a slot's piece is waited for before its next one");
   char* ring = (char*)ctx->stage;
   const int pieces = (int)((n + C - 1) / C), pos = ctx->stage_pos;
   ctx->stage_pos = (pos + pieces) % S;
@@ -269,20 +170,25 @@ int d2h(cpsz_b200_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t s
     return CPSZ_OK;
   };
   const int ahead = S / 2;  // transfers in flight; the other slots are being copied out
-  auto drive = [&](std::atomic<int>& open, std::vector<std::atomic<int>>& done) -> int {
+  if (pool.parallel()) {
+    CopyPool::Job job(pool, work);
+    job.arm();
+    CPSZ_CUDA_TRY(cudaEventRecord(ctx->stage_arm, st));
     for (int k = 0; k < pieces && k < ahead; k++) CPSZ_TRY(issue(k));
+    CPSZ_CUDA_TRY(cudaEventSynchronize(ctx->stage_arm));  // the kernels before the copy are done
+    job.arm();  // (again: those that had nothing to do for a millisecond sleep)
     for (int k = 0; k < pieces; k++) {
       CPSZ_CUDA_TRY(cudaEventSynchronize(ctx->stage_ev[slot(k)]));
-      open.store(k + 1, std::memory_order_release);
+      job.open(k + 1);
       const int q = k + ahead;
       if (q < pieces) {
-        if (q >= S) wait_for(done[q - S]);
+        if (q >= S) job.wait(q - S);
         CPSZ_TRY(issue(q));
       }
     }
+    job.help();
     return CPSZ_OK;
-  };
-  if (pool.parallel()) return pool.run(pieces, work, drive);
+  }
   for (int k = 0; k < pieces; k++) {
     CPSZ_TRY(issue(k));
     CPSZ_CUDA_TRY(cudaEventSynchronize(ctx->stage_ev[slot(k)]));
@@ -296,7 +202,7 @@ int Upload::send_whole(cpsz_b200_ctx* ctx, uint8_t* dst, cudaStream_t st) const 
   CPSZ_TRY(upload_reserve(ctx, bytes_));
   char* h = (char*)ctx->up_pinned;
   for (const Piece& p : pieces_) {
-    CopyPool::get().copy(h + p.at, p.src, p.n);
+    parallel_copy(h + p.at, p.src, p.n);
     memset(h + p.at + p.n, 0, p.pad);
   }
   CPSZ_CUDA_TRY(cudaMemcpyAsync(dst, h, bytes_, cudaMemcpyHostToDevice, st));

@@ -3,8 +3,9 @@
 // Device and page-locked host memory are copied directly (enqueued on `st`).
 // Pageable host memory of 1 MiB or more moves through the context's pinned
 // ring (kStageSlots slots of kStageBytes) with the host copies spread over a
-// small thread pool, piece by piece, the pieces' DMA overlapping the others'
-// host copies.  For pageable memory both calls return once the host
+// small thread pool (copy_pool.h), piece by piece, the pieces' DMA overlapping
+// the others' host copies.  Transfers of several contexts share the pool's
+// threads and wait for one another nowhere.  For pageable memory both calls return once the host
 // side is complete: after h2d the source may be reused, after d2h the
 // destination holds the data.  Device-side ordering is that of `st`.
 #pragma once
