@@ -343,9 +343,14 @@ __global__ void __launch_bounds__(STRIP_NT, STRIP_CTAS) strip_unpass_kernel(Stri
                                                                 int nsc, unsigned int ns, int* flag) {
   __shared__ StripShared sh;
   const StripUnpass P = blockIdx.y ? P1 : P0;
-  if (threadIdx.x == 0) sh.idx = atomicAdd(reinterpret_cast<unsigned int*>(P.status + ns), 1u);
+  if (threadIdx.x == 0) {
+    const bool again = decode_again(flag);
+    const unsigned int t = atomicAdd(reinterpret_cast<unsigned int*>(P.status + ns), 1u);
+    sh.idx = again ? ns : t;
+  }
   __syncthreads();
   const unsigned int s = sh.idx;
+  if (s >= ns) return;
   const StripGeom g = strip_geom(s, r1, r2, nsc);
   const int E = g.h * g.W, phase = (int)(g.out0 & 7);
   uint16_t* const img = sh.img + phase;

@@ -24,6 +24,10 @@ constexpr int FLAG_HUFF_CORRUPT = 4;  // a Huffman stream does not decode to the
 constexpr int FLAG_RAW_RANGE = 8;     // an unpredictable-value index fell outside the stored list
 constexpr int FLAG_OUT_CAPACITY = 16; // an output stream did not fit its buffer
 constexpr int FLAG_HUFF_RESYNC = 32;  // a Huffman stream needs more synchronisation rounds (launch_huff_decode)
+#ifdef __CUDACC__
+// Whether the decoder before this kernel asked for another attempt (it alone raises the flag).
+__device__ __forceinline__ bool decode_again(const int* flag) { return (*(const volatile int*)flag & FLAG_HUFF_RESYNC) != 0; }
+#endif
 
 // ---- 2D error bounds ---------------------------------------------------------
 // The bound kernel beside the wavefront runs unit by unit: a unit is a
@@ -306,7 +310,8 @@ struct HuffDecJob {
 // Up to three streams at once.  A stream whose subsequences did not settle in
 // the fixed rounds raises FLAG_HUFF_RESYNC (its output is then incomplete):
 // the caller decodes again with settle, which waits on the host until they
-// have.  A stream that does not decode to n symbols raises FLAG_HUFF_CORRUPT.
+// have.  The decompressors' kernels queued behind the decoder leave at once
+// then (decode_again), so what the caller gets is decoded once.  A stream that does not decode to n symbols raises FLAG_HUFF_CORRUPT.
 // tmp: huff_decode_tmp_bytes(jobs, nj).
 size_t huff_decode_tmp_bytes(const HuffDecJob* jobs, int nj);
 int launch_huff_decode(cpsz_b200_ctx* ctx, const HuffDecJob* jobs, int nj, void* tmp, bool settle);

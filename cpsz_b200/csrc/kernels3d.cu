@@ -316,6 +316,7 @@ __global__ void __launch_bounds__(CH_NT) prep3d_kernel(const uint8_t* __restrict
                                                        float4* __restrict__ pairs, LibmFn Lg, float* __restrict__ U,
                                                        float* __restrict__ V, float* __restrict__ W,
                                                        int* __restrict__ flag) {
+  if (decode_again(flag)) return;
   __shared__ uint8_t s_raw[CH_NT / 32][32 * CH_PER_T];  // the warps' raw points
   const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
   uint8_t iv[CH_PER_T];

@@ -52,7 +52,9 @@ __global__ void __launch_bounds__(256) log2d_kernel(const float* __restrict__ U,
 
 __global__ void __launch_bounds__(256) exp2d_kernel(float* __restrict__ U, float* __restrict__ V,
                                                     const uint8_t* __restrict__ sign_u,
-                                                    const uint8_t* __restrict__ sign_v, size_t n, LibmFn Ex) {
+                                                    const uint8_t* __restrict__ sign_v, size_t n, LibmFn Ex,
+                                                    const int* __restrict__ flag) {
+  if (decode_again(flag)) return;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += stride) {
     const unsigned byte_bit = 7u - (unsigned)(idx & 7);
@@ -90,7 +92,7 @@ int launch_log2d(cpsz_b200_ctx* ctx, const float* U, const float* V, const uint8
 int launch_exp2d(cpsz_b200_ctx* ctx, float* U, float* V, const uint8_t* sign_u, const uint8_t* sign_v, size_t n,
                  const LibmFn& Ex) {
   if (n == 0) return CPSZ_OK;
-  exp2d_kernel<<<grid_of(ctx, n), 256, 0, ctx->stream>>>(U, V, sign_u, sign_v, n, Ex);
+  exp2d_kernel<<<grid_of(ctx, n), 256, 0, ctx->stream>>>(U, V, sign_u, sign_v, n, Ex, ctx->d_flag);
   count_launch(ctx);
   return check_launch("exp2d_kernel");
 }

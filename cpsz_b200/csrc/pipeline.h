@@ -68,6 +68,13 @@ int compress_3d(cpsz_b200_ctx* ctx, const float* U, const float* V, const float*
 int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_size, size_t r1, size_t r2, size_t r3,
                   float* U, float* V, float* W);
 
+// Decompression to host memory: whether the decoders just queued on
+// ctx->stream ask for another attempt (decode_again) is read on the second
+// stream, beside the kernels behind them (probe), and is known before anything
+// is copied to the caller (seen).
+int probe_decode_again(cpsz_b200_ctx* ctx);
+int seen_decode_again(cpsz_b200_ctx* ctx, bool* again);
+
 // Copies n bytes from device memory to `dst`, which may be host or device memory.
 int copy_out(cpsz_b200_ctx* ctx, void* dst, const void* d_src, size_t n);
 // Copies n bytes from `src` (host or device) into device memory `d_dst`.

@@ -390,7 +390,8 @@ int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
   } aux_drain;
 
   // A stream whose subsequences did not settle in the decoder's fixed rounds
-  // (FLAG_HUFF_RESYNC) is decoded again, with rounds until they have.
+  // (FLAG_HUFF_RESYNC) is decoded again, with rounds until they have; what is
+  // queued behind the first attempt then does nothing.
   for (int attempt = 0;; attempt++) {
     const bool settle = attempt > 0;
     CPSZ_CUDA_TRY(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), st));
@@ -410,6 +411,11 @@ int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
         if (k < 2) CPSZ_TRY(launch_huff_decode(ctx, &dec[k], 1, dtmp[k], settle));
       }
     }
+    const bool probe = !settle && !dev_out;
+    if (probe) {
+      aux_drain.s = ctx->aux;
+      CPSZ_TRY(probe_decode_again(ctx));
+    }
     mark(ctx, "prep3d");
     CPSZ_TRY(launch_chunk_count_3d(ctx, false, ids, N, chunk_cnt));
     CPSZ_TRY(launch_scan_u32(ctx, chunk_cnt, chunk_off, nchunks, scan_tmp));
@@ -417,6 +423,11 @@ int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
     mark(ctx, "wave3d_decompress");
     CPSZ_TRY(launch_wave3d(ctx, true, pairs, rec, nullptr, signs, smap, &lt, dU, dV, dW, r1, r2, r3, wave_sync));
     mark(ctx, "d2h");
+    if (probe) {
+      bool again = false;
+      CPSZ_TRY(seen_decode_again(ctx, &again));
+      if (again) continue;
+    }
     if (!dev_out) {
       CPSZ_TRY(d2h(ctx, U_out, dU, 4 * N, st));
       CPSZ_TRY(d2h(ctx, V_out, dV, 4 * N, st));

@@ -484,7 +484,11 @@ __device__ __forceinline__ void wave2d_body(const WaveField* __restrict__ fields
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int strip = warp % WAVE_WARPS;  // the strip a compute warp runs, or its helper serves
   for (;;) {
-    if (threadIdx.x == 0) sh.item = atomicAdd(queue, 1);
+    if (threadIdx.x == 0) {
+      const bool again = DECOMP && decode_again(flag);
+      const int next = atomicAdd(queue, 1);
+      sh.item = again ? n_items : next;
+    }
     for (int k = threadIdx.x; k < (WAVE_WARPS + 1) * RING; k += blockDim.x) (&sh.ring[0][0])[k] = 0ull;
     if (threadIdx.x < WAVE_WARPS) sh.cons[threadIdx.x] = 0;
     __syncthreads();

@@ -409,7 +409,11 @@ __global__ void __launch_bounds__(W3_THREADS, 1) wave3d_kernel(const W3Args a) {
   bool aborted = false;  // the boundary warp's lanes: a wait has expired; no more waiting
   for (;;) {
     __syncthreads();  // the previous unit's results are stored
-    if (threadIdx.x == 0) M.unit = atomicAdd(a.sync, 1);
+    if (threadIdx.x == 0) {
+      const bool again = DECOMP && decode_again(a.flag);
+      const int next = atomicAdd(a.sync, 1);
+      M.unit = again ? units : next;
+    }
     __syncthreads();
     W3Unit U;
     U.u = M.unit;
@@ -432,7 +436,8 @@ __global__ void __launch_bounds__(W3_THREADS, 1) wave3d_kernel(const W3Args a) {
 __global__ void __launch_bounds__(256) exp3d_kernel(const float4* __restrict__ in, const float4* __restrict__ rec,
                                                     const uint8_t* __restrict__ signs, size_t sign_bytes, LibmFn Ex,
                                                     float* __restrict__ U, float* __restrict__ V,
-                                                    float* __restrict__ W, size_t n) {
+                                                    float* __restrict__ W, size_t n, const int* __restrict__ flag) {
+  if (decode_again(flag)) return;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += stride) {
     if (__float_as_int(in[idx].w) != 0) continue;
@@ -488,7 +493,7 @@ int launch_wave3d(cpsz_b200_ctx* ctx, bool decompress, const float4* in, float4*
   const size_t n = (size_t)r1 * r2 * r3;
   const size_t blocks = (n + 255) / 256, cap = (size_t)ctx->num_sms * 8;
   exp3d_kernel<<<(int)(blocks < cap ? blocks : cap), 256, 0, ctx->stream>>>(in, rec, signs, sign_bytes, L->exp2f, U,
-                                                                            V, W, n);
+                                                                            V, W, n, ctx->d_flag);
   count_launch(ctx);
   return check_launch("exp3d_kernel");
 }

@@ -4,6 +4,8 @@ Any code and id sequence is a valid blob, so the streams aim at the decoder's
 own edges: codes longer than one and both look-up tables, trees of every index
 width, streams that end at, before and after a subsequence's or a tile's end,
 and fixed-length codes that never synchronise (the settling rounds)."""
+import os
+import re
 import struct
 
 import numpy as np
@@ -168,3 +170,63 @@ def test_gpu_decoder_node_arrays_that_are_no_tree(ctx, oracle, kind, chain):
     du, dv = cpsz_b200.sz_decompress_cp_preserve_2d_offline(made, r1, r2, ctx=ctx)
     assert_bits_equal(du, ou)
     assert_bits_equal(dv, ov)
+
+
+def upload_whole():
+    """The library's limit for blobs that go up in one piece (bytes)."""
+    src = os.path.join(os.path.dirname(cpsz_b200.__file__), "csrc", "transfer.h")
+    m = re.search(r"UPLOAD_WHOLE = \(size_t\)(\d+) << (\d+)", open(src).read())
+    return int(m.group(1)) << int(m.group(2))
+
+
+@pytest.mark.parametrize("r1,r2", [(400, 903), (1700, 3001)])
+@pytest.mark.parametrize("which", ["ids", "u", "all"])
+@pytest.mark.parametrize("device", [False, True])
+def test_gpu_decoder_settles_streams_sent_whole_or_one_by_one(ctx, oracle, r1, r2, which, device):
+    """Streams that never synchronise in a blob that goes up whole and in one
+    above the limit, whose streams go up and are decoded one by one; into host
+    arrays and into device memory (what is queued behind the first attempt
+    must leave both to the second)."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(r1)
+    n = r1 * r2
+    kinds = {"ids": ("wide", "wide"), "u": ("fixed3", "wide"), "all": ("fixed3", "fixed16")}[which]
+    codes = [np.asarray(streams(k, n, rng)) for k in kinds]
+    blob = blob_2d(oracle, ids_of("cauchy" if which == "u" else "fixed3", 2 * n, rng), codes, r1, r2, rng)
+    assert (len(blob) > upload_whole()) == (r1 > 1000)
+    if device:
+        out = [torch.full((r1, r2), 7.0, device="cuda") for _ in range(2)]
+    else:
+        out = [np.full((r1, r2), 7.0, np.float32) for _ in range(2)]
+    cpsz_b200.sz_decompress_cp_preserve_2d_offline(blob, r1, r2, *out, ctx=ctx)
+    # (the made-up values grow past the largest float: inf - inf is a NaN, which
+    # x86 and the GPU encode differently)
+    for a, b in zip(out, oracle.decompress_2d(blob, r1, r2)):
+        assert_bits_equal(a.cpu().numpy() if device else a, b, nan_equal=True)
+
+
+@pytest.mark.parametrize("shape", [(20, 33, 47), (100, 160, 110)])
+@pytest.mark.parametrize("kind", ["fixed3", "wide"])
+@pytest.mark.parametrize("device", [False, True])
+def test_gpu_3d_decoder_settles_streams_sent_whole_or_one_by_one(ctx, oracle, shape, kind, device):
+    """The same for volumes: made-up id and code streams, most points raw."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(shape[0])
+    n = int(np.prod(shape))
+    ids = rng.permutation(np.arange(n) % 8) + 5 if kind == "fixed3" else rng.integers(5, 12, n)
+    ids = np.where(rng.random(n) < 0.65, np.where(rng.random(n) < 0.5, 0, 24), ids)
+    npred = int(((ids != 0) & (ids != 24)).sum())
+    codes = np.asarray(streams(kind, 3 * npred, rng)).clip(1, 65535)
+    raw = np.exp2(rng.uniform(-3, 3, 3 * (n - npred))).astype(np.float32) * rng.choice([-1, 1], 3 * (n - npred))
+    signs = rng.integers(0, 256, 3 * ((n - 1) // 8 + 1), np.uint8).tobytes()
+    blob = struct.pack("<ii", 2, 32768) + signs + struct.pack("<Q", raw.size) + raw.astype(np.float32).tobytes() + \
+        struct.pack("<Q", n) + oracle.huffman_encode(512, ids.astype(np.int32)) + struct.pack("<Q", codes.size) + \
+        oracle.huffman_encode(131072, codes.astype(np.int32))
+    assert (len(blob) > upload_whole()) == (n > 1 << 20)
+    if device:
+        out = [torch.full(shape, 7.0, device="cuda") for _ in range(3)]
+    else:
+        out = [np.full(shape, 7.0, np.float32) for _ in range(3)]
+    cpsz_b200.sz_decompress_cp_preserve_3d_online_log(blob, *shape, *out, ctx=ctx)
+    for a, b in zip(out, oracle.decompress_3d(blob, *shape)):
+        assert_bits_equal(a.cpu().numpy() if device else a, b)
