@@ -64,7 +64,7 @@ constexpr long long DEC_SPIN_LIMIT = 1ll << 22;  // look-back polls before givin
 //          payload, so a look-up takes up to 12 symbols there
 // A pattern that no code ends in: 0 symbols, bits 16-31 the pattern's
 // second-level table; in the count entry COUNT_LONG | that table.
-// Second-level entry: symbol << 8 | code length, or 0x80 | node << 8.
+// Second-level entry: symbol << 8 | code length, or 0x80 | node << 8 (node 0: walk from the root).
 constexpr uint32_t COUNT_LONG = 0x8000u;
 
 struct DecTree {
@@ -81,7 +81,7 @@ struct DecStream {
   uint32_t* lut1;   // write entries: LUT1 words, then LUT1 payload words
   uint16_t* lutc;   // count entries
   uint32_t* lut2;
-  unsigned lut2_cap;  // second-level tables there is room for; a pattern's table may number past it
+  unsigned lut2_cap;  // second-level tables of single patterns; the one behind them is for all patterns past them
   unsigned* lut2_n;
   uint8_t* rel;     // start of each subsequence, bits after its nominal start
   uint8_t* texit;   // exit of each scan tile, bits after its end
@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(256) dec_table_kernel(const __grid_constant__ 
   __shared__ int s_n;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) s_n = 0;
+  if (blockIdx.x == 0 && S.lut2_cap < LUT1) S.lut2[(size_t)S.lut2_cap * LUT2 + threadIdx.x] = 0x80u;
   __syncthreads();
   if (threadIdx.x < TAB_PAT) {
     const uint32_t pat = blockIdx.x * TAB_PAT + lane;
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(256) dec_table_kernel(const __grid_constant__ 
     uint32_t hi16 = (uint32_t)(pay & 0xffffu), count = (uint32_t)(len0 << 8 | bits_all << 4 | nall);
     if (n == 0) {
       const int q = atomicAdd(&s_n, 1);
-      const unsigned t = atomicAdd(S.lut2_n, 1u);
+      const unsigned t = min(atomicAdd(S.lut2_n, 1u), S.lut2_cap);
       s_node[q] = node;
       s_tab[q] = t;
       hi16 = t;
@@ -227,9 +228,10 @@ __device__ __forceinline__ void stage_bits(const DecStream& S, long long g0, uin
 }
 
 // The rest of a code that the tables do not end: from `node`, whose code has
-// `l` bits.  Returns symbol << 8 | length, 0 beyond MAX_CODE.
-__device__ __noinline__ uint32_t deep_code(DecTree T, Bits b, int pos, uint32_t node, int l) {
-  while (l < MAX_CODE) {
+// LUT1_BITS + LUT2_BITS bits, or from the root (node 0: a pattern without a
+// table).  Returns symbol << 8 | length, 0 beyond MAX_CODE.
+__device__ __noinline__ uint32_t deep_code(DecTree T, Bits b, int pos, uint32_t node) {
+  for (int l = node ? LUT1_BITS + LUT2_BITS : 0; l < MAX_CODE;) {
     const int at = pos + l;
     const uint32_t bit = (b.word(at >> 5) >> (31 - (at & 31))) & 1u;
     const TreeNode nd = tree_node(T, node);
@@ -242,12 +244,10 @@ __device__ __noinline__ uint32_t deep_code(DecTree T, Bits b, int pos, uint32_t 
 }
 
 // A code over 12 bits (second-level table `t`, next8 its bits after them):
-// symbol << 8 | length; 0: no code.  A pattern past the tables' room has none
-// (lut2_cap): its code is walked from the root.
+// symbol << 8 | length; 0: no code.
 __device__ __forceinline__ uint32_t long_code(const DecStream& S, Bits b, int pos, uint32_t t, uint32_t next8) {
-  if (t >= S.lut2_cap) return deep_code(S.tree, b, pos, 0, 0);
   const uint32_t e = __ldg(S.lut2 + (size_t)t * LUT2 + next8);
-  return e & 0x80u ? deep_code(S.tree, b, pos, e >> 8, LUT1_BITS + LUT2_BITS) : e;
+  return e & 0x80u ? deep_code(S.tree, b, pos, e >> 8) : e;
 }
 
 // Length of the one code at `pos` (lut: count entries).
@@ -605,11 +605,11 @@ DecLayout dec_layout(const HuffDecJob& j) {
   // Patterns that no code ends in are paths to inner nodes at depth 12: in a
   // tree fewer than half its nodes.  A node array whose nodes are shared (both
   // children one node, say: huff_parse takes any children with larger numbers)
-  // can have up to 4096 of them whatever its size; those past this room have
-  // no table.
+  // can have up to 4096 of them whatever its size: those past this room share
+  // one table more, whose entries have the code walked from the root.
   L.lut2_cap = std::min<size_t>(LUT1, (size_t)j.node_count / 2 + 1);
   L.zero = align_up(8 * L.write_tiles + 16, 256);
-  L.rest = align_up(10 * (size_t)LUT1, 256) + align_up(4 * L.lut2_cap * LUT2, 256) + align_up(L.nsub + 1, 256) +
+  L.rest = align_up(10 * (size_t)LUT1, 256) + align_up(4 * (L.lut2_cap + 1) * LUT2, 256) + align_up(L.nsub + 1, 256) +
            align_up(L.scan_tiles + 1, 256) + align_up(2 * (L.nsub + 1), 256);
   return L;
 }
@@ -682,7 +682,7 @@ int launch_huff_decode(cpsz_b200_ctx* ctx, const HuffDecJob* jobs, int nj, void*
     };
     S.lut1 = (uint32_t*)take(10 * (size_t)LUT1);
     S.lutc = (uint16_t*)(S.lut1 + 2 * LUT1);
-    S.lut2 = (uint32_t*)take(4 * lay[k].lut2_cap * LUT2);
+    S.lut2 = (uint32_t*)take(4 * (lay[k].lut2_cap + 1) * LUT2);
     S.rel = (uint8_t*)take(lay[k].nsub + 1);
     S.texit = (uint8_t*)take(lay[k].scan_tiles + 1);
     S.cnt = (uint16_t*)take(2 * (lay[k].nsub + 1));
