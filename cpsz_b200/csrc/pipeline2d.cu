@@ -667,6 +667,12 @@ int run_pass(cpsz_b200_ctx* ctx, std::vector<Job2D>& jobs, const StageTap* tap, 
     // below), so serialised execution costs that wait, not a failure.
     CPSZ_TRY(preload_eb2d());
     CPSZ_TRY(preload_wave2d());
+    for (const Job2D& j : jobs)
+      if (!j.dev_in) {  // a band and the row below it are copied at once
+        const size_t band = 4 * (size_t)std::min(j.r1, band_rows(j) + 1) * j.r2;
+        CPSZ_TRY(transfer_reserve(ctx, j.U_in, band));
+        CPSZ_TRY(transfer_reserve(ctx, j.V_in, band));
+      }
     hi_drain.s = ctx->hi;
     CPSZ_CUDA_TRY(cudaEventRecord(ctx->ev[3], st));
     CPSZ_CUDA_TRY(cudaStreamWaitEvent(ctx->hi, ctx->ev[3], 0));

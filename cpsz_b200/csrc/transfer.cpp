@@ -90,6 +90,10 @@ HostKind host_kind(const void* p) {
   return HOST_PAGEABLE;
 }
 
+int transfer_reserve(cpsz_b200_ctx* ctx, const void* host, size_t n) {
+  return n >= kStageMin && host_kind(host) == HOST_PAGEABLE ? stage_reserve(ctx) : CPSZ_OK;
+}
+
 int h2d(cpsz_b200_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t st) {
   if (!n) return CPSZ_OK;
   const HostKind k = host_kind(src);

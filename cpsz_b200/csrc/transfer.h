@@ -21,6 +21,9 @@ HostKind host_kind(const void* p);
 
 int h2d(cpsz_b200_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t st);
 int d2h(cpsz_b200_ctx* ctx, void* dst, const void* src, size_t n, cudaStream_t st);
+// Whatever a copy of n bytes between the device and `host` allocates the first
+// time (the ring: 64 MB, some 25 ms), before work that must not wait for it.
+int transfer_reserve(cpsz_b200_ctx* ctx, const void* host, size_t n);
 
 // Several host pieces that go up to one device buffer: add() places a piece
 // (256-byte aligned, `pad` zero bytes behind it) and returns its offset there;

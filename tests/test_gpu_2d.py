@@ -186,6 +186,23 @@ def test_gpu_histogram_follower_that_gives_up_recounts(oracle):
         c.close()
 
 
+def test_gpu_first_host_call_does_not_hold_up_the_wavefront(ctx, oracle):
+    """A context's first copy from pageable memory allocates its page-locked
+    ring (64 MB, some 25 ms), which must not happen while a wavefront waits for
+    the bounds of the rows being copied: with the wait's limit at 15 ms the
+    first call of a new context runs no wavefront twice."""
+    U, V = W.cfg0_like(10, 1000, 1100)
+    expect = oracle.compress_2d(U, V, 0.1)
+    assert_blob_equal_2d(cpsz_b200.sz_compress_cp_preserve_2d_offline(U, V, max_pwr_eb=0.1, ctx=ctx), expect)
+    c = cpsz_b200.Context(0)
+    try:
+        c.debug_band_wait(15_000_000, unreachable=False)
+        assert_blob_equal_2d(cpsz_b200.sz_compress_cp_preserve_2d_offline(U, V, max_pwr_eb=0.1, ctx=c), expect)
+        assert c.wave_reruns == 0
+    finally:
+        c.close()
+
+
 def test_gpu_serialised_launches_still_compress(tmp_path):
     """With every launch serialised (CUDA_LAUNCH_BLOCKING=1, as under tools that
     run kernels one at a time) the wavefront waits for bounds that no kernel
