@@ -149,8 +149,10 @@ class CopyPool {
     for (auto& t : workers_) t.join();
   }
   static CopyPool& get() {
-    const unsigned hw = std::thread::hardware_concurrency();
-    static CopyPool p((int)std::min(8u, hw > 1 ? hw - 1 : 0u));
+    static CopyPool p([] {
+      const unsigned hw = std::thread::hardware_concurrency();
+      return (int)std::min(8u, hw > 1 ? hw - 1 : 0u);
+    }());
     return p;
   }
   bool parallel() const { return !workers_.empty(); }
