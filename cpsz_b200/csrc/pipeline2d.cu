@@ -1426,12 +1426,13 @@ int decompress_2d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
   unsigned int* h_cnt = (unsigned int*)ctx->pinned + 16;
 
   // a copy from the caller's page-locked blob must not outlive the call
-  struct AuxDrain {
+  struct Drain {
     cudaStream_t s = nullptr;
-    ~AuxDrain() {
+    ~Drain() {
       if (s) cudaStreamSynchronize(s);
     }
-  } aux_drain;
+  } aux_drain, main_drain;
+  main_drain.s = st;
 
   // A stream whose subsequences did not settle in the decoder's fixed rounds
   // (FLAG_HUFF_RESYNC) is decoded again, with rounds until they have; what is
@@ -1493,7 +1494,8 @@ int decompress_2d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
     }
     mark(ctx, "end");
     int flag = 0;
-    CPSZ_TRY(read_flag(ctx, &flag));
+    CPSZ_TRY(read_flag(ctx, &flag));  // synchronizes the stream
+    main_drain.s = nullptr;
     if ((flag & FLAG_HUFF_RESYNC) && !settle) continue;
     if (flag) return flag_error(flag);
     break;

@@ -382,12 +382,13 @@ int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
     dec[k].out = k ? (void*)codes : (void*)ids;
   }
   // a copy from the caller's page-locked blob must not outlive the call
-  struct AuxDrain {
+  struct Drain {
     cudaStream_t s = nullptr;
-    ~AuxDrain() {
+    ~Drain() {
       if (s) cudaStreamSynchronize(s);
     }
-  } aux_drain;
+  } aux_drain, main_drain;
+  main_drain.s = st;
 
   // A stream whose subsequences did not settle in the decoder's fixed rounds
   // (FLAG_HUFF_RESYNC) is decoded again, with rounds until they have; what is
@@ -435,7 +436,8 @@ int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_siz
     }
     mark(ctx, "end");
     int flag = 0;
-    CPSZ_TRY(read_flag3(ctx, &flag));
+    CPSZ_TRY(read_flag3(ctx, &flag));  // synchronizes the stream
+    main_drain.s = nullptr;
     if ((flag & FLAG_HUFF_RESYNC) && !settle) continue;
     if (flag) return flag_error3(flag);
     break;

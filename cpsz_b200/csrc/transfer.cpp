@@ -45,11 +45,11 @@ void stream_copy(char* d, const char* s, size_t n) {
 // dst[0, n) = src[0, n), by the calling thread and the copy threads.
 void parallel_copy(void* dst, const void* src, size_t n) {
   constexpr size_t P = (size_t)256 << 10;
-  CopyPool& pool = CopyPool::get();
-  if (n < 2 * P || !pool.parallel()) {
+  if (n < 2 * P || !CopyPool::get().parallel()) {
     memcpy(dst, src, n);
     return;
   }
+  CopyPool& pool = CopyPool::get();
   auto work = [&](int k) { stream_copy((char*)dst + k * P, (const char*)src + k * P, std::min(P, n - k * P)); };
   CopyPool::Job job(pool, work);
   job.open((int)((n + P - 1) / P));
@@ -58,6 +58,9 @@ void parallel_copy(void* dst, const void* src, size_t n) {
 
 // copies at least this large from or to pageable memory go through the ring
 constexpr size_t kStageMin = (size_t)1 << 20;
+// page-locked pieces of an image at least this large go up by themselves
+// instead of through its staging
+constexpr size_t kDirectMin = (size_t)256 << 10;
 
 int stage_reserve(cpsz_b200_ctx* ctx) {
   if (ctx->stage) return CPSZ_OK;
@@ -205,12 +208,25 @@ int Upload::send_whole(cpsz_b200_ctx* ctx, uint8_t* dst, cudaStream_t st) const 
   if (!bytes_) return CPSZ_OK;
   CPSZ_TRY(upload_reserve(ctx, bytes_));
   char* h = (char*)ctx->up_pinned;
+  size_t from = 0, to = 0;  // staged and not yet sent
+  auto flush = [&]() -> int {
+    if (to > from) CPSZ_CUDA_TRY(cudaMemcpyAsync(dst + from, h + from, to - from, cudaMemcpyHostToDevice, st));
+    from = to;
+    return CPSZ_OK;
+  };
   for (const Piece& p : pieces_) {
+    if (p.n >= kDirectMin && host_kind(p.src) == HOST_PINNED) {
+      CPSZ_TRY(flush());
+      CPSZ_CUDA_TRY(cudaMemcpyAsync(dst + p.at, p.src, p.n, cudaMemcpyHostToDevice, st));
+      if (p.pad) CPSZ_CUDA_TRY(cudaMemsetAsync(dst + p.at + p.n, 0, p.pad, st));
+      from = to = p.at + p.n + p.pad;
+      continue;
+    }
     parallel_copy(h + p.at, p.src, p.n);
     memset(h + p.at + p.n, 0, p.pad);
+    to = p.at + p.n + p.pad;
   }
-  CPSZ_CUDA_TRY(cudaMemcpyAsync(dst, h, bytes_, cudaMemcpyHostToDevice, st));
-  return CPSZ_OK;
+  return flush();
 }
 
 int Upload::send_part(cpsz_b200_ctx* ctx, uint8_t* dst, int part, cudaStream_t st) const {

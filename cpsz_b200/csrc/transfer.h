@@ -29,8 +29,9 @@ int transfer_reserve(cpsz_b200_ctx* ctx, const void* host, size_t n);
 // (256-byte aligned, `pad` zero bytes behind it) and returns its offset there;
 // cut() ends a part.  Either the whole image goes up in one copy from the
 // context's page-locked staging (send_whole: no other copy from it may be in
-// flight), or part by part (send_part, h2d's rules).  Sources are read when
-// they are sent.
+// flight; large pieces that are page-locked themselves go up from where they
+// are, in their own copies, and are read until these have run), or part by
+// part (send_part, h2d's rules).  Sources are read when they are sent.
 class Upload {
  public:
   size_t add(const void* src, size_t n, size_t pad = 0) {
@@ -54,7 +55,7 @@ class Upload {
   size_t bytes_ = 0;
   int part_ = 0;
 };
-// Images up to this size go up whole: one copy, one decoder launch for all
+// Images up to this size go up whole: one upload, one decoder launch for all
 // streams and no gap between them; above it the staging copy takes longer than
 // decoding a stream while the next one travels.  Whole against in parts, 2D
 // decompression from a host blob: 3.1 MB 0.56 and 0.75 ms, 6.2 MB 0.80 and 0.95,

@@ -7,6 +7,7 @@ import pytest
 
 import cpsz_b200
 from cpsz_b200 import workloads as W
+from tests._util import assert_bits_equal
 
 pytestmark = pytest.mark.gpu
 
@@ -72,3 +73,26 @@ def test_3d_pageable_and_device_give_equal_results(ctx):
     cpsz_b200.sz_decompress_cp_preserve_3d_online_log(ref, *U.shape, *b, ctx=ctx)
     for x, y in zip(a, b):
         assert x.tobytes() == y.cpu().numpy().tobytes()
+
+
+@pytest.mark.parametrize("r1,r2", [(60, 70), (500, 700), (1300, 1900)])
+def test_page_locked_blobs(ctx, oracle, r1, r2):
+    """Blobs in page-locked memory, whose larger sections go up from where they
+    are, at odd addresses; one of few bytes, which goes through the staging."""
+    import ctypes
+
+    import torch
+
+    U, V = W.cfg0_like(r1, r1, r2)
+    blob = cpsz_b200.sz_compress_cp_preserve_2d_offline(U, V, max_pwr_eb=0.05, ctx=ctx)
+    ou, ov = oracle.decompress_2d(blob, r1, r2)
+    for shift in (0, 1, 6):
+        mem = torch.empty(len(blob) + 8, dtype=torch.uint8).pin_memory()
+        mem[shift:shift + len(blob)] = torch.frombuffer(bytearray(blob), dtype=torch.uint8)
+        src = ctypes.cast(mem.data_ptr() + shift, ctypes.c_char_p)
+        du, dv = np.zeros((r1, r2), np.float32), np.zeros((r1, r2), np.float32)
+        rc = cpsz_b200.lib().cpsz_b200_decompress_2d_offline_f32(ctx.handle, src, len(blob), r1, r2, du.ctypes.data,
+                                                                 dv.ctypes.data)
+        assert rc == 0
+        assert_bits_equal(du, ou)
+        assert_bits_equal(dv, ov)
