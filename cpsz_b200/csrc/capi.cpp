@@ -145,9 +145,9 @@ int cpsz_b200_compress_2d_stages(cpsz_b200_ctx* ctx, const float* U, const float
   uint8_t* d_ids = nullptr;
   uint16_t* d_codes = nullptr;
   float* d_recon = nullptr;
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&d_ids, 2 * N + 16));
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&d_codes, 4 * N + 16));
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&d_recon, 8 * N + 16));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&d_ids, 2 * N + 16));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&d_codes, 4 * N + 16));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&d_recon, 8 * N + 16));
   StageTap tap;
   tap.ids = d_ids;
   tap.codes_blocks[0] = d_codes;
@@ -196,12 +196,12 @@ int cpsz_b200_debug_eb2d(cpsz_b200_ctx* ctx, const float* U, const float* V, siz
   double *deb = nullptr, *dtab = nullptr;
   uint8_t* dids = nullptr;
   unsigned long long* dh = nullptr;
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&dU, 4 * N));
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&dV, 4 * N));
-  if (eb_out) CPSZ_CUDA_TRY(cudaMalloc((void**)&deb, 8 * N));
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&dids, 2 * N));
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&dtab, QUANT_TAB_MAX * 8));
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&dh, 256 * 8));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dU, 4 * N));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dV, 4 * N));
+  if (eb_out) CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&deb, 8 * N));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dids, 2 * N));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dtab, QUANT_TAB_MAX * 8));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dh, 256 * 8));
   cudaMemcpy(dU, U, 4 * N, cudaMemcpyHostToDevice);
   cudaMemcpy(dV, V, 4 * N, cudaMemcpyHostToDevice);
   cudaMemcpy(dtab, qt.t, QUANT_TAB_MAX * 8, cudaMemcpyHostToDevice);
@@ -235,7 +235,7 @@ int cpsz_b200_debug_wave_trace(cpsz_b200_ctx* ctx, size_t len, long long* out) {
   ctx->d_wave_trace = nullptr;
   ctx->wave_trace_len = 0;
   if (len) {
-    CPSZ_CUDA_TRY(cudaMalloc((void**)&ctx->d_wave_trace, len * 8));
+    CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&ctx->d_wave_trace, len * 8));
     CPSZ_CUDA_TRY(cudaMemset(ctx->d_wave_trace, 0, len * 8));
     ctx->wave_trace_len = len;
   }
@@ -383,12 +383,12 @@ int cpsz_b200_debug_eb3d(cpsz_b200_ctx* ctx, const float* U, const float* V, con
   float* dF = nullptr;
   double *deb = nullptr, *dtab = nullptr;
   uint8_t* dids = nullptr;
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&dF, 12 * N));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dF, 12 * N));
   void* dscr = nullptr;
-  if (eb_out) CPSZ_CUDA_TRY(cudaMalloc((void**)&deb, 8 * N));
-  else CPSZ_CUDA_TRY(cudaMalloc(&dscr, eb3d_scratch_bytes(N)));
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&dids, N));
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&dtab, QUANT_TAB_MAX * 8));
+  if (eb_out) CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&deb, 8 * N));
+  else CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dscr, eb3d_scratch_bytes(N)));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dids, N));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dtab, QUANT_TAB_MAX * 8));
   cudaMemcpy(dF, U, 4 * N, cudaMemcpyHostToDevice);
   cudaMemcpy(dF + N, V, 4 * N, cudaMemcpyHostToDevice);
   cudaMemcpy(dF + 2 * N, W, 4 * N, cudaMemcpyHostToDevice);
@@ -413,9 +413,9 @@ int cpsz_b200_debug_umma_gemm(cpsz_b200_ctx* ctx, const uint16_t* A, const uint1
   if (!A || !B || !D) return set_error(CPSZ_ERR_INVALID, "null pointer");
   void *dA = nullptr, *dB = nullptr;
   float* dD = nullptr;
-  CPSZ_CUDA_TRY(cudaMalloc(&dA, 128 * 128 * 2));
-  CPSZ_CUDA_TRY(cudaMalloc(&dB, 128 * 128 * 2));
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&dD, 128 * 128 * 4));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dA, 128 * 128 * 2));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dB, 128 * 128 * 2));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dD, 128 * 128 * 4));
   cudaMemcpy(dA, A, 128 * 128 * 2, cudaMemcpyHostToDevice);
   cudaMemcpy(dB, B, 128 * 128 * 2, cudaMemcpyHostToDevice);
   cudaMemset(dD, 0, 128 * 128 * 4);
@@ -444,8 +444,8 @@ int cpsz_b200_debug_libm(cpsz_b200_ctx* ctx, int which, const float* in, size_t 
   LibmTables lt;
   CPSZ_TRY(libm_tables_device(ctx, &lt));
   float *di = nullptr, *dout = nullptr;
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&di, 4 * n));
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&dout, 4 * n));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&di, 4 * n));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&dout, 4 * n));
   cudaMemcpy(di, in, 4 * n, cudaMemcpyHostToDevice);
   int rc = launch_libm_eval(ctx, which, di, n, lt, dout);
   cudaStreamSynchronize(ctx->stream);
@@ -459,7 +459,7 @@ int cpsz_b200_debug_filter_premises(cpsz_b200_ctx* ctx, double* out, size_t n) {
   RESOLVE(ctx);
   if (!out || n < (size_t)FP_ROOT_HI) return set_error(CPSZ_ERR_INVALID, "need %d output doubles", (int)FP_ROOT_HI);
   unsigned* d = nullptr;
-  CPSZ_CUDA_TRY(cudaMalloc((void**)&d, FP_COUNT * sizeof(unsigned)));
+  CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&d, FP_COUNT * sizeof(unsigned)));
   unsigned h[FP_COUNT];
   int rc = launch_filter_premises(ctx, d);
   if (rc == CPSZ_OK) {
@@ -497,7 +497,7 @@ struct CpInputs {
         continue;
       }
       void* p = nullptr;
-      CPSZ_CUDA_TRY(cudaMalloc(&p, 4 * n));
+      CPSZ_CUDA_TRY(dev_malloc(ctx, (void**)&p, 4 * n));
       owned.push_back(p);
       CPSZ_CUDA_TRY(cudaMemcpyAsync(p, in[f], 4 * n, cudaMemcpyHostToDevice, ctx->stream));
       d[f] = (const float*)p;

@@ -159,8 +159,8 @@ struct DevMem {
   ~DevMem() {
     if (p) cudaFree(p);
   }
-  int alloc(size_t bytes) {
-    CPSZ_CUDA_TRY(cudaMalloc(&p, bytes));
+  int alloc(cpsz_b200_ctx* ctx, size_t bytes) {
+    CPSZ_CUDA_TRY(dev_malloc(ctx, &p, bytes));
     return CPSZ_OK;
   }
 };
@@ -173,7 +173,7 @@ int ensure_scratch(cpsz_b200_mlp* m, size_t bytes) {
     m->scratch = nullptr;
     m->scratch_cap = 0;
   }
-  CPSZ_CUDA_TRY(cudaMalloc(&m->scratch, bytes));
+  CPSZ_CUDA_TRY(dev_malloc(m->ctx, &m->scratch, bytes));
   m->scratch_cap = bytes;
   return CPSZ_OK;
 }
@@ -195,12 +195,22 @@ int compress_2d_learned(cpsz_b200_ctx* ctx, cpsz_b200_mlp* mlp, const float* U_i
   cudaStream_t st = ctx->stream;
   const bool dev_in = is_device_ptr(U_in) && is_device_ptr(V_in);
   // workspace of the loop (the compressor's own arena is reused by every
-  // pass), kept by the context: a cudaMalloc and cudaFree per call wait for
-  // the device and cost 1 to 10 ms
+  // pass), kept by the context up to kLoopKeep bytes: a cudaMalloc and cudaFree
+  // per call wait for the device and cost a millisecond and now and then tens
+  // (2048 x 2048, 9 passes: 16.4 ms kept, 17.4 to 25 without; above the limit
+  // 3000 x 3200 takes 32)
   const size_t bytes = align_up(8 * N, 256) * 2 + align_up(QUANT_TAB_MAX * 8, 256) + align_up(4 * N, 256) * 3 +
                        align_up(2 * N, 256) +
                        align_up(ncell, 256) * 2 + align_up(N, 256) * 2 + 4096 + (dev_in ? 0 : align_up(8 * N, 256));
   CPSZ_TRY(loop_reserve(ctx, bytes));
+  struct LoopUse {
+    cpsz_b200_ctx* ctx;
+    explicit LoopUse(cpsz_b200_ctx* c) : ctx(c) { c->loop_used = true; }
+    ~LoopUse() {
+      ctx->loop_used = false;
+      if (ctx->loop_cap > cpsz_b200_ctx::kLoopKeep) loop_release(ctx);
+    }
+  } loop_use(ctx);
   uint8_t* w = (uint8_t*)ctx->loop_mem;
   auto take = [&](size_t b) {
     void* p = w;
@@ -471,7 +481,7 @@ int cpsz_b200_mlp_features_2d(cpsz_b200_ctx* ctx, const float* U, const float* V
   if (!U || !V || !eb_analytic || !idx || !X) return set_error(CPSZ_ERR_INVALID, "null argument");
   const size_t N = r1 * r2;
   DevMem mem;
-  CPSZ_TRY(mem.alloc(8 * N + 8 * N + 4 * n + 256 * n + 4096));
+  CPSZ_TRY(mem.alloc(ctx, 8 * N + 8 * N + 4 * n + 256 * n + 4096));
   uint8_t* p = (uint8_t*)mem.p;
   float* dU = (float*)p;
   float* dV = dU + N;
@@ -497,7 +507,7 @@ int cpsz_b200_mlp_propose_2d(cpsz_b200_mlp* mlp, const float* U, const float* V,
   if (r1 * r2 == 0 || r1 * r2 > (size_t)INT32_MAX) return set_error(CPSZ_ERR_UNSUPPORTED, "field size out of range");
   const size_t N = r1 * r2;
   DevMem mem;
-  CPSZ_TRY(mem.alloc(8 * N + 8 * N + 4 * N + 4096));
+  CPSZ_TRY(mem.alloc(ctx, 8 * N + 8 * N + 4 * N + 4096));
   uint8_t* p = (uint8_t*)mem.p;
   float* dU = (float*)p;
   float* dV = dU + N;
@@ -557,7 +567,7 @@ int cpsz_b200_learned_labels_2d(cpsz_b200_ctx* ctx, const float* U, const float*
   if (!U || !V || !eb_analytic || !idx || !t_out) return set_error(CPSZ_ERR_INVALID, "null argument");
   const size_t N = r1 * r2;
   DevMem mem;
-  CPSZ_TRY(mem.alloc(16 * N + 8 * n + 4096));
+  CPSZ_TRY(mem.alloc(ctx, 16 * N + 8 * n + 4096));
   uint8_t* p = (uint8_t*)mem.p;
   float* dU = (float*)p;
   float* dV = dU + N;

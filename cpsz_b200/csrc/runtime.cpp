@@ -213,7 +213,7 @@ int arena_reserve(cpsz_b200_ctx* ctx, size_t bytes) {
     ctx->arena.base = nullptr;
     ctx->arena.cap = 0;
   }
-  cudaError_t e = cudaMalloc((void**)&ctx->arena.base, bytes);
+  cudaError_t e = dev_malloc(ctx, (void**)&ctx->arena.base, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return set_error(CPSZ_ERR_NOMEM, "device workspace of %zu bytes: %s", bytes, cudaGetErrorString(e));
@@ -248,14 +248,25 @@ int pinned_reserve(cpsz_b200_ctx* ctx, size_t bytes) {
   return CPSZ_OK;
 }
 
+void loop_release(cpsz_b200_ctx* ctx) {
+  if (!ctx->loop_mem) return;
+  cudaStreamSynchronize(ctx->stream);
+  cudaFree(ctx->loop_mem);
+  ctx->loop_mem = nullptr;
+  ctx->loop_cap = 0;
+}
+
+cudaError_t dev_malloc(cpsz_b200_ctx* ctx, void** p, size_t bytes) {
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation || !ctx->loop_mem || ctx->loop_used) return e;
+  cudaGetLastError();
+  loop_release(ctx);
+  return cudaMalloc(p, bytes);
+}
+
 int loop_reserve(cpsz_b200_ctx* ctx, size_t bytes) {
   if (ctx->loop_cap >= bytes) return CPSZ_OK;
-  if (ctx->loop_mem) {
-    cudaStreamSynchronize(ctx->stream);
-    cudaFree(ctx->loop_mem);
-    ctx->loop_mem = nullptr;
-    ctx->loop_cap = 0;
-  }
+  loop_release(ctx);
   bytes = align_up(bytes, 1 << 20);
   cudaError_t e = cudaMalloc(&ctx->loop_mem, bytes);
   if (e != cudaSuccess) {

@@ -95,8 +95,12 @@ struct cpsz_b200_ctx {
   cudaEvent_t up_ev[kUploadChunks] = {};
   cpsz::Arena arena;
   // workspace of the learned bounds' loop, beside the arena its passes use
+  // (loop_reserve): kept between calls up to kLoopKeep bytes, and given back
+  // when another allocation of the context does not fit beside it
+  static constexpr size_t kLoopKeep = (size_t)256 << 20;
   void* loop_mem = nullptr;
   size_t loop_cap = 0;
+  bool loop_used = false;  // a learned call is running
   // pinned ring for bulk copies of pageable host memory (transfer.h)
   static constexpr int kStageSlots = 32;
   static constexpr size_t kStageBytes = (size_t)2 << 20;
@@ -147,6 +151,9 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 int pinned_reserve(cpsz_b200_ctx* ctx, size_t bytes);
 // Grows ctx->loop_mem to at least `bytes`.
 int loop_reserve(cpsz_b200_ctx* ctx, size_t bytes);
+void loop_release(cpsz_b200_ctx* ctx);
+// cudaMalloc; where it fails, a kept loop workspace is given up for it.
+cudaError_t dev_malloc(cpsz_b200_ctx* ctx, void** p, size_t bytes);
 // Grows ctx->up_pinned to at least `bytes` (its old contents are dropped:
 // call it only when no copy from it is in flight).
 int upload_reserve(cpsz_b200_ctx* ctx, size_t bytes);

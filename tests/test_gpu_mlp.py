@@ -210,3 +210,58 @@ def test_learned_bounds_never_exceed_max_pwr_eb(ctx):
         assert _within_relative_bound(U, dU, eb) == 0 and _within_relative_bound(V, dV, eb) == 0
         r = cpsz_b200.cp_check_2d(U, V, dU, dV, ctx=ctx)
         assert r["lost_or_spurious"] == 0 and r["type_changed"] == 0, (r, st)
+
+
+def _used(call):
+    """Device memory (bytes) that `call` leaves allocated."""
+    import torch
+
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    call()
+    torch.cuda.synchronize()
+    return before - torch.cuda.mem_get_info()[0]
+
+
+def test_gpu_loop_workspace_is_bounded_and_given_back():
+    """The learned call's workspace stays with the context up to 256 MB; a
+    larger one goes when the call ends, and a kept one goes when the context's
+    next allocation does not fit beside it."""
+    torch = pytest.importorskip("torch")
+    torch.zeros(1, device="cuda")
+    mult = lambda U: np.full(U.shape, 1.0, np.float32)  # noqa: E731
+    big, mid, plain = W.cfg0_like(21, 3000, 3200), W.cfg0_like(22, 1500, 1500), W.cfg0_like(23, 2200, 2400)
+    compress = cpsz_b200.sz_compress_cp_preserve_2d_offline
+    # what contexts hold after plain calls alone
+    a = cpsz_b200.Context(0)
+    arena_big = _used(lambda: compress(*big, max_pwr_eb=0.1, ctx=a))
+    a.close()
+    a = cpsz_b200.Context(0)
+    arena_mid = _used(lambda: compress(*mid, max_pwr_eb=0.1, ctx=a))
+    a.close()
+    a = cpsz_b200.Context(0)
+    arena_plain = _used(lambda: compress(*plain, max_pwr_eb=0.1, ctx=a))
+    expect = compress(*plain, max_pwr_eb=0.1, ctx=a)
+    a.close()
+    c = cpsz_b200.Context(0)
+    held = []
+    try:
+        # 36 bytes a vertex and the fields: 345 and 99 MB
+        kept = _used(lambda: cpsz_b200.compress_2d_learned(*mid, 0.1, log2_mult=mult(mid[0]), ctx=c)) - arena_mid
+        assert 60 << 20 < kept < 256 << 20
+        # fill the device: the plain call's larger workspace fits only in the loop's place
+        free = torch.cuda.mem_get_info()[0] - (arena_plain - arena_mid - kept // 2)
+        held.append(torch.empty(free, dtype=torch.uint8, device="cuda"))
+        assert compress(*plain, max_pwr_eb=0.1, ctx=c) == expect
+        held.clear()
+        torch.cuda.empty_cache()
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+        c.close()
+    c = cpsz_b200.Context(0)
+    try:
+        left = _used(lambda: cpsz_b200.compress_2d_learned(*big, 0.1, log2_mult=mult(big[0]), ctx=c))
+        assert left < arena_big + (64 << 20)
+    finally:
+        c.close()
