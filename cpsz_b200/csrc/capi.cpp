@@ -340,7 +340,7 @@ int cpsz_b200_compress_3d_offline_log_f32_into(cpsz_b200_ctx* ctx, const float* 
   if (!out || !blob_size) return set_error(CPSZ_ERR_INVALID, "null output pointer");
   RESOLVE(ctx);
   Blob3D b;
-  CPSZ_TRY(compress_3d(ctx, U, V, W, r1, r2, r3, max_pwr_eb, &b, is_device_ptr(out) ? out : nullptr, out_cap));
+  CPSZ_TRY(compress_3d(ctx, U, V, W, r1, r2, r3, max_pwr_eb, &b, on_ctx_device(ctx, out) ? out : nullptr, out_cap));
   *blob_size = b.size;
   if (b.size > out_cap) return set_error(CPSZ_ERR_INVALID, "output capacity %zu < blob size %zu", out_cap, b.size);
   if (b.d_blob != out) CPSZ_TRY(copy_out(ctx, out, b.d_blob, b.size));

@@ -1188,8 +1188,10 @@ int compress_2d(cpsz_b200_ctx* ctx, const float* U_in, const float* V_in, size_t
   jobs[0].log_form = log_form;
   jobs[0].eb_ext = eb_ext;
   if (host_out && host_kind(host_out) == HOST_DEVICE) {
-    jobs[0].dev_out = host_out;
-    jobs[0].dev_cap = host_cap;
+    if (on_ctx_device(ctx, host_out)) {  // (another device's memory gets a copy)
+      jobs[0].dev_out = host_out;
+      jobs[0].dev_cap = host_cap;
+    }
   } else {
     jobs[0].host_out = host_out;
     jobs[0].host_cap = host_cap;
@@ -1207,7 +1209,7 @@ int compress_2d_batch(cpsz_b200_ctx* ctx, int n, const float* const* U, const fl
                       const size_t* r2, const double* ebs, unsigned char* out, size_t out_cap, size_t* offsets) {
   if (n < 0 || (n > 0 && (!U || !V || !r1 || !r2 || !ebs))) return set_error(CPSZ_ERR_INVALID, "null batch argument");
   if (!out || !offsets) return set_error(CPSZ_ERR_INVALID, "null output");
-  const bool dev_out = is_device_ptr(out);
+  const bool dev_out = on_ctx_device(ctx, out);
   size_t at = 0;
   int k0 = 0;
   offsets[0] = 0;

@@ -160,6 +160,8 @@ int upload_reserve(cpsz_b200_ctx* ctx, size_t bytes);
 
 // Pointer kind: true if `p` is device (or managed) memory usable by kernels.
 bool is_device_ptr(const void* p);
+// Memory that the context's kernels may write: its device's, or managed.
+bool on_ctx_device(const cpsz_b200_ctx* ctx, const void* p);
 
 inline void count_launch(cpsz_b200_ctx* ctx, int n = 1) { ctx->launches += (uint64_t)n; }
 // Stage marks: when timing is on, records an event named `name` on the stream;
