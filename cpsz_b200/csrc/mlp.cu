@@ -582,7 +582,8 @@ int set_smem(K kernel, int bytes) {
 
 int launch_umma_selftest(cpsz_b200_ctx* ctx, const void* A, const void* B, float* D) {
   const int smem = 2 * umma::TILE_BYTES + 64;
-  static bool attr = false;
+  static bool attrs[64] = {};  // per device, as the attribute is
+  bool& attr = attrs[ctx->device & 63];
   if (!attr) {
     CPSZ_CUDA_TRY(cudaFuncSetAttribute(umma_selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr = true;
@@ -595,7 +596,8 @@ int launch_umma_selftest(cpsz_b200_ctx* ctx, const void* A, const void* B, float
 
 int launch_mlp_forward(cpsz_b200_ctx* ctx, const MlpParams& w, const void* X, const float* U, const float* V,
                        const double* eb_a, int r1, int r2, int M, float* y, void* H1, void* H2) {
-  static bool attr = false;
+  static bool attrs[64] = {};  // per device, as the attribute is
+  bool& attr = attrs[ctx->device & 63];
   if (!attr) {
     CPSZ_TRY(set_smem(mlp_fwd_kernel<false>, FWD_SMEM));
     CPSZ_TRY(set_smem(mlp_fwd_kernel<true>, FWD_SMEM));
@@ -623,7 +625,8 @@ int launch_mlp_forward(cpsz_b200_ctx* ctx, const MlpParams& w, const void* X, co
 
 int launch_mlp_backward(cpsz_b200_ctx* ctx, const MlpParams& w, const void* X, const void* H1, const void* H2,
                         const float* y, const float* t, int M, float grad_scale, float* loss) {
-  static bool attr = false;
+  static bool attrs[64] = {};  // per device, as the attribute is
+  bool& attr = attrs[ctx->device & 63];
   if (!attr) {
     CPSZ_TRY(set_smem(mlp_bwd_kernel, BWD_SMEM));
     attr = true;

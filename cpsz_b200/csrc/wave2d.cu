@@ -548,15 +548,15 @@ int launch_wave2d(cpsz_b200_ctx* ctx, bool decompress, const WaveField* d_fields
                   int n_items, int* d_queue, size_t points, cudaStream_t stream, int mode) {
   if (n_items <= 0) return CPSZ_OK;
   if (!stream) stream = ctx->stream;
-  static bool attr_set[3] = {false, false, false};
+  static bool attr_set[64][3] = {};  // per device, as the attribute is
   const bool beside = mode == WAVE_BESIDE && !decompress;
   const void* fn = decompress ? (const void*)wave2d_kernel<true>
                               : beside ? (const void*)wave2d_beside_kernel : (const void*)wave2d_kernel<false>;
   const int which = decompress ? 1 : beside ? 2 : 0;
-  if (!attr_set[which]) {
+  if (!attr_set[ctx->device & 63][which]) {
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDynSmem);
     if (e != cudaSuccess) return set_error(CPSZ_ERR_CUDA, "wave2d smem attribute: %s", cudaGetErrorString(e));
-    attr_set[which] = true;
+    attr_set[ctx->device & 63][which] = true;
   }
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, WAVE_THREADS, kDynSmem);
