@@ -395,7 +395,9 @@ int launch_zstd_frame(cpsz_b200_ctx* ctx, const uint8_t* d_in, size_t n, uint8_t
   if (!g_tables_ready[ctx->device & 63]) {
     zstd::Tables T;
     zstd::build_tables(&T);
-    CPSZ_CUDA_TRY(cudaMemcpyToSymbol(c_tables, &T, sizeof(T)));
+    // (in place before any stream's kernel reads them: the context's streams do not wait for the default one)
+    CPSZ_CUDA_TRY(cudaMemcpyToSymbolAsync(c_tables, &T, sizeof(T), 0, cudaMemcpyHostToDevice, st));
+    CPSZ_CUDA_TRY(cudaStreamSynchronize(st));
     g_tables_ready[ctx->device & 63] = true;
   }
   const long long nb = n ? (long long)((n + ZBLK - 1) / ZBLK) : 0;
