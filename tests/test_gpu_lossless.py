@@ -2,6 +2,11 @@
 (the decoder behind the reference's sz_lossless_decompress) reads every frame
 back to the input bytes, from host and device buffers, for empty, one-byte,
 constant (RLE), incompressible and real compressor blobs."""
+import os
+import shutil
+import struct
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -71,3 +76,33 @@ def test_block_edges(ctx, n, kind):
         a[-20:] = 5
     frame = _roundtrip(a.tobytes(), ctx)
     assert len(frame) <= cpsz_b200.lib().cpsz_b200_lossless_bound(n)
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_frames_equal_the_format_header_s_coder(ctx, tmp_path):
+    """Every frame byte for byte: tests/zstd_frame_check.cpp reads the blocks'
+    sequences back and writes them again with the host coder of
+    cpsz_b200/csrc/zstd_format.h."""
+    rng = np.random.default_rng(9)
+    U, V = W.cfg0_like(24, 700, 900)
+    inputs = [b"", b"\x07", bytes(20000), rng.integers(0, 256, 30001, np.uint8).tobytes(),
+              cpsz_b200.sz_compress_cp_preserve_2d_offline(U, V, max_pwr_eb=0.1, ctx=ctx),
+              cpsz_b200.sz_compress_cp_preserve_2d_offline(U, V, max_pwr_eb=0.01, ctx=ctx)]
+    for n in (5, 33, 100, 8191, 8192, 8193, 70001):
+        for alphabet, run in ((2, 1), (4, 1), (256, 3), (16, 40), (256, 4096)):
+            a = np.repeat(rng.integers(0, alphabet, n // run + 1), run)[:n].astype(np.uint8)
+            if n > 600:  # a distant repeat, so that every offset code occurs
+                a[-300:] = a[:300]
+            inputs.append(a.tobytes())
+    path = tmp_path / "frames"
+    with open(path, "wb") as f:
+        for data in inputs:
+            frame = _roundtrip(data, ctx)
+            f.write(struct.pack("<QQ", len(data), len(frame)) + data + frame)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    exe = str(tmp_path / "zframe")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-I", os.path.join(root, "cpsz_b200", "csrc"), "-o", exe,
+                    os.path.join(root, "tests", "zstd_frame_check.cpp")], check=True)
+    r = subprocess.run([exe, str(path)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and "ALL OK" in r.stdout, r.stdout + r.stderr
+    assert int(r.stdout.split(" compressed")[0].split()[-1]) > 100
