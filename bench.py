@@ -500,7 +500,7 @@ def run_product(args, rank, world, device):
 
     stages = {k: statistics.mean(v) for k, v in stage_acc.items()}
     n = int(np.prod(shape))
-    roof = product_roofline(kind, n, stages, clk.summary().get("sm_mhz"))
+    roof = product_roofline(kind, n, stages, clk.summary().get("sm_mhz"), PRESENT_INSTR_PER_POINT)
     return {
         "value": value, "ms": ms, "e2e_ms": e2e_ms, "dec_ms": dec_ms, "blob": len(blob), "size_dev": size,
         "lossless": len(lossless), "lossless_gpu": lossless_gpu, "raw": raw_bytes, "stages": stages, "roofline": roof,
@@ -509,12 +509,13 @@ def run_product(args, rank, world, device):
     }
 
 
-def product_roofline(kind, n, stages, sm_mhz):
+def product_roofline(kind, n, stages, sm_mhz, instr_per_point=None):
     """The roofline of the step's dominant kernel (the stage with the longest
     CUDA-event time among those with algorithmic bytes) for a field of `n`
     points: its algorithmic bytes over the stage time against the measured
     copy bandwidth, its DRAM traffic, and for a kernel bound by instruction
-    issue its issue roofline.  None when no such stage was timed."""
+    issue its issue roofline (from the counts in instr_per_point, see
+    issue_roofline).  None when no such stage was timed."""
     comps = 2 if kind == "2d" else 3
     # algorithmic bytes per launch of each stage's dominant kernel
     alg = {"eb2d": 4 * comps * n + comps * n,  # read fields, write one id byte per component
@@ -533,7 +534,7 @@ def product_roofline(kind, n, stages, sm_mhz):
     roof = {"bound": "hbm", "kernel": dom, "achieved": round(ach, 2), "peak": peak, "unit": "GB/s",
             "frac": round(ach / peak, 4), "traffic": round(tr * n) if tr else None, "peak_source": peak_kind,
             "algorithmic_bytes": alg[dom]}
-    issue = issue_roofline(dom, n, stages[dom], sm_mhz)
+    issue = issue_roofline(dom, n, stages[dom], sm_mhz, instr_per_point)
     if issue:
         roof["issue"] = issue
     return roof
@@ -541,22 +542,22 @@ def product_roofline(kind, n, stages, sm_mhz):
 
 # Warp instructions per point of a kernel that is bound by instruction issue
 # rather than by HBM, from one ncu capture of it on the 4096^2 case
-# (smsp__inst_executed.sum: 404,377,736 for 16.8 M vertices).  The capture is of
-# an earlier version of the kernel; the present one executes 300,591,438 there,
-# so its share of the issue peak is 0.743 of the one computed here (the line
-# carries both counts).
+# (smsp__inst_executed.sum for 16.8 M vertices).  The line takes the present
+# kernel's; the other is an earlier version's, the default of the functions
+# below, whose tests hold that capture's figures.
+PRESENT_INSTR_PER_POINT = {"eb2d": 300591438 / 4096 ** 2}
 INSTR_PER_POINT = {"eb2d": 404377736 / 4096 ** 2}
 B200_SMS = 148
 ISSUE_PER_SM_CYCLE = 4  # one warp instruction a cycle on each of an SM's four schedulers
 
 
-def issue_roofline(kernel, points, ms, sm_mhz):
+def issue_roofline(kernel, points, ms, sm_mhz, instr_per_point=None):
     """The issue roofline of `kernel` over a launch of `points` points that
     took `ms`: its warp instructions (scaled from the captured case by the
     points) a second against 4 a cycle on each of the 148 SMs at the SM clock
-    sampled during the run; None when the kernel has no captured count or no
-    clock was sampled."""
-    per = INSTR_PER_POINT.get(kernel)
+    sampled during the run; None when the kernel has no captured count
+    (instr_per_point, else INSTR_PER_POINT) or no clock was sampled."""
+    per = (instr_per_point or INSTR_PER_POINT).get(kernel)
     if per is None or not sm_mhz or not ms or ms <= 0:
         return None
     instr = per * points
@@ -564,8 +565,7 @@ def issue_roofline(kernel, points, ms, sm_mhz):
     peak = B200_SMS * ISSUE_PER_SM_CYCLE * float(sm_mhz) * 1e6 / 1e9
     return {"achieved": round(achieved, 2), "peak": round(peak, 2), "unit": "G warp instructions/s",
             "frac": round(achieved / peak, 4), "instructions": round(instr),
-            "min_ms": round(instr / (peak * 1e9) * 1e3, 4),
-            "count": "an earlier version's 404,377,736 at 4096^2; the present kernel's 300,591,438 there"}
+            "min_ms": round(instr / (peak * 1e9) * 1e3, 4)}
 
 
 def cp_and_bound_check(kind, fields, decoded, eb, ctx):

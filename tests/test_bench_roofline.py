@@ -62,3 +62,15 @@ def test_product_roofline_without_a_clock_or_an_issue_count():
     assert r3["traffic"] is None
     assert bench.product_roofline("2d", 100, {"host_trees": 1.0}, 1965.0) is None
     assert bench.product_roofline("2d", 100, {}, 1965.0) is None
+
+
+def test_the_line_takes_the_present_kernel_s_count():
+    """The present bound kernel's capture: 300,591,438 warp instructions at
+    4096^2, in 0.409 ms at 69 % of the issue slots."""
+    present = bench.PRESENT_INSTR_PER_POINT
+    r = bench.issue_roofline("eb2d", 4096 ** 2, 0.409, 1800.0, present)
+    assert r["instructions"] == 300591438 and "count" not in r
+    assert r["frac"] == pytest.approx(300591438 / 0.409e-3 / (148 * 4 * 1.8e9), abs=1e-4)
+    line = bench.product_roofline("2d", 8192 ** 2, STAGES_2D, 1965.0, present)
+    assert line["issue"]["instructions"] == 4 * 300591438
+    assert line["issue"]["min_ms"] == pytest.approx(4 * 300591438 / (148 * 4 * 1.965e9) * 1e3, rel=1e-3)
