@@ -177,8 +177,9 @@ struct StripShared {
   unsigned long long excl;
 };
 
-// Zeros of this thread's run of the image (elements [24 tid, 24 tid + 24)),
-// and of all earlier threads'; total in every thread.  All threads call it.
+// Zeros of this thread's run of the image (the STRIP_RUN elements from
+// STRIP_RUN tid on), and of all earlier threads'; total in every thread.  All
+// threads call it.
 __device__ __forceinline__ unsigned strip_zeros(StripShared& sh, const uint16_t* img, int E, unsigned& before,
                                                 unsigned& total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -319,7 +320,7 @@ struct StripUnpass {
   const float* unpred;         // unpredictable values, block order
   unsigned long long n_unpred;
   float2* pair;                // raster (pitch r2)
-  unsigned long long* status;  // as in StripPass
+  unsigned long long* status;  // as in StripJob
   unsigned* total;
   int id_shift;                // p = 2^(id_shift * id) * 2^-52: 2 (offline), 1 (offline_log)
 };

@@ -67,8 +67,8 @@ int cpsz_b200_compress_2d_offline_f32_into(cpsz_b200_ctx* ctx, const float* U, c
   RESOLVE(ctx);
   Blob2D b;
   // host memory: the sections are written there as they are produced; a
-  // device buffer: the blob is built in place when the buffer has room for
-  // the blob's bound, else copied there
+  // device buffer: the blob is built in place when the buffer has room for it
+  // (compress_2d), else copied there
   CPSZ_TRY(compress_2d(ctx, U, V, r1, r2, max_pwr_eb, &b, nullptr, nullptr, out, out_cap));
   *blob_size = b.size;
   if (b.d_blob && b.d_blob != out) {

@@ -197,8 +197,8 @@ int compress_2d_learned(cpsz_b200_ctx* ctx, cpsz_b200_mlp* mlp, const float* U_i
   // workspace of the loop (the compressor's own arena is reused by every
   // pass), kept by the context up to kLoopKeep bytes: a cudaMalloc and cudaFree
   // per call wait for the device and cost a millisecond and now and then tens
-  // (2048 x 2048, 9 passes: 16.4 ms kept, 17.4 to 25 without; above the limit
-  // 3000 x 3200 takes 32)
+  // (2048 x 2048 16.4 ms kept, 17.4 to 25 without; above the limit 3000 x 3200
+  // takes 32)
   const size_t bytes = align_up(8 * N, 256) * 2 + align_up(QUANT_TAB_MAX * 8, 256) + align_up(4 * N, 256) * 3 +
                        align_up(2 * N, 256) +
                        align_up(ncell, 256) * 2 + align_up(N, 256) * 2 + 4096 + (dev_in ? 0 : align_up(8 * N, 256));

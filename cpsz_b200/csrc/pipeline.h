@@ -41,9 +41,11 @@ int build_wave_items(int nfields, const int* r1s, std::vector<WaveItem>& items);
 // eb_ext (optional, device, N doubles): per-vertex bounds to quantize instead
 // of the derived ones (the learned-bound path).  host_out (optional, of
 // host_cap bytes): host memory gets the blob written there directly
-// (out->d_blob is then not set); a device buffer with room for the blob's
-// bound gets the blob built in place (out->d_blob == host_out), else the blob
-// is built in the workspace (out->d_blob) and the caller copies it.
+// (out->d_blob is then not set); a buffer in the context's device's memory gets
+// the blob built in place (out->d_blob == host_out) if it has room for it and 8
+// bytes more (a field large enough to pack its ids early: for the blob's
+// bound); else the blob is built in the workspace (out->d_blob) and the caller
+// copies it.
 // log_form: the offline_log blob (src/sz_compress_cp_preserve_2d.cpp:285-379)
 // instead of the offline one.
 int compress_2d(cpsz_b200_ctx* ctx, const float* U, const float* V, size_t r1, size_t r2, double max_pwr_eb,
@@ -61,8 +63,8 @@ struct Blob3D {
   size_t n_unpred = 0;  // floats (3 per unpredictable point)
   size_t n_codes = 0;   // codes (3 per predicted point)
 };
-// dev_out (optional): device memory of dev_cap bytes that gets the blob if it
-// has room (out->d_blob == dev_out then).
+// dev_out (optional): memory of the context's device, dev_cap bytes, that gets
+// the blob if it has room (out->d_blob == dev_out then).
 int compress_3d(cpsz_b200_ctx* ctx, const float* U, const float* V, const float* W, size_t r1, size_t r2, size_t r3,
                 double max_pwr_eb, Blob3D* out, unsigned char* dev_out = nullptr, size_t dev_cap = 0);
 int decompress_3d(cpsz_b200_ctx* ctx, const unsigned char* blob, size_t blob_size, size_t r1, size_t r2, size_t r3,
